@@ -20,7 +20,6 @@
 
 namespace cpppt_gb300 {
 
-
 __device__ __forceinline__ void stage_top_nodes(const DevScene& S, uint4* snodes) {
     const int n = min(S.n_nodes, kSmemNodes) * 4;
     for (int i = threadIdx.x; i < n; i += blockDim.x) snodes[i] = __ldg(S.nodes + i);
@@ -88,14 +87,14 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_any(
 void launch_trace_closest(const DevScene& S, const float* rays, int n, float4* hits, int* counter, uint32_t* status,
                           int num_sms, cudaStream_t st) {
     if (n <= 0) return;
-    const int blocks = min(num_sms * kTraceBlocksPerSM, (n + kTraceThreads - 1) / kTraceThreads);
+    const int blocks = min(num_sms * kTraceBlocksPerSM, n);
     k_trace_closest<<<blocks, kTraceThreads, kSmemNodeBytes, st>>>(S, rays, n, hits, counter, status);
 }
 
 void launch_trace_any(const DevScene& S, const float* rays, int n, uint8_t* occ, int* counter, uint32_t* status,
                       int num_sms, cudaStream_t st) {
     if (n <= 0) return;
-    const int blocks = min(num_sms * kTraceBlocksPerSM, (n + kTraceThreads - 1) / kTraceThreads);
+    const int blocks = min(num_sms * kTraceBlocksPerSM, n);
     k_trace_any<<<blocks, kTraceThreads, kSmemNodeBytes, st>>>(S, rays, n, occ, counter, status);
 }
 

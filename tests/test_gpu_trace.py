@@ -82,3 +82,21 @@ def test_empty_and_degenerate_inputs(gpu_lib):
     rays = np.array([[0.5, 0.5, 5.0, 0, 0, 1, np.inf], [0.5, 0.5, 0.5, 0, 1, 0, 0.0]], np.float32)
     idx, t, _, _ = gs.trace_closest(rays)
     assert idx[0] == -1 and idx[1] == -1
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 151, 153, 1000, 4863, 4865, 9729, 77823, 77825, 155649])
+def test_batch_sizes_around_the_ray_distribution(gpu_lib, n):
+    """Batches around the warp, SM and fetch sizes of the traversal kernels:
+    every ray is answered once, with the answer it has in any other batch."""
+    from cpppt.lib import GpuScene
+    from oracle.oracle import Oracle
+    sc = scenes.soup(seed=2, n_spheres=60, freq=3, width=64, height=64)
+    rays = scenes.hit_ray_batch(sc, n, seed=12)
+    oi, ot = Oracle("port").scene(sc).trace_closest(rays)
+    gs = GpuScene(sc)
+    gi, gt, _, _ = gs.trace_closest(rays)
+    assert np.array_equal(gi, oi)
+    assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
+    sh = rays.copy()
+    sh[:, 6] = np.where(oi >= 0, ot * np.where(np.arange(n) % 2, 0.5, 1.5), 1.0).astype(np.float32)
+    assert np.array_equal(gs.trace_any(sh), Oracle("port").scene(sc).trace_any(sh))
