@@ -367,7 +367,7 @@ void render_batch(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float* cons
     }
     *b->h_ctr = init;
     ck(cudaMemcpyAsync(b->d_ctr, b->h_ctr, sizeof(WaveCounters), cudaMemcpyHostToDevice, st), "init counters");
-    launch_generate(b->arena, b->pb, 1, b->d_ctr, b->d_jobs, n_jobs, st);  // fills buffer 0
+    launch_generate(b->pb, 1, b->d_ctr, b->d_jobs, n_jobs, b->num_sms, st, false);  // fills buffer 0
     // the whole loop on the device: one graph launch, one read of the counters
     ck(cudaGraphLaunch(b->graph, st), "graph launch");
     ck(cudaMemcpyAsync(b->h_ctr, b->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");

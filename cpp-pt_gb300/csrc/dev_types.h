@@ -95,8 +95,14 @@ constexpr uint32_t kStatusRoundLimit = 16u;    // a device-driven render loop re
 
 // Wavefront counters, one block of device memory per scene.
 struct WaveCounters {
-    int32_t n_cur, n_next, n_shadow, n_fin;  // n_fin: finished paths of the learned-guide integrator
-    int32_t fetch_ext, fetch_sh, free_top, n_rec;  // free_top: vertex-slot free list; n_rec: training records
+    int32_t n_cur, n_next, n_shadow;
+    union {
+        int32_t n_fin;      // learned-guide integrator: finished paths
+        int32_t n_shadow1;  // plain renders: shadow rays of the iterations that read path buffer 1 (n_shadow: buffer 0)
+    };
+    int32_t fetch_ext, fetch_sh;
+    int32_t free_top;  // vertex-slot free list
+    int32_t n_rec;     // training records
     uint32_t status;
     float film_safe;  // |contribution| below this cannot carry a film sum out of the 32.32 range
     uint32_t rounds;      // loop bodies run by a device-driven render (k_round_control)
@@ -107,6 +113,11 @@ struct WaveCounters {
     unsigned long long stat_nonfinite;         // contributions dropped because they were inf/NaN
     unsigned long long stat_film_overflow;     // contributions the 32.32 film could not hold
 };
+
+// A plain render's wavefront has nothing left: no path, no work, no shadow ray.
+__host__ __device__ inline bool wave_done(const WaveCounters& c) {
+    return c.n_cur == 0 && c.work_next >= c.work_total && c.n_shadow == 0 && c.n_shadow1 == 0;
+}
 
 // film_safe for a render of at most `per_pixel` film contributions per pixel
 // and channel: a sum of contributions below 2^31 / per_pixel stays below

@@ -307,7 +307,8 @@ constexpr int kMaxCapacity = 1 << CPPPT_MAX_WAVE_LOG2;
 #ifndef CPPPT_NN_WAVE_LOG2
 #define CPPPT_NN_WAVE_LOG2 20
 #endif
-constexpr int kItersPerGraph = 16;  // even: buffers alternate
+constexpr int kItersPerGraph = 16;   // of the learned-guide and SD-tree renders between host steps; even: buffers alternate
+constexpr int kItersPerBody = 20;    // of a plain render's device-driven loop body; even
 
 // The scene's wavefront buffers for `capacity` paths in flight (192 B per
 // path, kept for later renders).  Returns the paths in flight the render
@@ -851,13 +852,13 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     // the render parameters live in the scene's one-entry job table and the
     // counters, so the graph stays valid across renders
     if (!direct && !s->graph)
-        ck(build_render_graph(s->dev, s->pb, s->d_ctr, s->film, s->d_job, 1, kItersPerGraph, s->num_sms, st,
+        ck(build_render_graph(s->dev, s->pb, s->d_ctr, s->film, s->d_job, 1, kItersPerBody, s->num_sms, st,
                               &s->graph),
            "render graph");
     ck(cudaEventRecord(s->ev0, st), "event");
     ck(cudaMemsetAsync(s->film, 0, sizeof(unsigned long long) * film_n, st), "memset film");
     const unsigned long long max_rounds = 64 + (total / (unsigned long long)capacity + 2) *
-                                                   (unsigned long long)(desc->max_depth + 2) * 4 / kItersPerGraph;
+                                                   (unsigned long long)(desc->max_depth + 2) * 4 / kItersPerBody;
     WaveCounters init{};
     init.work_total = total;
     init.film_safe = film_safe_bound((double)desc->spp * (2.0 * desc->max_depth + 2.0));
@@ -868,7 +869,7 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     s->h_job->integrator = desc->mode == PT_MODE_NEE ? kIntegratorNEE
                            : desc->mode == PT_MODE_PT ? kIntegratorPT : kIntegratorMIS;
     ck(cudaMemcpyAsync(s->d_job, s->h_job, sizeof(DevBatchJob), cudaMemcpyHostToDevice, st), "job table");
-    launch_generate(s->dev, s->pb, 1, s->d_ctr, s->d_job, 1, st);  // fills buffer 0
+    launch_generate(s->pb, 1, s->d_ctr, s->d_job, 1, s->num_sms, st, false);  // fills buffer 0
     double launches = 2;
     std::vector<cudaEvent_t> tev;
     unsigned long long rounds = 0;
@@ -879,12 +880,12 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
         ck(cudaStreamSynchronize(st), "render");
         check_status(s, s->h_ctr->status);
         rounds = s->h_ctr->rounds;
-        launches += (double)rounds * (kKernelsPerIteration * kItersPerGraph + 1);
+        launches += (double)rounds * (kKernelsPerIteration * kItersPerBody + 1);
     }
     while (direct) {
         {
-            // the graph's work, launched one kernel at a time
-            for (int k = 0; k < kItersPerGraph; k++) {
+            // the graph's work with the two kinds of rays in launches of their own, one kernel at a time
+            for (int k = 0; k < kItersPerBody; k++) {
                 const int cur = k & 1;
                 cudaEvent_t e[4] = {nullptr, nullptr, nullptr, nullptr};
                 if (timed)
@@ -894,17 +895,17 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
                 if (timed) ck(cudaEventRecord(e[1], st), "event");
                 launch_shade(s->dev, s->pb, cur, s->d_ctr, s->film, s->d_job, st);
                 if (timed) ck(cudaEventRecord(e[2], st), "event");
-                launch_shadow(s->dev, s->pb, s->d_ctr, s->film, s->num_sms, st);
+                launch_shadow(s->dev, s->pb, cur, s->d_ctr, s->film, s->num_sms, st);
                 if (timed) ck(cudaEventRecord(e[3], st), "event");
-                launch_generate(s->dev, s->pb, cur, s->d_ctr, s->d_job, 1, st);
+                launch_generate(s->pb, cur, s->d_ctr, s->d_job, 1, s->num_sms, st, true);
             }
         }
-        launches += kKernelsPerIteration * kItersPerGraph;
+        launches += 5 * kItersPerBody;
         ck(cudaMemcpyAsync(s->h_ctr, s->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");
         ck(cudaStreamSynchronize(st), "render");
         check_status(s, s->h_ctr->status);
         rounds++;
-        if (s->h_ctr->n_cur == 0 && s->h_ctr->work_next >= s->h_ctr->work_total) break;
+        if (wave_done(*s->h_ctr)) break;
         if (rounds > max_rounds) throw Fail(PT_ERR_LIMIT, "render did not converge within the iteration bound");
     }
     launch_film_resolve(s->film, d_dst ? d_dst : s->d_out, film_n, 1.0 / (double)desc->spp, st);

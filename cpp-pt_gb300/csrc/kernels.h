@@ -28,6 +28,17 @@ struct PathBuffers {
     int capacity;
 };
 
+// One of the two path buffers, and the shadow queue, as a kernel's arguments
+// (pointers picked on the host: a run-time index into PathBuffers would copy
+// the argument to local memory).
+struct PathIO {
+    float4 *o, *d, *thr;
+    int4* info;
+};
+struct ShadowIO {
+    float4 *o, *d, *c;
+};
+
 struct RenderParams {
     int spp;
     int spp_axis;        // >0: spp = spp_axis^2, stratified as pathtracerMIS.h:148-153
@@ -41,16 +52,25 @@ struct RenderParams {
 // The stages of one wavefront iteration reading path buffer `cur` (writing
 // 1 - cur): extend (closest hit), shade (BSDF, NEE, MIS, RR, compaction),
 // shadow (any hit + film), generate (new camera paths) + advance (counters).
+// Plain renders run launch_wave_iteration; the separate extend and shadow
+// launches serve the learned-guide and SD-tree wavefronts and the renders
+// that time or count the two kinds of rays apart.
 void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, int num_sms, cudaStream_t st,
                    bool count = false);
 // jobs: device table of n_jobs DevBatchJob (one entry for a single-scene
 // render; several for a batch over a merged arena, ascending work ranges).
 void launch_shade(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                   const DevBatchJob* jobs, cudaStream_t st);
-void launch_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film, int num_sms,
-                   cudaStream_t st);
-void launch_generate(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs,
-                     int n_jobs, cudaStream_t st);
+void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
+                   int num_sms, cudaStream_t st);
+// shadows_traced: the iteration's own shadow rays have been traced
+// (launch_shadow), not only those of the iteration before.
+void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs, int n_jobs, int num_sms,
+                     cudaStream_t st, bool shadows_traced);
+// A whole iteration as renders run it: the extension rays together with the
+// shadow rays of the iteration before (one launch), shade, generate, advance.
+void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
+                           const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st);
 // The whole wavefront loop of a plain render (PT_MODE_MIS / NEE / PT, single
 // scene or batch) as one executable graph: a conditional WHILE node whose
 // body runs `iters` (even) iterations and then a round-control kernel that
@@ -63,7 +83,7 @@ cudaError_t build_render_graph(const DevScene& S, const PathBuffers& B, WaveCoun
                                cudaGraphExec_t* out);
 // The job-table entry of a single-scene render of S with parameters P.
 DevBatchJob single_job(const DevScene& S, const RenderParams& P);
-constexpr int kKernelsPerIteration = 5;
+constexpr int kKernelsPerIteration = 4;  // of launch_wave_iteration
 // Allocation-free render: the wavefront of launch_* above with its scratch in
 // a file-scope __device__ array (see render.cu).  Synchronises `st`.
 // limit_hit is set when the iteration bound ran out; the kernels' status

@@ -2,12 +2,13 @@
 // (PathtracerMIS::integrate/render, src/renderer/pathtracerMIS.h:29-167).
 //
 // Wavefront layout: path state lives in HBM as structure-of-arrays, two
-// copies (current / next).  One iteration = extend (closest hit for every
-// live path) -> shade (emission + MIS, BSDF sample, NEE shadow ray, Russian
-// roulette; survivors are appended compactly to the next buffer with
-// warp-aggregated atomics) -> shadow (any hit; unoccluded NEE contributions
-// go to the film) -> generate (new camera paths fill the next buffer up to
-// capacity from a global work counter) -> advance (one thread swaps counts).
+// copies (current / next).  One iteration = trace (closest hit for every live
+// path, then any hit for the shadow rays the iteration before queued, whose
+// unoccluded NEE contributions go to the film) -> shade (emission + MIS, BSDF
+// sample, NEE shadow ray, Russian roulette; survivors are appended compactly
+// to the next buffer with warp-aggregated atomics) -> generate (new camera
+// paths fill the next buffer up to capacity from a global work counter) ->
+// advance (one thread swaps counts).
 // All sizes are read from device counters, so an iteration needs no host
 // round trip and a chain of iterations is captured once in a CUDA graph.
 #include <cuda_runtime.h>
@@ -109,16 +110,12 @@ __device__ __forceinline__ void film_add(unsigned long long* film, size_t pix, f
     film_add_rgb(film, pix, r, g, b, ctr);
 }
 
+// The extension rays of a path buffer.
 template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(DevScene S, PathBuffers B, int cur, WaveCounters* ctr) {
-    extern __shared__ uint4 snodes[];
-    const int n = ctr->n_cur;
-    if (n == 0) return;  // drained wavefront: skip staging
-    stage_top_nodes(S, snodes);
-    const float4* __restrict__ O = B.o[cur];
-    const float4* __restrict__ D = B.d[cur];
-    float4* __restrict__ Hout = B.hit;
-    TraceCount cnt{0u, 0u};
+__device__ __forceinline__ void extend_queue(const DevScene& S, const uint4* snodes, const PathIO& in,
+                                             float4* __restrict__ Hout, int n, WaveCounters* ctr, TraceCount& cnt) {
+    const float4* __restrict__ O = in.o;
+    const float4* __restrict__ D = in.d;
     persistent_trace<false, COUNT>(
         S, snodes, n, &ctr->fetch_ext, &ctr->status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
@@ -129,6 +126,39 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(Dev
             if (root != kTravDone) root = __float_as_uint(b.w);  // the path's scene root (0 unbatched)
         },
         [&](int i, const HitRec& h) { Hout[i] = make_float4(h.t, __int_as_float(h.prim), h.beta, h.gamma); });
+}
+
+// The shadow rays of a queue; the unoccluded ones' contributions go to the film.
+__device__ __forceinline__ void shadow_queue(const DevScene& S, const uint4* snodes, const ShadowIO& Q, int n,
+                                             WaveCounters* ctr, unsigned long long* __restrict__ film, bool own_first) {
+    TraceCount cnt{0u, 0u};
+    persistent_trace<true, false>(
+        S, snodes, n, &ctr->fetch_sh, &ctr->status, cnt,
+        [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
+            const float4 a = Q.o[i], b = Q.d[i];
+            o = make_float3(a.x, a.y, a.z);
+            d = make_float3(b.x, b.y, b.z);
+            tmax = a.w;
+            if (root != kTravDone) root = __float_as_uint(Q.c[i].w);
+        },
+        [&](int i, const HitRec& h) {
+            if (h.prim < 0) {  // unoccluded: the NEE contribution reaches the film
+                const float4 c = Q.c[i];
+                film_add(film, (uint32_t)__float_as_int(Q.d[i].w), c.x, c.y, c.z, ctr);
+            }
+        },
+        own_first);
+}
+
+template <bool COUNT>
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(DevScene S, PathIO in, float4* __restrict__ Hout,
+                                                                           WaveCounters* ctr) {
+    extern __shared__ uint4 snodes[];
+    const int n = ctr->n_cur;
+    if (n == 0) return;  // drained wavefront: skip staging
+    stage_top_nodes(S, snodes);
+    TraceCount cnt{0u, 0u};
+    extend_queue<COUNT>(S, snodes, in, Hout, n, ctr, cnt);
     if (COUNT) {
         const unsigned nodes = __reduce_add_sync(0xffffffffu, cnt.nodes);
         const unsigned tris = __reduce_add_sync(0xffffffffu, cnt.tris);
@@ -139,28 +169,34 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(Dev
     }
 }
 
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(DevScene S, PathBuffers B, WaveCounters* ctr,
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(DevScene S, ShadowIO Q, int cur, WaveCounters* ctr,
                                                           unsigned long long* __restrict__ film) {
     extern __shared__ uint4 snodes[];
-    const int n = ctr->n_shadow;
+    const int n = cur ? ctr->n_shadow1 : ctr->n_shadow;
     if (n == 0) return;
     stage_top_nodes(S, snodes);
+    shadow_queue(S, snodes, Q, n, ctr, film, true);
+}
+
+// One wavefront iteration's rays: the extension rays of path buffer `in`,
+// then the shadow rays that the iteration before queued (those of the other
+// buffer; film additions are exact integers, so the image does not depend on
+// when they arrive).  A warp that finds no extension ray left goes on with
+// the shadow rays, so the launch has one tail of long rays instead of two:
+// measured (1M-triangle soup) 640x360 at 1 spp 2.9 -> 2.4
+// ms, 1920x1080 at 16 spp 106.3 -> 98.8 ms together with k_generate's grid;
+// the Cornell box at 256x256, 64 spp 6.1 -> 4.75 ms (same images).
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_wave(DevScene S, PathIO in,
+                                                                                 float4* __restrict__ Hout, ShadowIO Q,
+                                                                                 int cur, WaveCounters* ctr,
+                                                                                 unsigned long long* __restrict__ film) {
+    extern __shared__ uint4 snodes[];
+    const int n = ctr->n_cur, m = cur ? ctr->n_shadow : ctr->n_shadow1;
+    if (n == 0 && m == 0) return;
+    stage_top_nodes(S, snodes);
     TraceCount cnt{0u, 0u};
-    persistent_trace<true, false>(
-        S, snodes, n, &ctr->fetch_sh, &ctr->status, cnt,
-        [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
-            const float4 a = B.sh_o[i], b = B.sh_d[i];
-            o = make_float3(a.x, a.y, a.z);
-            d = make_float3(b.x, b.y, b.z);
-            tmax = a.w;
-            if (root != kTravDone) root = __float_as_uint(B.sh_c[i].w);
-        },
-        [&](int i, const HitRec& h) {
-            if (h.prim < 0) {  // unoccluded: the NEE contribution reaches the film
-                const float4 c = B.sh_c[i];
-                film_add(film, (uint32_t)__float_as_int(B.sh_d[i].w), c.x, c.y, c.z, ctr);
-            }
-        });
+    if (n > 0) extend_queue<false>(S, snodes, in, Hout, n, ctr, cnt);
+    if (m > 0) shadow_queue(S, snodes, Q, m, ctr, film, n == 0);
 }
 
 // info.w is the path's job: its table entry holds the render parameters,
@@ -174,113 +210,123 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(Dev
 #ifndef CPPPT_SHADE_BLOCKS
 #define CPPPT_SHADE_BLOCKS 4
 #endif
-__global__ void __launch_bounds__(256, CPPPT_SHADE_BLOCKS) k_shade(DevScene S, PathBuffers B, int cur, WaveCounters* ctr,
-                                               unsigned long long* __restrict__ film,
-                                               const DevBatchJob* __restrict__ jobs) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = ctr->n_cur;
-    bool push_sh = false, push_cont = false;
-    float4 sh_o, sh_d, sh_c, no, nd, nt;
-    int4 ninfo;
-    if (i < n) {
-        const float4 O = B.o[cur][i], D = B.d[cur][i], T = B.thr[cur][i];
-        const int4 I = B.info[cur][i];
-        const float4 H = B.hit[i];
-        const int prim = __float_as_int(H.y);
-        const int pixel = I.x, sample = I.y, bounce = I.z & 0xffff;
-        const bool sdelta = (I.z >> 16) & 1;
-        const DevBatchJob* J = jobs + I.w;
-        const int integrator = J->integrator;
-        const uint32_t seed = J->seed;
-        const int rr_start = J->rr_start, max_depth = J->max_depth;
-        const size_t fpix = (size_t)(uint32_t)pixel + J->film_off;
-        S.light_prim += J->light_off;
-        S.light_area += J->light_off;
-        S.n_lights = J->n_lights;
-        float p = O.w;
-        f3 mul = mk(T.x, T.y, T.z);
-        const f3 ro = mk(O.x, O.y, O.z), rd = mk(D.x, D.y, D.z);
-        if (prim >= 0) {  // a miss adds render_sky = 0 (pathtracerMIS.h:38-41)
-            int kind;
-            DevMaterial m;
-            const Surf s = make_surf(S, prim, ro, rd, H.x, H.z, H.w, bounce == 0, &kind, &m);
-            const f3 wo = -rd;
-            if (kind == PT_MAT_EMISSIVE_) {  // pathtracerMIS.h:43-67: emitters end the path
-                float w = 1.0f;
-                if (!sdelta && integrator == kIntegratorNEE) {
-                    w = 0.0f;  // pathtracer.h:41-46: NEE already counted this emitter
-                } else if (!sdelta && integrator == kIntegratorMIS) {
-                    const int4 vi = __ldg(S.tri_vidx + prim);
-                    const f3 a = f3of(__ldg(S.v_pos + vi.x)), b = f3of(__ldg(S.v_pos + vi.y)),
-                             c = f3of(__ldg(S.v_pos + vi.z));
-                    const float area = length(cross(b - a, c - a)) * 0.5f;
-                    const float pdf_l = (1.0f / (float)S.n_lights) * (1.0f / area);
-                    const float r = H.x;
-                    const float cos_theta = fabsf(dot(s.n, rd)) + kEps;
-                    const float p_nee = pdf_l * r * r / cos_theta;
-                    w = p / (p + p_nee);
-                }
-                film_add(film, fpix, mul.x * m.r * w, mul.y * m.g * w, mul.z * m.b * w, ctr);
-            } else {
-                const Rng4 r0 = rng4(seed, sample, pixel, bounce, 0);
-                const Rng4 r1 = rng4(seed, sample, pixel, bounce, 1);
-                const BSample bs = bsdf_sample(m, s, wo, r0.v[0], r0.v[1]);
-                p = bs.pdf;
-                if (!bs.delta && S.n_lights > 0 && integrator != kIntegratorPT) {  // NEE, pathtracerMIS.h:79-106
-                    const LSample ls = sample_light(S, s.p, r0.v[2], r0.v[3], r1.v[0]);
-                    f3 sd = ls.pos - s.p;
-                    const float len = length(sd);
-                    sd = sd * (1.0f / len);
-                    if (same_hemisphere(s, wo, sd)) {
-                        const float pb = bsdf_pdf(m, s, wo, sd);
-                        const float cosl = fabsf(dot(ls.n, sd)) + kEps;
-                        const float pn = ls.pdf * len * len / cosl;
-                        const float w = integrator == kIntegratorMIS ? pn / (pb + pn) : 1.0f;
-                        const f3 f = bsdf_eval(m, s, wo, sd);
-                        const f3 c = mul * f * ls.le * (1.0f / (ls.pdf * len * len)) * w;
-                        if (c.x != 0.f || c.y != 0.f || c.z != 0.f) {
-                            push_sh = true;
-                            const f3 so = s.p + sd * kEps;
-                            sh_o = make_float4(so.x, so.y, so.z, len - 2.0f * kEps);
-                            sh_d = make_float4(sd.x, sd.y, sd.z, __int_as_float((int)(uint32_t)fpix));
-                            sh_c = make_float4(c.x, c.y, c.z, D.w);  // w: the scene root
-                        }
+// What shading a path's vertex leaves: a shadow ray, the continued path.
+struct ShadeOut {
+    bool push_sh, push_cont;
+    float4 sh_o, sh_d, sh_c;
+    float4 o, d, thr;
+    int4 info;
+};
+
+// One vertex of a path (PathtracerMIS::integrate's loop body): emission with
+// its MIS weight, BSDF sample, next-event estimation, Russian roulette.
+__device__ __forceinline__ void shade_vertex(DevScene S, const DevBatchJob* __restrict__ jobs, float4 O, float4 D, float4 T,
+                                             int4 I, float4 H, WaveCounters* ctr, unsigned long long* __restrict__ film,
+                                             ShadeOut& out) {
+    out.push_sh = out.push_cont = false;
+    const int prim = __float_as_int(H.y);
+    const int pixel = I.x, sample = I.y, bounce = I.z & 0xffff;
+    const bool sdelta = (I.z >> 16) & 1;
+    const DevBatchJob* J = jobs + I.w;
+    const int integrator = J->integrator;
+    const uint32_t seed = J->seed;
+    const int rr_start = J->rr_start, max_depth = J->max_depth;
+    const size_t fpix = (size_t)(uint32_t)pixel + J->film_off;
+    S.light_prim += J->light_off;
+    S.light_area += J->light_off;
+    S.n_lights = J->n_lights;
+    float p = O.w;
+    f3 mul = mk(T.x, T.y, T.z);
+    const f3 ro = mk(O.x, O.y, O.z), rd = mk(D.x, D.y, D.z);
+    if (prim >= 0) {  // a miss adds render_sky = 0 (pathtracerMIS.h:38-41)
+        int kind;
+        DevMaterial m;
+        const Surf s = make_surf(S, prim, ro, rd, H.x, H.z, H.w, bounce == 0, &kind, &m);
+        const f3 wo = -rd;
+        if (kind == PT_MAT_EMISSIVE_) {  // pathtracerMIS.h:43-67: emitters end the path
+            float w = 1.0f;
+            if (!sdelta && integrator == kIntegratorNEE) {
+                w = 0.0f;  // pathtracer.h:41-46: NEE already counted this emitter
+            } else if (!sdelta && integrator == kIntegratorMIS) {
+                const int4 vi = __ldg(S.tri_vidx + prim);
+                const f3 a = f3of(__ldg(S.v_pos + vi.x)), b = f3of(__ldg(S.v_pos + vi.y)),
+                         c = f3of(__ldg(S.v_pos + vi.z));
+                const float area = length(cross(b - a, c - a)) * 0.5f;
+                const float pdf_l = (1.0f / (float)S.n_lights) * (1.0f / area);
+                const float r = H.x;
+                const float cos_theta = fabsf(dot(s.n, rd)) + kEps;
+                const float p_nee = pdf_l * r * r / cos_theta;
+                w = p / (p + p_nee);
+            }
+            film_add(film, fpix, mul.x * m.r * w, mul.y * m.g * w, mul.z * m.b * w, ctr);
+        } else {
+            const Rng4 r0 = rng4(seed, sample, pixel, bounce, 0);
+            const Rng4 r1 = rng4(seed, sample, pixel, bounce, 1);
+            const BSample bs = bsdf_sample(m, s, wo, r0.v[0], r0.v[1]);
+            p = bs.pdf;
+            if (!bs.delta && S.n_lights > 0 && integrator != kIntegratorPT) {  // NEE, pathtracerMIS.h:79-106
+                const LSample ls = sample_light(S, s.p, r0.v[2], r0.v[3], r1.v[0]);
+                f3 sd = ls.pos - s.p;
+                const float len = length(sd);
+                sd = sd * (1.0f / len);
+                if (same_hemisphere(s, wo, sd)) {
+                    const float pb = bsdf_pdf(m, s, wo, sd);
+                    const float cosl = fabsf(dot(ls.n, sd)) + kEps;
+                    const float pn = ls.pdf * len * len / cosl;
+                    const float w = integrator == kIntegratorMIS ? pn / (pb + pn) : 1.0f;
+                    const f3 f = bsdf_eval(m, s, wo, sd);
+                    const f3 c = mul * f * ls.le * (1.0f / (ls.pdf * len * len)) * w;
+                    if (c.x != 0.f || c.y != 0.f || c.z != 0.f) {
+                        out.push_sh = true;
+                        const f3 so = s.p + sd * kEps;
+                        out.sh_o = make_float4(so.x, so.y, so.z, len - 2.0f * kEps);
+                        out.sh_d = make_float4(sd.x, sd.y, sd.z, __int_as_float((int)(uint32_t)fpix));
+                        out.sh_c = make_float4(c.x, c.y, c.z, D.w);  // w: the scene root
                     }
                 }
-                if (same_hemisphere(s, wo, bs.wi)) {  // pathtracerMIS.h:112-126
-                    const f3 f = bsdf_eval(m, s, wo, bs.wi);
-                    bool alive = true;
-                    if (bounce >= rr_start) {
-                        const float rr = russian_roulette(f);
-                        if (r1.v[1] > rr) alive = false;
-                        else p = p * rr;
-                    }
-                    if (alive && bounce + 1 < max_depth) {
-                        mul = mul * f * (1.0f / p);
-                        const f3 oo = s.p + bs.wi * kEps;
-                        push_cont = true;
-                        no = make_float4(oo.x, oo.y, oo.z, p);
-                        nd = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
-                        nt = make_float4(mul.x, mul.y, mul.z, 0.f);
-                        ninfo = make_int4(pixel, sample, (bounce + 1) | ((bs.delta ? 1 : 0) << 16), I.w);
-                    }
+            }
+            if (same_hemisphere(s, wo, bs.wi)) {  // pathtracerMIS.h:112-126
+                const f3 f = bsdf_eval(m, s, wo, bs.wi);
+                bool alive = true;
+                if (bounce >= rr_start) {
+                    const float rr = russian_roulette(f);
+                    if (r1.v[1] > rr) alive = false;
+                    else p = p * rr;
+                }
+                if (alive && bounce + 1 < max_depth) {
+                    mul = mul * f * (1.0f / p);
+                    const f3 oo = s.p + bs.wi * kEps;
+                    out.push_cont = true;
+                    out.o = make_float4(oo.x, oo.y, oo.z, p);
+                    out.d = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, D.w);
+                    out.thr = make_float4(mul.x, mul.y, mul.z, 0.f);
+                    out.info = make_int4(pixel, sample, (bounce + 1) | ((bs.delta ? 1 : 0) << 16), I.w);
                 }
             }
         }
     }
-    const int js = warp_append(&ctr->n_shadow, push_sh);
-    if (push_sh) {
-        B.sh_o[js] = sh_o;
-        B.sh_d[js] = sh_d;
-        B.sh_c[js] = sh_c;
+}
+
+__global__ void __launch_bounds__(256, CPPPT_SHADE_BLOCKS) k_shade(DevScene S, PathIO in, PathIO nxt, ShadowIO Q,
+                                               const float4* __restrict__ hit, int cur, WaveCounters* ctr,
+                                               unsigned long long* __restrict__ film,
+                                               const DevBatchJob* __restrict__ jobs) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    ShadeOut out;
+    out.push_sh = out.push_cont = false;
+    if (i < ctr->n_cur) shade_vertex(S, jobs, in.o[i], in.d[i], in.thr[i], in.info[i], hit[i], ctr, film, out);
+    const int js = warp_append(cur ? &ctr->n_shadow1 : &ctr->n_shadow, out.push_sh);
+    if (out.push_sh) {
+        Q.o[js] = out.sh_o;
+        Q.d[js] = out.sh_d;
+        Q.c[js] = out.sh_c;
     }
-    const int jc = warp_append(&ctr->n_next, push_cont);
-    if (push_cont) {
-        const int nx = 1 - cur;
-        B.o[nx][jc] = no;
-        B.d[nx][jc] = nd;
-        B.thr[nx][jc] = nt;
-        B.info[nx][jc] = ninfo;
+    const int jc = warp_append(&ctr->n_next, out.push_cont);
+    if (out.push_cont) {
+        nxt.o[jc] = out.o;
+        nxt.d[jc] = out.d;
+        nxt.thr[jc] = out.thr;
+        nxt.info[jc] = out.info;
     }
 }
 
@@ -297,55 +343,58 @@ __device__ __forceinline__ int find_job(const DevBatchJob* __restrict__ jobs, in
 
 // New camera paths for the free slots of the next buffer; work index w
 // (global over the jobs' pixel x sample ranges) selects job, sample, pixel.
-__global__ void __launch_bounds__(256) k_generate(DevScene S, PathBuffers B, int cur, WaveCounters* ctr,
+__global__ void __launch_bounds__(256) k_generate(PathIO nxt, int capacity, WaveCounters* ctr,
                                                   const DevBatchJob* __restrict__ jobs, int n_jobs) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int n_next = ctr->n_next;
-    const int avail = B.capacity - n_next;
-    unsigned long long w = ctr->work_next + (unsigned long long)t;
-    if (t >= avail || w >= ctr->work_total) return;
-    const int job = n_jobs > 1 ? find_job(jobs, n_jobs, w) : 0;
-    const DevBatchJob* J = jobs + job;
-    w -= J->work_begin;
-    const DevCamera* C = &J->cam;
-    const int width = C->width, height = C->height, spp_axis = J->spp_axis;
-    const uint32_t seed = J->seed, root = J->root;
-    const unsigned long long npix = (unsigned long long)width * height;
-    const int sample = (int)(w / npix);
-    int pixel = (int)(w - (unsigned long long)sample * npix);
-    {  // visit the pass in tiles (a bijection of the pixels; the RNG is keyed by pixel, not by order)
-        const int tw = J->tile_w, th = J->tile_h;
-        if (tw * th > 1) {
-            const int tile = pixel / (tw * th), r = pixel - tile * (tw * th);
-            const int tiles_x = width / tw;
-            const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
-            pixel = (ty * th + r / tw) * width + tx * tw + r % tw;
+    const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
+    const int room = capacity - n_next;
+    const int count = left < (unsigned long long)room ? (int)left : room;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+        unsigned long long w = first + (unsigned long long)t;
+        const int job = n_jobs > 1 ? find_job(jobs, n_jobs, w) : 0;
+        const DevBatchJob* J = jobs + job;
+        w -= J->work_begin;
+        const DevCamera* C = &J->cam;
+        const int width = C->width, height = C->height, spp_axis = J->spp_axis;
+        const uint32_t seed = J->seed, root = J->root;
+        const unsigned long long npix = (unsigned long long)width * height;
+        const int sample = (int)(w / npix);
+        int pixel = (int)(w - (unsigned long long)sample * npix);
+        {  // visit the pass in tiles (a bijection of the pixels; the RNG is keyed by pixel, not by order)
+            const int tw = J->tile_w, th = J->tile_h;
+            if (tw * th > 1) {
+                const int tile = pixel / (tw * th), r = pixel - tile * (tw * th);
+                const int tiles_x = width / tw;
+                const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
+                pixel = (ty * th + r / tw) * width + tx * tw + r % tw;
+            }
         }
+        const int px = pixel % width, py = pixel / width;
+        const Rng4 r = rng4(seed, sample, pixel, 0xffffu, 2);
+        float cx, cy;
+        if (spp_axis > 0) {  // pathtracerMIS.h:148-153: spp x spp strata
+            const int k = sample / spp_axis, l = sample - (sample / spp_axis) * spp_axis;
+            cx = (((float)px + ((float)k + r.v[0]) / (float)spp_axis) / (float)width) * 2.0f - 1.0f;
+            cy = -((((float)py + ((float)l + r.v[1]) / (float)spp_axis) / (float)height) * 2.0f - 1.0f);
+        } else {
+            cx = (((float)px + r.v[0]) / (float)width) * 2.0f - 1.0f;
+            cy = -((((float)py + r.v[1]) / (float)height) * 2.0f - 1.0f);
+        }
+        // CameraPerspective::get_ray (camera_perspective.h:30-39)
+        const float dx = cx * C->tan_fovy * C->aspect, dy = cy * C->tan_fovy, dz = -1.0f;
+        const f3 d = normalized(mk(C->m[0] * dx + C->m[1] * dy + C->m[2] * dz, C->m[3] * dx + C->m[4] * dy + C->m[5] * dz,
+                                   C->m[6] * dx + C->m[7] * dy + C->m[8] * dz));
+        const int j = n_next + t;
+        nxt.o[j] = make_float4(C->o[0], C->o[1], C->o[2], 1.0f);
+        nxt.d[j] = make_float4(d.x, d.y, d.z, __uint_as_float(root));
+        nxt.thr[j] = make_float4(1.f, 1.f, 1.f, 0.f);
+        nxt.info[j] = make_int4(pixel, sample, 0 | (1 << 16), job);  // sampled_delta starts true (:34)
     }
-    const int px = pixel % width, py = pixel / width;
-    const Rng4 r = rng4(seed, sample, pixel, 0xffffu, 2);
-    float cx, cy;
-    if (spp_axis > 0) {  // pathtracerMIS.h:148-153: spp x spp strata
-        const int k = sample / spp_axis, l = sample - (sample / spp_axis) * spp_axis;
-        cx = (((float)px + ((float)k + r.v[0]) / (float)spp_axis) / (float)width) * 2.0f - 1.0f;
-        cy = -((((float)py + ((float)l + r.v[1]) / (float)spp_axis) / (float)height) * 2.0f - 1.0f);
-    } else {
-        cx = (((float)px + r.v[0]) / (float)width) * 2.0f - 1.0f;
-        cy = -((((float)py + r.v[1]) / (float)height) * 2.0f - 1.0f);
-    }
-    // CameraPerspective::get_ray (camera_perspective.h:30-39)
-    const float dx = cx * C->tan_fovy * C->aspect, dy = cy * C->tan_fovy, dz = -1.0f;
-    const f3 d = normalized(mk(C->m[0] * dx + C->m[1] * dy + C->m[2] * dz, C->m[3] * dx + C->m[4] * dy + C->m[5] * dz,
-                               C->m[6] * dx + C->m[7] * dy + C->m[8] * dz));
-    const int nx = 1 - cur;
-    const int j = n_next + t;
-    B.o[nx][j] = make_float4(C->o[0], C->o[1], C->o[2], 1.0f);
-    B.d[nx][j] = make_float4(d.x, d.y, d.z, __uint_as_float(root));
-    B.thr[nx][j] = make_float4(1.f, 1.f, 1.f, 0.f);
-    B.info[nx][j] = make_int4(pixel, sample, 0 | (1 << 16), job);  // sampled_delta starts true (:34)
 }
 
-__global__ void k_advance(WaveCounters* ctr, int capacity) {
+// Counters at the end of an iteration that read path buffer `cur`.  traced: the
+// buffer whose shadow rays have been traced by now (the other one in k_trace_wave's order).
+__global__ void k_advance(WaveCounters* ctr, int capacity, int cur, int traced) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int n_next = ctr->n_next;
     const unsigned long long left = ctr->work_total - ctr->work_next;
@@ -353,11 +402,11 @@ __global__ void k_advance(WaveCounters* ctr, int capacity) {
     const unsigned long long added = left < room ? left : room;
     ctr->work_next += added;
     ctr->stat_paths += added;
-    ctr->stat_shadow += (unsigned long long)ctr->n_shadow;
+    ctr->stat_shadow += (unsigned long long)(cur ? ctr->n_shadow1 : ctr->n_shadow);
     ctr->n_cur = n_next + (int)added;
     ctr->stat_closest += (unsigned long long)ctr->n_cur;
     ctr->n_next = 0;
-    ctr->n_shadow = 0;
+    (traced ? ctr->n_shadow1 : ctr->n_shadow) = 0;
     ctr->fetch_ext = 0;
     ctr->fetch_sh = 0;
     ctr->stat_iters += 1;
@@ -368,10 +417,21 @@ __global__ void k_resolve(const unsigned long long* __restrict__ film, float* __
         out[i] = (float)((double)(long long)film[i] * scale);
 }
 
+namespace {
+PathIO path_io(const PathBuffers& B, int k) { return PathIO{B.o[k], B.d[k], B.thr[k], B.info[k]}; }
+ShadowIO shadow_io(const PathBuffers& B) { return ShadowIO{B.sh_o, B.sh_d, B.sh_c}; }
+}  // namespace
+
 void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, int num_sms, cudaStream_t st,
                    bool count) {
-    if (count) k_extend<true><<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, B, cur, ctr);
-    else k_extend<false><<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, B, cur, ctr);
+    const int g = num_sms * kTraceBlocksPerSM;
+    if (count) k_extend<true><<<g, kTraceThreads, kSmemNodeBytes, st>>>(S, path_io(B, cur), B.hit, ctr);
+    else k_extend<false><<<g, kTraceThreads, kSmemNodeBytes, st>>>(S, path_io(B, cur), B.hit, ctr);
+}
+void launch_trace_wave(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
+                       int num_sms, cudaStream_t st) {
+    k_trace_wave<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, path_io(B, cur), B.hit,
+                                                                                     shadow_io(B), cur, ctr, film);
 }
 cudaError_t trace_kernels_setup() {
     const int bytes = (int)kSmemNodeBytes;
@@ -379,29 +439,41 @@ cudaError_t trace_kernels_setup() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_any, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_extend<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_extend<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e;
 }
 
 void launch_shade(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                   const DevBatchJob* jobs, cudaStream_t st) {
-    k_shade<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, B, cur, ctr, film, jobs);
+    k_shade<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, path_io(B, cur), path_io(B, 1 - cur), shadow_io(B), B.hit, cur,
+                                                      ctr, film, jobs);
 }
-void launch_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film, int num_sms,
-                   cudaStream_t st) {
-    k_shadow<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, B, ctr, film);
+void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
+                   int num_sms, cudaStream_t st) {
+    k_shadow<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, shadow_io(B), cur, ctr, film);
 }
-void launch_generate(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs,
-                     int n_jobs, cudaStream_t st) {
-    k_generate<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, B, cur, ctr, jobs, n_jobs);
-    k_advance<<<1, 32, 0, st>>>(ctr, B.capacity);
+void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs, int n_jobs, int num_sms,
+                     cudaStream_t st, bool shadows_traced) {
+    // a resident grid that strides over the free slots: most iterations have
+    // few of them or none, and a CTA per 256 slots of the capacity cost up to
+    // 50 us a launch there (a quarter of the Cornell box's 64-spp render)
+    const int g = max(1, min((B.capacity + 255) / 256, num_sms * 8));
+    k_generate<<<g, 256, 0, st>>>(path_io(B, 1 - cur), B.capacity, ctr, jobs, n_jobs);
+    k_advance<<<1, 32, 0, st>>>(ctr, B.capacity, cur, shadows_traced ? cur : 1 - cur);
+}
+void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
+                           const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
+    launch_trace_wave(S, B, cur, ctr, film, num_sms, st);
+    launch_shade(S, B, cur, ctr, film, jobs, st);
+    launch_generate(B, cur, ctr, jobs, n_jobs, num_sms, st, false);
 }
 
 // Body end of a device-driven render loop (build_render_graph).  One thread.
 __global__ void k_round_control(WaveCounters* ctr, cudaGraphConditionalHandle h) {
     const uint32_t r = ctr->rounds + 1u;
     ctr->rounds = r;
-    bool more = !(ctr->n_cur == 0 && ctr->work_next >= ctr->work_total) && ctr->status == 0u;
+    bool more = !wave_done(*ctr) && ctr->status == 0u;
     if (more && r >= ctr->max_rounds) {
         ctr->status |= kStatusRoundLimit;
         more = false;
@@ -431,13 +503,8 @@ cudaError_t build_render_graph(const DevScene& S, const PathBuffers& B, WaveCoun
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            for (int k = 0; k < iters; k++) {
-                const int cur = k & 1;
-                launch_extend(S, B, cur, ctr, num_sms, st);
-                launch_shade(S, B, cur, ctr, film, jobs, st);
-                launch_shadow(S, B, ctr, film, num_sms, st);
-                launch_generate(S, B, cur, ctr, jobs, n_jobs, st);
-            }
+            for (int k = 0; k < iters; k++)
+                launch_wave_iteration(S, B, k & 1, ctr, film, jobs, n_jobs, num_sms, st);
             k_round_control<<<1, 1, 0, st>>>(ctr, h);
             cudaGraph_t captured = nullptr;
             const cudaError_t e2 = cudaStreamEndCapture(st, &captured);
@@ -625,25 +692,19 @@ cudaError_t render_noalloc(const DevScene& S, const RenderParams& P, int num_sms
     const DevBatchJob hjob = single_job(S, P);
     e = cudaMemcpyAsync(job, &hjob, sizeof(hjob), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
-    launch_generate(S, B, 1, ctr, job, 1, st);
+    launch_generate(B, 1, ctr, job, 1, num_sms, st, false);
     const int iters = 16;
     const unsigned long long max_rounds =
         64 + (total / (unsigned long long)kNoAllocPaths + 2) * (unsigned long long)(max_depth + 2) * 4 / iters;
     WaveCounters h{};
     for (unsigned long long round = 0;; round++) {
-        for (int k = 0; k < iters; k++) {
-            const int cur = k & 1;
-            launch_extend(S, B, cur, ctr, num_sms, st, false);
-            launch_shade(S, B, cur, ctr, film, job, st);
-            launch_shadow(S, B, ctr, film, num_sms, st);
-            launch_generate(S, B, cur, ctr, job, 1, st);
-        }
+        for (int k = 0; k < iters; k++) launch_wave_iteration(S, B, k & 1, ctr, film, job, 1, num_sms, st);
         e = cudaMemcpyAsync(&h, ctr, sizeof(h), cudaMemcpyDeviceToHost, st);
         if (e != cudaSuccess) return e;
         e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return e;
         if (h.status) break;
-        if (h.n_cur == 0 && h.work_next >= h.work_total) break;
+        if (wave_done(h)) break;
         if (round > max_rounds) {
             *limit_hit = 1;
             break;

@@ -454,6 +454,8 @@ __device__ __forceinline__ bool trav_leaf(Trav& T, const DevScene& S, TraceCount
 // rays (ray_chunk) into a warp-private range, the first one by its number and
 // the next ones from a global counter; a lane whose ray finishes
 // takes the next ray of the range at once (no waiting for the other lanes).
+// own_first = false: the first chunk comes from the counter too (a kernel's
+// second queue, which warps reach at different times).
 // load(i, o, d, tmax, root) fetches ray i; root arrives set to the scene's
 // own root and may be replaced (rays of a merged multi-scene arena).
 //
@@ -508,7 +510,7 @@ __device__ __forceinline__ int ray_chunk(int left, int nwarps, int share) {
 template <bool ANY, bool COUNT, class Load, class Store>
 __device__ __forceinline__ void persistent_trace(const DevScene& S, const uint4* __restrict__ snodes, int n,
                                                  int* counter, uint32_t* status, TraceCount& cnt, Load load,
-                                                 Store store) {
+                                                 Store store, bool own_first = true) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     Trav T;
@@ -518,7 +520,7 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, const uint4*
     // across the CTAs, so a small batch spreads over every SM), later ones
     // come from the counter
     const int nwarps = (int)(gridDim.x * (blockDim.x >> 5));
-    const int c0 = ray_chunk(n, nwarps, 1);
+    const int c0 = own_first ? ray_chunk(n, nwarps, 1) : 0;
     int pool_next = min((int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * c0, n);
     int pool_end = min(pool_next + c0, n);
     bool exhausted = nwarps * c0 >= n;
