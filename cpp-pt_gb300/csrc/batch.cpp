@@ -343,7 +343,9 @@ void render_batch(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float* cons
     std::memcpy(b->h_jobs, table.data(), sizeof(DevBatchJob) * n_jobs);
     ck(cudaMemcpyAsync(b->d_jobs, b->h_jobs, sizeof(DevBatchJob) * n_jobs, cudaMemcpyHostToDevice, st), "jobs");
     const pt_batch::GraphKey key{b->film, n_jobs, capacity, t.iters_per_graph};
-    if (!b->graph || !(b->graph_key == key)) {
+    // a render that the first generate holds whole and k_finish takes at once needs no loop
+    const bool loop = total > (unsigned long long)std::min(kFinishPaths, capacity);
+    if (loop && (!b->graph || !(b->graph_key == key))) {
         if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         ck(build_render_graph(b->arena, b->pb, b->d_ctr, b->film, b->d_jobs, n_jobs, t.iters_per_graph, b->num_sms, st,
                               &b->graph),
@@ -369,7 +371,8 @@ void render_batch(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float* cons
     ck(cudaMemcpyAsync(b->d_ctr, b->h_ctr, sizeof(WaveCounters), cudaMemcpyHostToDevice, st), "init counters");
     launch_generate(b->pb, 1, b->d_ctr, b->d_jobs, n_jobs, b->num_sms, st, false);  // fills buffer 0
     // the whole loop on the device: one graph launch, one read of the counters
-    ck(cudaGraphLaunch(b->graph, st), "graph launch");
+    if (loop) ck(cudaGraphLaunch(b->graph, st), "graph launch");
+    launch_finish(b->arena, b->pb, b->d_ctr, b->film, b->d_jobs, b->num_sms, st);
     ck(cudaMemcpyAsync(b->h_ctr, b->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");
     ck(cudaStreamSynchronize(st), "batch render");
     {
@@ -380,7 +383,7 @@ void render_batch(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float* cons
         if (status & kStatusRoundLimit) throw Fail(PT_ERR_LIMIT, "batch render did not converge within the iteration bound");
     }
     const unsigned long long rounds = b->h_ctr->rounds;
-    double launches = 2 + (double)rounds * (kKernelsPerIteration * t.iters_per_graph + 1);
+    double launches = 2 + (double)rounds * (kKernelsPerIteration * t.iters_per_graph + 1) + 1;
     for (int i = 0; i < n_jobs; i++) {
         const pt_batch::Member& m = b->members[jobs[i].scene];
         const size_t off = 3 * (size_t)table[i].film_off;
@@ -398,7 +401,7 @@ void render_batch(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float* cons
     R.paths = (double)b->h_ctr->stat_paths;
     R.closest_rays = (double)b->h_ctr->stat_closest;
     R.shadow_rays = (double)b->h_ctr->stat_shadow;
-    R.iterations = (double)b->h_ctr->stat_iters;
+    R.iterations = (double)b->h_ctr->stat_iters + (double)b->h_ctr->n_next;
     R.render_ms = ms;
     R.kernel_launches = launches;
     R.nonfinite = (double)b->h_ctr->stat_nonfinite;

@@ -101,8 +101,14 @@ struct WaveCounters {
         int32_t n_shadow1;  // plain renders: shadow rays of the iterations that read path buffer 1 (n_shadow: buffer 0)
     };
     int32_t fetch_ext, fetch_sh;
-    int32_t free_top;  // vertex-slot free list
-    int32_t n_rec;     // training records
+    union {
+        int32_t free_top;  // learned-guide and SD-tree renders: vertex-slot free list
+        int32_t n_finish;  // plain renders: paths left to k_finish
+    };
+    union {
+        int32_t n_rec;       // learned-guide renders: training records
+        int32_t finish_buf;  // plain renders: the path buffer that holds them
+    };
     uint32_t status;
     float film_safe;  // |contribution| below this cannot carry a film sum out of the 32.32 range
     uint32_t rounds;      // loop bodies run by a device-driven render (k_round_control)
@@ -113,11 +119,6 @@ struct WaveCounters {
     unsigned long long stat_nonfinite;         // contributions dropped because they were inf/NaN
     unsigned long long stat_film_overflow;     // contributions the 32.32 film could not hold
 };
-
-// A plain render's wavefront has nothing left: no path, no work, no shadow ray.
-__host__ __device__ inline bool wave_done(const WaveCounters& c) {
-    return c.n_cur == 0 && c.work_next >= c.work_total && c.n_shadow == 0 && c.n_shadow1 == 0;
-}
 
 // film_safe for a render of at most `per_pixel` film contributions per pixel
 // and channel: a sum of contributions below 2^31 / per_pixel stays below

@@ -851,7 +851,9 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     const bool direct = timed || count;
     // the render parameters live in the scene's one-entry job table and the
     // counters, so the graph stays valid across renders
-    if (!direct && !s->graph)
+    // a render that the first generate holds whole and k_finish takes at once needs no loop
+    const bool loop = total > (unsigned long long)std::min(kFinishPaths, capacity);
+    if (!direct && loop && !s->graph)
         ck(build_render_graph(s->dev, s->pb, s->d_ctr, s->film, s->d_job, 1, kItersPerBody, s->num_sms, st,
                               &s->graph),
            "render graph");
@@ -869,18 +871,19 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     s->h_job->integrator = desc->mode == PT_MODE_NEE ? kIntegratorNEE
                            : desc->mode == PT_MODE_PT ? kIntegratorPT : kIntegratorMIS;
     ck(cudaMemcpyAsync(s->d_job, s->h_job, sizeof(DevBatchJob), cudaMemcpyHostToDevice, st), "job table");
-    launch_generate(s->pb, 1, s->d_ctr, s->d_job, 1, s->num_sms, st, false);  // fills buffer 0
+    launch_generate(s->pb, 1, s->d_ctr, s->d_job, 1, s->num_sms, st, direct);  // fills buffer 0
     double launches = 2;
     std::vector<cudaEvent_t> tev;
     unsigned long long rounds = 0;
     if (!direct) {
         // the whole loop on the device: one graph launch, one read of the counters
-        ck(cudaGraphLaunch(s->graph, st), "graph launch");
+        if (loop) ck(cudaGraphLaunch(s->graph, st), "graph launch");
+        launch_finish(s->dev, s->pb, s->d_ctr, s->film, s->d_job, s->num_sms, st);
         ck(cudaMemcpyAsync(s->h_ctr, s->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");
         ck(cudaStreamSynchronize(st), "render");
         check_status(s, s->h_ctr->status);
         rounds = s->h_ctr->rounds;
-        launches += (double)rounds * (kKernelsPerIteration * kItersPerBody + 1);
+        launches += (double)rounds * (kKernelsPerIteration * kItersPerBody + 1) + 1;
     }
     while (direct) {
         {
@@ -905,7 +908,7 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
         ck(cudaStreamSynchronize(st), "render");
         check_status(s, s->h_ctr->status);
         rounds++;
-        if (wave_done(*s->h_ctr)) break;
+        if (s->h_ctr->n_cur == 0 && s->h_ctr->work_next >= s->h_ctr->work_total) break;
         if (rounds > max_rounds) throw Fail(PT_ERR_LIMIT, "render did not converge within the iteration bound");
     }
     launch_film_resolve(s->film, d_dst ? d_dst : s->d_out, film_n, 1.0 / (double)desc->spp, st);
@@ -919,7 +922,7 @@ void render_impl(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     R.paths = (double)s->h_ctr->stat_paths;
     R.closest_rays = (double)s->h_ctr->stat_closest;
     R.shadow_rays = (double)s->h_ctr->stat_shadow;
-    R.iterations = (double)s->h_ctr->stat_iters;
+    R.iterations = (double)s->h_ctr->stat_iters + (double)s->h_ctr->n_next;
     R.render_ms = ms;
     R.kernel_launches = launches + 1;
     R.extend_nodes = (double)s->h_ctr->stat_nodes;
@@ -1202,7 +1205,7 @@ pt_status pt_render_device_noalloc(pt_scene* s, const pt_render_desc* desc, floa
         R.paths = (double)h.stat_paths;
         R.closest_rays = (double)h.stat_closest;
         R.shadow_rays = (double)h.stat_shadow;
-        R.iterations = (double)h.stat_iters;
+        R.iterations = (double)h.stat_iters + (double)h.n_next;
         R.nonfinite = (double)h.stat_nonfinite;
         R.film_overflow = (double)h.stat_film_overflow;
         s->stats = R;

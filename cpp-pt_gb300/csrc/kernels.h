@@ -71,6 +71,14 @@ void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const Dev
 // shadow rays of the iteration before (one launch), shade, generate, advance.
 void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                            const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st);
+// Paths that k_finish takes once no work is left (render.cu); a render of no
+// more than these needs no wavefront iteration at all.
+constexpr int kFinishPaths = 65536;
+// After the last iteration: its shadow rays and the paths k_advance left to
+// k_finish (n_finish), to their ends.  The longest warp's passes are in
+// ctr->n_next afterwards.
+void launch_finish(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
+                   const DevBatchJob* jobs, int num_sms, cudaStream_t st);
 // The whole wavefront loop of a plain render (PT_MODE_MIS / NEE / PT, single
 // scene or batch) as one executable graph: a conditional WHILE node whose
 // body runs `iters` (even) iterations and then a round-control kernel that

@@ -580,4 +580,39 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, const uint4*
     }
 }
 
+// Traces one ray per lane (active lanes' T, set up by trav_init) to the end:
+// the closest hit, or with `any` until the first hit (the same test against
+// the ray's own max_t, which best.t holds until then).  All 32 lanes call it.
+__device__ __forceinline__ void warp_trace(const DevScene& S, Trav& T, TravStack& K, bool active, bool any,
+                                           uint32_t* status) {
+    TraceCount cnt{0u, 0u};
+    while (true) {
+        const bool live = active && (T.cur != kTravDone || T.leaf != kTravDone);
+        const unsigned act = __ballot_sync(0xffffffffu, live);
+        if (act == 0) break;
+        unsigned wait, inner;
+        do {
+            if (live && is_inner(T.cur)) {
+                if (++T.steps > S.step_limit) trav_abort(T, status, kStatusIterLimit);
+                else if (T.cur_t > cull_dist(T)) trav_pop(T, K);
+                else trav_node<false, false>(T, K, S, nullptr, status, cnt);
+            }
+            if (live && T.leaf == kTravDone && is_leaf(T.cur)) {
+                T.leaf = T.cur;
+                trav_pop(T, K);
+            }
+            wait = __ballot_sync(0xffffffffu, live && T.leaf != kTravDone && !is_inner(T.cur));
+            inner = __ballot_sync(0xffffffffu, live && is_inner(T.cur));
+        } while (inner != 0 && CPPPT_LEAF_WAIT_DIV * __popc(wait) < __popc(act));
+        if (live && T.leaf != kTravDone) {
+            ++T.steps;
+            trav_leaf<false, false>(T, S, cnt);
+            if (any && T.best.prim >= 0) {
+                T.cur = kTravDone;
+                T.sp = 0;
+            }
+        }
+    }
+}
+
 }  // namespace cpppt_gb300

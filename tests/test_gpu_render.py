@@ -205,3 +205,20 @@ def test_render_argument_errors(gpu_lib):
         gs.render(0)
     with pytest.raises(PtError):
         gs.render(4, max_depth=0)
+
+
+@pytest.mark.parametrize("width,height,spp", [(1, 1, 1), (37, 1, 3), (64, 64, 1), (152, 32, 1), (256, 256, 1),
+                                              (257, 256, 1), (256, 257, 2)])
+def test_last_paths_give_the_wavefronts_image(gpu_lib, width, height, spp):
+    """Renders around the number of paths that are finished in one launch
+    (65536) give the image of the wavefront that traces every iteration
+    separately (PT_FLAG_TIME_KERNELS), bit for bit, in every mode."""
+    from cpppt.lib import FLAG_TIME_KERNELS, MODE_MIS, MODE_NEE, MODE_PT, GpuScene
+    gs = GpuScene(scenes.soup(seed=5, n_spheres=120, freq=3, width=width, height=height, extent=8.0))
+    for mode in (MODE_MIS, MODE_NEE, MODE_PT):
+        got = gs.render(spp, max_depth=10, seed=3, mode=mode)
+        st = gs.stats()
+        want = gs.render(spp, max_depth=10, seed=3, mode=mode, flags=FLAG_TIME_KERNELS)
+        wt = gs.stats()
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+        assert all(st[k] == wt[k] for k in ("paths", "closest_rays", "shadow_rays"))
