@@ -989,15 +989,12 @@ __global__ void __launch_bounds__(256) k_finish_nn(NNPathData PD, WaveCounters* 
 __global__ void __launch_bounds__(kTraceThreads) k_shadow_nn(DevScene S, PathBuffers B, WaveCounters* ctr,
                                                    unsigned long long* __restrict__ film, NNPathData PD,
                                                    const DevBatchJob* __restrict__ jobs) {
-    extern __shared__ uint4 snodes[];
+    extern __shared__ uint32_t s_stack[];
     const int n = ctr->n_shadow;
     if (n == 0) return;
-    const int nn = min(S.n_nodes, kSmemNodes) * 4;
-    for (int k = threadIdx.x; k < nn; k += blockDim.x) snodes[k] = __ldg(S.nodes + k);
-    __syncthreads();
     TraceCount cnt{0u, 0u};
     persistent_trace<true, false>(
-        S, snodes, n, &ctr->fetch_sh, &ctr->status, cnt,
+        S, s_stack, n, &ctr->fetch_sh, &ctr->status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
             const float4 a = B.sh_o[i], b = B.sh_d[i];
             o = make_float3(a.x, a.y, a.z);
@@ -1020,7 +1017,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_shadow_nn(DevScene S, PathBuf
 }
 
 cudaError_t nn_shadow_smem_limit() {
-    return cudaFuncSetAttribute(k_shadow_nn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemNodeBytes);
+    return cudaFuncSetAttribute(k_shadow_nn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTraceSmem);
 }
 
 // Camera paths (stratified like pathtracerMIS.h:148-153) with a vertex slot.
@@ -1110,7 +1107,7 @@ void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const Ren
 }
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    k_shadow_nn<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, B, ctr, film, PD, jobs);
+    k_shadow_nn<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kTraceSmem, st>>>(S, B, ctr, film, PD, jobs);
 }
 void launch_nn_generate(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
                         const DevBatchJob* jobs, int n_jobs, cudaStream_t st) {

@@ -21,12 +21,6 @@
 
 namespace cpppt_gb300 {
 
-__device__ __forceinline__ void stage_top_nodes(const DevScene& S, uint4* snodes) {
-    const int n = min(S.n_nodes, kSmemNodes) * 4;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) snodes[i] = __ldg(S.nodes + i);
-    __syncthreads();
-}
-
 // Each warp takes 32 consecutive work items at a time from a global counter
 // (persistent threads); returns the first index, or >= n when done.
 __device__ __forceinline__ int warp_fetch(int* counter, int n) {
@@ -59,11 +53,10 @@ __device__ __forceinline__ int warp_append(int* counter, bool pred) {
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_closest(DevScene S, const float* __restrict__ rays, int n,
                                                                  float4* __restrict__ hits, int* counter,
                                                                  uint32_t* status) {
-    extern __shared__ uint4 snodes[];
-    stage_top_nodes(S, snodes);
+    extern __shared__ uint32_t s_stack[];
     TraceCount cnt{0u, 0u};
     persistent_trace<false, false>(
-        S, snodes, n, counter, status, cnt,
+        S, s_stack, n, counter, status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
             const float* r = rays + 7 * (size_t)i;
             o = make_float3(r[0], r[1], r[2]);
@@ -76,11 +69,10 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_clos
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_any(DevScene S, const float* __restrict__ rays, int n,
                                                              uint8_t* __restrict__ occ, int* counter,
                                                              uint32_t* status) {
-    extern __shared__ uint4 snodes[];
-    stage_top_nodes(S, snodes);
+    extern __shared__ uint32_t s_stack[];
     TraceCount cnt{0u, 0u};
     persistent_trace<true, false>(
-        S, snodes, n, counter, status, cnt,
+        S, s_stack, n, counter, status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
             const float* r = rays + 7 * (size_t)i;
             o = make_float3(r[0], r[1], r[2]);
@@ -94,14 +86,14 @@ void launch_trace_closest(const DevScene& S, const float* rays, int n, float4* h
                           int num_sms, cudaStream_t st) {
     if (n <= 0) return;
     const int blocks = min(num_sms * kTraceBlocksPerSM, n);
-    k_trace_closest<<<blocks, kTraceThreads, kSmemNodeBytes, st>>>(S, rays, n, hits, counter, status);
+    k_trace_closest<<<blocks, kTraceThreads, kTraceSmem, st>>>(S, rays, n, hits, counter, status);
 }
 
 void launch_trace_any(const DevScene& S, const float* rays, int n, uint8_t* occ, int* counter, uint32_t* status,
                       int num_sms, cudaStream_t st) {
     if (n <= 0) return;
     const int blocks = min(num_sms * kTraceBlocksPerSM, n);
-    k_trace_any<<<blocks, kTraceThreads, kSmemNodeBytes, st>>>(S, rays, n, occ, counter, status);
+    k_trace_any<<<blocks, kTraceThreads, kTraceSmem, st>>>(S, rays, n, occ, counter, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -117,12 +109,12 @@ __device__ __forceinline__ void film_add(unsigned long long* film, size_t pix, f
 
 // The extension rays of a path buffer.
 template <bool COUNT>
-__device__ __forceinline__ void extend_queue(const DevScene& S, const uint4* snodes, const PathIO& in,
+__device__ __forceinline__ void extend_queue(const DevScene& S, uint32_t* s_stack, const PathIO& in,
                                              float4* __restrict__ Hout, int n, WaveCounters* ctr, TraceCount& cnt) {
     const float4* __restrict__ O = in.o;
     const float4* __restrict__ D = in.d;
     persistent_trace<false, COUNT>(
-        S, snodes, n, &ctr->fetch_ext, &ctr->status, cnt,
+        S, s_stack, n, &ctr->fetch_ext, &ctr->status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
             const float4 a = O[i], b = D[i];
             o = make_float3(a.x, a.y, a.z);
@@ -134,11 +126,12 @@ __device__ __forceinline__ void extend_queue(const DevScene& S, const uint4* sno
 }
 
 // The shadow rays of a queue; the unoccluded ones' contributions go to the film.
-__device__ __forceinline__ void shadow_queue(const DevScene& S, const uint4* snodes, const ShadowIO& Q, int n,
+template <int THREADS>
+__device__ __forceinline__ void shadow_queue(const DevScene& S, uint32_t* s_stack, const ShadowIO& Q, int n,
                                              WaveCounters* ctr, unsigned long long* __restrict__ film, bool own_first) {
     TraceCount cnt{0u, 0u};
-    persistent_trace<true, false>(
-        S, snodes, n, &ctr->fetch_sh, &ctr->status, cnt,
+    persistent_trace<true, false, THREADS>(
+        S, s_stack, n, &ctr->fetch_sh, &ctr->status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
             const float4 a = Q.o[i], b = Q.d[i];
             o = make_float3(a.x, a.y, a.z);
@@ -158,12 +151,11 @@ __device__ __forceinline__ void shadow_queue(const DevScene& S, const uint4* sno
 template <bool COUNT>
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(DevScene S, PathIO in, float4* __restrict__ Hout,
                                                                            WaveCounters* ctr) {
-    extern __shared__ uint4 snodes[];
+    extern __shared__ uint32_t s_stack[];
     const int n = ctr->n_cur;
-    if (n == 0) return;  // drained wavefront: skip staging
-    stage_top_nodes(S, snodes);
+    if (n == 0) return;  // drained wavefront
     TraceCount cnt{0u, 0u};
-    extend_queue<COUNT>(S, snodes, in, Hout, n, ctr, cnt);
+    extend_queue<COUNT>(S, s_stack, in, Hout, n, ctr, cnt);
     if (COUNT) {
         const unsigned nodes = __reduce_add_sync(0xffffffffu, cnt.nodes);
         const unsigned tris = __reduce_add_sync(0xffffffffu, cnt.tris);
@@ -176,11 +168,10 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(Dev
 
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(DevScene S, ShadowIO Q, int cur, WaveCounters* ctr,
                                                           unsigned long long* __restrict__ film) {
-    extern __shared__ uint4 snodes[];
+    extern __shared__ uint32_t s_stack[];
     const int n = cur ? ctr->n_shadow1 : ctr->n_shadow;
     if (n == 0) return;
-    stage_top_nodes(S, snodes);
-    shadow_queue(S, snodes, Q, n, ctr, film, true);
+    shadow_queue<kTraceThreads>(S, s_stack, Q, n, ctr, film, true);
 }
 
 // One wavefront iteration's rays: the extension rays of path buffer `in`,
@@ -195,13 +186,12 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_wave
                                                                                  float4* __restrict__ Hout, ShadowIO Q,
                                                                                  int cur, WaveCounters* ctr,
                                                                                  unsigned long long* __restrict__ film) {
-    extern __shared__ uint4 snodes[];
+    extern __shared__ uint32_t s_stack[];
     const int n = ctr->n_cur, m = cur ? ctr->n_shadow : ctr->n_shadow1;
     if (n == 0 && m == 0) return;
-    stage_top_nodes(S, snodes);
     TraceCount cnt{0u, 0u};
-    if (n > 0) extend_queue<false>(S, snodes, in, Hout, n, ctr, cnt);
-    if (m > 0) shadow_queue(S, snodes, Q, m, ctr, film, n == 0);
+    if (n > 0) extend_queue<false>(S, s_stack, in, Hout, n, ctr, cnt);
+    if (m > 0) shadow_queue<kTraceThreads>(S, s_stack, Q, m, ctr, film, n == 0);
 }
 
 // info.w is the path's job: its table entry holds the render parameters,
@@ -449,7 +439,8 @@ __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
     const DevBatchJob* __restrict__ jobs) {
     const unsigned full = 0xffffffffu;
     const int m = ctr->n_shadow + ctr->n_shadow1;  // at most one of them is non-zero
-    if (m > 0) shadow_queue(S, nullptr, Q, m, ctr, film, true);
+    extern __shared__ uint32_t s_stack[];
+    if (m > 0) shadow_queue<kFinishThreads>(S, s_stack, Q, m, ctr, film, true);
     const int n = ctr->n_finish;
     if (n == 0) return;
     const PathIO in = ctr->finish_buf ? b1 : b0;
@@ -467,7 +458,7 @@ __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
     I = make_int4(0, 0, 0, 0);
     unsigned n_closest = 0, n_shadow = 0;
     int passes = 0;
-    TravStack K;
+    TravStack<false, kFinishThreads> K(s_stack);
     while (true) {
         const unsigned idle = __ballot_sync(full, lane < 16 && !alive);
         if (idle) {
@@ -544,20 +535,22 @@ ShadowIO shadow_io(const PathBuffers& B) { return ShadowIO{B.sh_o, B.sh_d, B.sh_
 void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, int num_sms, cudaStream_t st,
                    bool count) {
     const int g = num_sms * kTraceBlocksPerSM;
-    if (count) k_extend<true><<<g, kTraceThreads, kSmemNodeBytes, st>>>(S, path_io(B, cur), B.hit, ctr);
-    else k_extend<false><<<g, kTraceThreads, kSmemNodeBytes, st>>>(S, path_io(B, cur), B.hit, ctr);
+    if (count) k_extend<true><<<g, kTraceThreads, kTraceSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
+    else k_extend<false><<<g, kTraceThreads, kTraceSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
 }
 void launch_trace_wave(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                        int num_sms, cudaStream_t st) {
-    k_trace_wave<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, path_io(B, cur), B.hit,
+    k_trace_wave<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kTraceSmem, st>>>(S, path_io(B, cur), B.hit,
                                                                                      shadow_io(B), cur, ctr, film);
 }
 cudaError_t trace_kernels_setup() {
-    const int bytes = (int)kSmemNodeBytes;
+    const int bytes = (int)kTraceSmem;
     cudaError_t e = cudaFuncSetAttribute(k_trace_closest, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_any, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_extend<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_extend<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trace_smem_bytes(kFinishThreads));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e;
@@ -570,7 +563,7 @@ void launch_shade(const DevScene& S, const PathBuffers& B, int cur, WaveCounters
 }
 void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                    int num_sms, cudaStream_t st) {
-    k_shadow<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kSmemNodeBytes, st>>>(S, shadow_io(B), cur, ctr, film);
+    k_shadow<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kTraceSmem, st>>>(S, shadow_io(B), cur, ctr, film);
 }
 void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs, int n_jobs, int num_sms,
                      cudaStream_t st, bool shadows_traced) {
@@ -590,7 +583,7 @@ void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, Wav
 
 void launch_finish(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                    const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    k_finish<<<num_sms, kFinishThreads, 0, st>>>(S, path_io(B, 0), path_io(B, 1),
+    k_finish<<<num_sms, kFinishThreads, trace_smem_bytes(kFinishThreads), st>>>(S, path_io(B, 0), path_io(B, 1),
                                                                             shadow_io(B), ctr, film, jobs);
 }
 

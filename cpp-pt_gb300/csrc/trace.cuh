@@ -5,60 +5,12 @@
 
 namespace cpppt_gb300 {
 
-// Launch shape of the traversal kernels (threads per CTA, resident CTAs per
-// SM; the grid is the latter times the SM count) and the number of top wide
-// nodes (breadth-first, so the top levels) each CTA stages in shared memory.
-// Measured on the 1M-triangle soup at 1080p, 64 spp.  With the earlier node
-// phase (full child sort, 64-ray chunks), staging paid: 256x4 with 256
-// nodes 273.0 Mpaths/s, 512x2 with 1024 nodes 275.2, 1024x1 with 2048
-// nodes 277.3, with 3072 nodes 256.7 (L1 squeezed); 5 and 6 CTAs of 256
-// threads (48 and 40 registers, spilling) 264.9 and 234.5.  With the
-// current node phase the whole L1 serves better: 1024x1 with 2048 nodes
-// 303.1, 1536 306.2, 1024 305.9, 512 308.8, 256 310.1, 128 310.6, none
-// 310.4-310.8; without staging 512x2 310.0 and 256x4 309.4.  So no nodes
-// are staged (the mechanism stays for other scenes and shapes).
-#ifndef CPPPT_TRACE_THREADS
-#define CPPPT_TRACE_THREADS 1024
-#endif
-#ifndef CPPPT_TRACE_BLOCKS_PER_SM
-#define CPPPT_TRACE_BLOCKS_PER_SM 1
-#endif
-#ifndef CPPPT_SMEM_NODES
-#define CPPPT_SMEM_NODES 0
-#endif
-// Child slab distances two children at a time with the packed f32x2 adds
-// and FMAs of sm_100 and later (1) or one at a time (0); same results
-// (bit-identical images).  Measured on the 1M-triangle soup at 1080p, 64 spp:
-// 280.8 against 277.5 Mpaths/s (closest-hit kernel -0.9 %, shadow -2.4 %).
-#ifndef CPPPT_TRACE_F32X2
-#define CPPPT_TRACE_F32X2 1
-#endif
-// Any-hit queries push their children in slot order without sorting (1) or
-// nearest first like closest-hit queries (0).  Measured on the 1M-triangle
-// soup at 1080p, 64 spp: shadow kernel 148.2 -> 137.3 ms, 281.2 -> 287.9
-// Mpaths/s, bit-identical images (an occlusion answer does not depend on the
-// visiting order).
-#ifndef CPPPT_ANY_UNSORTED
-#define CPPPT_ANY_UNSORTED 1
-#endif
-// Closest-hit queries: the nearest child next and the others pushed in slot
-// order (1), or all pushed far to near after a full sort (0).  Measured as
-// above: closest-hit kernel 258.0 -> 250.3 ms, 286.9 -> 291.8 Mpaths/s,
-// bit-identical images (culling compares each popped entry with the best
-// hit, so the push order changes the work, never the answer).
-#ifndef CPPPT_CLOSEST_PARTIAL
-#define CPPPT_CLOSEST_PARTIAL 1
-#endif
-// Any-hit queries keep no entry distances (an occlusion query never culls
-// below its own max_t, so the distances are not needed) (1), or keep them (0).
-// Measured as above: shadow kernel 137.4 -> 136.4 ms.
-#ifndef CPPPT_ANY_LEAN
-#define CPPPT_ANY_LEAN 1
-#endif
-constexpr int kTraceThreads = CPPPT_TRACE_THREADS;
-constexpr int kTraceBlocksPerSM = CPPPT_TRACE_BLOCKS_PER_SM;
-constexpr int kSmemNodes = CPPPT_SMEM_NODES;
-constexpr size_t kSmemNodeBytes = (size_t)kSmemNodes * 64;  // dynamic shared memory of a traversal CTA
+// Launch shape of the traversal kernels: threads per CTA and resident CTAs
+// per SM (the grid is the latter times the SM count); 64 registers.  1024 x 1:
+// 1.8M closest-hit rays on the 1M-triangle soup 967 us, 512 x 2 981 us; more
+// threads (48 or 40 registers, spilling) were slower.
+constexpr int kTraceThreads = 1024;
+constexpr int kTraceBlocksPerSM = 1;
 constexpr int kStackSize = kTraversalStackSize;
 // Nodes whose entry distance exceeds best_t * (1 + 2^-8) are skipped.  The
 // margin covers the rounding of the reference's Cramer-rule t (triangle.h:41-57)
@@ -149,12 +101,6 @@ __device__ __forceinline__ bool ref_box_exact(float4 lo, float4 hi, float3 o, fl
     return tmax > 0.f;
 }
 
-// byte c of w as a float: one byte permute builds 2^23 + b, one exact
-// subtraction removes 2^23 (keeps the integer pipe free for the min/max)
-__device__ __forceinline__ float byte_to_float(uint32_t w, int c) {
-    return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7540u | (uint32_t)c)) - 8388608.0f;
-}
-
 // Packed pairs of floats (two children per instruction on sm_100 and later:
 // add.f32x2 / fma.f32x2 round each half exactly as add.f32 / fma.rn.f32).
 typedef unsigned long long f32x2;
@@ -176,7 +122,9 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-// slab distances of byte children c and c + 1 of w: q B + A, with q exact
+// slab distances of byte children c and c + 1 of w: q B + A.  A byte permute
+// builds 2^23 + q, an exact subtraction removes 2^23 (the integer pipe stays
+// free for the min / max).
 __device__ __forceinline__ void slab2(uint32_t w, int c, f32x2 B2, f32x2 A2, float& t0, float& t1) {
     const f32x2 q = pk2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7540u | (uint32_t)c)),
                         __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7540u | (uint32_t)(c + 1))));
@@ -203,10 +151,11 @@ struct TraceCount {
 };
 
 constexpr uint32_t kTravDone = 0xffffffffu;  // never a valid node or leaf reference
+constexpr uint32_t kTravPop = 0xfffffffeu;   // take the next entry off the stack (never a valid reference either)
 constexpr uint32_t kLeafRef = 0x80000000u;
 
-__device__ __forceinline__ bool is_inner(uint32_t r) { return !(r & kLeafRef); }  // kTravDone has the bit set
-__device__ __forceinline__ bool is_leaf(uint32_t r) { return (r & kLeafRef) && r != kTravDone; }
+__device__ __forceinline__ bool is_inner(uint32_t r) { return (int32_t)r >= 0; }  // kTravDone and kTravPop have the leaf bit set
+__device__ __forceinline__ bool is_leaf(uint32_t r) { return r - kLeafRef < kTravPop - kLeafRef; }
 
 struct Trav {
     float3 o, d;
@@ -220,10 +169,44 @@ struct Trav {
     HitRec best;
 };
 
-// Traversal stack of one lane: {node reference, entry distance bits}, one
-// 8-byte local-memory access per push and pop.
-struct TravStack {
-    uint2 e[kStackSize];
+// Traversal stack of one lane: node references, and for closest-hit queries
+// their entry distances.  The first entries lie in shared memory
+// ([entry][thread], no bank conflicts whatever the lanes' depths), the rare
+// rest in local memory.  Wholly in local memory the lanes' different depths
+// made every access a scatter over lines that compete with the tree for L1:
+// the any-hit kernel wrote 14 sectors per store and more to L2 than it read
+// (1.8M shadow rays on the 1M-triangle soup 888 us, 797 us once it stores only
+// the references it keeps, 774 us with them in shared memory); closest hits
+// 1070 -> 1042 us.  Entries swept 3-16: the 120 KB of ten leave L1 enough.
+constexpr int kShortStack = 10;  // shared entries of a closest-hit lane (8 bytes each)
+constexpr int kShortAny = 10;    // of an any-hit lane (4 bytes: an occlusion query culls nothing but by its own max_t)
+// The two kinds have regions of their own: in a kernel that traces both, a warp
+// may be at the second queue while another is still at the first.
+constexpr size_t trace_smem_bytes(int threads) { return (size_t)(8 * kShortStack + 4 * kShortAny) * threads; }
+constexpr size_t kTraceSmem = trace_smem_bytes(kTraceThreads);
+template <bool ANY, int THREADS>
+struct TravStack;
+template <int THREADS>
+struct TravStack<false, THREADS> {
+    uint2* s;  // this thread's column
+    uint2 e[kStackSize - kShortStack];
+    __device__ __forceinline__ explicit TravStack(uint32_t* smem) : s(reinterpret_cast<uint2*>(smem) + threadIdx.x) {}
+    __device__ __forceinline__ void put(int k, uint32_t r, uint32_t tb) {
+        if (k < kShortStack) s[k * THREADS] = make_uint2(r, tb);
+        else e[k - kShortStack] = make_uint2(r, tb);
+    }
+    __device__ __forceinline__ uint2 get(int k) const { return k < kShortStack ? s[k * THREADS] : e[k - kShortStack]; }
+};
+template <int THREADS>
+struct TravStack<true, THREADS> {
+    uint32_t* s;
+    uint32_t e[kStackSize - kShortAny];
+    __device__ __forceinline__ explicit TravStack(uint32_t* smem) : s(smem + 2 * kShortStack * THREADS + threadIdx.x) {}
+    __device__ __forceinline__ void put(int k, uint32_t r, uint32_t) {
+        if (k < kShortAny) s[k * THREADS] = r;
+        else e[k - kShortAny] = r;
+    }
+    __device__ __forceinline__ uint2 get(int k) const { return make_uint2(k < kShortAny ? s[k * THREADS] : e[k - kShortAny], 0u); }
 };
 
 // root: wide-node index where the traversal starts (0 for a scene of its own;
@@ -258,11 +241,12 @@ __device__ __forceinline__ void trav_init(Trav& T, float3 o, float3 d, float tma
 __device__ __forceinline__ float cull_dist(const Trav& T) { return T.best.t * kCullScale + 1e-6f; }
 
 // Next stacked node that is still in front of the best hit.
-__device__ __forceinline__ void trav_pop(Trav& T, const TravStack& K) {
+template <class Stack>
+__device__ __forceinline__ void trav_pop(Trav& T, const Stack& K) {
     const float cull = cull_dist(T);
     while (T.sp > 0) {
         T.sp--;
-        const uint2 e = K.e[T.sp];
+        const uint2 e = K.get(T.sp);
         if (__uint_as_float(e.y) <= cull) {
             T.cur = e.x;
             T.cur_t = __uint_as_float(e.y);
@@ -279,22 +263,27 @@ __device__ __forceinline__ void trav_abort(Trav& T, uint32_t* status, uint32_t b
     T.sp = 0;
 }
 
-// One inner node (T.cur): the children the ray enters in front of the best
-// hit, nearest first; far children are pushed.  (Any-hit rays use the same
-// order: skipping the sort measured 2% slower on the bench, since near
-// occluders end a shadow ray sooner.)
-template <bool ANY, bool COUNT>
-__device__ __forceinline__ void trav_node(Trav& T, TravStack& K, const DevScene& S, const uint4* __restrict__ snodes,
-                                          uint32_t* status, TraceCount& cnt) {
+// 32 bytes of a node in one load (sm_100 and later).
+__device__ __forceinline__ void ld256(const uint4* p, uint4& a, uint4& b) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+        : "l"(p));
+}
+
+// One inner node (T.cur): a child that the ray enters in front of the best
+// hit is next -- the nearest for a closest-hit query, the first in slot order
+// for an any-hit query -- and the other entered children are pushed unsorted
+// (culling compares each popped entry with the best hit, so the order changes
+// the work, never the answer; sorting them cost more than it saved).  kTravPop
+// when no child is entered.  Two 256-bit loads instead of four of 128 bits:
+// 1080p, 16 spp on the 1M-triangle soup 89.6 -> 88.3 ms.
+template <bool ANY, bool COUNT, class Stack>
+__device__ __forceinline__ void trav_node(Trav& T, Stack& K, const DevScene& S, uint32_t* status, TraceCount& cnt) {
     if (COUNT) cnt.nodes++;
-    const uint32_t cur = T.cur;
+    const uint4* np = S.nodes + 4 * (size_t)T.cur;
     uint4 w0, w1, w2, w3;
-    if (cur < (uint32_t)kSmemNodes) {
-        w0 = snodes[4 * cur]; w1 = snodes[4 * cur + 1]; w2 = snodes[4 * cur + 2]; w3 = snodes[4 * cur + 3];
-    } else {
-        const uint4* np = S.nodes + 4 * (size_t)cur;
-        w0 = __ldg(np); w1 = __ldg(np + 1); w2 = __ldg(np + 2); w3 = __ldg(np + 3);
-    }
+    ld256(np, w0, w1);
+    ld256(np + 2, w2, w3);
     const float cull = cull_dist(T);
     // slab distance of quantised coordinate q on axis k:
     //   (p + q s - o) / d = q (s/d) + (p - o)/d = q B + A
@@ -310,8 +299,7 @@ __device__ __forceinline__ void trav_node(Trav& T, TravStack& K, const DevScene&
     const uint32_t ny = nys ? w2.x : w1.y, fy = nys ? w1.y : w2.x;
     const uint32_t nz = nzs ? w2.y : w1.z, fz = nzs ? w1.z : w2.y;
     uint32_t key[4];
-#if CPPPT_TRACE_F32X2
-    // children in pairs: the same roundings as the scalar form below
+    // children in pairs (packed adds and FMAs, the roundings of scalar ones)
     const f32x2 BX = pk2(bx, bx), BY = pk2(by, by), BZ = pk2(bz, bz);
     const f32x2 AX = pk2(ax, ax), AY = pk2(ay, ay), AZ = pk2(az, az);
 #pragma unroll
@@ -328,92 +316,45 @@ __device__ __forceinline__ void trav_node(Trav& T, TravStack& K, const DevScene&
             const float tn = fmax3(tnx[h], tny[h], fmaxf(tnz[h], 0.0f));
             const float tf = fmin3(tfx[h], tfy[h], fminf(tfz[h], cull));
             const bool hit = tn <= tf * 1.0000005f;
-            if (ANY && CPPPT_ANY_LEAN) key[c + h] = hit ? 0u : 0xffffffffu;
+            if (ANY) key[c + h] = hit ? 0u : 0xffffffffu;
             else key[c + h] = hit ? ((__float_as_uint(tn) & ~3u) | (uint32_t)(c + h)) : 0xffffffffu;
         }
     }
-#else
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const float tnx = fmaf(byte_to_float(nx, c), bx, ax);
-        const float tny = fmaf(byte_to_float(ny, c), by, ay);
-        const float tnz = fmaf(byte_to_float(nz, c), bz, az);
-        const float tfx = fmaf(byte_to_float(fx, c), bx, ax);
-        const float tfy = fmaf(byte_to_float(fy, c), by, ay);
-        const float tfz = fmaf(byte_to_float(fz, c), bz, az);
-        const float tn = fmax3(tnx, tny, fmaxf(tnz, 0.0f));
-        const float tf = fmin3(tfx, tfy, fminf(tfz, cull));
-        const bool hit = tn <= tf * 1.0000005f;
-        key[c] = hit ? ((__float_as_uint(tn) & ~3u) | (uint32_t)c) : 0xffffffffu;
-    }
-#endif
     // Indexed by constants only: with a run-time index (the nearest child's) the
     // array lives in local memory, a 16-byte store and a load per node visit
     // (closest hits of 1.8M rays on the 1M-triangle soup 1057 us, with selects
     // 1026 us; 1M rays in the 192k-triangle room 325 -> 318 us).
     const uint32_t refs[4] = {w2.z, w2.w, w3.x, w3.y};
-#if CPPPT_ANY_UNSORTED
-    if (ANY) {  // any hit: children in slot order, no sorting
+    if (ANY) {
         if (T.sp + 3 > S.stack_limit) {
             trav_abort(T, status, kStatusStackOverflow);
             return;
         }
-        uint32_t nxt = kTravDone, nxt_t = 0u;
+        uint32_t nxt = kTravPop;
 #pragma unroll
         for (int c = 3; c >= 0; c--) {
             const bool v = key[c] != 0xffffffffu;
-            K.e[T.sp] = make_uint2(nxt, nxt_t);
-            T.sp += (v && nxt != kTravDone) ? 1 : 0;
+            if (v && nxt != kTravPop) K.put(T.sp++, nxt, 0u);
             nxt = v ? refs[c] : nxt;
-            nxt_t = v ? (key[c] & ~3u) : nxt_t;
-        }
-        if (nxt == kTravDone) {
-            trav_pop(T, K);
-            return;
         }
         T.cur = nxt;
-        T.cur_t = __uint_as_float(nxt_t);
+        T.cur_t = 0.f;
         return;
     }
-#endif
-#if CPPPT_CLOSEST_PARTIAL
-    if (!ANY) {  // nearest child next, the others pushed in slot order
-        const uint32_t m = min(min(key[0], key[1]), min(key[2], key[3]));
-        if (m == 0xffffffffu) {
-            trav_pop(T, K);
-            return;
-        }
-        if (T.sp + 3 > S.stack_limit) {
-            trav_abort(T, status, kStatusStackOverflow);
-            return;
-        }
-#pragma unroll
-        for (int c = 3; c >= 0; c--)
-            if (key[c] != 0xffffffffu && key[c] != m) K.e[T.sp++] = make_uint2(refs[c], key[c] & ~3u);
-        T.cur = (m & 2u) ? ((m & 1u) ? refs[3] : refs[2]) : ((m & 1u) ? refs[1] : refs[0]);
-        T.cur_t = __uint_as_float(m & ~3u);
-        return;
-    }
-#endif
-#define CSWAP(a, b) { uint32_t lo_ = min(key[a], key[b]), hi_ = max(key[a], key[b]); key[a] = lo_; key[b] = hi_; }
-    CSWAP(0, 1) CSWAP(2, 3) CSWAP(0, 2) CSWAP(1, 3) CSWAP(1, 2)
-#undef CSWAP
-    if (key[0] == 0xffffffffu) {
-        trav_pop(T, K);
+    const uint32_t m = min(min(key[0], key[1]), min(key[2], key[3]));
+    if (m == 0xffffffffu) {
+        T.cur = kTravPop;
         return;
     }
     if (T.sp + 3 > S.stack_limit) {
         trav_abort(T, status, kStatusStackOverflow);
         return;
     }
-    // far children first; an invalid key is written but not counted
 #pragma unroll
-    for (int k = 3; k >= 1; k--) {
-        K.e[T.sp] = make_uint2(refs[key[k] & 3u], key[k] & ~3u);
-        T.sp += (key[k] != 0xffffffffu) ? 1 : 0;
-    }
-    T.cur = refs[key[0] & 3u];
-    T.cur_t = __uint_as_float(key[0] & ~3u);
+    for (int c = 3; c >= 0; c--)
+        if (key[c] != 0xffffffffu && key[c] != m) K.put(T.sp++, refs[c], key[c] & ~3u);
+    T.cur = (m & 2u) ? ((m & 1u) ? refs[3] : refs[2]) : ((m & 1u) ? refs[1] : refs[0]);
+    T.cur_t = __uint_as_float(m & ~3u);
 }
 
 // The postponed leaf T.leaf.  Returns true when an any-hit query is answered.
@@ -450,71 +391,89 @@ __device__ __forceinline__ bool trav_leaf(Trav& T, const DevScene& S, TraceCount
     return false;
 }
 
-// Persistent ray loop.  Each warp takes chunks of up to kChunk consecutive
-// rays (ray_chunk) into a warp-private range, the first one by its number and
-// the next ones from a global counter; a lane whose ray finishes
-// takes the next ray of the range at once (no waiting for the other lanes).
-// own_first = false: the first chunk comes from the counter too (a kernel's
-// second queue, which warps reach at different times).
-// load(i, o, d, tmax, root) fetches ray i; root arrives set to the scene's
-// own root and may be replaced (rays of a merged multi-scene arena).
+// One node phase and one leaf phase of a warp, n_act of whose lanes have rays
+// (the others' cur and leaf are kTravDone).  Leaves are postponed as in Aila
+// and Laine 2009, "Understanding the efficiency of ray traversal on GPUs": a
+// lane that reaches a leaf parks it and keeps descending inner nodes; the node
+// phase goes on while more than two thirds of the lanes with rays can (have a
+// node, or a stacked entry to take), then the lanes with a parked leaf test its
+// triangles together.  The result does not depend on the visiting order: the
+// closest hit is the minimum over the tested triangles of (t, -rank), and a
+// node is culled only when its entry distance lies behind the best hit.
 //
-// Every iteration has a node phase and a leaf phase (leaves are postponed
-// as in Aila and Laine 2009, "Understanding the efficiency of ray traversal
-// on GPUs"): a lane that reaches a leaf parks it and keeps descending inner
-// nodes; the node phase repeats until a third of the warp's active lanes
-// cannot continue without their leaf, or no lane has an inner node left,
-// and then the lanes with a parked leaf test its triangles together.
-// Inner-node and triangle code run with most lanes converged instead of
-// alternating per lane.  Measured on the 1M-triangle soup with an earlier
-// node phase: a quarter 238.7 Mpaths/s against 232.5 at one half, 232.0 at
-// one eighth and 215 at any waiting lane; repeating the node phase instead
-// of one node step per iteration 247 against 237 (the current figures are
-// below).  The result does not depend on the visiting order: the closest
-// hit is the minimum over the tested triangles of (t, -rank), and a node is
-// culled only when its entry distance lies behind the best hit found so far.
-// Rays a warp takes from the global counter at a time, and the leaf-phase
-// trigger (a leaf phase once 1/CPPPT_LEAF_WAIT_DIV of the active lanes wait
-// on a parked leaf).  Measured on the 1M-triangle soup at 1080p, 64 spp, with
-// the node phase above: chunk 64 / quarter 292.5 Mpaths/s, chunk 128 277.0,
-// chunk 32 300.9, chunk 16 302.0; with a third: chunk 64 294.6, chunk 32
-// 302.8, chunk 16 303.1; with a sixth (chunk 64) 287.7.  Smaller chunks
-// balance the lanes' and warps' uneven ray lengths better, above all at
-// the end of a launch.
-#ifndef CPPPT_RAY_CHUNK
-#define CPPPT_RAY_CHUNK 16
-#endif
-#ifndef CPPPT_LEAF_WAIT_DIV
-#define CPPPT_LEAF_WAIT_DIV 3
-#endif
-// The same trigger for any-hit queries, measured apart: a half 308.7, a
-// third 310.8, a fifth 310.4, an eighth 308.1 Mpaths/s.
-#ifndef CPPPT_LEAF_WAIT_DIV_ANY
-#define CPPPT_LEAF_WAIT_DIV_ANY CPPPT_LEAF_WAIT_DIV
-#endif
-constexpr int kChunk = CPPPT_RAY_CHUNK;
+// There is one place for each kind of work -- taking an entry off the stack,
+// visiting a node, parking a leaf -- and the warp reconverges before the node:
+// with the pops inlined where they arise (no child entered, leaf parked, entry
+// culled), lanes went through the same code one group after another.  Finished
+// lanes count as unable to go on, so they get a new ray soon.  Measured
+// (1M-triangle soup, with the stack above) 1.8M closest-hit rays 1042 -> 967
+// us, shadow rays 774 -> 739 us, 1M rays in the 192k-triangle room 324 -> 297
+// us, 1080p at 16 spp 94.8 -> 88.2 ms.  Phase end at a half of the lanes 91.5
+// ms, three fifths 89.5, three quarters 89.6; counting only lanes that wait on
+// a leaf (a third of them) 90.5.
+template <bool ANY, bool COUNT, class Stack>
+__device__ __forceinline__ void trav_round(const DevScene& S, Trav& T, Stack& K, int n_act, uint32_t* status,
+                                           TraceCount& cnt) {
+    unsigned go;
+    do {
+        if (T.cur == kTravPop) trav_pop(T, K);
+        __syncwarp();
+        if (is_inner(T.cur)) {
+            if (++T.steps > S.step_limit) trav_abort(T, status, kStatusIterLimit);
+            else trav_node<ANY, COUNT>(T, K, S, status, cnt);
+        }
+        if (is_leaf(T.cur) && T.leaf == kTravDone) {
+            T.leaf = T.cur;
+            T.cur = kTravPop;
+        }
+        if (T.cur == kTravPop && T.sp == 0) T.cur = kTravDone;
+        go = __ballot_sync(0xffffffffu, is_inner(T.cur) || T.cur == kTravPop);
+    } while (3 * __popc(go) > 2 * n_act);
+    if (T.leaf != kTravDone) {
+        ++T.steps;
+        if (!trav_leaf<ANY, COUNT>(T, S, cnt)) {
+            if (!ANY && T.cur != kTravDone && T.cur_t > cull_dist(T)) T.cur = kTravPop;
+            if (is_leaf(T.cur)) {
+                T.leaf = T.cur;
+                T.cur = kTravPop;
+            }
+        }
+    }
+}
+
 // Rays per fetch when `left` rays remain for `nwarps` warps (`share` chunks
 // each): kChunk while there are many, down to one for the last ones, so that
 // a small batch (or the end of a large one) is spread over all warps.  A warp
-// whose 16 rays take different ways through the tree runs the union of their
+// whose rays take different ways through the tree runs the union of their
 // steps, and the launch ends with its slowest warp.  Measured (1M-triangle
 // soup) against 16 rays a fetch from one CTA per 1024 rays: 1000 shadow rays
-// 136 -> 54 us, 30,001 closest-hit rays 194 -> 125 us, 200,001 226 -> 222 us,
-// 1.8M rays unchanged; the first fetch at half the even share 144 us
-// (30,001 rays), at a quarter 171 us, since half the rays then wait for a
-// second fetch.
+// 136 -> 54 us, 30,001 closest-hit rays 194 -> 125 us; the first fetch at half
+// the even share 144 us (30,001 rays), at a quarter 171 us, since half the rays
+// then wait for a second fetch.  kChunk 8, 16, 24, 32, 48, 64: 1080p at 16 spp
+// 92.0, 87.7, 87.2, 86.8, 86.6, 86.5 ms, 1M rays in the 192k-triangle room 336,
+// 291, 289, 283, 294, 319 us.
+constexpr int kChunk = 32;
 __device__ __forceinline__ int ray_chunk(int left, int nwarps, int share) {
     return min(kChunk, max(1, left / (share * nwarps)));
 }
 
-template <bool ANY, bool COUNT, class Load, class Store>
-__device__ __forceinline__ void persistent_trace(const DevScene& S, const uint4* __restrict__ snodes, int n,
-                                                 int* counter, uint32_t* status, TraceCount& cnt, Load load,
+// Persistent ray loop.  Each warp takes chunks of up to kChunk consecutive
+// rays (ray_chunk) into a warp-private range, the first one by its number and
+// the next ones from a global counter; between rounds every lane whose ray
+// has finished takes the next one, across the end of the range if need be (a
+// lane left idle until the next fetch cost 4 % at 1080p).
+// own_first = false: the first chunk comes from the counter too (a kernel's
+// second queue, which warps reach at different times).
+// load(i, o, d, tmax, root) fetches ray i; root arrives set to the scene's
+// own root and may be replaced (rays of a merged multi-scene arena).
+template <bool ANY, bool COUNT, int THREADS = kTraceThreads, class Load, class Store>
+__device__ __forceinline__ void persistent_trace(const DevScene& S, uint32_t* __restrict__ smem, int n, int* counter, uint32_t* status, TraceCount& cnt, Load load,
                                                  Store store, bool own_first = true) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     Trav T;
-    TravStack K;
+    TravStack<ANY, THREADS> K(smem);
+    T.cur = T.leaf = kTravDone;
     int ray = -1;
     // warp-uniform ray range; the first one is the warp's own (warps numbered
     // across the CTAs, so a small batch spreads over every SM), later ones
@@ -527,53 +486,37 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, const uint4*
     while (true) {
         const unsigned idle = __ballot_sync(0xffffffffu, ray < 0);
         if (idle) {
-            if (pool_next >= pool_end && !exhausted) {
+            const int want = __popc(idle), avail = pool_end - pool_next;
+            int next = pool_end, end = pool_end;  // the range after the present one
+            if (avail < want && !exhausted) {
                 const int chunk = ray_chunk(n - pool_end, nwarps, 2);
                 int base = 0;
                 if (lane == 0) base = atomicAdd(counter, chunk);
-                base = __shfl_sync(0xffffffffu, base, 0) + nwarps * c0;
-                pool_next = base;
-                pool_end = min(base + chunk, n);
-                if (base + chunk >= n) exhausted = true;
+                next = min(__shfl_sync(0xffffffffu, base, 0) + nwarps * c0, n);
+                end = min(next + chunk, n);
+                exhausted = end >= n;
             }
-            const int avail = max(0, pool_end - pool_next);
-            if (avail > 0) {
-                const int r = __popc(idle & lt_mask);
-                if (ray < 0 && r < avail) {
-                    ray = pool_next + r;
-                    float3 o, d;
-                    float tmax;
-                    uint32_t root = S.n_tris > 0 ? 0u : kTravDone;
-                    load(ray, o, d, tmax, root);
-                    trav_init(T, o, d, tmax, root);
-                }
-                pool_next += min(avail, __popc(idle));
+            const int r = __popc(idle & lt_mask);
+            const int i = r < avail ? pool_next + r : next + (r - avail);
+            if (ray < 0 && (r < avail || i < end)) {
+                ray = i;
+                float3 o, d;
+                float tmax;
+                uint32_t root = S.n_tris > 0 ? 0u : kTravDone;
+                load(ray, o, d, tmax, root);
+                trav_init(T, o, d, tmax, root);
+            }
+            if (avail >= want) {
+                pool_next += want;
+            } else {
+                pool_next = min(next + (want - avail), end);
+                pool_end = end;
             }
         }
-        const bool active = ray >= 0;
-        const unsigned act = __ballot_sync(0xffffffffu, active);
+        const unsigned act = __ballot_sync(0xffffffffu, ray >= 0);
         if (act == 0) break;
-        unsigned wait, inner;
-        do {
-            if (active && is_inner(T.cur)) {
-                if (++T.steps > S.step_limit) trav_abort(T, status, kStatusIterLimit);
-                else if (T.cur_t > cull_dist(T)) trav_pop(T, K);
-                else trav_node<ANY, COUNT>(T, K, S, snodes, status, cnt);
-            }
-            if (active && T.leaf == kTravDone && is_leaf(T.cur)) {
-                T.leaf = T.cur;
-                trav_pop(T, K);
-            }
-            const bool waiting = active && T.leaf != kTravDone && !is_inner(T.cur);
-            wait = __ballot_sync(0xffffffffu, waiting);
-            inner = __ballot_sync(0xffffffffu, active && is_inner(T.cur));
-        } while (inner != 0 && (ANY ? CPPPT_LEAF_WAIT_DIV_ANY : CPPPT_LEAF_WAIT_DIV) * __popc(wait) < __popc(act));
-        // leaf phase (the node phase ended because enough lanes wait or none can descend)
-        if (active && T.leaf != kTravDone) {
-            ++T.steps;
-            if (trav_leaf<ANY, COUNT>(T, S, cnt)) T.leaf = kTravDone;
-        }
-        if (active && T.cur == kTravDone && T.leaf == kTravDone) {
+        trav_round<ANY, COUNT>(S, T, K, __popc(act), status, cnt);
+        if (ray >= 0 && T.cur == kTravDone && T.leaf == kTravDone) {
             store(ray, T.best);
             ray = -1;
         }
@@ -583,34 +526,18 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, const uint4*
 // Traces one ray per lane (active lanes' T, set up by trav_init) to the end:
 // the closest hit, or with `any` until the first hit (the same test against
 // the ray's own max_t, which best.t holds until then).  All 32 lanes call it.
-__device__ __forceinline__ void warp_trace(const DevScene& S, Trav& T, TravStack& K, bool active, bool any,
+template <class Stack>
+__device__ __forceinline__ void warp_trace(const DevScene& S, Trav& T, Stack& K, bool active, bool any,
                                            uint32_t* status) {
     TraceCount cnt{0u, 0u};
+    if (!active) T.cur = T.leaf = kTravDone;
     while (true) {
-        const bool live = active && (T.cur != kTravDone || T.leaf != kTravDone);
-        const unsigned act = __ballot_sync(0xffffffffu, live);
+        const unsigned act = __ballot_sync(0xffffffffu, T.cur != kTravDone || T.leaf != kTravDone);
         if (act == 0) break;
-        unsigned wait, inner;
-        do {
-            if (live && is_inner(T.cur)) {
-                if (++T.steps > S.step_limit) trav_abort(T, status, kStatusIterLimit);
-                else if (T.cur_t > cull_dist(T)) trav_pop(T, K);
-                else trav_node<false, false>(T, K, S, nullptr, status, cnt);
-            }
-            if (live && T.leaf == kTravDone && is_leaf(T.cur)) {
-                T.leaf = T.cur;
-                trav_pop(T, K);
-            }
-            wait = __ballot_sync(0xffffffffu, live && T.leaf != kTravDone && !is_inner(T.cur));
-            inner = __ballot_sync(0xffffffffu, live && is_inner(T.cur));
-        } while (inner != 0 && CPPPT_LEAF_WAIT_DIV * __popc(wait) < __popc(act));
-        if (live && T.leaf != kTravDone) {
-            ++T.steps;
-            trav_leaf<false, false>(T, S, cnt);
-            if (any && T.best.prim >= 0) {
-                T.cur = kTravDone;
-                T.sp = 0;
-            }
+        trav_round<false, false>(S, T, K, __popc(act), status, cnt);
+        if (any && T.best.prim >= 0) {
+            T.cur = T.leaf = kTravDone;
+            T.sp = 0;
         }
     }
 }
