@@ -1017,7 +1017,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_shadow_nn(DevScene S, PathBuf
 }
 
 cudaError_t nn_shadow_smem_limit() {
-    return cudaFuncSetAttribute(k_shadow_nn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTraceSmem);
+    return cudaFuncSetAttribute(k_shadow_nn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trace_smem(false, true, kTraceThreads));
 }
 
 // Camera paths (stratified like pathtracerMIS.h:148-153) with a vertex slot.
@@ -1107,7 +1107,7 @@ void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const Ren
 }
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    k_shadow_nn<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kTraceSmem, st>>>(S, B, ctr, film, PD, jobs);
+    k_shadow_nn<<<num_sms * kTraceBlocksPerSM, kTraceThreads, trace_smem(false, true, kTraceThreads), st>>>(S, B, ctr, film, PD, jobs);
 }
 void launch_nn_generate(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
                         const DevBatchJob* jobs, int n_jobs, cudaStream_t st) {

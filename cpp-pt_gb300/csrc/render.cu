@@ -21,14 +21,10 @@
 
 namespace cpppt_gb300 {
 
-// Each warp takes 32 consecutive work items at a time from a global counter
-// (persistent threads); returns the first index, or >= n when done.
-__device__ __forceinline__ int warp_fetch(int* counter, int n) {
-    int base = 0;
-    if ((threadIdx.x & 31) == 0) base = atomicAdd(counter, 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    return base;
-}
+constexpr size_t kClosestSmem = trace_smem(true, false, kTraceThreads);
+constexpr size_t kAnySmem = trace_smem(false, true, kTraceThreads);
+constexpr size_t kBothSmem = trace_smem(true, true, kTraceThreads);
+constexpr size_t kBothAnyWord = kClosestSmem / 4;  // the any-hit region of a kernel with both
 
 __device__ __forceinline__ float4 shfl4(float4 v, int src) {
     return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
@@ -86,14 +82,14 @@ void launch_trace_closest(const DevScene& S, const float* rays, int n, float4* h
                           int num_sms, cudaStream_t st) {
     if (n <= 0) return;
     const int blocks = min(num_sms * kTraceBlocksPerSM, n);
-    k_trace_closest<<<blocks, kTraceThreads, kTraceSmem, st>>>(S, rays, n, hits, counter, status);
+    k_trace_closest<<<blocks, kTraceThreads, kClosestSmem, st>>>(S, rays, n, hits, counter, status);
 }
 
 void launch_trace_any(const DevScene& S, const float* rays, int n, uint8_t* occ, int* counter, uint32_t* status,
                       int num_sms, cudaStream_t st) {
     if (n <= 0) return;
     const int blocks = min(num_sms * kTraceBlocksPerSM, n);
-    k_trace_any<<<blocks, kTraceThreads, kTraceSmem, st>>>(S, rays, n, occ, counter, status);
+    k_trace_any<<<blocks, kTraceThreads, kAnySmem, st>>>(S, rays, n, occ, counter, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -191,7 +187,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_wave
     if (n == 0 && m == 0) return;
     TraceCount cnt{0u, 0u};
     if (n > 0) extend_queue<false>(S, s_stack, in, Hout, n, ctr, cnt);
-    if (m > 0) shadow_queue<kTraceThreads>(S, s_stack, Q, m, ctr, film, n == 0);
+    if (m > 0) shadow_queue<kTraceThreads>(S, s_stack + kBothAnyWord, Q, m, ctr, film, n == 0);
 }
 
 // info.w is the path's job: its table entry holds the render parameters,
@@ -434,13 +430,15 @@ __global__ void k_advance(WaveCounters* ctr, int capacity, int cur, int traced, 
 // last 64k paths are a small part).  512 threads per SM with 128 registers;
 // 1024 with 64 (spilling) 2262 us, two CTAs of 256 2190 us.
 constexpr int kFinishThreads = 512;
+constexpr size_t kFinishSmem = trace_smem(true, true, kFinishThreads);
+constexpr size_t kFinishAnyWord = trace_smem(true, false, kFinishThreads) / 4;
 __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
     DevScene S, PathIO b0, PathIO b1, ShadowIO Q, WaveCounters* ctr, unsigned long long* __restrict__ film,
     const DevBatchJob* __restrict__ jobs) {
     const unsigned full = 0xffffffffu;
     const int m = ctr->n_shadow + ctr->n_shadow1;  // at most one of them is non-zero
     extern __shared__ uint32_t s_stack[];
-    if (m > 0) shadow_queue<kFinishThreads>(S, s_stack, Q, m, ctr, film, true);
+    if (m > 0) shadow_queue<kFinishThreads>(S, s_stack + kFinishAnyWord, Q, m, ctr, film, true);
     const int n = ctr->n_finish;
     if (n == 0) return;
     const PathIO in = ctr->finish_buf ? b1 : b0;
@@ -458,7 +456,7 @@ __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
     I = make_int4(0, 0, 0, 0);
     unsigned n_closest = 0, n_shadow = 0;
     int passes = 0;
-    TravStack<false, kFinishThreads> K(s_stack);
+    TravStack<false, kFinishThreads> K(s_stack, S.stack_limit);
     while (true) {
         const unsigned idle = __ballot_sync(full, lane < 16 && !alive);
         if (idle) {
@@ -488,7 +486,7 @@ __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
         passes++;
         n_closest += __popc(live);
         Trav T;
-        trav_init(T, make_float3(O.x, O.y, O.z), make_float3(D.x, D.y, D.z),
+        trav_init(T, K.base, make_float3(O.x, O.y, O.z), make_float3(D.x, D.y, D.z),
                   pending ? O.w : __int_as_float(0x7f800000),
                   S.n_tris > 0 ? __float_as_uint(pending ? C.w : D.w) : kTravDone);
         warp_trace(S, T, K, alive || pending, pending, &ctr->status);
@@ -535,24 +533,25 @@ ShadowIO shadow_io(const PathBuffers& B) { return ShadowIO{B.sh_o, B.sh_d, B.sh_
 void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, int num_sms, cudaStream_t st,
                    bool count) {
     const int g = num_sms * kTraceBlocksPerSM;
-    if (count) k_extend<true><<<g, kTraceThreads, kTraceSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
-    else k_extend<false><<<g, kTraceThreads, kTraceSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
+    if (count) k_extend<true><<<g, kTraceThreads, kClosestSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
+    else k_extend<false><<<g, kTraceThreads, kClosestSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
 }
 void launch_trace_wave(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                        int num_sms, cudaStream_t st) {
-    k_trace_wave<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kTraceSmem, st>>>(S, path_io(B, cur), B.hit,
+    k_trace_wave<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kBothSmem, st>>>(S, path_io(B, cur), B.hit,
                                                                                      shadow_io(B), cur, ctr, film);
 }
 cudaError_t trace_kernels_setup() {
-    const int bytes = (int)kTraceSmem;
-    cudaError_t e = cudaFuncSetAttribute(k_trace_closest, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_any, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_extend<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_extend<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trace_smem_bytes(kFinishThreads));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trace_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const auto limit = [](const void* f, size_t bytes) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    cudaError_t e = limit((const void*)k_trace_closest, kClosestSmem);
+    if (e == cudaSuccess) e = limit((const void*)k_trace_any, kAnySmem);
+    if (e == cudaSuccess) e = limit((const void*)k_extend<true>, kClosestSmem);
+    if (e == cudaSuccess) e = limit((const void*)k_extend<false>, kClosestSmem);
+    if (e == cudaSuccess) e = limit((const void*)k_shadow, kAnySmem);
+    if (e == cudaSuccess) e = limit((const void*)k_trace_wave, kBothSmem);
+    if (e == cudaSuccess) e = limit((const void*)k_finish, kFinishSmem);
     return e;
 }
 
@@ -563,7 +562,7 @@ void launch_shade(const DevScene& S, const PathBuffers& B, int cur, WaveCounters
 }
 void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                    int num_sms, cudaStream_t st) {
-    k_shadow<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kTraceSmem, st>>>(S, shadow_io(B), cur, ctr, film);
+    k_shadow<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kAnySmem, st>>>(S, shadow_io(B), cur, ctr, film);
 }
 void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs, int n_jobs, int num_sms,
                      cudaStream_t st, bool shadows_traced) {
@@ -583,7 +582,7 @@ void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, Wav
 
 void launch_finish(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                    const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    k_finish<<<num_sms, kFinishThreads, trace_smem_bytes(kFinishThreads), st>>>(S, path_io(B, 0), path_io(B, 1),
+    k_finish<<<num_sms, kFinishThreads, kFinishSmem, st>>>(S, path_io(B, 0), path_io(B, 1),
                                                                             shadow_io(B), ctr, film, jobs);
 }
 

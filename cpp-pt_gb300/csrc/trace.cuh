@@ -27,6 +27,28 @@ struct HitRec {
     int32_t rank;
 };
 
+// Packed pairs of floats (two children per instruction on sm_100 and later:
+// add.f32x2 / fma.f32x2 round each half exactly as add.f32 / fma.rn.f32).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ void upk2(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 __device__ __forceinline__ float m3r(float a, float b, float c) { return __fmul_rn(__fmul_rn(a, b), c); }
 
 // Triangle::intersect up to acceptance (triangle.h:18-80): Cramer's rule with
@@ -101,27 +123,6 @@ __device__ __forceinline__ bool ref_box_exact(float4 lo, float4 hi, float3 o, fl
     return tmax > 0.f;
 }
 
-// Packed pairs of floats (two children per instruction on sm_100 and later:
-// add.f32x2 / fma.f32x2 round each half exactly as add.f32 / fma.rn.f32).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float a, float b) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-    return d;
-}
-__device__ __forceinline__ void upk2(f32x2 v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 // slab distances of byte children c and c + 1 of w: q B + A.  A byte permute
 // builds 2^23 + q, an exact subtraction removes 2^23 (the integer pipe stays
 // free for the min / max).
@@ -151,21 +152,24 @@ struct TraceCount {
 };
 
 constexpr uint32_t kTravDone = 0xffffffffu;  // never a valid node or leaf reference
-constexpr uint32_t kTravPop = 0xfffffffeu;   // take the next entry off the stack (never a valid reference either)
+constexpr uint32_t kTravPop = 0x7fffffffu;   // take the next entry off the stack (never a valid node either)
 constexpr uint32_t kLeafRef = 0x80000000u;
 
-__device__ __forceinline__ bool is_inner(uint32_t r) { return (int32_t)r >= 0; }  // kTravDone and kTravPop have the leaf bit set
-__device__ __forceinline__ bool is_leaf(uint32_t r) { return r - kLeafRef < kTravPop - kLeafRef; }
+// kTravDone is the only reference with the leaf bit that is no leaf, and
+// kTravPop the only one without it that is no node
+__device__ __forceinline__ bool is_inner(uint32_t r) { return r < kTravPop; }
+__device__ __forceinline__ bool is_leaf(uint32_t r) { return (int32_t)r < -1; }
+__device__ __forceinline__ bool can_go(uint32_t r) { return (int32_t)r >= 0; }  // a node, or an entry to take
 
 struct Trav {
     float3 o, d;
     float idx, idy, idz, oix, oiy, oiz;
-    float tmax0;
     uint32_t neg;   // bit k: direction component k is negative
     uint32_t cur;   // next node or leaf to visit (kTravDone: nothing left on the stack)
     float cur_t;    // entry distance of cur
     uint32_t leaf;  // leaf postponed to the warp's next leaf phase (kTravDone: none)
-    int sp, steps;
+    uint32_t sp;    // stack top (TravStack)
+    int steps;
     HitRec best;
 };
 
@@ -174,48 +178,77 @@ struct Trav {
 // ([entry][thread], no bank conflicts whatever the lanes' depths), the rare
 // rest in local memory.  Wholly in local memory the lanes' different depths
 // made every access a scatter over lines that compete with the tree for L1:
-// the any-hit kernel wrote 14 sectors per store and more to L2 than it read
-// (1.8M shadow rays on the 1M-triangle soup 888 us, 797 us once it stores only
-// the references it keeps, 774 us with them in shared memory); closest hits
-// 1070 -> 1042 us.  Entries swept 3-16: the 120 KB of ten leave L1 enough.
-constexpr int kShortStack = 10;  // shared entries of a closest-hit lane (8 bytes each)
-constexpr int kShortAny = 10;    // of an any-hit lane (4 bytes: an occlusion query culls nothing but by its own max_t)
-// The two kinds have regions of their own: in a kernel that traces both, a warp
-// may be at the second queue while another is still at the first.
-constexpr size_t trace_smem_bytes(int threads) { return (size_t)(8 * kShortStack + 4 * kShortAny) * threads; }
-constexpr size_t kTraceSmem = trace_smem_bytes(kTraceThreads);
+// the any-hit kernel wrote 14 sectors per store and more to L2 than it read.
+// The top is kept as the shared-memory address of the next entry, so a push is
+// a store and an add; addresses past the region stand for the entries in local
+// memory, and pushes go the short way while three more entries fit the region.
+// Measured (1M-triangle soup, 1.8M closest-hit / shadow rays): all in local
+// memory 1070 / 797 us, seven entries by index 1042 / 775 us; with addresses
+// and 6, 8, 10, 12, 13 or 16 closest-hit entries 988, 948, 898, 862, 854, 852
+// us, and 6, 8, 10, 12, 14 or 18 any-hit entries 693, 666, 637, 609, 604, 603
+// us; 13 and 14 are 160 KB of an SM.
+constexpr int kShortStack = 13;  // shared entries of a closest-hit lane (8 bytes each)
+constexpr int kShortAny = 14;    // of an any-hit lane (4 bytes: an occlusion query culls nothing but by its own max_t)
+// Bytes of the region of one kind of query.  A kernel that traces both has two
+// regions: a warp may be at the second queue while another is at the first.
+constexpr size_t stack_bytes(bool any, int threads) { return (size_t)(any ? 4 * kShortAny : 8 * kShortStack) * threads; }
+constexpr size_t trace_smem(bool closest, bool any, int threads) {
+    return (closest ? stack_bytes(false, threads) : 0) + (any ? stack_bytes(true, threads) : 0);
+}
 template <bool ANY, int THREADS>
-struct TravStack;
-template <int THREADS>
-struct TravStack<false, THREADS> {
-    uint2* s;  // this thread's column
-    uint2 e[kStackSize - kShortStack];
-    __device__ __forceinline__ explicit TravStack(uint32_t* smem) : s(reinterpret_cast<uint2*>(smem) + threadIdx.x) {}
-    __device__ __forceinline__ void put(int k, uint32_t r, uint32_t tb) {
-        if (k < kShortStack) s[k * THREADS] = make_uint2(r, tb);
-        else e[k - kShortStack] = make_uint2(r, tb);
+struct TravStack {
+    static constexpr int kShared = ANY ? kShortAny : kShortStack;
+    static constexpr uint32_t kEntry = ANY ? 4u : 8u, kStep = kEntry * THREADS;
+    uint32_t base;       // the thread's column
+    uint32_t end;        // end of the region, the same for all threads: entries at or above it are local
+    uint32_t fast;       // below it three more entries fit the region and the stack limit
+    uint32_t ref[kStackSize - kShared];
+    uint32_t t[ANY ? 1 : kStackSize - kShared];
+    __device__ __forceinline__ TravStack(uint32_t* smem, int stack_limit) {
+        const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(smem);
+        base = s0 + kEntry * threadIdx.x;
+        end = s0 + kShared * kStep;
+        const int f = min(kShared, stack_limit) - 2;
+        fast = s0 + (f > 0 ? (uint32_t)f * kStep : 0u);
     }
-    __device__ __forceinline__ uint2 get(int k) const { return k < kShortStack ? s[k * THREADS] : e[k - kShortStack]; }
-};
-template <int THREADS>
-struct TravStack<true, THREADS> {
-    uint32_t* s;
-    uint32_t e[kStackSize - kShortAny];
-    __device__ __forceinline__ explicit TravStack(uint32_t* smem) : s(smem + 2 * kShortStack * THREADS + threadIdx.x) {}
-    __device__ __forceinline__ void put(int k, uint32_t r, uint32_t) {
-        if (k < kShortAny) s[k * THREADS] = r;
-        else e[k - kShortAny] = r;
+    // entries on the stack
+    __device__ __forceinline__ int depth(uint32_t sp) const { return (int)((sp - base) / kStep); }
+    __device__ __forceinline__ void put_shared(uint32_t& sp, uint32_t r, uint32_t tb) const {
+        if (ANY) asm volatile("st.shared.b32 [%0], %1;" ::"r"(sp), "r"(r));
+        else asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(sp), "r"(r), "r"(tb));
+        sp += kStep;
     }
-    __device__ __forceinline__ uint2 get(int k) const { return make_uint2(k < kShortAny ? s[k * THREADS] : e[k - kShortAny], 0u); }
+    __device__ __forceinline__ void put(uint32_t& sp, uint32_t r, uint32_t tb) {
+        if (sp < end) {
+            put_shared(sp, r, tb);
+            return;
+        }
+        const uint32_t k = (sp - end) / kStep;
+        ref[k] = r;
+        if (!ANY) t[k] = tb;
+        sp += kStep;
+    }
+    __device__ __forceinline__ uint2 take(uint32_t& sp) const {
+        sp -= kStep;
+        uint2 e = make_uint2(0u, 0u);
+        if (sp < end) {
+            if (ANY) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(e.x) : "r"(sp));
+            else asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(e.x), "=r"(e.y) : "r"(sp));
+        } else {
+            const uint32_t k = (sp - end) / kStep;
+            e.x = ref[k];
+            if (!ANY) e.y = t[k];
+        }
+        return e;
+    }
 };
 
 // root: wide-node index where the traversal starts (0 for a scene of its own;
 // the scene's first node inside a merged multi-scene arena; kTravDone for a
 // scene without triangles).
-__device__ __forceinline__ void trav_init(Trav& T, float3 o, float3 d, float tmax0, uint32_t root) {
+__device__ __forceinline__ void trav_init(Trav& T, uint32_t stack_base, float3 o, float3 d, float tmax0, uint32_t root) {
     T.o = o;
     T.d = d;
-    T.tmax0 = tmax0;
     T.best.t = tmax0;
     T.best.prim = -1;
     T.best.rank = -1;
@@ -234,7 +267,7 @@ __device__ __forceinline__ void trav_init(Trav& T, float3 o, float3 d, float tma
     T.cur = root;
     T.cur_t = 0.f;
     T.leaf = kTravDone;
-    T.sp = 0;
+    T.sp = stack_base;
     T.steps = 0;
 }
 
@@ -244,9 +277,8 @@ __device__ __forceinline__ float cull_dist(const Trav& T) { return T.best.t * kC
 template <class Stack>
 __device__ __forceinline__ void trav_pop(Trav& T, const Stack& K) {
     const float cull = cull_dist(T);
-    while (T.sp > 0) {
-        T.sp--;
-        const uint2 e = K.get(T.sp);
+    while (T.sp != K.base) {
+        const uint2 e = K.take(T.sp);
         if (__uint_as_float(e.y) <= cull) {
             T.cur = e.x;
             T.cur_t = __uint_as_float(e.y);
@@ -260,7 +292,6 @@ __device__ __forceinline__ void trav_abort(Trav& T, uint32_t* status, uint32_t b
     atomicOr(status, bit);
     T.cur = kTravDone;
     T.leaf = kTravDone;
-    T.sp = 0;
 }
 
 // 32 bytes of a node in one load (sm_100 and later).
@@ -326,16 +357,21 @@ __device__ __forceinline__ void trav_node(Trav& T, Stack& K, const DevScene& S, 
     // 1026 us; 1M rays in the 192k-triangle room 325 -> 318 us).
     const uint32_t refs[4] = {w2.z, w2.w, w3.x, w3.y};
     if (ANY) {
-        if (T.sp + 3 > S.stack_limit) {
-            trav_abort(T, status, kStatusStackOverflow);
-            return;
-        }
-        uint32_t nxt = kTravPop;
-#pragma unroll
-        for (int c = 3; c >= 0; c--) {
-            const bool v = key[c] != 0xffffffffu;
-            if (v && nxt != kTravPop) K.put(T.sp++, nxt, 0u);
-            nxt = v ? refs[c] : nxt;
+        const bool v0 = key[0] == 0u, v1 = key[1] == 0u, v2 = key[2] == 0u, v3 = key[3] == 0u;
+        const bool p1 = v1 && v0, p2 = v2 && (v0 || v1), p3 = v3 && (v0 || v1 || v2);
+        const uint32_t nxt = v0 ? refs[0] : (v1 ? refs[1] : (v2 ? refs[2] : (v3 ? refs[3] : kTravPop)));
+        if (T.sp < K.fast) {
+            if (p3) K.put_shared(T.sp, refs[3], 0u);
+            if (p2) K.put_shared(T.sp, refs[2], 0u);
+            if (p1) K.put_shared(T.sp, refs[1], 0u);
+        } else {
+            if (K.depth(T.sp) + 3 > S.stack_limit) {
+                trav_abort(T, status, kStatusStackOverflow);
+                return;
+            }
+            if (p3) K.put(T.sp, refs[3], 0u);
+            if (p2) K.put(T.sp, refs[2], 0u);
+            if (p1) K.put(T.sp, refs[1], 0u);
         }
         T.cur = nxt;
         T.cur_t = 0.f;
@@ -346,13 +382,19 @@ __device__ __forceinline__ void trav_node(Trav& T, Stack& K, const DevScene& S, 
         T.cur = kTravPop;
         return;
     }
-    if (T.sp + 3 > S.stack_limit) {
-        trav_abort(T, status, kStatusStackOverflow);
-        return;
-    }
+    if (T.sp < K.fast) {
 #pragma unroll
-    for (int c = 3; c >= 0; c--)
-        if (key[c] != 0xffffffffu && key[c] != m) K.put(T.sp++, refs[c], key[c] & ~3u);
+        for (int c = 3; c >= 0; c--)
+            if (key[c] != 0xffffffffu && key[c] != m) K.put_shared(T.sp, refs[c], key[c]);
+    } else {
+        if (K.depth(T.sp) + 3 > S.stack_limit) {
+            trav_abort(T, status, kStatusStackOverflow);
+            return;
+        }
+#pragma unroll
+        for (int c = 3; c >= 0; c--)
+            if (key[c] != 0xffffffffu && key[c] != m) K.put(T.sp, refs[c], key[c]);
+    }
     T.cur = (m & 2u) ? ((m & 1u) ? refs[3] : refs[2]) : ((m & 1u) ? refs[1] : refs[0]);
     T.cur_t = __uint_as_float(m & ~3u);
 }
@@ -368,8 +410,8 @@ __device__ __forceinline__ bool trav_leaf(Trav& T, const DevScene& S, TraceCount
         const float4* tp = S.tris + 3 * (size_t)(start + k);
         const float4 A = __ldg(tp), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
         float t, beta, gamma;
-        // ANY: the reference tests against the ray's own max_t
-        if (!tri_exact(A, E1, E2, T.o, T.d, ANY ? T.tmax0 : T.best.t, t, beta, gamma)) continue;
+        // ANY: best.t is the ray's own max_t until the first hit
+        if (!tri_exact(A, E1, E2, T.o, T.d, T.best.t, t, beta, gamma)) continue;
         const int32_t rank = __float_as_int(A.w);
         if (!ANY && !(t < T.best.t || rank > T.best.rank)) continue;  // equal t: the later-visited wins
         const int32_t parent = __float_as_int(E1.w);
@@ -384,7 +426,6 @@ __device__ __forceinline__ bool trav_leaf(Trav& T, const DevScene& S, TraceCount
         T.best.gamma = gamma;
         if (ANY) {
             T.cur = kTravDone;
-            T.sp = 0;
             return true;
         }
     }
@@ -419,16 +460,17 @@ __device__ __forceinline__ void trav_round(const DevScene& S, Trav& T, Stack& K,
         if (T.cur == kTravPop) trav_pop(T, K);
         __syncwarp();
         if (is_inner(T.cur)) {
-            if (++T.steps > S.step_limit) trav_abort(T, status, kStatusIterLimit);
-            else trav_node<ANY, COUNT>(T, K, S, status, cnt);
+            ++T.steps;
+            trav_node<ANY, COUNT>(T, K, S, status, cnt);
         }
         if (is_leaf(T.cur) && T.leaf == kTravDone) {
             T.leaf = T.cur;
             T.cur = kTravPop;
         }
-        if (T.cur == kTravPop && T.sp == 0) T.cur = kTravDone;
-        go = __ballot_sync(0xffffffffu, is_inner(T.cur) || T.cur == kTravPop);
+        if (T.cur == kTravPop && T.sp == K.base) T.cur = kTravDone;
+        go = __ballot_sync(0xffffffffu, can_go(T.cur));
     } while (3 * __popc(go) > 2 * n_act);
+    if (T.steps > S.step_limit) trav_abort(T, status, kStatusIterLimit);
     if (T.leaf != kTravDone) {
         ++T.steps;
         if (!trav_leaf<ANY, COUNT>(T, S, cnt)) {
@@ -457,6 +499,7 @@ __device__ __forceinline__ int ray_chunk(int left, int nwarps, int share) {
     return min(kChunk, max(1, left / (share * nwarps)));
 }
 
+// smem: the stacks' shared region (stack_bytes(ANY, THREADS)).
 // Persistent ray loop.  Each warp takes chunks of up to kChunk consecutive
 // rays (ray_chunk) into a warp-private range, the first one by its number and
 // the next ones from a global counter; between rounds every lane whose ray
@@ -472,8 +515,9 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, uint32_t* __
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     Trav T;
-    TravStack<ANY, THREADS> K(smem);
+    TravStack<ANY, THREADS> K(smem, S.stack_limit);
     T.cur = T.leaf = kTravDone;
+    T.steps = 0;
     int ray = -1;
     // warp-uniform ray range; the first one is the warp's own (warps numbered
     // across the CTAs, so a small batch spreads over every SM), later ones
@@ -504,7 +548,7 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, uint32_t* __
                 float tmax;
                 uint32_t root = S.n_tris > 0 ? 0u : kTravDone;
                 load(ray, o, d, tmax, root);
-                trav_init(T, o, d, tmax, root);
+                trav_init(T, K.base, o, d, tmax, root);
             }
             if (avail >= want) {
                 pool_next += want;
@@ -537,7 +581,6 @@ __device__ __forceinline__ void warp_trace(const DevScene& S, Trav& T, Stack& K,
         trav_round<false, false>(S, T, K, __popc(act), status, cnt);
         if (any && T.best.prim >= 0) {
             T.cur = T.leaf = kTravDone;
-            T.sp = 0;
         }
     }
 }

@@ -100,3 +100,29 @@ def test_batch_sizes_around_the_ray_distribution(gpu_lib, n):
     sh = rays.copy()
     sh[:, 6] = np.where(oi >= 0, ot * np.where(np.arange(n) % 2, 0.5, 1.5), 1.0).astype(np.float32)
     assert np.array_equal(gs.trace_any(sh), Oracle("port").scene(sc).trace_any(sh))
+
+
+def test_stacks_beyond_their_shared_part(gpu_lib):
+    """Overlapping spheres need more stack entries than the kernels keep in
+    shared memory (13 of a closest-hit lane, 14 of an any-hit lane): with the
+    stack limited to those the queries report an overflow, with the default
+    limit they give the oracle's answers."""
+    from cpppt.lib import GpuScene, PtError
+    from oracle.oracle import Oracle
+    sc = scenes.soup(seed=3, n_spheres=300, freq=4, width=64, height=64, extent=1.0)
+    rays = scenes.hit_ray_batch(sc, 1 << 14, seed=13)
+    osc = Oracle("port").scene(sc)
+    oi, ot = osc.trace_closest(rays)
+    sh = rays.copy()
+    sh[:, 6] = np.where(oi >= 0, ot * np.where(np.arange(len(rays)) % 2, 0.99, 1.01), 1.0).astype(np.float32)
+    gs = GpuScene(sc)
+    for limit, query in ((13, lambda: gs.trace_closest(rays)), (14, lambda: gs.trace_any(sh))):
+        assert gpu_lib.pt_debug_traversal_limits(gs.h, 0, limit) == 0
+        with pytest.raises(PtError) as e:
+            query()
+        assert e.value.status == 4 and "stack overflow" in str(e.value)
+    assert gpu_lib.pt_debug_traversal_limits(gs.h, 0, 0) == 0
+    gi, gt, _, _ = gs.trace_closest(rays)
+    assert np.array_equal(gi, oi)
+    assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
+    assert np.array_equal(gs.trace_any(sh), osc.trace_any(sh))
