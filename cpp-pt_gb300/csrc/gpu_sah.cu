@@ -17,9 +17,14 @@
 //     (k_split_big); the chunks then scatter their primitives into the other
 //     order buffer, left side first, each chunk offset by the left counts of
 //     the chunks before it (k_scatter_big).
-//   subtrees    (nodes of at most kSmallSeg primitives): one CTA builds the
-//     whole subtree depth first from a stack in shared memory
-//     (k_subtree), with the same binning, decision and stable partition.
+//   subtrees    (nodes of at most kSmallSeg primitives): one CTA splits the
+//     node depth first from a stack in shared memory, with the same binning,
+//     decision and stable partition, down to nodes of kTinySeg (k_subtree);
+//     one warp builds each of those with its primitives in registers
+//     (k_tiny).  A CTA stepping through every node of a 4096-primitive subtree
+//     (barriers, 96 bins to clear and scan, for nodes of a few triangles) took
+//     23 ms of the 192k-triangle room's 36 ms scene creation and 29 ms of a
+//     10k-triangle scene's 32 ms; now 0.5 ms of either.
 //   collapse    breadth-first, one launch set per 4-wide level: each entry
 //     gathers its up-to-4 children (the child of largest SAH area opened
 //     first, as the host does), an exclusive scan gives the next level's
@@ -50,9 +55,11 @@ namespace {
 
 constexpr int kSahBins = 32;         // SahBuilder::kBins
 constexpr int kDepthLimit = 56;      // SAH splits are tried above this depth
-constexpr int kSmallSeg = 4096;      // nodes up to this size: one CTA builds the subtree
+constexpr int kSmallSeg = 1024;      // nodes up to this size: one CTA splits them down to kTinySeg
+constexpr int kTinySeg = 32;         // nodes up to this size: one warp builds the subtree
 constexpr int kChunk = 4096;         // primitives per CTA in the top levels
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;        // of the top levels' CTAs
+constexpr int kSubThreads = 128;   // of a subtree's CTA
 constexpr int kStack = 128;          // subtree stack entries (tree depth is at most 56 + 27)
 constexpr int kBinFields = 13;       // count, box lo xyz, box hi xyz, centroid lo xyz, centroid hi xyz
 constexpr int kBinWords = 3 * kSahBins * kBinFields;
@@ -73,6 +80,25 @@ __device__ __forceinline__ float unkey(uint32_t k) {
 __device__ __forceinline__ float sah_area(const float lo[3], const float hi[3]) {
     const float dx = __fsub_rn(hi[0], lo[0]), dy = __fsub_rn(hi[1], lo[1]), dz = __fsub_rn(hi[2], lo[2]);
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dy), __fmul_rn(dy, dz)), __fmul_rn(dz, dx));
+}
+
+// SahBuilder's cost of a split, and its bits for an unsigned minimum (costs are
+// sums of products of box extents and counts; one that is not a number or
+// negative counts as none, as in the host's comparison with +inf).
+__device__ __forceinline__ float sah_cost(const float llo[3], const float lhi[3], uint32_t lc, const float rlo[3],
+                                          const float rhi[3], uint32_t rc) {
+    return __fadd_rn(__fmul_rn(sah_area(llo, lhi), __uint2float_rn(lc)),
+                     __fmul_rn(sah_area(rlo, rhi), __uint2float_rn(rc)));
+}
+__device__ __forceinline__ uint32_t cost_bits(float c) { return c >= 0.f ? __float_as_uint(c) : 0x7f800000u; }
+
+// Whether a node of `count` primitives stays a leaf (best: the cheapest
+// split's cost, axis < 0 for none).
+__device__ __forceinline__ bool sah_leaf(const float lo[3], const float hi[3], int count, int max_leaf, int axis,
+                                         float best) {
+    const float area = sah_area(lo, hi);
+    return count <= max_leaf &&
+           (axis < 0 || __fadd_rn(best, __fmul_rn(area, 1.0f)) >= __fmul_rn(area, __int2float_rn(count)));
 }
 
 struct Prims {
@@ -182,30 +208,32 @@ __device__ __forceinline__ void warp_scan(uint32_t& cnt, uint32_t k[12], bool su
 }
 
 // The host's split decision from the bins (SahBuilder::build): warp w < 3
-// evaluates axis w; the first strict minimum over (axis, bin) wins.  Writes
-// *out (leaf, axis or fallback) from thread 0; the caller synchronises.
-// The node's box and centroid bounds come from s.key.  All threads of the
-// CTA call it (it synchronises once).
+// evaluates axis w (lane = bin); the first strict minimum over (axis, bin)
+// wins, and the lane that holds the winning split writes the two sides' counts
+// and bounds from its scans.  *out is complete after the caller's next
+// __syncthreads.  The node's box and centroid bounds come from s.key.  All
+// threads of the CTA call it (it synchronises once).
 __device__ void decide(const uint32_t* bins, const Seg& s, int max_leaf, Split* out, float* s_cost, int* s_bin) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float lo[3], hi[3], clo[3], chi[3];
     seg_bounds(s.key, lo, hi, clo, chi);
     const bool try_sah = s.depth < kDepthLimit;
+    uint32_t pc = 0, pk[12], rk[12];
     if (warp < 3) {
         const int a = warp;
         float best = __int_as_float(0x7f800000);  // +inf
         int bbin = -1;
         if (try_sah && chi[a] > clo[a]) {
             const uint32_t* B = bins + (a * kSahBins + lane) * kBinFields;
-            uint32_t pc = B[0], sc = B[0], pk[12], sk[12];
+            uint32_t sc = B[0], sk[12];
+            pc = B[0];
             for (int f = 0; f < 12; f++) pk[f] = sk[f] = B[1 + f];
             warp_scan(pc, pk, false);
             warp_scan(sc, sk, true);
             // right side of the split after bin `lane`: the suffix from lane + 1
             const uint32_t rc = __shfl_down_sync(0xffffffffu, sc, 1);
-            uint32_t rk[12];
             for (int f = 0; f < 12; f++) rk[f] = __shfl_down_sync(0xffffffffu, sk[f], 1);
-            float cost = __int_as_float(0x7fffffff);  // NaN: no candidate
+            uint32_t cost = 0x7f800000u;  // +inf: no candidate (a NaN cost is none either)
             if (lane < kSahBins - 1 && pc != 0 && rc != 0) {
                 float llo[3], lhi[3], rlo[3], rhi[3];
                 for (int k = 0; k < 3; k++) {
@@ -214,16 +242,13 @@ __device__ void decide(const uint32_t* bins, const Seg& s, int max_leaf, Split* 
                     rlo[k] = unkey(~rk[k]);
                     rhi[k] = unkey(rk[3 + k]);
                 }
-                cost = __fadd_rn(__fmul_rn(sah_area(llo, lhi), __uint2float_rn(pc)),
-                                 __fmul_rn(sah_area(rlo, rhi), __uint2float_rn(rc)));
+                cost = cost_bits(sah_cost(llo, lhi, pc, rlo, rhi, rc));
             }
             // first strict minimum below +inf: the sequential scan's choice
-            for (int b = 0; b < kSahBins - 1; b++) {
-                const float cb = __shfl_sync(0xffffffffu, cost, b);
-                if (cb < best) {
-                    best = cb;
-                    bbin = b;
-                }
+            const uint32_t m = __reduce_min_sync(0xffffffffu, cost);
+            if (m < 0x7f800000u) {
+                best = __uint_as_float(m);
+                bbin = __ffs(__ballot_sync(0xffffffffu, cost == m)) - 1;
             }
         }
         if (lane == 0) {
@@ -232,33 +257,27 @@ __device__ void decide(const uint32_t* bins, const Seg& s, int max_leaf, Split* 
         }
     }
     __syncthreads();
+    float best = __int_as_float(0x7f800000);
+    int axis = -1;
+    for (int a = 0; a < 3; a++)
+        if (s_bin[a] >= 0 && s_cost[a] < best) {
+            best = s_cost[a];
+            axis = a;
+        }
+    const bool leaf = sah_leaf(lo, hi, s.count, max_leaf, axis, best);
     if (threadIdx.x == 0) {
-        float best = __int_as_float(0x7f800000);
-        int axis = -1;
-        for (int a = 0; a < 3; a++)
-            if (s_bin[a] >= 0 && s_cost[a] < best) {
-                best = s_cost[a];
-                axis = a;
-            }
-        const float area = sah_area(lo, hi);
-        const float leaf_cost = __fmul_rn(area, __int2float_rn(s.count));
-        const float trav = __fmul_rn(area, 1.0f);
-        out->leaf = s.count <= max_leaf && (axis < 0 || __fadd_rn(best, trav) >= leaf_cost);
-        out->axis = out->leaf ? -1 : axis;
+        out->leaf = leaf;
+        out->axis = leaf ? -1 : axis;
         out->bin = axis >= 0 ? s_bin[axis] : -1;
-        out->nleft = 0;
-        if (!out->leaf && axis >= 0) {
-            out->lo = clo[axis];
-            out->scale = __fdiv_rn((float)kSahBins, __fsub_rn(chi[axis], clo[axis]));
-            for (int f = 0; f < 12; f++) out->lkey[f] = out->rkey[f] = 0;
-            uint32_t nl = 0;
-            for (int b = 0; b < kSahBins; b++) {
-                const uint32_t* B = bins + (axis * kSahBins + b) * kBinFields;
-                uint32_t* K = b <= out->bin ? out->lkey : out->rkey;
-                if (b <= out->bin) nl += B[0];
-                for (int f = 0; f < 12; f++) K[f] = max(K[f], B[1 + f]);
-            }
-            out->nleft = (int)nl;
+        if (leaf || axis < 0) out->nleft = 0;
+    }
+    if (!leaf && axis >= 0 && warp == axis && lane == s_bin[axis]) {
+        out->lo = clo[axis];
+        out->scale = __fdiv_rn((float)kSahBins, __fsub_rn(chi[axis], clo[axis]));
+        out->nleft = (int)pc;
+        for (int f = 0; f < 12; f++) {
+            out->lkey[f] = pk[f];
+            out->rkey[f] = rk[f];
         }
     }
 }
@@ -410,22 +429,38 @@ __global__ void __launch_bounds__(kThreads) k_bin_chunks(Prims P, const Chunk* _
     }
 }
 
+// A node of at most kTinySeg primitives, for the warp that builds its subtree.
+struct Tiny {
+    int32_t start, node;
+    int16_t count, buf;
+    int32_t depth;
+};
+
+// counts: [0] next large nodes, [1] CTA subtree roots, [2] node ids, [3] status,
+// [4] warp subtree roots
 struct LevelOut {
-    Seg* big;        // next level's large nodes
-    Seg* small;      // subtree roots
-    int32_t* counts;  // [0] next large nodes, [1] subtree roots, [2] node ids, [3] status
+    Seg* big;    // next level's large nodes
+    Seg* small;  // CTA subtree roots
+    Tiny* tiny;  // warp subtree roots (room for one per primitive)
+    int32_t* counts;
     int32_t max_big, max_small, max_nodes;
 };
+
+__device__ __forceinline__ void emit_tiny(Tiny* tiny, int32_t* counts, const Seg& c) {
+    tiny[atomicAdd(counts + 4, 1)] = Tiny{c.start, c.node, (int16_t)c.count, (int16_t)c.buf, c.depth};
+}
 
 __device__ __forceinline__ void emit_seg(const LevelOut& L, const Seg& c) {
     if (c.count > kSmallSeg) {
         const int j = atomicAdd(L.counts + 0, 1);
         if (j < L.max_big) L.big[j] = c;
         else atomicOr(L.counts + 3, kErrRange);
-    } else {
+    } else if (c.count > kTinySeg) {
         const int j = atomicAdd(L.counts + 1, 1);
         if (j < L.max_small) L.small[j] = c;
         else atomicOr(L.counts + 3, kErrRange);
+    } else {
+        emit_tiny(L.tiny, L.counts, c);
     }
 }
 
@@ -504,18 +539,19 @@ __global__ void __launch_bounds__(kThreads) k_scatter_big(Prims P, const Chunk* 
 }
 
 // ---------------------------------------------------------------------------
-// Subtrees: one CTA per root, depth first.
+// Subtrees: one CTA per root splits depth first, down to nodes of kTinySeg.
 // ---------------------------------------------------------------------------
 struct SubCtx {
     Prims P;
     int32_t* ord[2];
     int32_t* out_order;
     Node2* nodes;
-    int32_t* counts;  // [2] node ids, [3] status
+    Tiny* tiny;
+    int32_t* counts;
     int32_t max_leaf, max_nodes;
 };
 
-__global__ void __launch_bounds__(kThreads) k_subtree(const Seg* __restrict__ roots, SubCtx C) {
+__global__ void __launch_bounds__(kSubThreads) k_subtree(const Seg* __restrict__ roots, SubCtx C) {
     __shared__ uint32_t bins[kBinWords];
     __shared__ Seg stack[kStack];
     __shared__ Seg s;
@@ -523,7 +559,7 @@ __global__ void __launch_bounds__(kThreads) k_subtree(const Seg* __restrict__ ro
     __shared__ int sp_top;
     __shared__ float s_cost[3];
     __shared__ int s_bin[3];
-    __shared__ int s_warp[kThreads / 32];
+    __shared__ int s_warp[kSubThreads / 32];
     if (threadIdx.x == 0) {
         stack[0] = roots[blockIdx.x];
         sp_top = 1;
@@ -614,12 +650,154 @@ __global__ void __launch_bounds__(kThreads) k_subtree(const Seg* __restrict__ ro
                 }
                 r.start = s.start + l.count;
                 r.count = s.count - l.count;
-                stack[sp_top] = r;
-                stack[sp_top + 1] = l;
-                sp_top += 2;
+                for (const Seg& c : {r, l}) {
+                    if (c.count > kTinySeg) stack[sp_top++] = c;
+                    else emit_tiny(C.tiny, C.counts, c);
+                }
             }
         }
         __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small subtrees: one warp per root of at most kTinySeg primitives, one
+// primitive per lane in registers.  A node is the set of lanes that hold its
+// primitives (every node's primitives stay in insertion order, so a
+// primitive's place within its node is the number of the node's lanes below
+// it) and the place of its first primitive; nothing moves until the leaves are
+// written.  The split costs come from a loop over the node's primitives with
+// one lane per split bin, which for nodes this small is far less work than
+// filling and scanning 96 bins: most nodes of a tree are here.
+// ---------------------------------------------------------------------------
+constexpr int kTinyWarps = 4;  // warps per CTA
+
+__global__ void __launch_bounds__(32 * kTinyWarps) k_tiny(const Tiny* __restrict__ roots, int n_roots, SubCtx C) {
+    struct Item {
+        uint32_t lanes;
+        int32_t node, begin, depth;
+    };
+    __shared__ Item s_stack[kTinyWarps][kTinySeg];  // disjoint lane sets
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r = blockIdx.x * kTinyWarps + warp;
+    if (r >= n_roots) return;
+    const Tiny root = roots[r];
+    float lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f}, cen[3] = {0.f, 0.f, 0.f};
+    int id = 0;
+    if (lane < root.count) {
+        id = C.ord[root.buf][root.start + lane];
+        const float4 l = C.P.lo[id], h = C.P.hi[id];
+        lo[0] = l.x; lo[1] = l.y; lo[2] = l.z;
+        hi[0] = h.x; hi[1] = h.y; hi[2] = h.z;
+        cen[0] = l.w; cen[1] = h.w; cen[2] = C.P.cz[id];
+    }
+    Item* stack = s_stack[warp];
+    Item it{root.count == 32 ? full : (1u << root.count) - 1u, root.node, root.start, root.depth};
+    int top = 0;
+    for (;;) {
+        const bool mine = (it.lanes >> lane) & 1u;
+        const int count = __popc(it.lanes);
+        float nlo[3], nhi[3], clo[3], chi[3];
+        for (int a = 0; a < 3; a++) {
+            nlo[a] = unkey(~__reduce_max_sync(full, mine ? ~fkey(lo[a]) : 0u));
+            nhi[a] = unkey(__reduce_max_sync(full, mine ? fkey(hi[a]) : 0u));
+            clo[a] = unkey(~__reduce_max_sync(full, mine ? ~fkey(cen[a]) : 0u));
+            chi[a] = unkey(__reduce_max_sync(full, mine ? fkey(cen[a]) : 0u));
+        }
+        // the cheapest split: axis, bin and cost as in decide()
+        int axis = -1, bin = -1;
+        float best = __int_as_float(0x7f800000);
+        uint32_t b3 = 0;  // this lane's primitive's bins, one byte per axis
+        if (count > 1 && it.depth < kDepthLimit) {
+            for (int a = 0; a < 3; a++)
+                if (chi[a] > clo[a])
+                    b3 |= (uint32_t)bin_of(cen[a], clo[a], __fdiv_rn((float)kSahBins, __fsub_rn(chi[a], clo[a]))) << (8 * a);
+            float l0[3][3], l1[3][3], r0[3][3], r1[3][3];  // per axis: left box, right box of the split after bin `lane`
+            int lc[3] = {0, 0, 0};
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    l0[a][k] = r0[a][k] = __int_as_float(0x7f800000);
+                    l1[a][k] = r1[a][k] = __int_as_float(0xff800000);
+                }
+            for (uint32_t left = it.lanes; left; left &= left - 1u) {
+                const int i = __ffs(left) - 1;
+                const uint32_t bi = __shfl_sync(full, b3, i);
+                float plo[3], phi[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    plo[k] = __shfl_sync(full, lo[k], i);
+                    phi[k] = __shfl_sync(full, hi[k], i);
+                }
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    if ((int)((bi >> (8 * a)) & 0xffu) <= lane) {
+                        lc[a]++;
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            l0[a][k] = fminf(l0[a][k], plo[k]);
+                            l1[a][k] = fmaxf(l1[a][k], phi[k]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            r0[a][k] = fminf(r0[a][k], plo[k]);
+                            r1[a][k] = fmaxf(r1[a][k], phi[k]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                uint32_t cost = 0x7f800000u;
+                if (chi[a] > clo[a] && lane < kSahBins - 1 && lc[a] > 0 && lc[a] < count)
+                    cost = cost_bits(sah_cost(l0[a], l1[a], (uint32_t)lc[a], r0[a], r1[a], (uint32_t)(count - lc[a])));
+                const uint32_t m = __reduce_min_sync(full, cost);
+                if (m < 0x7f800000u && __uint_as_float(m) < best) {
+                    best = __uint_as_float(m);
+                    axis = a;
+                    bin = __ffs(__ballot_sync(full, cost == m)) - 1;
+                }
+            }
+        }
+        const bool leaf = count <= 1 || sah_leaf(nlo, nhi, count, C.max_leaf, axis, best);
+        int kids = -1;
+        if (!leaf) {
+            if (lane == 0) kids = atomicAdd(C.counts + 2, 2);
+            kids = __shfl_sync(full, kids, 0);
+        }
+        if (lane == 0) {
+            if (it.node < C.max_nodes) {
+                Node2 nd;
+                for (int a = 0; a < 3; a++) {
+                    nd.lo[a] = nlo[a];
+                    nd.hi[a] = nhi[a];
+                }
+                nd.left = kids;
+                nd.right = leaf ? -1 : kids + 1;
+                nd.start = it.begin;
+                nd.count = leaf ? count : 0;
+                C.nodes[it.node] = nd;
+            }
+            if (!leaf && kids + 2 > C.max_nodes) atomicOr(C.counts + 3, kErrRange);
+        }
+        if (leaf) {
+            if (mine) C.out_order[it.begin + __popc(it.lanes & ((1u << lane) - 1u))] = id;
+            if (top == 0) break;
+            it = stack[--top];
+            continue;
+        }
+        // the left side: the lower bins, or the first half where no split exists
+        const bool left = mine && (axis >= 0 ? (int)((b3 >> (8 * axis)) & 0xffu) <= bin
+                                             : __popc(it.lanes & ((1u << lane) - 1u)) < count / 2);
+        const uint32_t ml = __ballot_sync(full, left), mr = it.lanes & ~ml;
+        __syncwarp();
+        if (lane == 0) stack[top] = Item{mr, kids + 1, it.begin + __popc(ml), it.depth + 1};
+        __syncwarp();
+        top++;
+        it = Item{ml, kids, it.begin, it.depth + 1};
     }
 }
 
@@ -811,7 +989,7 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
     } hguard{h};
 
     const int max_big = n / kSmallSeg + 2;
-    const int max_small = 4 * (n / kSmallSeg) + 16;
+    const int max_small = n / kTinySeg + 16;  // they hold more than kTinySeg primitives each, and share none
     const int max_chunks = n / kChunk + max_big + 2;
     float* d_tv = dmalloc<float>(owned, 9 * (size_t)n);
     float4* plo = dmalloc<float4>(owned, n);
@@ -828,7 +1006,8 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
     uint32_t* gbins = dmalloc<uint32_t>(owned, (size_t)max_big * kBinWords);
     uint32_t* key6 = dmalloc<uint32_t>(owned, 6);
     float* d_delta = dmalloc<float>(owned, 1);
-    int32_t* counts = dmalloc<int32_t>(owned, 4);  // next big, small, node ids, status
+    Tiny* tiny = dmalloc<Tiny>(owned, n);
+    int32_t* counts = dmalloc<int32_t>(owned, 5);  // LevelOut::counts
 
     ck(cudaMemcpyAsync(d_tv, tri_v, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice, st), "upload");
     ck(cudaMemsetAsync(key6, 0, 6 * sizeof(uint32_t), st), "memset");
@@ -841,9 +1020,13 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
     root.buf = 0;
     root.has_bounds = 1;
     Seg* d_root = n > kSmallSeg ? big[0] : small;
+    if (n <= kTinySeg) {
+        const Tiny t{0, 0, (int16_t)n, 0, 0};
+        ck(cudaMemcpyAsync(tiny, &t, sizeof(Tiny), cudaMemcpyHostToDevice, st), "root");
+    }
     ck(cudaMemcpyAsync(d_root, &root, sizeof(Seg), cudaMemcpyHostToDevice, st), "root");
     // next-level large nodes, subtree roots, node ids (the root is node 0), status
-    const int32_t init[4] = {0, n > kSmallSeg ? 0 : 1, 1, 0};
+    const int32_t init[5] = {0, n > kTinySeg && n <= kSmallSeg ? 1 : 0, 1, 0, n <= kTinySeg ? 1 : 0};
     ck(cudaMemcpyAsync(counts, init, sizeof(init), cudaMemcpyHostToDevice, st), "counts");
     k_scene_bounds<<<grid_for(3 * n, 256), 256, 0, st>>>(d_tv, n, key6);
     k_prims<<<grid_for(n, 256), 256, 0, st>>>(d_tv, n, key6, plo, phi, pcz, ord[0], d_root, d_delta);
@@ -869,7 +1052,7 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
         ck(cudaMemsetAsync(gbins, 0, sizeof(uint32_t) * kBinWords * (size_t)n_big, st), "memset");
         ck(cudaMemsetAsync(counts, 0, sizeof(int32_t), st), "memset");
         k_bin_chunks<<<(int)hch.size(), kThreads, 0, st>>>(P, d_chunks, big[cur], ord[cur], gbins, chunk_cnt);
-        LevelOut L{big[1 - cur], small, counts, max_big, max_small, 2 * n};
+        LevelOut L{big[1 - cur], small, tiny, counts, max_big, max_small, 2 * n};
         k_split_big<<<n_big, kThreads, 0, st>>>(big[cur], gbins, splits, nodes, L, max_leaf, cur);
         k_scatter_big<<<(int)hch.size(), kThreads, 0, st>>>(P, d_chunks, big[cur], splits, chunk_cnt, ord[cur],
                                                             ord[1 - cur]);
@@ -884,11 +1067,17 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
     ck(cudaMemcpyAsync(h, counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "counts");
     ck(cudaStreamSynchronize(st), "counts");
     const int n_small = h[1];
-    SubCtx C{P, {ord[0], ord[1]}, out_order, nodes, counts, max_leaf, 2 * n};
-    if (n_small > 0) k_subtree<<<n_small, kThreads, 0, st>>>(small, C);
+    SubCtx C{P, {ord[0], ord[1]}, out_order, nodes, tiny, counts, max_leaf, 2 * n};
+    if (n_small > 0) k_subtree<<<n_small, kSubThreads, 0, st>>>(small, C);
     ck(cudaGetLastError(), "subtrees");
-    ck(cudaMemcpyAsync(h, counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "counts");
+    ck(cudaMemcpyAsync(h, counts, 5 * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "counts");
     ck(cudaStreamSynchronize(st), "subtrees");
+    if (h[3] != 0) throw std::runtime_error("device SAH build: subtree stack or node overflow");
+    const int n_tiny = h[4];
+    if (n_tiny > 0) k_tiny<<<(n_tiny + kTinyWarps - 1) / kTinyWarps, 32 * kTinyWarps, 0, st>>>(tiny, n_tiny, C);
+    ck(cudaGetLastError(), "small subtrees");
+    ck(cudaMemcpyAsync(h, counts, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "counts");
+    ck(cudaStreamSynchronize(st), "small subtrees");
     if (h[3] != 0) throw std::runtime_error("device SAH build: subtree stack or node overflow");
     const int n_node2 = h[2];
     if (n_node2 < 1 || n_node2 > 2 * n - 1) throw std::runtime_error("device SAH build: node count out of range");
