@@ -517,7 +517,7 @@ void render_batch_slot(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float*
     }
     *b->h_ctr = init;
     ck(cudaMemcpyAsync(b->d_ctr, b->h_ctr, sizeof(WaveCounters), cudaMemcpyHostToDevice, st), "init counters");
-    launch_nn_generate(b->arena, b->pb, 1, b->d_ctr, PD, b->d_jobs, n_jobs, st);  // fills buffer 0
+    launch_nn_generate(b->pb, 1, b->d_ctr, PD, b->d_jobs, n_jobs, b->num_sms, st);  // fills buffer 0
     const unsigned long long max_rounds =
         64 + (total / (unsigned long long)capacity + 2 + (unsigned long long)n_jobs) *
                  (unsigned long long)(max_depth + 2) * 4 / (unsigned long long)t.iters_per_graph;
@@ -535,7 +535,7 @@ void render_batch_slot(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float*
             launch_nn_shade(b->arena, b->pb, cur, P, b->d_ctr, b->film, b->nn_params, PD, guided, b->d_jobs, st);
             launch_nn_shadow(b->arena, b->pb, b->d_ctr, b->film, PD, b->d_jobs, b->num_sms, st);
             launch_nn_finish(PD, b->d_ctr, b->d_nnjobs, max_depth, capacity, st);
-            launch_nn_generate(b->arena, b->pb, cur, b->d_ctr, PD, b->d_jobs, n_jobs, st);
+            launch_nn_generate(b->pb, cur, b->d_ctr, PD, b->d_jobs, n_jobs, b->num_sms, st);
             launches += guided ? 7 : 6;
         }
         ck(cudaMemcpyAsync(b->h_ctr, b->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");

@@ -735,7 +735,7 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
     init.film_safe = film_safe_bound((double)desc->spp * (2.0 * desc->max_depth + 2.0));
     *s->h_ctr = init;
     ck(cudaMemcpyAsync(s->d_ctr, s->h_ctr, sizeof(WaveCounters), cudaMemcpyHostToDevice, st), "init counters");
-    launch_nn_generate(s->dev, s->pb, 1, s->d_ctr, PD, s->d_job, 1, st);
+    launch_nn_generate(s->pb, 1, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
     double launches = 3;
     const unsigned long long max_rounds =
         64 + (total / (unsigned long long)capacity + 2) * (unsigned long long)(desc->max_depth + 2) * 4 / kItersPerGraph;
@@ -753,7 +753,7 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
             launch_nn_shade(s->dev, s->pb, cur, P, s->d_ctr, s->film, params, PD, guided, s->d_job, st);
             launch_nn_shadow(s->dev, s->pb, s->d_ctr, s->film, PD, s->d_job, s->num_sms, st);
             launch_nn_finish(PD, s->d_ctr, s->d_nnjob, P.max_depth, capacity, st);
-            launch_nn_generate(s->dev, s->pb, cur, s->d_ctr, PD, s->d_job, 1, st);
+            launch_nn_generate(s->pb, cur, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
             launches += guided ? 7 : 6;
         }
         ck(cudaMemcpyAsync(s->h_ctr, s->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");

@@ -38,6 +38,8 @@ struct PathIO {
 struct ShadowIO {
     float4 *o, *d, *c;
 };
+inline PathIO path_io(const PathBuffers& B, int k) { return PathIO{B.o[k], B.d[k], B.thr[k], B.info[k]}; }
+inline ShadowIO shadow_io(const PathBuffers& B) { return ShadowIO{B.sh_o, B.sh_d, B.sh_c}; }
 
 struct RenderParams {
     int spp;

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_forward_debug(const DevN
 // Guide parameters for every live path's hit (run between extend and shade),
 // each path with its job's network.
 template <bool ONEBLOB>
-__global__ void __launch_bounds__(kTcInferThreads) k_nn_infer(DevScene S, PathBuffers B, int cur, WaveCounters* ctr,
+__global__ void __launch_bounds__(kTcInferThreads) k_nn_infer(DevScene S, PathIO in, const float4* __restrict__ hit, WaveCounters* ctr,
                                                               const DevNNJob* __restrict__ nnj,
                                                               float4* __restrict__ params) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -257,19 +257,19 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_infer(DevScene S, PathBu
     tc_infer_loop<ONEBLOB>(
         n, smem, nnj, &ctr->status,
         [&](int i, NNIn& v, int& job) {
-            const float4 H = B.hit[i];
+            const float4 H = hit[i];
             const int prim = __float_as_int(H.y);
             if (prim < 0) return false;
             const int4 vi = __ldg(S.tri_vidx + prim);
             if (S.mats[vi.w].kind == PT_MAT_EMISSIVE_) return false;
-            const float4 O = B.o[cur][i], D = B.d[cur][i];
+            const float4 O = in.o[i], D = in.d[i];
             const f3 d = mk(D.x, D.y, D.z);
             const float beta = H.z, gamma = H.w, alpha = 1.0f - (gamma + beta);
             v.pn = mk(O.x, O.y, O.z) + d * H.x;
             v.n = normalized(f3of(__ldg(S.v_nrm + vi.x)) * alpha + f3of(__ldg(S.v_nrm + vi.y)) * beta +
                              f3of(__ldg(S.v_nrm + vi.z)) * gamma);
             v.wo = -d;
-            job = (int)((uint32_t)B.info[cur][i].z >> kNNJobShift);
+            job = (int)((uint32_t)in.info[i].z >> kNNJobShift);
             return true;
         },
         [&](int i, const float* prm) { nn_pack_mixture(prm, params + kNNMixF4 * (size_t)i); });
@@ -627,8 +627,8 @@ void launch_nn_forward_debug(const DevNNJob* nnj, const float* in, int n, float*
 void launch_nn_infer(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const DevNNJob* nnj,
                      float4* params, int num_sms, cudaStream_t st, bool oneblob) {
     // four CTAs of 128 threads per SM fit in shared memory (48 KB each)
-    if (oneblob) k_nn_infer<true><<<num_sms * 4, kTcInferThreads, nn_smem_infer(), st>>>(S, B, cur, ctr, nnj, params);
-    else k_nn_infer<false><<<num_sms * 4, kTcInferThreads, nn_smem_infer(), st>>>(S, B, cur, ctr, nnj, params);
+    if (oneblob) k_nn_infer<true><<<num_sms * 4, kTcInferThreads, nn_smem_infer(), st>>>(S, path_io(B, cur), B.hit, ctr, nnj, params);
+    else k_nn_infer<false><<<num_sms * 4, kTcInferThreads, nn_smem_infer(), st>>>(S, path_io(B, cur), B.hit, ctr, nnj, params);
 }
 // Zeroes each task's gradient and loss (and, with prep, its T sum).
 __global__ void k_nn_task_zero(const NNTrainTask* __restrict__ tasks, int prep) {
@@ -715,7 +715,8 @@ __device__ __forceinline__ int warp_append_nn(int* counter, bool pred) {
 // 4: film total after the vertex's own NEE (rgb), wi valid (non-delta)
 // 5: film total before the NEE (rgb), p_bsdf(wi_nee)  6: wi_nee xyz, NEE valid.
 constexpr int kNNVert = kNNVertFloat4;
-__global__ void __launch_bounds__(256, 2) k_shade_nn(DevScene S, PathBuffers B, int cur, RenderParams P,
+constexpr int kShadeNNThreads = 256;
+__global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, PathBuffers B, PathIO in, PathIO nxt, RenderParams P,
                                                   WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                   const float4* __restrict__ params, NNPathData PD, int guided,
                                                   const DevBatchJob* __restrict__ jobs) {
@@ -726,8 +727,8 @@ __global__ void __launch_bounds__(256, 2) k_shade_nn(DevScene S, PathBuffers B, 
     int4 ninfo;
     int slot = -1, fin_bounce = 0, fin_nv = 0;
     if (i < n) {
-        const float4 O = B.o[cur][i], D = B.d[cur][i], Tp = B.thr[cur][i];
-        const int4 I = B.info[cur][i];
+        const float4 O = in.o[i], D = in.d[i], Tp = in.thr[i];
+        const int4 I = in.info[i];
         const float4 H = B.hit[i];
         const int prim = __float_as_int(H.y);
         const int pixel = I.x, sample = I.y, bounce = I.z & 0xffff;
@@ -866,22 +867,42 @@ __global__ void __launch_bounds__(256, 2) k_shade_nn(DevScene S, PathBuffers B, 
         if (fin_nv < bounce) fin_nv = bounce;
         release = done;
     }
-    const int js = warp_append_nn(&ctr->n_shadow, push_sh);
+    // one addition to each queue's counter per CTA (as k_shade)
+    __shared__ int s_count[3][kShadeNNThreads / 32], s_base[3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m_sh = __ballot_sync(0xffffffffu, push_sh), m_cont = __ballot_sync(0xffffffffu, push_cont),
+                   m_fin = __ballot_sync(0xffffffffu, release);
+    if (lane == 0) {
+        s_count[0][warp] = __popc(m_sh);
+        s_count[1][warp] = __popc(m_cont);
+        s_count[2][warp] = __popc(m_fin);
+    }
+    __syncthreads();
+    if (lane == 0 && warp < 3) {
+        int total = 0;
+        for (int w = 0; w < kShadeNNThreads / 32; w++) {
+            const int q = s_count[warp][w];
+            s_count[warp][w] = total;
+            total += q;
+        }
+        if (total) s_base[warp] = atomicAdd(warp == 0 ? &ctr->n_shadow : (warp == 1 ? &ctr->n_next : &ctr->n_fin), total);
+    }
+    __syncthreads();
+    const unsigned below = (1u << lane) - 1u;
     if (push_sh) {
+        const int js = s_base[0] + s_count[0][warp] + __popc(m_sh & below);
         B.sh_o[js] = sh_o;
         B.sh_d[js] = sh_d;
         B.sh_c[js] = sh_c;
     }
-    const int jc = warp_append_nn(&ctr->n_next, push_cont);
     if (push_cont) {
-        const int nx = 1 - cur;
-        B.o[nx][jc] = no;
-        B.d[nx][jc] = nd;
-        B.thr[nx][jc] = nt;
-        B.info[nx][jc] = ninfo;
+        const int jc = s_base[1] + s_count[1][warp] + __popc(m_cont & below);
+        nxt.o[jc] = no;
+        nxt.d[jc] = nd;
+        nxt.thr[jc] = nt;
+        nxt.info[jc] = ninfo;
     }
-    const int jf = warp_append_nn(&ctr->n_fin, release);
-    if (release) PD.fin[jf] = make_int4(slot, fin_bounce, fin_nv, 0);
+    if (release) PD.fin[s_base[2] + s_count[2][warp] + __popc(m_fin & below)] = make_int4(slot, fin_bounce, fin_nv, 0);
 }
 
 // Finished paths.  Two records per vertex, both MIS-weighted one-sample
@@ -1021,61 +1042,62 @@ cudaError_t nn_shadow_smem_limit() {
 }
 
 // Camera paths (stratified like pathtracerMIS.h:148-153) with a vertex slot.
-__global__ void __launch_bounds__(256) k_generate_nn(DevScene S, PathBuffers B, int cur, WaveCounters* ctr,
-                                                     NNPathData PD, const DevBatchJob* __restrict__ jobs,
+__global__ void __launch_bounds__(256) k_generate_nn(PathIO nxt, int capacity, WaveCounters* ctr, NNPathData PD,
+                                                     const DevBatchJob* __restrict__ jobs,
                                                      int n_jobs) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n_next = ctr->n_next;
-    const int avail = min(B.capacity - n_next, ctr->free_top);
-    unsigned long long w = ctr->work_next + (unsigned long long)t;
-    if (t >= avail || w >= ctr->work_total) return;
-    int job = 0;
-    if (n_jobs > 1) {  // job ranges ascend (as find_job in render.cu)
-        int lo = 0, hi = n_jobs - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(&jobs[mid].work_begin) <= w) lo = mid;
-            else hi = mid - 1;
+    const int n_next = ctr->n_next, free_top = ctr->free_top;
+    const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
+    const int avail = min(capacity - n_next, free_top);
+    const int count = left < (unsigned long long)avail ? (int)left : avail;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+        unsigned long long w = first + (unsigned long long)t;
+        int job = 0;
+        if (n_jobs > 1) {  // job ranges ascend (as find_job in render.cu)
+            int lo = 0, hi = n_jobs - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (__ldg(&jobs[mid].work_begin) <= w) lo = mid;
+                else hi = mid - 1;
+            }
+            job = lo;
         }
-        job = lo;
+        const DevBatchJob* J = jobs + job;
+        w -= J->work_begin;
+        const DevCamera* C = &J->cam;
+        const int width = C->width, height = C->height, spp_axis = J->spp_axis;
+        const unsigned long long npix = (unsigned long long)width * height;
+        const int sample = (int)(w / npix);
+        int pixel = (int)(w - (unsigned long long)sample * npix);
+        if (J->tile_w * J->tile_h > 1) {  // tiled pass order (a bijection of the pixels)
+            const int tw = J->tile_w, th = J->tile_h;
+            const int tile = pixel / (tw * th), r = pixel - tile * (tw * th);
+            const int tiles_x = width / tw;
+            const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
+            pixel = (ty * th + r / tw) * width + tx * tw + r % tw;
+        }
+        const int px = pixel % width, py = pixel / width;
+        const Rng4 r = rng4(J->seed, sample, pixel, 0xffffu, 2);
+        float cx, cy;
+        if (spp_axis > 0) {  // pathtracerMIS.h:148-153
+            const int k = sample / spp_axis, l = sample - (sample / spp_axis) * spp_axis;
+            cx = (((float)px + ((float)k + r.v[0]) / (float)spp_axis) / (float)width) * 2.0f - 1.0f;
+            cy = -((((float)py + ((float)l + r.v[1]) / (float)spp_axis) / (float)height) * 2.0f - 1.0f);
+        } else {
+            cx = (((float)px + r.v[0]) / (float)width) * 2.0f - 1.0f;
+            cy = -((((float)py + r.v[1]) / (float)height) * 2.0f - 1.0f);
+        }
+        const float dx = cx * C->tan_fovy * C->aspect, dy = cy * C->tan_fovy, dz = -1.0f;
+        const f3 d = normalized(mk(C->m[0] * dx + C->m[1] * dy + C->m[2] * dz, C->m[3] * dx + C->m[4] * dy + C->m[5] * dz,
+                                   C->m[6] * dx + C->m[7] * dy + C->m[8] * dz));
+        const int j = n_next + t;
+        const int slot = PD.slot_stack[free_top - 1 - t];
+        PD.acc[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+        PD.slot_job[slot] = job;
+        nxt.o[j] = make_float4(C->o[0], C->o[1], C->o[2], 1.0f);
+        nxt.d[j] = make_float4(d.x, d.y, d.z, __uint_as_float(J->root));
+        nxt.thr[j] = make_float4(1.f, 1.f, 1.f, 0.f);
+        nxt.info[j] = make_int4(pixel, sample, (1 << 16) | (job << kNNJobShift), slot);  // sampled_delta starts true
     }
-    const DevBatchJob* J = jobs + job;
-    w -= J->work_begin;
-    const DevCamera* C = &J->cam;
-    const int width = C->width, height = C->height, spp_axis = J->spp_axis;
-    const unsigned long long npix = (unsigned long long)width * height;
-    const int sample = (int)(w / npix);
-    int pixel = (int)(w - (unsigned long long)sample * npix);
-    if (J->tile_w * J->tile_h > 1) {  // tiled pass order (a bijection of the pixels)
-        const int tw = J->tile_w, th = J->tile_h;
-        const int tile = pixel / (tw * th), r = pixel - tile * (tw * th);
-        const int tiles_x = width / tw;
-        const int ty = tile / tiles_x, tx = tile - ty * tiles_x;
-        pixel = (ty * th + r / tw) * width + tx * tw + r % tw;
-    }
-    const int px = pixel % width, py = pixel / width;
-    const Rng4 r = rng4(J->seed, sample, pixel, 0xffffu, 2);
-    float cx, cy;
-    if (spp_axis > 0) {  // pathtracerMIS.h:148-153
-        const int k = sample / spp_axis, l = sample - (sample / spp_axis) * spp_axis;
-        cx = (((float)px + ((float)k + r.v[0]) / (float)spp_axis) / (float)width) * 2.0f - 1.0f;
-        cy = -((((float)py + ((float)l + r.v[1]) / (float)spp_axis) / (float)height) * 2.0f - 1.0f);
-    } else {
-        cx = (((float)px + r.v[0]) / (float)width) * 2.0f - 1.0f;
-        cy = -((((float)py + r.v[1]) / (float)height) * 2.0f - 1.0f);
-    }
-    const float dx = cx * C->tan_fovy * C->aspect, dy = cy * C->tan_fovy, dz = -1.0f;
-    const f3 d = normalized(mk(C->m[0] * dx + C->m[1] * dy + C->m[2] * dz, C->m[3] * dx + C->m[4] * dy + C->m[5] * dz,
-                               C->m[6] * dx + C->m[7] * dy + C->m[8] * dz));
-    const int nx = 1 - cur;
-    const int j = n_next + t;
-    const int slot = PD.slot_stack[ctr->free_top - 1 - t];
-    PD.acc[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
-    PD.slot_job[slot] = job;
-    B.o[nx][j] = make_float4(C->o[0], C->o[1], C->o[2], 1.0f);
-    B.d[nx][j] = make_float4(d.x, d.y, d.z, __uint_as_float(J->root));
-    B.thr[nx][j] = make_float4(1.f, 1.f, 1.f, 0.f);
-    B.info[nx][j] = make_int4(pixel, sample, (1 << 16) | (job << kNNJobShift), slot);  // sampled_delta starts true
 }
 
 __global__ void k_advance_nn(WaveCounters* ctr, int capacity) {
@@ -1103,15 +1125,17 @@ __global__ void k_advance_nn(WaveCounters* ctr, int capacity) {
 void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                      unsigned long long* film, const float4* params, const NNPathData& PD, bool guided,
                      const DevBatchJob* jobs, cudaStream_t st) {
-    k_shade_nn<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, B, cur, P, ctr, film, params, PD, guided ? 1 : 0, jobs);
+    k_shade_nn<<<(B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st>>>(S, B, path_io(B, cur), path_io(B, 1 - cur), P, ctr, film, params, PD, guided ? 1 : 0, jobs);
 }
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
     k_shadow_nn<<<num_sms * kTraceBlocksPerSM, kTraceThreads, trace_smem(false, true, kTraceThreads), st>>>(S, B, ctr, film, PD, jobs);
 }
-void launch_nn_generate(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
-                        const DevBatchJob* jobs, int n_jobs, cudaStream_t st) {
-    k_generate_nn<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, B, cur, ctr, PD, jobs, n_jobs);
+void launch_nn_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
+                        const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
+    // a resident grid over the free slots (as the plain wavefront's)
+    k_generate_nn<<<std::max(1, std::min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st>>>(
+        path_io(B, 1 - cur), B.capacity, ctr, PD, jobs, n_jobs);
     k_advance_nn<<<1, 32, 0, st>>>(ctr, B.capacity);
 }
 void launch_nn_finish(const NNPathData& PD, WaveCounters* ctr, const DevNNJob* nnj, int max_depth, int capacity,

@@ -112,8 +112,8 @@ void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const Ren
                      const DevBatchJob* jobs, cudaStream_t st);
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st);
-void launch_nn_generate(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
-                        const DevBatchJob* jobs, int n_jobs, cudaStream_t st);
+void launch_nn_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
+                        const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st);
 // Emits the training records of the paths that finished this iteration (after
 // the shadow stage, so their last NEE is counted) and frees their slots.
 void launch_nn_finish(const NNPathData& PD, WaveCounters* ctr, const DevNNJob* nnj, int max_depth, int capacity,

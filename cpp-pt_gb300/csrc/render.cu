@@ -539,11 +539,6 @@ __global__ void k_resolve(const unsigned long long* __restrict__ film, float* __
         out[i] = (float)((double)(long long)film[i] * scale);
 }
 
-namespace {
-PathIO path_io(const PathBuffers& B, int k) { return PathIO{B.o[k], B.d[k], B.thr[k], B.info[k]}; }
-ShadowIO shadow_io(const PathBuffers& B) { return ShadowIO{B.sh_o, B.sh_d, B.sh_c}; }
-}  // namespace
-
 void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, int num_sms, cudaStream_t st,
                    bool count) {
     const int g = num_sms * kTraceBlocksPerSM;
