@@ -506,7 +506,7 @@ void render_batch_slot(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float*
     P.flags = flags;
     ck(cudaEventRecord(b->ev0, st), "event");
     ck(cudaMemsetAsync(b->film, 0, sizeof(unsigned long long) * 3 * pixels, st), "memset film");
-    launch_init_slots(PD.slot_stack, capacity, st);
+    if (train) launch_init_slots(PD.slot_stack, capacity, st);
     WaveCounters init{};
     init.work_total = total;
     init.free_top = capacity;
@@ -529,14 +529,17 @@ void render_batch_slot(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float*
     while (true) {
         for (int k = 0; k < t.iters_per_graph; k++) {
             const int cur = k & 1;
-            launch_extend(b->arena, b->pb, cur, b->d_ctr, b->num_sms, st);
+            if (train) launch_extend(b->arena, b->pb, cur, b->d_ctr, b->num_sms, st);
+            else launch_trace_wave(b->arena, b->pb, cur, b->d_ctr, b->film, b->num_sms, st);
             if (guided)
                 launch_nn_infer(b->arena, b->pb, cur, b->d_ctr, b->d_nnjobs, b->nn_params, b->num_sms, st, oneblob);
             launch_nn_shade(b->arena, b->pb, cur, P, b->d_ctr, b->film, b->nn_params, PD, guided, b->d_jobs, st);
-            launch_nn_shadow(b->arena, b->pb, b->d_ctr, b->film, PD, b->d_jobs, b->num_sms, st);
-            launch_nn_finish(PD, b->d_ctr, b->d_nnjobs, max_depth, capacity, st);
+            if (train) {
+                launch_nn_shadow(b->arena, b->pb, b->d_ctr, b->film, PD, b->d_jobs, b->num_sms, st);
+                launch_nn_finish(PD, b->d_ctr, b->d_nnjobs, max_depth, capacity, st);
+            }
             launch_nn_generate(b->pb, cur, b->d_ctr, PD, b->d_jobs, n_jobs, b->num_sms, st);
-            launches += guided ? 7 : 6;
+            launches += (guided ? 5 : 4) + (train ? 2 : 0);
         }
         ck(cudaMemcpyAsync(b->h_ctr, b->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");
         if (train)
@@ -570,7 +573,7 @@ void render_batch_slot(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float*
             }
         }
         rounds++;
-        if (b->h_ctr->n_cur == 0 && b->h_ctr->work_next >= b->h_ctr->work_total) break;
+        if (train ? b->h_ctr->n_cur == 0 && b->h_ctr->work_next >= b->h_ctr->work_total : wave_done(*b->h_ctr)) break;
         if (rounds > max_rounds) throw Fail(PT_ERR_LIMIT, "batch render did not converge within the iteration bound");
     }
     if (train)

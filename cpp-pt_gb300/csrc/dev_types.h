@@ -120,6 +120,11 @@ struct WaveCounters {
     unsigned long long stat_film_overflow;     // contributions the 32.32 film could not hold
 };
 
+// Nothing is left of a wavefront whose shadow rays are traced an iteration late.
+inline bool wave_done(const WaveCounters& c) {
+    return c.n_cur == 0 && c.work_next >= c.work_total && c.n_shadow == 0 && c.n_shadow1 == 0;
+}
+
 // film_safe for a render of at most `per_pixel` film contributions per pixel
 // and channel: a sum of contributions below 2^31 / per_pixel stays below
 // 2^31, the largest value the signed 32.32 fixed-point film holds.

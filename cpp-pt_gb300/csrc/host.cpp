@@ -727,7 +727,7 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
     ck(cudaMemcpyAsync(s->d_nnjob, s->h_nnjob, sizeof(DevNNJob), cudaMemcpyHostToDevice, st), "guide job table");
     ck(cudaEventRecord(s->ev0, st), "event");
     ck(cudaMemsetAsync(s->film, 0, sizeof(unsigned long long) * film_n, st), "memset film");
-    launch_init_slots(PD.slot_stack, capacity, st);
+    if (train) launch_init_slots(PD.slot_stack, capacity, st);
     WaveCounters init{};
     init.work_total = total;
     init.free_top = capacity;
@@ -746,15 +746,20 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
     for (unsigned long long round = 0;; round++) {
         for (int k = 0; k < kItersPerGraph; k++) {
             const int cur = k & 1;
-            launch_extend(s->dev, s->pb, cur, s->d_ctr, s->num_sms, st);
+            // without records to collect, nothing waits for a path's shadow ray:
+            // it is traced with the next iteration's extension rays
+            if (train) launch_extend(s->dev, s->pb, cur, s->d_ctr, s->num_sms, st);
+            else launch_trace_wave(s->dev, s->pb, cur, s->d_ctr, s->film, s->num_sms, st);
             if (guided)
                 launch_nn_infer(s->dev, s->pb, cur, s->d_ctr, s->d_nnjob, params, s->num_sms, st,
                                 s->nn_cfg.encoding == PT_NN_ENC_ONEBLOB);
             launch_nn_shade(s->dev, s->pb, cur, P, s->d_ctr, s->film, params, PD, guided, s->d_job, st);
-            launch_nn_shadow(s->dev, s->pb, s->d_ctr, s->film, PD, s->d_job, s->num_sms, st);
-            launch_nn_finish(PD, s->d_ctr, s->d_nnjob, P.max_depth, capacity, st);
+            if (train) {
+                launch_nn_shadow(s->dev, s->pb, s->d_ctr, s->film, PD, s->d_job, s->num_sms, st);
+                launch_nn_finish(PD, s->d_ctr, s->d_nnjob, P.max_depth, capacity, st);
+            }
             launch_nn_generate(s->pb, cur, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
-            launches += guided ? 7 : 6;
+            launches += (guided ? 5 : 4) + (train ? 2 : 0);
         }
         ck(cudaMemcpyAsync(s->h_ctr, s->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");
         ck(cudaStreamSynchronize(st), "render");
@@ -782,7 +787,7 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
             ck(cudaMemcpyAsync(s->d_nnjob, s->h_nnjob, sizeof(DevNNJob), cudaMemcpyHostToDevice, st),
                "guide job table");
         n0 = rec_left >= 0 ? rec_left : s->h_ctr->n_rec;
-        if (s->h_ctr->n_cur == 0 && s->h_ctr->work_next >= s->h_ctr->work_total) break;
+        if (train ? s->h_ctr->n_cur == 0 && s->h_ctr->work_next >= s->h_ctr->work_total : wave_done(*s->h_ctr)) break;
         if (round > max_rounds) throw Fail(PT_ERR_LIMIT, "render did not converge within the iteration bound");
     }
     if (train) s->nn_rec_count = rec_left >= 0 ? rec_left : std::min(s->h_ctr->n_rec, rec_cap);

@@ -69,6 +69,12 @@ void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounter
 // (launch_shadow), not only those of the iteration before.
 void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const DevBatchJob* jobs, int n_jobs, int num_sms,
                      cudaStream_t st, bool shadows_traced);
+// The parts of launch_wave_iteration that the learned-guide wavefront uses
+// when it does not train: the extension rays with the shadow rays of the
+// iteration before, and the counters.
+void launch_trace_wave(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
+                       int num_sms, cudaStream_t st);
+void launch_advance(WaveCounters* ctr, int capacity, int cur, cudaStream_t st);
 // A whole iteration as renders run it: the extension rays together with the
 // shadow rays of the iteration before (one launch), shade, generate, advance.
 void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,

@@ -716,7 +716,7 @@ __device__ __forceinline__ int warp_append_nn(int* counter, bool pred) {
 // 5: film total before the NEE (rgb), p_bsdf(wi_nee)  6: wi_nee xyz, NEE valid.
 constexpr int kNNVert = kNNVertFloat4;
 constexpr int kShadeNNThreads = 256;
-__global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, PathBuffers B, PathIO in, PathIO nxt, RenderParams P,
+__global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, PathBuffers B, PathIO in, PathIO nxt, int cur, RenderParams P,
                                                   WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                   const float4* __restrict__ params, NNPathData PD, int guided,
                                                   const DevBatchJob* __restrict__ jobs) {
@@ -818,7 +818,8 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
                             const f3 so = s.p + sd * kEps;
                             sh_o = make_float4(so.x, so.y, so.z, len - 2.0f * kEps);
                             sh_d = make_float4(sd.x, sd.y, sd.z, __int_as_float((int)(uint32_t)fpix));
-                            sh_c = make_float4(cc.x, cc.y, cc.z, __int_as_float(slot));
+                            // w: the path's slot while training, else the scene root (as k_shade)
+                            sh_c = make_float4(cc.x, cc.y, cc.z, train ? __int_as_float(slot) : D.w);
                         }
                     }
                 }
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
         // records are emitted once this vertex's shadow ray has resolved
         fin_bounce = bounce;
         if (fin_nv < bounce) fin_nv = bounce;
-        release = done;
+        release = done && train;  // without records no slot is held
     }
     // one addition to each queue's counter per CTA (as k_shade)
     __shared__ int s_count[3][kShadeNNThreads / 32], s_base[3];
@@ -885,7 +886,9 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
             s_count[warp][w] = total;
             total += q;
         }
-        if (total) s_base[warp] = atomicAdd(warp == 0 ? &ctr->n_shadow : (warp == 1 ? &ctr->n_next : &ctr->n_fin), total);
+        // while training n_shadow and n_fin; else the counters of k_shade
+        int* n_shadow = PD.rec_cap == 0 && cur ? &ctr->n_shadow1 : &ctr->n_shadow;
+        if (total) s_base[warp] = atomicAdd(warp == 0 ? n_shadow : (warp == 1 ? &ctr->n_next : &ctr->n_fin), total);
     }
     __syncthreads();
     const unsigned below = (1u << lane) - 1u;
@@ -1047,7 +1050,8 @@ __global__ void __launch_bounds__(256) k_generate_nn(PathIO nxt, int capacity, W
                                                      int n_jobs) {
     const int n_next = ctr->n_next, free_top = ctr->free_top;
     const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
-    const int avail = min(capacity - n_next, free_top);
+    const bool slots = PD.rec_cap > 0;  // vertex slots are for training records
+    const int avail = slots ? min(capacity - n_next, free_top) : capacity - n_next;
     const int count = left < (unsigned long long)avail ? (int)left : avail;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
         unsigned long long w = first + (unsigned long long)t;
@@ -1090,9 +1094,12 @@ __global__ void __launch_bounds__(256) k_generate_nn(PathIO nxt, int capacity, W
         const f3 d = normalized(mk(C->m[0] * dx + C->m[1] * dy + C->m[2] * dz, C->m[3] * dx + C->m[4] * dy + C->m[5] * dz,
                                    C->m[6] * dx + C->m[7] * dy + C->m[8] * dz));
         const int j = n_next + t;
-        const int slot = PD.slot_stack[free_top - 1 - t];
-        PD.acc[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
-        PD.slot_job[slot] = job;
+        int slot = 0;
+        if (slots) {
+            slot = PD.slot_stack[free_top - 1 - t];
+            PD.acc[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+            PD.slot_job[slot] = job;
+        }
         nxt.o[j] = make_float4(C->o[0], C->o[1], C->o[2], 1.0f);
         nxt.d[j] = make_float4(d.x, d.y, d.z, __uint_as_float(J->root));
         nxt.thr[j] = make_float4(1.f, 1.f, 1.f, 0.f);
@@ -1125,7 +1132,7 @@ __global__ void k_advance_nn(WaveCounters* ctr, int capacity) {
 void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                      unsigned long long* film, const float4* params, const NNPathData& PD, bool guided,
                      const DevBatchJob* jobs, cudaStream_t st) {
-    k_shade_nn<<<(B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st>>>(S, B, path_io(B, cur), path_io(B, 1 - cur), P, ctr, film, params, PD, guided ? 1 : 0, jobs);
+    k_shade_nn<<<(B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st>>>(S, B, path_io(B, cur), path_io(B, 1 - cur), cur, P, ctr, film, params, PD, guided ? 1 : 0, jobs);
 }
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
@@ -1136,7 +1143,8 @@ void launch_nn_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const 
     // a resident grid over the free slots (as the plain wavefront's)
     k_generate_nn<<<std::max(1, std::min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st>>>(
         path_io(B, 1 - cur), B.capacity, ctr, PD, jobs, n_jobs);
-    k_advance_nn<<<1, 32, 0, st>>>(ctr, B.capacity);
+    if (PD.rec_cap > 0) k_advance_nn<<<1, 32, 0, st>>>(ctr, B.capacity);
+    else launch_advance(ctr, B.capacity, cur, st);
 }
 void launch_nn_finish(const NNPathData& PD, WaveCounters* ctr, const DevNNJob* nnj, int max_depth, int capacity,
                       cudaStream_t st) {

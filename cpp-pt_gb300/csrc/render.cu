@@ -582,6 +582,9 @@ void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const Dev
     k_generate<<<g, 256, 0, st>>>(path_io(B, 1 - cur), B.capacity, ctr, jobs, n_jobs);
     k_advance<<<1, 32, 0, st>>>(ctr, B.capacity, cur, shadows_traced ? cur : 1 - cur, shadows_traced ? 0 : kFinishPaths);
 }
+void launch_advance(WaveCounters* ctr, int capacity, int cur, cudaStream_t st) {
+    k_advance<<<1, 32, 0, st>>>(ctr, capacity, cur, 1 - cur, 0);
+}
 void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                            const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
     launch_trace_wave(S, B, cur, ctr, film, num_sms, st);
