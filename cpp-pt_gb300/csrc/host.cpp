@@ -304,9 +304,12 @@ constexpr int kMaxCapacity = 1 << CPPPT_MAX_WAVE_LOG2;
 // 3.3e-3 against 4.7e-4 at 2^20); with records sampled evenly (the keep
 // probability) it learned faster but then took very bright samples
 // (relMSE 8.8e-3 at 10 s).  So 2^20.
-#ifndef CPPPT_NN_WAVE_LOG2
-#define CPPPT_NN_WAVE_LOG2 20
-#endif
+constexpr int kTrainCapacity = 1 << 20;
+// Without training (a frozen guide, or BSDF sampling alone) there are no
+// records and the image does not depend on the paths in flight: 192 B of path
+// state and 128 B of mixture each.  The slit room at 1280x720, 4 spp, frozen
+// guide: 2^20 12.46 ms, 2^21 11.95, 2^22 11.19.
+constexpr int kFrozenCapacity = 1 << 22;
 constexpr int kItersPerGraph = 16;   // of the learned-guide and SD-tree renders between host steps; even: buffers alternate
 constexpr int kItersPerBody = 20;    // of a plain render's device-driven loop body; even
 
@@ -559,27 +562,43 @@ NNNorm scene_norm(const pt_scene* s) {
     return N;
 }
 
-// Per-path buffers of the slot-based wavefront, kept by the scene and grown
-// on demand (capacity paths; vertex records for `depth` vertices per path
-// when training; guide parameters when the guide is used).
-NNPathData nn_path_buffers(pt_scene* s, int capacity, int depth) {
-    const bool grow = capacity > s->nnpd_cap || depth > s->nnpd_depth;
-    if (grow) {
+// Per-path buffers of the learned-guide wavefront, kept by the scene and grown
+// on demand: the guide's mixtures for `capacity` paths (guided), and vertex
+// records and slots for `depth` vertices per path (training, depth > 0).
+// Returns the paths in flight the render uses: `capacity`, or fewer (down to
+// 2^20) when the device cannot hold the mixtures of that many.
+int nn_path_buffers(pt_scene* s, int capacity, int depth, bool guided) {
+    if (guided && capacity > s->nn_params_cap) {
+        if (s->nn_params) cudaFree(s->nn_params);
+        s->nn_params = nullptr;
+        s->nn_params_cap = 0;
+        for (int c = capacity;; c = std::max(1 << 20, c / 2)) {
+            void* p = nullptr;
+            const cudaError_t e = cudaMalloc(&p, sizeof(float4) * (size_t)c * kNNMixF4);
+            if (e == cudaSuccess) {
+                s->nn_params = static_cast<float4*>(p);
+                s->nn_params_cap = c;
+                break;
+            }
+            if (c <= (1 << 20)) ck(e, "cudaMalloc");
+            cudaGetLastError();  // an allocation failure is not sticky
+        }
+    }
+    if (guided) capacity = std::min(capacity, s->nn_params_cap);
+    if (depth > 0 && (capacity > s->nnpd_cap || depth > s->nnpd_depth)) {
         for (void* p : s->nnpd_owned) cudaFree(p);
         s->nnpd_owned.clear();
         s->nnpd = NNPathData{};
-        s->nn_params = nullptr;
         s->nnpd_cap = std::max(capacity, s->nnpd_cap);
         s->nnpd_depth = std::max(depth, s->nnpd_depth);
         const int cap = s->nnpd_cap;
-        s->nnpd.vert = dalloc<float4>(s->nnpd_owned, (size_t)cap * std::max(1, s->nnpd_depth) * kNNVertFloat4);
+        s->nnpd.vert = dalloc<float4>(s->nnpd_owned, (size_t)cap * s->nnpd_depth * kNNVertFloat4);
         s->nnpd.acc = dalloc<float4>(s->nnpd_owned, cap);
         s->nnpd.slot_stack = dalloc<int>(s->nnpd_owned, cap);
         s->nnpd.slot_job = dalloc<int>(s->nnpd_owned, cap);
         s->nnpd.fin = dalloc<int4>(s->nnpd_owned, cap);
-        s->nn_params = dalloc<float4>(s->nnpd_owned, (size_t)cap * kNNMixF4);
     }
-    return s->nnpd;
+    return capacity;
 }
 
 // Overlapped training rounds of one or several scenes' guides (declared
@@ -702,9 +721,13 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
     P.flags = desc->flags;
     const unsigned long long total = (unsigned long long)s->width * s->height * (unsigned long long)desc->spp;
     const int film_n = 3 * s->width * s->height;
-    const int capacity =
-        ensure_wave(s, (int)std::min<unsigned long long>(1 << CPPPT_NN_WAVE_LOG2, (total + 1023) / 1024 * 1024), film_n);
-    NNPathData PD = nn_path_buffers(s, capacity, train ? P.max_depth : 0);
+    int capacity = ensure_wave(
+        s, (int)std::min<unsigned long long>(train ? kTrainCapacity : kFrozenCapacity, (total + 1023) / 1024 * 1024),
+        film_n);
+    capacity = nn_path_buffers(s, capacity, train ? P.max_depth : 0, guided);
+    PathBuffers pb = s->pb;  // kernels fill at most `capacity` paths of the scene's buffers
+    pb.capacity = capacity;
+    NNPathData PD = s->nnpd;
     const int batch = s->nn_cfg.batch;
     const int rec_cap = std::min(kNNRecordCap, s->nn_cfg.steps_per_round * batch);
     PD.rec_cap = train ? rec_cap : 0;
@@ -735,7 +758,7 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
     init.film_safe = film_safe_bound((double)desc->spp * (2.0 * desc->max_depth + 2.0));
     *s->h_ctr = init;
     ck(cudaMemcpyAsync(s->d_ctr, s->h_ctr, sizeof(WaveCounters), cudaMemcpyHostToDevice, st), "init counters");
-    launch_nn_generate(s->pb, 1, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
+    launch_nn_generate(pb, 1, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
     double launches = 3;
     const unsigned long long max_rounds =
         64 + (total / (unsigned long long)capacity + 2) * (unsigned long long)(desc->max_depth + 2) * 4 / kItersPerGraph;
@@ -748,17 +771,17 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
             const int cur = k & 1;
             // without records to collect, nothing waits for a path's shadow ray:
             // it is traced with the next iteration's extension rays
-            if (train) launch_extend(s->dev, s->pb, cur, s->d_ctr, s->num_sms, st);
-            else launch_trace_wave(s->dev, s->pb, cur, s->d_ctr, s->film, s->num_sms, st);
+            if (train) launch_extend(s->dev, pb, cur, s->d_ctr, s->num_sms, st);
+            else launch_trace_wave(s->dev, pb, cur, s->d_ctr, s->film, s->num_sms, st);
             if (guided)
-                launch_nn_infer(s->dev, s->pb, cur, s->d_ctr, s->d_nnjob, params, s->num_sms, st,
+                launch_nn_infer(s->dev, pb, cur, s->d_ctr, s->d_nnjob, params, s->num_sms, st,
                                 s->nn_cfg.encoding == PT_NN_ENC_ONEBLOB);
-            launch_nn_shade(s->dev, s->pb, cur, P, s->d_ctr, s->film, params, PD, guided, s->d_job, st);
+            launch_nn_shade(s->dev, pb, cur, P, s->d_ctr, s->film, params, PD, guided, s->d_job, st);
             if (train) {
-                launch_nn_shadow(s->dev, s->pb, s->d_ctr, s->film, PD, s->d_job, s->num_sms, st);
+                launch_nn_shadow(s->dev, pb, s->d_ctr, s->film, PD, s->d_job, s->num_sms, st);
                 launch_nn_finish(PD, s->d_ctr, s->d_nnjob, P.max_depth, capacity, st);
             }
-            launch_nn_generate(s->pb, cur, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
+            launch_nn_generate(pb, cur, s->d_ctr, PD, s->d_job, 1, s->num_sms, st);
             launches += (guided ? 5 : 4) + (train ? 2 : 0);
         }
         ck(cudaMemcpyAsync(s->h_ctr, s->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");

@@ -182,8 +182,9 @@ struct pt_scene {
     int nn_rec_count = 0;
     float nn_keep = 1.0f;  // probability that a finished path leaves training records (adapted per round)
     int* h_rec_left = nullptr;  // pinned staging word for the kept-record count
-    NNPathData nnpd{};          // per-path buffers of the slot-based wavefront (grown on demand)
-    float4* nn_params = nullptr;
+    NNPathData nnpd{};          // per-path buffers of the training wavefront (grown on demand)
+    float4* nn_params = nullptr;  // the guide's mixtures, nn_params_cap paths
+    int nn_params_cap = 0;
     int nnpd_cap = 0, nnpd_depth = 0;
     std::vector<void*> nnpd_owned;
     pt_nn_config nn_cfg{3e-3f, 0.3f, 0.9f, 1 << 16, PT_NN_CHI2, 16, PT_NN_ENC_FREQ, 1};
@@ -191,6 +192,7 @@ struct pt_scene {
     ~pt_scene() {
         for (void* p : nn_owned) cudaFree(p);
         for (void* p : nnpd_owned) cudaFree(p);
+        if (nn_params) cudaFree(nn_params);
         if (graph) cudaGraphExecDestroy(graph);
         for (void* p : owned) cudaFree(p);
         for (void* p : pb_owned) cudaFree(p);

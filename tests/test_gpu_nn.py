@@ -203,3 +203,25 @@ def test_passes_take_several_steps_per_batch(gpu_lib):
     assert batches >= 4 and batches == int(batches), st
     assert st["steps"] == 3 * batches, st
     assert np.isfinite(img).all() and img.mean() > 0
+
+
+@pytest.mark.parametrize("spp", [4, 300, 1200])
+def test_frozen_render_after_other_renders(gpu_lib, spp):
+    """A frozen-guide render gives the same image whatever the scene rendered
+    before: its wavefront (at most 2^22 paths) keeps to its own size inside
+    larger path buffers, and follows a training render with vertex records."""
+    from cpppt import scenes
+    from cpppt.lib import FLAG_NN_FREEZE, MODE_MIS, MODE_NN, GpuScene
+    sc = scenes.slit_room(seed=4, n_boxes=20, box_subdiv=1, width=72, height=64)
+    fresh = GpuScene(sc)
+    fresh.nn_reset(3)
+    want = fresh.render(spp, max_depth=6, seed=2, mode=MODE_NN, flags=FLAG_NN_FREEZE)
+    gs = GpuScene(sc)
+    gs.render(1500, max_depth=4, seed=1, mode=MODE_MIS)  # 6.9M paths in flight
+    gs.nn_reset(3)
+    got = gs.render(spp, max_depth=6, seed=2, mode=MODE_NN, flags=FLAG_NN_FREEZE)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    gs.render(4, max_depth=6, seed=5, mode=MODE_NN)  # trains: records and slots
+    gs.nn_reset(3)
+    again = gs.render(spp, max_depth=6, seed=2, mode=MODE_NN, flags=FLAG_NN_FREEZE)
+    assert np.array_equal(again.view(np.uint32), want.view(np.uint32))
