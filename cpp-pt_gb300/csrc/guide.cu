@@ -98,17 +98,6 @@ __device__ __forceinline__ void sd_splat(const DevSDTree& T, float rad, f3 p, f3
     atomicAdd(T.dtree_rad + t, rad);
 }
 
-__device__ __forceinline__ int warp_append_ppg(int* counter, bool pred) {
-    const unsigned mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return -1;
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return pred ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
-}
-
 // Backward products and splats of a finished path (ppg.h:131-141): only when
 // the last vertex carries radiance; vertex k receives max-channel of the
 // product of the factors of vertices k..n-1.
@@ -136,8 +125,9 @@ __device__ __forceinline__ void set_vertex_rad(const PPGVerts& V, int slot, int 
     V.vr[i] = r.z;
 }
 
-__global__ void __launch_bounds__(256) k_shade_ppg(DevScene S, PathBuffers B, int cur, RenderParams P,
-                                                   WaveCounters* ctr, unsigned long long* __restrict__ film,
+constexpr int kShadePPGThreads = 256;
+__global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, PathIO in, PathIO nxt,
+                                                   const float4* __restrict__ hit, RenderParams P, WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                    DevSDTree T, PPGVerts V, int* slot_stack) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
@@ -146,9 +136,9 @@ __global__ void __launch_bounds__(256) k_shade_ppg(DevScene S, PathBuffers B, in
     int4 ninfo;
     int slot = -1;
     if (i < n) {
-        const float4 O = B.o[cur][i], D = B.d[cur][i], Tp = B.thr[cur][i];
-        const int4 I = B.info[cur][i];
-        const float4 H = B.hit[i];
+        const float4 O = in.o[i], D = in.d[i], Tp = in.thr[i];
+        const int4 I = in.info[i];
+        const float4 H = hit[i];
         const int prim = __float_as_int(H.y);
         const int pixel = I.x, sample = I.y, bounce = I.z & 0xffff;
         slot = I.w;
@@ -225,45 +215,64 @@ __global__ void __launch_bounds__(256) k_shade_ppg(DevScene S, PathBuffers B, in
             release = true;
         }
     }
-    const int jr = warp_append_ppg(&ctr->free_top, release);
-    if (release) slot_stack[jr] = slot;
-    const int jc = warp_append_ppg(&ctr->n_next, push_cont);
+    // one addition to each queue's counter per CTA (as k_shade)
+    __shared__ int s_count[2][kShadePPGThreads / 32], s_base[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m_free = __ballot_sync(0xffffffffu, release), m_cont = __ballot_sync(0xffffffffu, push_cont);
+    if (lane == 0) {
+        s_count[0][warp] = __popc(m_free);
+        s_count[1][warp] = __popc(m_cont);
+    }
+    __syncthreads();
+    if (lane == 0 && warp < 2) {
+        int total = 0;
+        for (int w = 0; w < kShadePPGThreads / 32; w++) {
+            const int q = s_count[warp][w];
+            s_count[warp][w] = total;
+            total += q;
+        }
+        if (total) s_base[warp] = atomicAdd(warp == 0 ? &ctr->free_top : &ctr->n_next, total);
+    }
+    __syncthreads();
+    const unsigned below = (1u << lane) - 1u;
+    if (release) slot_stack[s_base[0] + s_count[0][warp] + __popc(m_free & below)] = slot;
     if (push_cont) {
-        const int nx = 1 - cur;
-        B.o[nx][jc] = no;
-        B.d[nx][jc] = nd;
-        B.thr[nx][jc] = nt;
-        B.info[nx][jc] = ninfo;
+        const int jc = s_base[1] + s_count[1][warp] + __popc(m_cont & below);
+        nxt.o[jc] = no;
+        nxt.d[jc] = nd;
+        nxt.thr[jc] = nt;
+        nxt.info[jc] = ninfo;
     }
 }
 
 // Camera paths for PPG (ppg.h:174-186: one jittered sample per pixel per
 // pass, no strata), each with a vertex slot from the free list.
-__global__ void __launch_bounds__(256) k_generate_ppg(DevScene S, PathBuffers B, int cur, RenderParams P,
+__global__ void __launch_bounds__(256) k_generate_ppg(DevScene S, PathIO nxt, int capacity, RenderParams P,
                                                       WaveCounters* ctr, const int* slot_stack) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n_next = ctr->n_next;
-    const int avail = min(B.capacity - n_next, ctr->free_top);
-    const unsigned long long w = ctr->work_next + (unsigned long long)t;
-    if (t >= avail || w >= ctr->work_total) return;
-    const unsigned long long npix = (unsigned long long)P.width * P.height;
-    const int sample = (int)(w / npix);
-    const int pixel = (int)(w - (unsigned long long)sample * npix);
-    const int px = pixel % P.width, py = pixel / P.width;
-    const Rng4 r = rng4(P.seed, sample, pixel, 0xffffu, 2);
-    const float cx = (((float)px + r.v[0]) / (float)P.width) * 2.0f - 1.0f;
-    const float cy = -((((float)py + r.v[1]) / (float)P.height) * 2.0f - 1.0f);
-    const DevCamera& C = S.cam;
-    const float dx = cx * C.tan_fovy * C.aspect, dy = cy * C.tan_fovy, dz = -1.0f;
-    const f3 d = normalized(mk(C.m[0] * dx + C.m[1] * dy + C.m[2] * dz, C.m[3] * dx + C.m[4] * dy + C.m[5] * dz,
-                               C.m[6] * dx + C.m[7] * dy + C.m[8] * dz));
-    const int nx = 1 - cur;
-    const int j = n_next + t;
-    const int slot = slot_stack[ctr->free_top - 1 - t];
-    B.o[nx][j] = make_float4(C.o[0], C.o[1], C.o[2], 1.0f);
-    B.d[nx][j] = make_float4(d.x, d.y, d.z, 0.f);
-    B.thr[nx][j] = make_float4(1.f, 1.f, 1.f, 0.f);
-    B.info[nx][j] = make_int4(pixel, sample, 0, slot);
+    const int n_next = ctr->n_next, free_top = ctr->free_top;
+    const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
+    const int avail = min(capacity - n_next, free_top);
+    const int count = left < (unsigned long long)avail ? (int)left : avail;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+        const unsigned long long w = first + (unsigned long long)t;
+        const unsigned long long npix = (unsigned long long)P.width * P.height;
+        const int sample = (int)(w / npix);
+        const int pixel = (int)(w - (unsigned long long)sample * npix);
+        const int px = pixel % P.width, py = pixel / P.width;
+        const Rng4 r = rng4(P.seed, sample, pixel, 0xffffu, 2);
+        const float cx = (((float)px + r.v[0]) / (float)P.width) * 2.0f - 1.0f;
+        const float cy = -((((float)py + r.v[1]) / (float)P.height) * 2.0f - 1.0f);
+        const DevCamera& C = S.cam;
+        const float dx = cx * C.tan_fovy * C.aspect, dy = cy * C.tan_fovy, dz = -1.0f;
+        const f3 d = normalized(mk(C.m[0] * dx + C.m[1] * dy + C.m[2] * dz, C.m[3] * dx + C.m[4] * dy + C.m[5] * dz,
+                                   C.m[6] * dx + C.m[7] * dy + C.m[8] * dz));
+        const int j = n_next + t;
+        const int slot = slot_stack[free_top - 1 - t];
+        nxt.o[j] = make_float4(C.o[0], C.o[1], C.o[2], 1.0f);
+        nxt.d[j] = make_float4(d.x, d.y, d.z, 0.f);
+        nxt.thr[j] = make_float4(1.f, 1.f, 1.f, 0.f);
+        nxt.info[j] = make_int4(pixel, sample, 0, slot);
+    }
 }
 
 __global__ void k_advance_ppg(WaveCounters* ctr, int capacity) {
@@ -295,11 +304,14 @@ void launch_init_slots(int* slot_stack, int n, cudaStream_t st) {
 void launch_shade_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                       unsigned long long* film, const DevSDTree& T, const PPGVerts& V, int* slot_stack,
                       cudaStream_t st) {
-    k_shade_ppg<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, B, cur, P, ctr, film, T, V, slot_stack);
+    k_shade_ppg<<<(B.capacity + kShadePPGThreads - 1) / kShadePPGThreads, kShadePPGThreads, 0, st>>>(
+        S, path_io(B, cur), path_io(B, 1 - cur), B.hit, P, ctr, film, T, V, slot_stack);
 }
 void launch_generate_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
-                         const int* slot_stack, cudaStream_t st) {
-    k_generate_ppg<<<(B.capacity + 255) / 256, 256, 0, st>>>(S, B, cur, P, ctr, slot_stack);
+                         const int* slot_stack, int num_sms, cudaStream_t st) {
+    // a resident grid over the free slots (as the plain wavefront's)
+    k_generate_ppg<<<max(1, min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st>>>(S, path_io(B, 1 - cur), B.capacity,
+                                                                                       P, ctr, slot_stack);
     k_advance_ppg<<<1, 32, 0, st>>>(ctr, B.capacity);
 }
 

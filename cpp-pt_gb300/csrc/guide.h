@@ -34,6 +34,6 @@ void launch_shade_ppg(const DevScene& S, const PathBuffers& B, int cur, const Re
                       unsigned long long* film, const DevSDTree& T, const PPGVerts& V, int* slot_stack,
                       cudaStream_t st);
 void launch_generate_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
-                         const int* slot_stack, cudaStream_t st);
+                         const int* slot_stack, int num_sms, cudaStream_t st);
 
 }  // namespace cpppt_gb300

@@ -311,6 +311,12 @@ constexpr int kTrainCapacity = 1 << 20;
 // guide: 2^20 12.46 ms, 2^21 11.95, 2^22 11.19.
 constexpr int kFrozenCapacity = 1 << 22;
 constexpr int kItersPerGraph = 16;   // of the learned-guide and SD-tree renders between host steps; even: buffers alternate
+// Iterations between two looks at the counters: where all paths start at once
+// they end within `last` iterations (the depth, and one more where shadow rays
+// follow an iteration late), and the rest of sixteen would be empty launches.
+int iterations_per_check(unsigned long long work, int capacity, int last) {
+    return work <= (unsigned long long)capacity ? std::min(kItersPerGraph, (last + 1) & ~1) : kItersPerGraph;
+}
 constexpr int kItersPerBody = 20;    // of a plain render's device-driven loop body; even
 
 // The scene's wavefront buffers for `capacity` paths in flight (192 B per
@@ -375,6 +381,8 @@ void render_ppg(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     const unsigned long long max_pass = (unsigned long long)s->width * s->height * (unsigned long long)passes.back();
     const int capacity =
         ensure_wave(s, (int)std::min<unsigned long long>(1 << 20, (max_pass + 1023) / 1024 * 1024), film_n);
+    PathBuffers pb = s->pb;  // kernels fill at most `capacity` paths of the scene's buffers
+    pb.capacity = capacity;
     std::vector<void*> tmp;  // per-render buffers
     struct Free {
         std::vector<void*>& v;
@@ -430,18 +438,19 @@ void render_ppg(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
         init.film_safe = film_safe_bound((double)passes[l] * (2.0 * D + 2.0));
         *s->h_ctr = init;
         ck(cudaMemcpyAsync(s->d_ctr, s->h_ctr, sizeof(WaveCounters), cudaMemcpyHostToDevice, st), "init counters");
-        launch_generate_ppg(s->dev, s->pb, 1, P, s->d_ctr, slots, st);
+        launch_generate_ppg(s->dev, pb, 1, P, s->d_ctr, slots, s->num_sms, st);
         launches += 4;
         const unsigned long long max_rounds =
             64 + (work / (unsigned long long)capacity + 2) * (unsigned long long)(D + 2) * 4 / kItersPerGraph;
+        const int iters = iterations_per_check(work, capacity, D);
         for (unsigned long long round = 0;; round++) {
-            for (int k = 0; k < kItersPerGraph; k++) {
+            for (int k = 0; k < iters; k++) {
                 const int cur = k & 1;
-                launch_extend(s->dev, s->pb, cur, s->d_ctr, s->num_sms, st);
-                launch_shade_ppg(s->dev, s->pb, cur, P, s->d_ctr, s->film, T, V, slots, st);
-                launch_generate_ppg(s->dev, s->pb, cur, P, s->d_ctr, slots, st);
+                launch_extend(s->dev, pb, cur, s->d_ctr, s->num_sms, st);
+                launch_shade_ppg(s->dev, pb, cur, P, s->d_ctr, s->film, T, V, slots, st);
+                launch_generate_ppg(s->dev, pb, cur, P, s->d_ctr, slots, s->num_sms, st);
             }
-            launches += 4 * kItersPerGraph;
+            launches += 4 * iters;
             ck(cudaMemcpyAsync(s->h_ctr, s->d_ctr, sizeof(WaveCounters), cudaMemcpyDeviceToHost, st), "read counters");
             ck(cudaStreamSynchronize(st), "render");
             check_status(s, s->h_ctr->status);
@@ -766,8 +775,9 @@ void render_nn(pt_scene* s, const pt_render_desc* desc, float* d_dst, bool guide
     int rec_left = -1;  // records kept after the last round's training (-1: that round did not train)
     int n0 = init.n_rec;  // records held when the round started
     NNTrainPending pending;
+    const int iters = iterations_per_check(total, capacity, desc->max_depth + (train ? 0 : 1));
     for (unsigned long long round = 0;; round++) {
-        for (int k = 0; k < kItersPerGraph; k++) {
+        for (int k = 0; k < iters; k++) {
             const int cur = k & 1;
             // without records to collect, nothing waits for a path's shadow ray:
             // it is traced with the next iteration's extension rays
