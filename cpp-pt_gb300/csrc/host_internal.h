@@ -92,6 +92,42 @@ T* dupload(std::vector<void*>& owned, const std::vector<T>& v, cudaStream_t st) 
     return p;
 }
 
+// Device buffers by index, grown on demand and kept until the owner goes.
+struct Workspace {
+    struct Buf {
+        void* p = nullptr;
+        size_t bytes = 0;
+    };
+    std::vector<Buf> bufs;
+    Workspace() = default;
+    Workspace(const Workspace&) = delete;
+    Workspace& operator=(const Workspace&) = delete;
+    ~Workspace() {
+        for (Buf& b : bufs) cudaFree(b.p);
+    }
+    // Buffer i with room for n elements; what it held is lost when it grows
+    // (no work that uses it may be in flight then).
+    template <class T>
+    T* get(size_t i, size_t n) {
+        if (bufs.size() <= i) bufs.resize(i + 1);
+        Buf& b = bufs[i];
+        const size_t bytes = sizeof(T) * std::max<size_t>(1, n);
+        if (b.bytes < bytes) {
+            cudaFree(b.p);
+            b = Buf{};
+            ck(cudaMalloc(&b.p, bytes), "cudaMalloc");
+            b.bytes = bytes;
+        }
+        return static_cast<T*>(b.p);
+    }
+    template <class T>
+    T* upload(size_t i, const std::vector<T>& v, cudaStream_t st) {
+        T* p = get<T>(i, v.size());
+        if (!v.empty()) ck(cudaMemcpyAsync(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, st), "upload");
+        return p;
+    }
+};
+
 inline float fnorm3(float* v) {
     float l = std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
     float inv = 1.0f / l;
@@ -160,6 +196,8 @@ struct pt_scene {
     DevNNJob* h_nnjob = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     pt_render_stats stats{};
+
+    hostimpl::Workspace ppg;  // SD-tree renders: vertex records, slots and the pass's tree
 
     // learned guide
     bool nn_ready = false;
