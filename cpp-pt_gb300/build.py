@@ -55,7 +55,7 @@ def _commands(extra_cuda: list[str] | None = None):
     nvcc = _nvcc()
     common = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off"]
     jobs = []
-    for name in ("render.cu", "guide.cu", "nn.cu", "batch.cu", "gpu_bvh.cu", "gpu_sah.cu", "host.cpp", "batch.cpp", "bvh.cpp", "sdtree.cpp",
+    for name in ("render.cu", "guide.cu", "nn.cu", "batch.cu", "gpu_bvh.cu", "gpu_sah.cu", "gpu_scene.cu", "host.cpp", "batch.cpp", "bvh.cpp", "sdtree.cpp",
                  "image_io.cpp", "loader.cpp"):
         src = os.path.join(CSRC, name)
         out = os.path.join(OBJ, name + ".o")

@@ -578,15 +578,13 @@ __global__ void k_preorder(const NodeG* __restrict__ nodes, int lo, int hi, cons
 }
 
 __global__ void k_node_out(const NodeG* __restrict__ nodes, int n_nodes, const int32_t* __restrict__ pre,
-                           float* __restrict__ box, int32_t* __restrict__ parent) {
+                           float4* __restrict__ box, int32_t* __restrict__ parent) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_nodes) return;
     const NodeG& nd = nodes[i];
     const int p = pre[i];
-    for (int j = 0; j < 3; j++) {
-        box[6 * (size_t)p + j] = nd.lo[j];
-        box[6 * (size_t)p + 3 + j] = nd.hi[j];
-    }
+    box[2 * (size_t)p] = make_float4(nd.lo[0], nd.lo[1], nd.lo[2], 0.f);
+    box[2 * (size_t)p + 1] = make_float4(nd.hi[0], nd.hi[1], nd.hi[2], 0.f);
     parent[p] = nd.parent >= 0 ? pre[nd.parent] : -1;
 }
 
@@ -618,24 +616,15 @@ T* dmalloc(std::vector<void*>& owned, size_t n) {
 
 }  // namespace
 
-RefTopology build_ref_topology_device(const float* tri_v, int n, cudaStream_t st, RefBuildStats* stats) {
-    RefTopology t;
-    t.rank.assign(n, 0);
-    t.prim_parent.assign(n, -1);
-    if (n <= 0) return t;
-    std::vector<void*> owned;
-    struct Free {
-        std::vector<void*>& v;
-        ~Free() { for (void* p : v) cudaFree(p); }
-    } guard{owned};
+RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& scratch, DeviceBufs& keep,
+                       RefBuildStats* stats) {
+    std::vector<void*>& owned = scratch.v;
     int* h_cnt = nullptr;  // pinned: LevelOut::counts
     ck(cudaMallocHost(&h_cnt, 4 * sizeof(int)), "cudaMallocHost");
     struct FreeHost {
         int* p;
         ~FreeHost() { cudaFreeHost(p); }
     } hguard{h_cnt};
-    float* d_tv = dmalloc<float>(owned, 9 * (size_t)n);
-    ck(cudaMemcpyAsync(d_tv, tri_v, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice, st), "upload");
     PrimG* buf[2] = {dmalloc<PrimG>(owned, n), dmalloc<PrimG>(owned, n)};
     // a split leaves at least one primitive on each side, so there are fewer
     // internal nodes than primitives, and at most n segments on a level
@@ -692,34 +681,46 @@ RefTopology build_ref_topology_device(const float* tri_v, int n, cudaStream_t st
         const int lo = level_nodes[L], hi = level_nodes[L + 1];
         if (hi > lo) k_preorder<<<(hi - lo + 255) / 256, 256, 0, st>>>(nodes, lo, hi, size, pre);
     }
-    float* d_box = dmalloc<float>(owned, 6 * (size_t)n_nodes);
+    float4* d_box = dmalloc<float4>(keep.v, 2 * (size_t)n_nodes);
     int32_t* d_parent = dmalloc<int32_t>(owned, n_nodes);
     int32_t* d_rank = dmalloc<int32_t>(owned, n);
     int32_t* d_pp = dmalloc<int32_t>(owned, n);
     if (n_nodes > 0) k_node_out<<<(n_nodes + 255) / 256, 256, 0, st>>>(nodes, n_nodes, pre, d_box, d_parent);
     k_prim_out<<<(n + 255) / 256, 256, 0, st>>>(final_id, leaf_parent, n, pre, d_rank, d_pp);
     ck(cudaGetLastError(), "outputs");
-    t.leaf_order.resize(n);
-    t.node_box.resize(n_nodes);
-    t.node_parent.resize(n_nodes);
-    std::vector<float> hbox(6 * (size_t)n_nodes);
-    ck(cudaMemcpyAsync(t.leaf_order.data(), final_id, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st), "copy");
-    ck(cudaMemcpyAsync(t.rank.data(), d_rank, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st), "copy");
-    ck(cudaMemcpyAsync(t.prim_parent.data(), d_pp, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st), "copy");
-    if (n_nodes > 0) {
-        ck(cudaMemcpyAsync(hbox.data(), d_box, sizeof(float) * hbox.size(), cudaMemcpyDeviceToHost, st), "copy");
-        ck(cudaMemcpyAsync(t.node_parent.data(), d_parent, sizeof(int32_t) * n_nodes, cudaMemcpyDeviceToHost, st),
-           "copy");
-    }
     ck(cudaStreamSynchronize(st), "outputs");
-    for (int i = 0; i < n_nodes; i++)
-        for (int j = 0; j < 3; j++) {
-            t.node_box[i].lo[j] = hbox[6 * (size_t)i + j];
-            t.node_box[i].hi[j] = hbox[6 * (size_t)i + 3 + j];
-        }
     if (stats) {
         stats->levels = levels;
         stats->nodes = n_nodes;
+    }
+    return RefTree{final_id, d_rank, d_pp, d_parent, d_box, n_nodes};
+}
+
+RefTopology build_ref_topology_device(const float* tri_v, int n, cudaStream_t st, RefBuildStats* stats) {
+    RefTopology t;
+    t.rank.assign(n, 0);
+    t.prim_parent.assign(n, -1);
+    if (n <= 0) return t;
+    DeviceBufs scratch;
+    float* d_tv = dmalloc<float>(scratch.v, 9 * (size_t)n);
+    ck(cudaMemcpyAsync(d_tv, tri_v, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice, st), "upload");
+    const RefTree d = build_ref_tree(d_tv, n, st, scratch, scratch, stats);
+    t.leaf_order.resize(n);
+    t.node_box.resize(d.n_nodes);
+    t.node_parent.resize(d.n_nodes);
+    std::vector<float4> box(2 * (size_t)d.n_nodes);
+    auto copy = [&](void* dst, const void* src, size_t bytes) {
+        if (bytes) ck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st), "copy");
+    };
+    copy(t.leaf_order.data(), d.leaf_order, sizeof(int32_t) * n);
+    copy(t.rank.data(), d.rank, sizeof(int32_t) * n);
+    copy(t.prim_parent.data(), d.prim_parent, sizeof(int32_t) * n);
+    copy(box.data(), d.node_box, sizeof(float4) * box.size());
+    copy(t.node_parent.data(), d.node_parent, sizeof(int32_t) * d.n_nodes);
+    ck(cudaStreamSynchronize(st), "copies");
+    for (int i = 0; i < d.n_nodes; i++) {
+        std::memcpy(t.node_box[i].lo, &box[2 * (size_t)i], 12);
+        std::memcpy(t.node_box[i].hi, &box[2 * (size_t)i + 1], 12);
     }
     return t;
 }

@@ -973,14 +973,9 @@ int grid_for(int n, int threads) { return std::max(1, std::min((n + threads - 1)
 
 }  // namespace
 
-WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStream_t st, WideBuildStats* stats) {
-    if (max_leaf < 1 || max_leaf > 16) throw std::invalid_argument("max_leaf must be in [1,16]");
-    if (n <= 0) return build_wide_bvh(tri_v, n, max_leaf, 1);
-    std::vector<void*> owned;
-    struct Free {
-        std::vector<void*>& v;
-        ~Free() { for (void* p : v) cudaFree(p); }
-    } guard{owned};
+WideTree build_wide_tree(const float* d_tv, int n, int max_leaf, cudaStream_t st, DeviceBufs& scratch,
+                         DeviceBufs& keep, WideBuildStats* stats) {
+    std::vector<void*>& owned = scratch.v;
     int32_t* h = nullptr;  // pinned counters
     ck(cudaMallocHost(&h, 8 * sizeof(int32_t)), "cudaMallocHost");
     struct FreeHost {
@@ -991,7 +986,6 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
     const int max_big = n / kSmallSeg + 2;
     const int max_small = n / kTinySeg + 16;  // they hold more than kTinySeg primitives each, and share none
     const int max_chunks = n / kChunk + max_big + 2;
-    float* d_tv = dmalloc<float>(owned, 9 * (size_t)n);
     float4* plo = dmalloc<float4>(owned, n);
     float4* phi = dmalloc<float4>(owned, n);
     float* pcz = dmalloc<float>(owned, n);
@@ -1009,7 +1003,6 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
     Tiny* tiny = dmalloc<Tiny>(owned, n);
     int32_t* counts = dmalloc<int32_t>(owned, 5);  // LevelOut::counts
 
-    ck(cudaMemcpyAsync(d_tv, tri_v, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice, st), "upload");
     ck(cudaMemsetAsync(key6, 0, 6 * sizeof(uint32_t), st), "memset");
     // the root: node 0, bounds reduced by k_prims
     Seg root{};
@@ -1106,14 +1099,9 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
         qc = 1 - qc;
         if (base + nq > n_node2) throw std::runtime_error("device SAH build: collapse overflow");
     }
-    WideBVH out;
-    out.max_leaf = max_leaf;
-    out.max_depth = depth;
-    out.nodes.resize(base);
-    out.tri_order.resize(n);
-    ck(cudaMemcpyAsync(out.nodes.data(), wide, sizeof(WideNode) * (size_t)base, cudaMemcpyDeviceToHost, st), "nodes");
-    ck(cudaMemcpyAsync(out.tri_order.data(), out_order, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st), "order");
-    ck(cudaMemcpyAsync(&out.inflate, d_delta, sizeof(float), cudaMemcpyDeviceToHost, st), "delta");
+    // the binary tree bounds the buffer; the result keeps its own size
+    uint4* d_nodes = dmalloc<uint4>(keep.v, 4 * (size_t)base);
+    ck(cudaMemcpyAsync(d_nodes, wide, sizeof(WideNode) * (size_t)base, cudaMemcpyDeviceToDevice, st), "nodes");
     ck(cudaStreamSynchronize(st), "outputs");
     if (stats) {
         stats->top_levels = top_levels;
@@ -1121,6 +1109,26 @@ WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStrea
         stats->binary_nodes = n_node2;
         stats->wide_levels = depth;
     }
+    return WideTree{d_nodes, out_order, d_delta, base, depth};
+}
+
+WideBVH build_wide_bvh_device(const float* tri_v, int n, int max_leaf, cudaStream_t st, WideBuildStats* stats) {
+    if (max_leaf < 1 || max_leaf > 16) throw std::invalid_argument("max_leaf must be in [1,16]");
+    if (n <= 0) return build_wide_bvh(tri_v, n, max_leaf, 1);
+    DeviceBufs scratch;
+    float* d_tv = dmalloc<float>(scratch.v, 9 * (size_t)n);
+    ck(cudaMemcpyAsync(d_tv, tri_v, sizeof(float) * 9 * (size_t)n, cudaMemcpyHostToDevice, st), "upload");
+    const WideTree d = build_wide_tree(d_tv, n, max_leaf, st, scratch, scratch, stats);
+    WideBVH out;
+    out.max_leaf = max_leaf;
+    out.max_depth = d.max_depth;
+    out.nodes.resize(d.n_nodes);
+    out.tri_order.resize(n);
+    ck(cudaMemcpyAsync(out.nodes.data(), d.nodes, sizeof(WideNode) * (size_t)d.n_nodes, cudaMemcpyDeviceToHost, st),
+       "nodes");
+    ck(cudaMemcpyAsync(out.tri_order.data(), d.tri_order, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st), "order");
+    ck(cudaMemcpyAsync(&out.inflate, d.inflate, sizeof(float), cudaMemcpyDeviceToHost, st), "delta");
+    ck(cudaStreamSynchronize(st), "copies");
     return out;
 }
 

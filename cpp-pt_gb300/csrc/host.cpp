@@ -8,8 +8,10 @@
 #include "image_io.h"
 #include "loader.h"
 
-#include <thread>
+#include <initializer_list>
 #include <iterator>
+#include <thread>
+#include <type_traits>
 
 using namespace cpppt_gb300;
 using namespace cpppt_gb300::hostimpl;
@@ -53,96 +55,87 @@ void create_scene(const pt_scene_desc* d, pt_scene* s, const SceneTextures* tx =
     s->width = d->camera.width;
     s->height = d->camera.height;
 
-    // per-triangle vertex positions (a, b, c)
-    std::vector<float> tv(9 * (size_t)nt);
-    for (int t = 0; t < nt; t++)
-        for (int k = 0; k < 3; k++)
-            std::memcpy(&tv[9 * (size_t)t + 3 * k], d->vertices + 3 * (size_t)d->triangles[3 * t + k], 12);
+    // the caller's arrays; the scene's are made of them on the device
+    DeviceBufs scratch, wide_scratch, keep, wide_keep;
+    auto upload = [&](const auto* src, size_t count) {
+        auto* p = dalloc<std::remove_cv_t<std::remove_pointer_t<decltype(src)>>>(scratch.v, count);
+        if (count) ck(cudaMemcpyAsync(p, src, sizeof(*src) * count, cudaMemcpyHostToDevice, s->stream), "upload");
+        return p;
+    };
+    DevScene& S = s->dev;
+    const float* d_verts = upload(d->vertices, 3 * (size_t)nv);
+    const int32_t* d_tri = upload(d->triangles, 3 * (size_t)nt);
+    const int32_t* d_mat = upload(d->tri_material, nt);
+    float* tv = dalloc<float>(scratch.v, 9 * (size_t)nt);  // per-triangle vertex positions (a, b, c)
+    uint32_t* d_key = dalloc<uint32_t>(scratch.v, 6);
+    int4* vidx = dalloc<int4>(s->owned, nt);
+    ck(cudaMemsetAsync(d_key, 0, 6 * sizeof(uint32_t), s->stream), "memset");
+    launch_triangle_positions(d_verts, d_tri, d_mat, nt, tv, vidx, d_key, s->num_sms, s->stream);
+    uint32_t key[6];
+    ck(cudaMemcpyAsync(key, d_key, sizeof(key), cudaMemcpyDeviceToHost, s->stream), "bounds");
+    ck(cudaStreamSynchronize(s->stream), "triangle positions");
+    triangle_bounds(key, s->bounds_lo, s->bounds_hi);
 
     // the two device builds are independent: the 4-wide SAH tree from a
     // second host thread on a stream of its own
     auto t0 = std::chrono::steady_clock::now();
-    WideBVH wide;
+    WideTree wide;
     std::exception_ptr wide_err;
-    std::chrono::steady_clock::time_point t2;
+    std::chrono::steady_clock::time_point t2 = t0;
     const int dev = s->device;
     std::thread wide_th([&] {
         cudaStream_t ws = nullptr;
         try {
-            ck(cudaSetDevice(dev), "cudaSetDevice");
-            ck(cudaStreamCreateWithFlags(&ws, cudaStreamNonBlocking), "cudaStreamCreate");
-            wide = build_wide_bvh_device(tv.data(), nt, 4, ws);
+            if (nt > 0) {
+                ck(cudaSetDevice(dev), "cudaSetDevice");
+                ck(cudaStreamCreateWithFlags(&ws, cudaStreamNonBlocking), "cudaStreamCreate");
+                wide = build_wide_tree(tv, nt, 4, ws, wide_scratch, wide_keep);
+            }
         } catch (...) {
             wide_err = std::current_exception();
         }
         if (ws) cudaStreamDestroy(ws);
         t2 = std::chrono::steady_clock::now();
     });
-    RefTopology ref;
+    RefTree ref;
+    std::chrono::steady_clock::time_point t1;
+    float4 *vpos, *vnrm, *vbt;
     try {
-        ref = build_ref_topology_device(tv.data(), nt, s->stream);
+        if (nt > 0) ref = build_ref_tree(tv, nt, s->stream, scratch, keep);
+        t1 = std::chrono::steady_clock::now();
+        const float* d_nrm = upload(d->normals, 3 * (size_t)nv);
+        const float* d_tan = d->tangents ? upload(d->tangents, 3 * (size_t)nv) : nullptr;
+        vpos = dalloc<float4>(s->owned, nv);
+        vnrm = dalloc<float4>(s->owned, nv);
+        vbt = dalloc<float4>(s->owned, nv);
+        launch_vertices(d_verts, d_nrm, d_tan, nv, vpos, vnrm, vbt, s->stream);
     } catch (...) {
         wide_th.join();
         throw;
     }
-    auto t1 = std::chrono::steady_clock::now();
     wide_th.join();
     if (wide_err) std::rethrow_exception(wide_err);
     s->build_ref_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
     s->build_wide_ms = std::chrono::duration<double, std::milli>(t2 - t0).count();
+    if (nt == 0) {  // an empty root
+        const WideBVH w = build_wide_bvh(nullptr, 0, 4, 1);
+        wide.n_nodes = (int)w.nodes.size();
+        wide.max_depth = w.max_depth;
+        wide.nodes = dalloc<uint4>(wide_keep.v, 4 * w.nodes.size());
+        ck(cudaMemcpyAsync(wide.nodes, w.nodes.data(), sizeof(WideNode) * w.nodes.size(), cudaMemcpyHostToDevice,
+                           s->stream), "upload");
+        ck(cudaStreamSynchronize(s->stream), "upload");
+        ref.node_box = dalloc<float4>(keep.v, 0);
+    }
     s->wide_depth = wide.max_depth;
-    for (int k = 0; k < 3; k++) { s->bounds_lo[k] = INFINITY; s->bounds_hi[k] = -INFINITY; }
-    for (size_t i = 0; i < tv.size(); i += 3)
-        for (int k = 0; k < 3; k++) {
-            s->bounds_lo[k] = std::min(s->bounds_lo[k], tv[i + k]);
-            s->bounds_hi[k] = std::max(s->bounds_hi[k], tv[i + k]);
-        }
     if (3 * wide.max_depth + 4 > 64) throw Fail(PT_ERR_LIMIT, "wide BVH too deep for the traversal stack");
-
-    // traversal triangles in leaf order: {a, rank}, {b - a, parent}, {c - a, prim}
-    std::vector<float4> tris(3 * (size_t)nt);
-    for (int k = 0; k < nt; k++) {
-        const int p = wide.tri_order[k];
-        const float* v = &tv[9 * (size_t)p];
-        float a[3] = {v[0], v[1], v[2]};
-        float e1[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};  // triangle.h:40 (b - a)
-        float e2[3] = {v[6] - v[0], v[7] - v[1], v[8] - v[2]};  // triangle.h:41 (c - a)
-        int32_t rank = ref.rank[p], parent = ref.prim_parent[p];
-        float rf, pf, idf;
-        std::memcpy(&rf, &rank, 4);
-        std::memcpy(&pf, &parent, 4);
-        std::memcpy(&idf, &p, 4);
-        tris[3 * (size_t)k] = make_float4(a[0], a[1], a[2], rf);
-        tris[3 * (size_t)k + 1] = make_float4(e1[0], e1[1], e1[2], pf);
-        tris[3 * (size_t)k + 2] = make_float4(e2[0], e2[1], e2[2], idf);
-    }
-    std::vector<float4> rbox(2 * ref.node_box.size());
-    for (size_t i = 0; i < ref.node_box.size(); i++) {
-        const Box3& b = ref.node_box[i];
-        rbox[2 * i] = make_float4(b.lo[0], b.lo[1], b.lo[2], 0.f);
-        rbox[2 * i + 1] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.f);
-    }
-    // shading data
-    std::vector<int4> vidx(nt);
-    for (int t = 0; t < nt; t++)
-        vidx[t] = make_int4(d->triangles[3 * t], d->triangles[3 * t + 1], d->triangles[3 * t + 2], d->tri_material[t]);
-    std::vector<float4> vpos(nv), vnrm(nv), vbt(nv);
-    for (int v = 0; v < nv; v++) {
-        const float* p = d->vertices + 3 * (size_t)v;
-        const float* n = d->normals + 3 * (size_t)v;
-        float tg[3];
-        if (d->tangents) {
-            std::memcpy(tg, d->tangents + 3 * (size_t)v, 12);
-        } else {  // any vector perpendicular to the normal
-            float ax[3] = {std::fabs(n[1]) < 0.9f ? 0.f : 1.f, std::fabs(n[1]) < 0.9f ? 1.f : 0.f, 0.f};
-            fcross(ax, n, tg);
-            fnorm3(tg);
-        }
-        float bt[3];
-        fcross(n, tg, bt);  // loader.h:237
-        vpos[v] = make_float4(p[0], p[1], p[2], 0.f);
-        vnrm[v] = make_float4(n[0], n[1], n[2], 0.f);
-        vbt[v] = make_float4(bt[0], bt[1], bt[2], 0.f);
+    float4* tris = dalloc<float4>(s->owned, 3 * (size_t)nt);
+    launch_leaf_triangles(tv, wide.tri_order, ref.rank, ref.prim_parent, nt, tris, s->stream);
+    ck(cudaGetLastError(), "scene arrays");
+    // the trees' results belong to the scene
+    for (DeviceBufs* b : {&keep, &wide_keep}) {
+        s->owned.insert(s->owned.end(), b->v.begin(), b->v.end());
+        b->v.clear();
     }
     std::vector<DevMaterial> mats(nm);
     for (int i = 0; i < nm; i++) {
@@ -167,37 +160,42 @@ void create_scene(const pt_scene_desc* d, pt_scene* s, const SceneTextures* tx =
     for (int t = 0; t < nt; t++) {
         if (d->materials[d->tri_material[t]].kind != PT_MAT_EMISSIVE) continue;
         lprim.push_back(t);
-        const float* v = &tv[9 * (size_t)t];
-        float e1[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]}, e2[3] = {v[6] - v[0], v[7] - v[1], v[8] - v[2]}, c[3];
+        const float* v[3];
+        for (int k = 0; k < 3; k++) v[k] = d->vertices + 3 * (size_t)d->triangles[3 * t + k];
+        float e1[3], e2[3], c[3];
+        for (int a = 0; a < 3; a++) {
+            e1[a] = v[1][a] - v[0][a];
+            e2[a] = v[2][a] - v[0][a];
+        }
         fcross(e1, e2, c);
         larea.push_back(std::sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]) * 0.5f);
     }
-    std::vector<uint4> nodes(4 * wide.nodes.size());
-    std::memcpy(nodes.data(), wide.nodes.data(), sizeof(WideNode) * wide.nodes.size());
 
     s->n_verts = nv;
     s->n_mats = nm;
-    s->n_rbox = (int)ref.node_box.size();
-    DevScene& S = s->dev;
-    S.nodes = dupload(s->owned, nodes, s->stream);
-    S.n_nodes = (int)wide.nodes.size();
+    s->n_rbox = ref.n_nodes;
+    S.nodes = wide.nodes;
+    S.n_nodes = wide.n_nodes;
     S.n_tris = nt;
-    S.tris = dupload(s->owned, tris, s->stream);
-    S.ref_box = dupload(s->owned, rbox, s->stream);
-    S.tri_vidx = dupload(s->owned, vidx, s->stream);
-    S.v_pos = dupload(s->owned, vpos, s->stream);
-    S.v_nrm = dupload(s->owned, vnrm, s->stream);
-    S.v_btan = dupload(s->owned, vbt, s->stream);
+    S.tris = tris;
+    S.ref_box = ref.node_box;
+    S.tri_vidx = vidx;
+    S.v_pos = vpos;
+    S.v_nrm = vnrm;
+    S.v_btan = vbt;
     S.mats = dupload(s->owned, mats, s->stream);
     s->h_mats = mats;
     S.light_prim = dupload(s->owned, lprim, s->stream);
     S.light_area = dupload(s->owned, larea, s->stream);
     S.n_lights = (int)lprim.size();
     // image textures and uv (zero uv and an empty texture table without them)
-    std::vector<float2> uv(std::max(1, nv), make_float2(0.f, 0.f));
-    if (tx && tx->uv.size() >= 2 * (size_t)nv)
-        for (int v = 0; v < nv; v++) uv[v] = make_float2(tx->uv[2 * (size_t)v], tx->uv[2 * (size_t)v + 1]);
-    S.v_uv = dupload(s->owned, uv, s->stream);
+    const size_t n_uv = std::max(1, nv);
+    float2* uv = dalloc<float2>(s->owned, n_uv);
+    if (nv > 0 && tx && tx->uv.size() >= 2 * (size_t)nv)
+        ck(cudaMemcpyAsync(uv, tx->uv.data(), sizeof(float2) * n_uv, cudaMemcpyHostToDevice, s->stream), "upload");
+    else
+        ck(cudaMemsetAsync(uv, 0, sizeof(float2) * n_uv, s->stream), "memset");
+    S.v_uv = uv;
     std::vector<float> px = (tx && !tx->px.empty()) ? tx->px : std::vector<float>(1, 0.f);
     std::vector<int4> info = (tx && !tx->info.empty()) ? tx->info : std::vector<int4>(1, make_int4(0, 1, 1, 1));
     S.tex_px = dupload(s->owned, px, s->stream);

@@ -135,3 +135,59 @@ def test_device_wide_tree_full_size(gpu_lib, make):
     for _ in range(4):
         again = lib.wide_bvh(sc, on_device=True)[0]
         assert np.array_equal(again, nodes)
+
+
+@pytest.mark.parametrize("n", [0, 1, 4, 5, 32, 33, 255, 256, 257, 3001])
+def test_scene_arrays_at_block_edges(gpu_lib, n):
+    """The scene's arrays, assembled on the device: hits of the first n
+    triangles of a soup equal the oracle's bit for bit, and light areas and
+    materials follow (a render of the same triangles is finite and, without
+    triangles, black)."""
+    from dataclasses import replace
+
+    from cpppt.lib import GpuScene
+    from oracle.oracle import Oracle
+    full = scenes.soup(seed=5, n_spheres=60, freq=3, width=24, height=16)
+    tris = np.random.default_rng(1).permutation(full.triangles)[:n]
+    half = n // 2
+    sc = replace(full, triangles=np.ascontiguousarray(tris), mesh_tri_offset=np.array([0, half, n], np.int32),
+                 mesh_material=np.array([0, len(full.mat_kind) - 1], np.int32),
+                 mesh_vert_offset=np.array([0, 0, len(full.vertices)], np.int32))
+    rays = scenes.hit_ray_batch(full, 4096, seed=3)
+    gs = GpuScene(sc)
+    gi, gt, _, _ = gs.trace_closest(rays)
+    img = gs.render(2, 4)
+    assert np.isfinite(img).all()
+    if n == 0:
+        assert (gi < 0).all() and (img == 0).all()
+        return
+    oi, ot = Oracle("port").scene(sc).trace_closest(rays)
+    assert np.array_equal(gi, oi)
+    assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
+
+
+def test_scene_without_tangents_uses_perpendicular(gpu_lib, monkeypatch):
+    """A description without tangents renders as one with the unit vector
+    perpendicular to each normal, computed here in 32 bits operation by
+    operation: the same image bit for bit."""
+    from dataclasses import replace
+
+    from cpppt import lib
+    sc = scenes.slit_room(n_boxes=12, width=48, height=32)
+    f = np.float32
+    n = sc.normals.astype(f)
+    x = np.abs(n[:, 1]) < f(0.9)
+    a = np.stack([np.where(x, 0, 1), np.where(x, 1, 0), np.zeros(len(n))], 1).astype(f)
+    t = np.stack([a[:, 1] * n[:, 2] - a[:, 2] * n[:, 1], a[:, 2] * n[:, 0] - a[:, 0] * n[:, 2],
+                  a[:, 0] * n[:, 1] - a[:, 1] * n[:, 0]], 1)
+    inv = f(1) / np.sqrt((t[:, 0] * t[:, 0] + t[:, 1] * t[:, 1]) + t[:, 2] * t[:, 2])
+    given = lib.GpuScene(replace(sc, tangents=t * inv[:, None])).render(8, 6)
+
+    class NoTangents(lib.PtSceneDesc):
+        def __setattr__(self, name, value):
+            super().__setattr__(name, None if name == "tangents" else value)
+
+    monkeypatch.setattr(lib, "PtSceneDesc", NoTangents)
+    none = lib.GpuScene(sc).render(8, 6)
+    assert given.max() > 0
+    assert np.array_equal(given.view(np.uint32), none.view(np.uint32))
