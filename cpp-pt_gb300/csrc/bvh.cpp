@@ -402,50 +402,16 @@ uint32_t fbits(float f) {
     return u;
 }
 
-}  // namespace
-
-WideBVH build_wide_bvh(const float* tri_v, int n, int max_leaf, int n_threads) {
-    if (max_leaf < 1 || max_leaf > 16) throw std::invalid_argument("max_leaf must be in [1,16]");
-    WideBVH out;
-    out.max_leaf = max_leaf;
-    std::vector<AB> box(n > 0 ? n : 1);
-    std::vector<V3> cen(n > 0 ? n : 1);
-    AB scene;
-    for (int i = 0; i < n; i++) {
-        tri_box(tri_v + 9 * (size_t)i, &box[i]);
-        scene.unite(box[i]);
-    }
-    // Boxes are inflated by delta, far above the rounding error of the
-    // device slab test for rays starting inside or near the scene.
-    float ext = 0.0f, mag = 0.0f;
-    if (n > 0) {
-        for (int k = 0; k < 3; k++) {
-            ext = std::max(ext, scene.hi[k] - scene.lo[k]);
-            mag = std::max(mag, std::max(std::fabs(scene.hi[k]), std::fabs(scene.lo[k])));
-        }
-    }
-    float delta = (ext + mag + 1e-3f) * (1.0f / 262144.0f);
-    out.inflate = delta;
-    for (int i = 0; i < n; i++) {
-        box[i].lo = {box[i].lo.x - delta, box[i].lo.y - delta, box[i].lo.z - delta};
-        box[i].hi = {box[i].hi.x + delta, box[i].hi.y + delta, box[i].hi.z + delta};
-        cen[i] = {0.5f * (box[i].lo.x + box[i].hi.x), 0.5f * (box[i].lo.y + box[i].hi.y),
-                  0.5f * (box[i].lo.z + box[i].hi.z)};
-    }
-    out.tri_order.resize(n);
-    for (int i = 0; i < n; i++) out.tri_order[i] = i;
-
-    std::vector<Node2> nodes(n > 0 ? 2 * (size_t)n : 1);
-    std::atomic<int32_t> next{1};
-    if (n_threads <= 0) n_threads = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    SahBuilder sb{box, cen, nodes, next, out.tri_order.data(), max_leaf};
-    if (n > 0) sb.build(0, 0, n, 0, n_threads);
-    else { nodes[0].count = 0; }
-
-    // Collapse into 4-wide nodes, breadth first.
+// Wide nodes of the binary tree, breadth first, by the choices of the cheapest
+// collapse or (null) opening the child of largest area first.
+void emit_wide(const std::vector<Node2>& nodes, const std::vector<uint32_t>* choice, int n, WideBVH& out) {
+    auto left = [&](int32_t i) { return nodes[i].left; };
+    auto right = [&](int32_t i) { return nodes[i].right; };
     struct Item { int32_t n2; int depth; };
     std::vector<Item> queue;
     queue.push_back({0, 1});
+    out.nodes.clear();
+    out.max_depth = 0;
     out.nodes.reserve(n / 2 + 1);
     for (size_t qi = 0; qi < queue.size(); qi++) {
         int32_t n2 = queue[qi].n2;
@@ -456,22 +422,10 @@ WideBVH build_wide_bvh(const float* tri_v, int n, int max_leaf, int n_threads) {
         int nc = 0;
         if (nodes[n2].left < 0) {
             ch[nc++] = n2;  // a root that is a leaf
+        } else if (choice) {
+            nc = collapse_children(n2, left, right, [&](int32_t i) { return (*choice)[i]; }, ch);
         } else {
-            ch[nc++] = nodes[n2].left;
-            ch[nc++] = nodes[n2].right;
-            while (nc < 4) {
-                int pick = -1;
-                float best = -1.0f;
-                for (int i = 0; i < nc; i++)
-                    if (nodes[ch[i]].left >= 0 && nodes[ch[i]].box.sah_area() > best) {
-                        best = nodes[ch[i]].box.sah_area();
-                        pick = i;
-                    }
-                if (pick < 0) break;
-                int32_t c = ch[pick];
-                ch[pick] = nodes[c].left;
-                ch[nc++] = nodes[c].right;
-            }
+            nc = collapse_largest(n2, left, right, [&](int32_t i) { return nodes[i].box.sah_area(); }, ch);
         }
         WideNode wn;
         std::memset(&wn, 0, sizeof(wn));
@@ -529,6 +483,67 @@ WideBVH build_wide_bvh(const float* tri_v, int n, int max_leaf, int n_threads) {
         for (int i = 0; i < 4; i++) wn.w[10 + i] = refs[i];
         out.nodes.push_back(wn);
     }
+}
+
+}  // namespace
+
+WideBVH build_wide_bvh(const float* tri_v, int n, int max_leaf, int n_threads) {
+    if (max_leaf < 1 || max_leaf > 16) throw std::invalid_argument("max_leaf must be in [1,16]");
+    WideBVH out;
+    out.max_leaf = max_leaf;
+    std::vector<AB> box(n > 0 ? n : 1);
+    std::vector<V3> cen(n > 0 ? n : 1);
+    AB scene;
+    for (int i = 0; i < n; i++) {
+        tri_box(tri_v + 9 * (size_t)i, &box[i]);
+        scene.unite(box[i]);
+    }
+    // Boxes are inflated by delta, far above the rounding error of the
+    // device slab test for rays starting inside or near the scene.
+    float ext = 0.0f, mag = 0.0f;
+    if (n > 0) {
+        for (int k = 0; k < 3; k++) {
+            ext = std::max(ext, scene.hi[k] - scene.lo[k]);
+            mag = std::max(mag, std::max(std::fabs(scene.hi[k]), std::fabs(scene.lo[k])));
+        }
+    }
+    float delta = (ext + mag + 1e-3f) * (1.0f / 262144.0f);
+    out.inflate = delta;
+    for (int i = 0; i < n; i++) {
+        box[i].lo = {box[i].lo.x - delta, box[i].lo.y - delta, box[i].lo.z - delta};
+        box[i].hi = {box[i].hi.x + delta, box[i].hi.y + delta, box[i].hi.z + delta};
+        cen[i] = {0.5f * (box[i].lo.x + box[i].hi.x), 0.5f * (box[i].lo.y + box[i].hi.y),
+                  0.5f * (box[i].lo.z + box[i].hi.z)};
+    }
+    out.tri_order.resize(n);
+    for (int i = 0; i < n; i++) out.tri_order[i] = i;
+
+    std::vector<Node2> nodes(n > 0 ? 2 * (size_t)n : 1);
+    std::atomic<int32_t> next{1};
+    if (n_threads <= 0) n_threads = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    SahBuilder sb{box, cen, nodes, next, out.tri_order.data(), max_leaf};
+    if (n > 0) sb.build(0, 0, n, 0, n_threads);
+    else { nodes[0].count = 0; }
+
+    // the cheapest collapse, and the depth of the one that opens the largest child first
+    const int32_t n_nodes = next.load();
+    std::vector<float> cost(3 * (size_t)n_nodes, 0.0f);
+    std::vector<uint32_t> record(n_nodes, 0);
+    for (int32_t i = n_nodes - 1; i >= 0; i--) {  // children come after their parent
+        if (nodes[i].left < 0) continue;
+        int32_t ch[4];
+        const int nc = collapse_largest(
+            i, [&](int32_t k) { return nodes[k].left; }, [&](int32_t k) { return nodes[k].right; },
+            [&](int32_t k) { return nodes[k].box.sah_area(); }, ch);
+        uint32_t depth = 0;
+        for (int k = 0; k < nc; k++) depth = std::max(depth, record[ch[k]] >> kDepthShift);
+        record[i] = collapse_cost(nodes[i].box.sah_area(), &cost[3 * (size_t)nodes[i].left],
+                                  &cost[3 * (size_t)nodes[i].right], &cost[3 * (size_t)i]) |
+                    (depth + 1) << kDepthShift;
+    }
+    const bool deep = record[0] >> kDepthShift > (uint32_t)kMaxWideDepth;
+    emit_wide(nodes, deep ? nullptr : &record, n, out);
+    if (!deep && out.max_depth > kMaxWideDepth) emit_wide(nodes, nullptr, n, out);
     return out;
 }
 

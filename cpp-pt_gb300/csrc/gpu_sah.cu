@@ -26,9 +26,9 @@
 //     23 ms of the 192k-triangle room's 36 ms scene creation and 29 ms of a
 //     10k-triangle scene's 32 ms; now 0.5 ms of either.
 //   collapse    breadth-first, one launch set per 4-wide level: each entry
-//     gathers its up-to-4 children (the child of largest SAH area opened
-//     first, as the host does), an exclusive scan gives the next level's
-//     queue positions, and each entry quantises its children's boxes in
+//     gathers its up-to-4 children (collapse_children, by the choices that
+//     k_collapse_cost made bottom-up), an exclusive scan gives the next
+//     level's queue positions, and each entry quantises its children's boxes in
 //     double precision like the host (k_collapse, k_scan, k_emit).
 //
 // Bins hold, per axis and bin, the primitive count, the union of the boxes
@@ -806,31 +806,61 @@ __global__ void __launch_bounds__(32 * kTinyWarps) k_tiny(const Tiny* __restrict
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float node_area(const Node2& n) { return sah_area(n.lo, n.hi); }
 
+// parent[i] of every node but the root.
+__global__ void k_parents(const Node2* __restrict__ nodes, int n, int32_t* __restrict__ parent) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) parent[0] = -1;
+    if (i >= n || nodes[i].left < 0) return;
+    parent[nodes[i].left] = i;
+    parent[nodes[i].right] = i;
+}
+
+// Costs of the cheapest collapse, its choices, and the depth of the largest-
+// first one (a record is {cost[3], choices | depth << kDepthShift}, zero for a
+// leaf), bottom-up: a thread starts at each leaf and climbs; of a node's two
+// arrivals (counted in `seen`, zeroed) the first ends and the second, which
+// finds the records of all nodes below, goes on.  Bound by the latency of that
+// chain (about 25 levels).
+__global__ void k_collapse_cost(const Node2* __restrict__ nodes, int n, const int32_t* __restrict__ parent,
+                                int32_t* __restrict__ seen, float4* __restrict__ cost) {
+    const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
+    if (leaf >= n || nodes[leaf].left >= 0) return;
+    auto left = [&](int32_t k) { return nodes[k].left; };
+    auto right = [&](int32_t k) { return nodes[k].right; };
+    auto area = [&](int32_t k) { return node_area(nodes[k]); };
+    for (int i = parent[leaf]; i >= 0; i = parent[i]) {
+        __threadfence();
+        if (atomicAdd(seen + i, 1) == 0) return;
+        __threadfence();
+        const float4 a = __ldcg(cost + left(i)), b = __ldcg(cost + right(i));
+        const float l[3] = {a.x, a.y, a.z}, r[3] = {b.x, b.y, b.z};
+        float c[3];
+        uint32_t record = collapse_cost(area(i), l, r, c), depth = 0;
+        int32_t ch[4];
+        const int nc = collapse_largest(i, left, right, area, ch);
+        for (int k = 0; k < nc; k++) depth = max(depth, __float_as_uint(__ldcg(&cost[ch[k]].w)) >> kDepthShift);
+        record |= (depth + 1) << kDepthShift;
+        __stcg(cost + i, make_float4(c[0], c[1], c[2], __uint_as_float(record)));
+    }
+}
+
+// cost: k_collapse_cost's records, or null to open the largest child first.
 __global__ void k_collapse(const int32_t* __restrict__ q, int nq, const Node2* __restrict__ nodes,
-                           int4* __restrict__ ch_out, int32_t* __restrict__ nc_out, int32_t* __restrict__ nint_out) {
+                           const float4* __restrict__ cost, int4* __restrict__ ch_out, int32_t* __restrict__ nc_out,
+                           int32_t* __restrict__ nint_out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nq) return;
     const int n2 = q[i];
+    auto left = [&](int32_t k) { return nodes[k].left; };
+    auto right = [&](int32_t k) { return nodes[k].right; };
     int ch[4] = {-1, -1, -1, -1};
     int nc = 0;
     if (nodes[n2].left < 0) {
         ch[nc++] = n2;  // a root that is a leaf
+    } else if (cost) {
+        nc = collapse_children(n2, left, right, [&](int32_t k) { return __float_as_uint(cost[k].w); }, ch);
     } else {
-        ch[nc++] = nodes[n2].left;
-        ch[nc++] = nodes[n2].right;
-        while (nc < 4) {
-            int pick = -1;
-            float best = -1.0f;
-            for (int k = 0; k < nc; k++)
-                if (nodes[ch[k]].left >= 0 && node_area(nodes[ch[k]]) > best) {
-                    best = node_area(nodes[ch[k]]);
-                    pick = k;
-                }
-            if (pick < 0) break;
-            const int c = ch[pick];
-            ch[pick] = nodes[c].left;
-            ch[nc++] = nodes[c].right;
-        }
+        nc = collapse_largest(n2, left, right, [&](int32_t k) { return node_area(nodes[k]); }, ch);
     }
     int nint = 0;
     for (int k = 0; k < nc; k++)
@@ -1081,13 +1111,30 @@ WideTree build_wide_tree(const float* d_tv, int n, int max_leaf, cudaStream_t st
     int32_t* ncb = dmalloc<int32_t>(owned, n_node2);
     int32_t* offs = dmalloc<int32_t>(owned, n_node2);
     uint4* wide = dmalloc<uint4>(owned, 4 * (size_t)n_node2);
-    ck(cudaMemsetAsync(q[0], 0, sizeof(int32_t), st), "root queue");  // node 0
+    float4* cost = dmalloc<float4>(owned, n_node2);
+    int32_t* parent = ncb;  // until the collapse
+    int32_t* seen = offs;
+    ck(cudaMemsetAsync(cost, 0, sizeof(float4) * (size_t)n_node2, st), "memset");
+    ck(cudaMemsetAsync(seen, 0, sizeof(int32_t) * (size_t)n_node2, st), "memset");
+    k_parents<<<(n_node2 + 255) / 256, 256, 0, st>>>(nodes, n_node2, parent);
+    k_collapse_cost<<<(n_node2 + 255) / 256, 256, 0, st>>>(nodes, n_node2, parent, seen, cost);
     ck(cudaMemsetAsync(counts + 3, 0, sizeof(int32_t), st), "status");
-    int nq = 1, base = 0, qc = 0, depth = 0;
-    while (nq > 0) {
+    ck(cudaMemcpyAsync(h, &cost[0].w, sizeof(float), cudaMemcpyDeviceToHost, st), "depth");
+    ck(cudaStreamSynchronize(st), "collapse costs");
+    const float4* by = (uint32_t)h[0] >> kDepthShift > (uint32_t)kMaxWideDepth ? nullptr : cost;
+    int nq = 0, base = 0, qc = 0, depth = 0;
+    for (;;) {
+        if (nq == 0) {
+            // done, unless the cheapest collapse is too deep
+            if (depth > 0 && (depth <= kMaxWideDepth || !by)) break;
+            if (depth > 0) by = nullptr;
+            ck(cudaMemsetAsync(q[0], 0, sizeof(int32_t), st), "root queue");  // node 0
+            nq = 1;
+            base = qc = depth = 0;
+        }
         depth++;
         const int g = (nq + 255) / 256;
-        k_collapse<<<g, 256, 0, st>>>(q[qc], nq, nodes, chb, ncb, offs);
+        k_collapse<<<g, 256, 0, st>>>(q[qc], nq, nodes, by, chb, ncb, offs);
         k_scan<<<1, 1024, 0, st>>>(offs, nq, counts);
         k_emit<<<g, 256, 0, st>>>(q[qc], nq, base, base + nq, chb, ncb, offs, nodes, wide, q[1 - qc], counts + 3);
         ck(cudaGetLastError(), "collapse");

@@ -128,7 +128,8 @@ void create_scene(const pt_scene_desc* d, pt_scene* s, const SceneTextures* tx =
         ref.node_box = dalloc<float4>(keep.v, 0);
     }
     s->wide_depth = wide.max_depth;
-    if (3 * wide.max_depth + 4 > 64) throw Fail(PT_ERR_LIMIT, "wide BVH too deep for the traversal stack");
+    static_assert(3 * kMaxWideDepth + 4 <= 64, "");
+    if (wide.max_depth > kMaxWideDepth) throw Fail(PT_ERR_LIMIT, "wide BVH too deep for the traversal stack");
     float4* tris = dalloc<float4>(s->owned, 3 * (size_t)nt);
     launch_leaf_triangles(tv, wide.tri_order, ref.rank, ref.prim_parent, nt, tris, s->stream);
     ck(cudaGetLastError(), "scene arrays");

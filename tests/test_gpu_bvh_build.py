@@ -137,6 +137,47 @@ def test_device_wide_tree_full_size(gpu_lib, make):
         assert np.array_equal(again, nodes)
 
 
+def _chain(links, per):
+    """Clusters of `per` triangles along x, each three times closer to the origin."""
+    from dataclasses import replace
+    x = (np.float32(3) ** -np.arange(links, dtype=np.float32))[:, None] * (
+        1 + np.float32(0.01) * np.arange(per, dtype=np.float32))
+    x = x.reshape(-1)
+    z = np.zeros_like(x)
+    v = np.stack([np.stack([x, z, z], 1), np.stack([x, x * np.float32(.1), z], 1),
+                  np.stack([x, z, x * np.float32(.1)], 1)], 1).reshape(-1, 3).astype(np.float32)
+    n = len(v) // 3
+    sc = scenes.soup(seed=5, n_spheres=2, freq=1, width=8, height=8)
+    up, side = np.float32([[0, 0, 1]]), np.float32([[1, 0, 0]])
+    return replace(sc, vertices=v, normals=np.repeat(up, len(v), 0), tangents=np.repeat(side, len(v), 0),
+                   triangles=np.arange(len(v), dtype=np.int32).reshape(-1, 3),
+                   mesh_tri_offset=np.array([0, n], np.int32), mesh_vert_offset=np.array([0, len(v)], np.int32),
+                   mesh_material=np.array([0], np.int32))
+
+
+@pytest.mark.parametrize("links,per,depth", [(15, 4000, 18), (19, 4000, 19), (24, 4000, 24)],
+                         ids=["cheapest", "cheapest_too_deep", "both_too_deep"])
+def test_wide_tree_at_depth_limit(gpu_lib, links, per, depth):
+    """The cheapest collapse, or the largest-first one where the cheapest
+    exceeds the traversal's depth (20; 21 levels for 19 links); a scene whose
+    largest-first tree exceeds it is refused, though its cheapest would fit."""
+    from cpppt import lib
+    from oracle.oracle import Oracle
+    sc = _chain(links, per)
+    _same_wide(sc)
+    assert lib.wide_bvh(sc, on_device=False)[2] == depth
+    if depth > 20:
+        with pytest.raises(lib.PtError, match="too deep"):
+            lib.GpuScene(sc)
+        return
+    rays = scenes.hit_ray_batch(sc, 2048, seed=1)
+    gi, gt, _, _ = lib.GpuScene(sc).trace_closest(rays)
+    oi, ot = Oracle("port").scene(sc).trace_closest(rays)
+    assert (oi >= 0).any()
+    assert np.array_equal(gi, oi)
+    assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
+
+
 @pytest.mark.parametrize("n", [0, 1, 4, 5, 32, 33, 255, 256, 257, 3001])
 def test_scene_arrays_at_block_edges(gpu_lib, n):
     """The scene's arrays, assembled on the device: hits of the first n
