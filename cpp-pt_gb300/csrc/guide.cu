@@ -87,42 +87,36 @@ __device__ __forceinline__ BSample sd_sample(const DevSDTree& T, f3 p, float u0,
     return s;
 }
 
-// SDTree::splat (sdtree.h:514-524)
-__device__ __forceinline__ void sd_splat(const DevSDTree& T, float rad, f3 p, f3 dir) {
-    const int t = sd_dtree(T, p);
-    if (t < 0) return;
-    float area;
-    const int slot = sd_dleaf(T, t, atan2f(dir.y, dir.x), dir.z, &area);
-    if (slot >= 0) atomicAdd(T.slot_value + slot, rad);
-    atomicAdd(T.dtree_count + t, 1);
-    atomicAdd(T.dtree_rad + t, rad);
-}
-
-// Backward products and splats of a finished path (ppg.h:131-141): only when
-// the last vertex carries radiance; vertex k receives max-channel of the
-// product of the factors of vertices k..n-1.
-__device__ __forceinline__ void splat_path(const DevSDTree& T, const PPGVerts& V, int slot, int nv, int max_depth) {
-    if (nv <= 0) return;
-    const size_t base = (size_t)slot * (size_t)max_depth;
-    float4 b = V.vd[base + nv - 1];
-    f3 acc = mk(b.z, b.w, V.vr[base + nv - 1]);
-    if (!(acc.x > 0.f || acc.y > 0.f || acc.z > 0.f)) return;
-    for (int k = nv - 1; k >= 0; k--) {
-        const float4 a = V.vp[base + k];
-        const float4 bb = V.vd[base + k];
-        if (k < nv - 1) acc = acc * mk(bb.z, bb.w, V.vr[base + k]);
-        const float r = fmaxf(acc.x, fmaxf(acc.y, acc.z));
-        sd_splat(T, r, mk(a.x, a.y, a.z), mk(a.w, bb.x, bb.y));
+// SDTree::splat (sdtree.h:514-524), by the lanes that have one (`on`; the
+// whole warp calls).  The count and sum of a spatial leaf are added once per
+// warp for each leaf its lanes hit: few leaves take all of a pass's splats,
+// and additions to one address follow one another.
+__device__ __forceinline__ void sd_splat_warp(const DevSDTree& T, bool on, float rad, f3 p, f3 dir) {
+    const unsigned lane = threadIdx.x & 31u;
+    const int t = on ? sd_dtree(T, p) : -1;
+    if (t >= 0) {
+        float area;
+        const int slot = sd_dleaf(T, t, atan2f(dir.y, dir.x), dir.z, &area);
+        if (slot >= 0) atomicAdd(T.slot_value + slot, rad);
     }
-}
-
-__device__ __forceinline__ void set_vertex_rad(const PPGVerts& V, int slot, int k, int max_depth, f3 r) {
-    const size_t i = (size_t)slot * (size_t)max_depth + k;
-    float4 b = V.vd[i];
-    b.z = r.x;
-    b.w = r.y;
-    V.vd[i] = b;
-    V.vr[i] = r.z;
+    // the sum over the lanes of one leaf: in each step a lane takes in the next
+    // one of those that remain, and every second one leaves
+    const unsigned group = __match_any_sync(0xffffffffu, t);
+    const int rank = __popc(group & ((1u << lane) - 1u));
+    unsigned rest = group & (0xfffffffeu << lane);  // remaining lanes above this one
+    unsigned kept = group;
+    float sum = t >= 0 ? rad : 0.f;
+    for (int bit = 0; __any_sync(0xffffffffu, rest != 0); bit++) {
+        const int next = __ffs(rest);
+        const float x = __shfl_sync(0xffffffffu, sum, next ? next - 1 : (int)lane);
+        if (next) sum += x;
+        kept = __ballot_sync(0xffffffffu, (rank >> bit & 1) == 0) & kept;
+        rest &= kept;
+    }
+    if (t >= 0 && rank == 0) {
+        atomicAdd(T.dtree_count + t, __popc(group));
+        atomicAdd(T.dtree_rad + t, sum);
+    }
 }
 
 constexpr int kShadePPGThreads = 256;
@@ -134,7 +128,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
     bool push_cont = false, release = false;
     float4 no, nd, nt;
     int4 ninfo;
-    int slot = -1;
+    int slot = -1, n_splat = 0;  // vertices that take a splat (all of them, one per bounce, or none)
     if (i < n) {
         const float4 O = in.o[i], D = in.d[i], Tp = in.thr[i];
         const int4 I = in.info[i];
@@ -145,16 +139,10 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
         const int D_ = P.max_depth;
         f3 mul = mk(Tp.x, Tp.y, Tp.z);
         const f3 ro = mk(O.x, O.y, O.z), rd = mk(D.x, D.y, D.z);
-        const int nv = bounce;  // vertices recorded so far, this bounce's included (bounce > 0)
-        if (bounce > 0) {  // ppg.h:51-56: a vertex at the ray's origin with radiance 1
-            const size_t vi = (size_t)slot * D_ + (bounce - 1);
-            V.vp[vi] = make_float4(ro.x, ro.y, ro.z, rd.x);
-            V.vd[vi] = make_float4(rd.y, rd.z, 1.f, 1.f);
-            V.vr[vi] = 1.f;
-        }
+        f3 vrad = mk(1.f, 1.f, 1.f);  // ppg.h:51-56: a vertex at the ray's origin with radiance 1
         bool done = true;
         if (prim < 0) {  // sky = 0 (ppg.h:57-63)
-            if (bounce > 0) set_vertex_rad(V, slot, bounce - 1, D_, mk(0.f, 0.f, 0.f));
+            vrad = mk(0.f, 0.f, 0.f);
         } else {
             int kind;
             DevMaterial m;
@@ -162,7 +150,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
             const f3 wo = -rd;
             if (kind == PT_MAT_EMISSIVE_) {  // ppg.h:66-73
                 const f3 rad = mk(m.r, m.g, m.b);
-                if (bounce > 0) set_vertex_rad(V, slot, bounce - 1, D_, rad);
+                vrad = rad;
                 const f3 c = mul * rad;
                 film_add_rgb(film, pixel, c.x, c.y, c.z, ctr);
             } else {
@@ -194,7 +182,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
                         }
                         if (alive) {
                             const f3 nm = f * (weight / p);
-                            if (bounce > 0) set_vertex_rad(V, slot, bounce - 1, D_, nm);
+                            vrad = nm;
                             mul = mul * nm;
                             if (bounce + 1 < P.max_depth) {
                                 done = false;
@@ -210,14 +198,70 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
                 }
             }
         }
-        if (done) {
-            splat_path(T, V, slot, nv, D_);
-            release = true;
+        if (bounce > 0) {
+            const size_t vi = (size_t)slot * D_ + (bounce - 1);
+            V.vp[vi] = make_float4(ro.x, ro.y, ro.z, rd.x);
+            V.vd[vi] = make_float4(rd.y, rd.z, vrad.x, vrad.y);
+            V.vr[vi] = vrad.z;
         }
+        release = done;
+        // ppg.h:131-141: splats only when the last vertex carries radiance
+        if (done && (vrad.x > 0.f || vrad.y > 0.f || vrad.z > 0.f)) n_splat = bounce;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kShadePPGThreads / 32;
+    // Backward products and splats of the finished paths (ppg.h:131-141):
+    // vertex k receives the largest channel of the product of the factors of
+    // vertices k..n-1, taken from the last one down.  A thread per vertex of
+    // the CTA's finished paths, found in the running total of their vertices:
+    // the tree walks are chains of dependent loads, and one thread walking for
+    // vertex after vertex left the SM at 6 % of its issue slots (Cornell box
+    // 128x128, 64 spp: render 4.35 -> 3.60 ms with the sums per warp).
+    __shared__ int s_first[kShadePPGThreads], s_slot[kShadePPGThreads], s_nv[kShadePPGThreads], s_total[kWarps];
+    int incl = n_splat;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_total[warp] = incl;
+    __syncthreads();
+    int before = 0, n_verts = 0;
+    for (int w = 0; w < kWarps; w++) {
+        if (w < warp) before += s_total[w];
+        n_verts += s_total[w];
+    }
+    s_first[threadIdx.x] = before + incl - n_splat;
+    s_slot[threadIdx.x] = slot;
+    s_nv[threadIdx.x] = n_splat;
+    __syncthreads();
+    for (int j0 = 0; j0 < n_verts; j0 += kShadePPGThreads) {
+        const int j = j0 + (int)threadIdx.x;
+        const bool on = j < n_verts;
+        float rad = 0.f;
+        f3 vp = mk(0.f, 0.f, 0.f), vd = vp;
+        if (on) {
+            int path = 0;  // the last one that starts at or before j; those without vertices start with their successor
+            for (int step = kShadePPGThreads / 2; step > 0; step >>= 1)
+                if (s_first[path + step] <= j) path += step;
+            const int k = j - s_first[path];
+            const size_t base = (size_t)s_slot[path] * P.max_depth;
+            int v = s_nv[path] - 1;
+            float4 b = V.vd[base + v];
+            f3 acc = mk(b.z, b.w, V.vr[base + v]);
+            while (v > k) {
+                v--;
+                b = V.vd[base + v];
+                acc = acc * mk(b.z, b.w, V.vr[base + v]);
+            }
+            const float4 a = V.vp[base + k];
+            rad = fmaxf(acc.x, fmaxf(acc.y, acc.z));
+            vp = mk(a.x, a.y, a.z);
+            vd = mk(a.w, b.x, b.y);
+        }
+        sd_splat_warp(T, on, rad, vp, vd);
     }
     // one addition to each queue's counter per CTA (as k_shade)
-    __shared__ int s_count[2][kShadePPGThreads / 32], s_base[2];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int s_count[2][kWarps], s_base[2];
     const unsigned m_free = __ballot_sync(0xffffffffu, release), m_cont = __ballot_sync(0xffffffffu, push_cont);
     if (lane == 0) {
         s_count[0][warp] = __popc(m_free);
@@ -226,7 +270,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
     __syncthreads();
     if (lane == 0 && warp < 2) {
         int total = 0;
-        for (int w = 0; w < kShadePPGThreads / 32; w++) {
+        for (int w = 0; w < kWarps; w++) {
             const int q = s_count[warp][w];
             s_count[warp][w] = total;
             total += q;

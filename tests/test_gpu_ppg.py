@@ -40,3 +40,21 @@ def test_ppg_learns_and_reports_stats(gpu_lib):
     # passes of 1, 2, ..., 128 spp: 255 spp worth of paths
     assert st["paths"] == 64 * 64 * 255
     assert img.mean() > 0.05 and np.isfinite(img).all()
+
+
+@pytest.mark.parametrize("res,depth", [((1, 1), 32), ((17, 15), 2), ((16, 16), 3), ((33, 31), 40)],
+                         ids=["one_pixel", "partial_block", "full_block", "long_paths"])
+def test_ppg_splats_by_vertex(gpu_lib, res, depth):
+    """The splats of a CTA's finished paths, one thread per vertex: the tree
+    they train, and with it the image, is the same from run to run, and the
+    image's mean is that of BSDF sampling to the same depth (6 standard errors
+    over 16 seeds)."""
+    from cpppt.lib import MODE_PT, MODE_SDTREE, GpuScene
+    gs = GpuScene(scenes.cornell(*res))
+    guided = [gs.render(64, max_depth=depth, seed=s, mode=MODE_SDTREE) for s in range(16)]
+    again = [gs.render(64, max_depth=depth, seed=s, mode=MODE_SDTREE) for s in range(16)]
+    assert all(np.array_equal(a, b) for a, b in zip(guided, again))
+    plain = [gs.render(64, max_depth=depth, seed=s, mode=MODE_PT) for s in range(16)]
+    g, p = (np.array([x.astype(np.float64).mean() for x in v]) for v in (guided, plain))
+    se = np.sqrt(g.var(ddof=1) / len(g) + p.var(ddof=1) / len(p))
+    assert abs(g.mean() - p.mean()) <= 6 * se
