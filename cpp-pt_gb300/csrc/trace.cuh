@@ -303,11 +303,18 @@ __device__ __forceinline__ void ld256(const uint4* p, uint4& a, uint4& b) {
 
 // One inner node (T.cur): a child that the ray enters in front of the best
 // hit is next -- the nearest for a closest-hit query, the first in slot order
-// for an any-hit query -- and the other entered children are pushed unsorted
-// (culling compares each popped entry with the best hit, so the order changes
-// the work, never the answer; sorting them cost more than it saved).  kTravPop
-// when no child is entered.  Two 256-bit loads instead of four of 128 bits:
-// 1080p, 16 spp on the 1M-triangle soup 89.6 -> 88.3 ms.
+// for an any-hit query -- and the other entered children are pushed, for a
+// closest-hit query with the second nearest on top.  (Culling compares each
+// popped entry with the best hit, so the order changes the work, never the
+// answer.)  kTravPop when no child is entered.  The nearest two come from two
+// ordered pairs of children, with the references selected along: as many
+// instructions as finding the nearest alone by keys that carry the slot.
+// Against pushing in slot order: 1M rays in the 192k-triangle room 263 -> 207
+// us, 1.8M on the 1M-triangle soup 753 -> 731, 1080p at 16 spp there 75.1 ->
+// 74.0 ms, guided 720p in the room 10.8 -> 10.1 ms.  An any-hit query that
+// takes the nearest first: room 124 -> 132 us, the farthest first: soup 578
+// -> 715 us.  Two 256-bit loads instead of four of 128 bits: 1080p, 16 spp on
+// the 1M-triangle soup 89.6 -> 88.3 ms.
 template <bool ANY, bool COUNT, class Stack>
 __device__ __forceinline__ void trav_node(Trav& T, Stack& K, const DevScene& S, uint32_t* status, TraceCount& cnt) {
     if (COUNT) cnt.nodes++;
@@ -348,7 +355,7 @@ __device__ __forceinline__ void trav_node(Trav& T, Stack& K, const DevScene& S, 
             const float tf = fmin3(tfx[h], tfy[h], fminf(tfz[h], cull));
             const bool hit = tn <= tf * 1.0000005f;
             if (ANY) key[c + h] = hit ? 0u : 0xffffffffu;
-            else key[c + h] = hit ? ((__float_as_uint(tn) & ~3u) | (uint32_t)(c + h)) : 0xffffffffu;
+            else key[c + h] = hit ? __float_as_uint(tn) : 0xffffffffu;  // tn >= 0: ordered as its bits
         }
     }
     // Indexed by constants only: with a run-time index (the nearest child's) the
@@ -377,26 +384,40 @@ __device__ __forceinline__ void trav_node(Trav& T, Stack& K, const DevScene& S, 
         T.cur_t = 0.f;
         return;
     }
-    const uint32_t m = min(min(key[0], key[1]), min(key[2], key[3]));
-    if (m == 0xffffffffu) {
+    // the pairs (0, 1) and (2, 3), the nearer child first
+    const bool p = key[1] < key[0], q = key[3] < key[2];
+    const uint32_t ka = min(key[0], key[1]), kb = max(key[0], key[1]);
+    const uint32_t kc = min(key[2], key[3]), kd = max(key[2], key[3]);
+    const uint32_t ra = p ? refs[1] : refs[0], rb = p ? refs[0] : refs[1];
+    const uint32_t rc = q ? refs[3] : refs[2], rd = q ? refs[2] : refs[3];
+    const uint32_t k0 = min(ka, kc);
+    if (k0 == 0xffffffffu) {
         T.cur = kTravPop;
         return;
     }
+    // the pair with the nearest child, and the two children between it and the farthest
+    const bool f = kc < ka;
+    const uint32_t kn = f ? kd : kb, rn = f ? rd : rb;  // the nearest's neighbour
+    const uint32_t kf = max(ka, kc), rf = f ? ra : rc;  // the nearer child of the other pair
+    const uint32_t kl = f ? kb : kd, rl = f ? rb : rd;  // its farther one
+    const bool g = kn < kf;
+    const uint32_t k1 = min(kn, kf), r1 = g ? rn : rf;
+    const uint32_t k2 = max(kn, kf), r2 = g ? rf : rn;
     if (T.sp < K.fast) {
-#pragma unroll
-        for (int c = 3; c >= 0; c--)
-            if (key[c] != 0xffffffffu && key[c] != m) K.put_shared(T.sp, refs[c], key[c]);
+        if (kl != 0xffffffffu) K.put_shared(T.sp, rl, kl);
+        if (k2 != 0xffffffffu) K.put_shared(T.sp, r2, k2);
+        if (k1 != 0xffffffffu) K.put_shared(T.sp, r1, k1);
     } else {
         if (K.depth(T.sp) + 3 > S.stack_limit) {
             trav_abort(T, status, kStatusStackOverflow);
             return;
         }
-#pragma unroll
-        for (int c = 3; c >= 0; c--)
-            if (key[c] != 0xffffffffu && key[c] != m) K.put(T.sp, refs[c], key[c]);
+        if (kl != 0xffffffffu) K.put(T.sp, rl, kl);
+        if (k2 != 0xffffffffu) K.put(T.sp, r2, k2);
+        if (k1 != 0xffffffffu) K.put(T.sp, r1, k1);
     }
-    T.cur = (m & 2u) ? ((m & 1u) ? refs[3] : refs[2]) : ((m & 1u) ? refs[1] : refs[0]);
-    T.cur_t = __uint_as_float(m & ~3u);
+    T.cur = f ? rc : ra;
+    T.cur_t = __uint_as_float(k0);
 }
 
 // The postponed leaf T.leaf.  Returns true when an any-hit query is answered.
