@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
                                                    DevSDTree T, PPGVerts V, int* slot_stack) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
     bool push_cont = false, release = false;
     float4 no, nd, nt;
     int4 ninfo;

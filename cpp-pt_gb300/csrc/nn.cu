@@ -722,6 +722,7 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
                                                   const DevBatchJob* __restrict__ jobs) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
     bool push_sh = false, push_cont = false, release = false;
     float4 sh_o, sh_d, sh_c, no, nd, nt;
     int4 ninfo;
@@ -950,6 +951,7 @@ __global__ void __launch_bounds__(256) k_finish_nn(NNPathData PD, WaveCounters* 
                                                    const DevNNJob* __restrict__ nnj, int max_depth) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_fin;
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
     const unsigned lane = threadIdx.x & 31u;
     const bool release = i < n;
     int4 f = make_int4(0, 0, 0, 0);
