@@ -9,6 +9,7 @@
 // a free list: k_generate_ppg pops, terminating paths push.
 #include <cuda_runtime.h>
 
+#include "launch.cuh"
 #include "guide.h"
 #include "shade.cuh"
 
@@ -123,6 +124,7 @@ constexpr int kShadePPGThreads = 256;
 __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, PathIO in, PathIO nxt,
                                                    const float4* __restrict__ hit, RenderParams P, WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                    DevSDTree T, PPGVerts V, int* slot_stack) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
     if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
 // pass, no strata), each with a vertex slot from the free list.
 __global__ void __launch_bounds__(256) k_generate_ppg(DevScene S, PathIO nxt, int capacity, RenderParams P,
                                                       WaveCounters* ctr, const int* slot_stack) {
+    after_previous();
     const int n_next = ctr->n_next, free_top = ctr->free_top;
     const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
     const int avail = min(capacity - n_next, free_top);
@@ -321,6 +324,7 @@ __global__ void __launch_bounds__(256) k_generate_ppg(DevScene S, PathIO nxt, in
 }
 
 __global__ void k_advance_ppg(WaveCounters* ctr, int capacity) {
+    after_previous();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int n_next = ctr->n_next;
     const unsigned long long left = ctr->work_total - ctr->work_next;
@@ -349,15 +353,15 @@ void launch_init_slots(int* slot_stack, int n, cudaStream_t st) {
 void launch_shade_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                       unsigned long long* film, const DevSDTree& T, const PPGVerts& V, int* slot_stack,
                       cudaStream_t st) {
-    k_shade_ppg<<<(B.capacity + kShadePPGThreads - 1) / kShadePPGThreads, kShadePPGThreads, 0, st>>>(
+    launch_after(k_shade_ppg, (B.capacity + kShadePPGThreads - 1) / kShadePPGThreads, kShadePPGThreads, 0, st,
         S, path_io(B, cur), path_io(B, 1 - cur), B.hit, P, ctr, film, T, V, slot_stack);
 }
 void launch_generate_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                          const int* slot_stack, int num_sms, cudaStream_t st) {
     // a resident grid over the free slots (as the plain wavefront's)
-    k_generate_ppg<<<max(1, min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st>>>(S, path_io(B, 1 - cur), B.capacity,
+    launch_after(k_generate_ppg, max(1, min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st, S, path_io(B, 1 - cur), B.capacity,
                                                                                        P, ctr, slot_stack);
-    k_advance_ppg<<<1, 32, 0, st>>>(ctr, B.capacity);
+    launch_after(k_advance_ppg, 1, 32, 0, st, ctr, B.capacity);
 }
 
 }  // namespace cpppt_gb300

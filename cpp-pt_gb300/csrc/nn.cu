@@ -11,6 +11,7 @@
 
 #include <algorithm>
 
+#include "launch.cuh"
 #include "nn.h"
 #include "nn.cuh"
 #include "trace.cuh"
@@ -251,6 +252,7 @@ template <bool ONEBLOB>
 __global__ void __launch_bounds__(kTcInferThreads) k_nn_infer(DevScene S, PathIO in, const float4* __restrict__ hit, WaveCounters* ctr,
                                                               const DevNNJob* __restrict__ nnj,
                                                               float4* __restrict__ params) {
+    after_previous();
     extern __shared__ __align__(1024) unsigned char smem[];
     const int n = ctr->n_cur;
     if (n == 0) return;
@@ -627,8 +629,8 @@ void launch_nn_forward_debug(const DevNNJob* nnj, const float* in, int n, float*
 void launch_nn_infer(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const DevNNJob* nnj,
                      float4* params, int num_sms, cudaStream_t st, bool oneblob) {
     // four CTAs of 128 threads per SM fit in shared memory (48 KB each)
-    if (oneblob) k_nn_infer<true><<<num_sms * 4, kTcInferThreads, nn_smem_infer(), st>>>(S, path_io(B, cur), B.hit, ctr, nnj, params);
-    else k_nn_infer<false><<<num_sms * 4, kTcInferThreads, nn_smem_infer(), st>>>(S, path_io(B, cur), B.hit, ctr, nnj, params);
+    if (oneblob) launch_after(k_nn_infer<true>, num_sms * 4, kTcInferThreads, nn_smem_infer(), st, S, path_io(B, cur), B.hit, ctr, nnj, params);
+    else launch_after(k_nn_infer<false>, num_sms * 4, kTcInferThreads, nn_smem_infer(), st, S, path_io(B, cur), B.hit, ctr, nnj, params);
 }
 // Zeroes each task's gradient and loss (and, with prep, its T sum).
 __global__ void k_nn_task_zero(const NNTrainTask* __restrict__ tasks, int prep) {
@@ -720,6 +722,7 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
                                                   WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                   const float4* __restrict__ params, NNPathData PD, int guided,
                                                   const DevBatchJob* __restrict__ jobs) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
     if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
@@ -949,6 +952,7 @@ __device__ __forceinline__ void visit_records(const NNPathData& PD, int4 f, int 
 // capacity are dropped); the slots go back to the free list.
 __global__ void __launch_bounds__(256) k_finish_nn(NNPathData PD, WaveCounters* ctr,
                                                    const DevNNJob* __restrict__ nnj, int max_depth) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_fin;
     if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
@@ -1015,6 +1019,7 @@ __global__ void __launch_bounds__(256) k_finish_nn(NNPathData PD, WaveCounters* 
 __global__ void __launch_bounds__(kTraceThreads) k_shadow_nn(DevScene S, PathBuffers B, WaveCounters* ctr,
                                                    unsigned long long* __restrict__ film, NNPathData PD,
                                                    const DevBatchJob* __restrict__ jobs) {
+    after_previous();
     extern __shared__ uint32_t s_stack[];
     const int n = ctr->n_shadow;
     if (n == 0) return;
@@ -1050,6 +1055,7 @@ cudaError_t nn_shadow_smem_limit() {
 __global__ void __launch_bounds__(256) k_generate_nn(PathIO nxt, int capacity, WaveCounters* ctr, NNPathData PD,
                                                      const DevBatchJob* __restrict__ jobs,
                                                      int n_jobs) {
+    after_previous();
     const int n_next = ctr->n_next, free_top = ctr->free_top;
     const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
     const bool slots = PD.rec_cap > 0;  // vertex slots are for training records
@@ -1110,6 +1116,7 @@ __global__ void __launch_bounds__(256) k_generate_nn(PathIO nxt, int capacity, W
 }
 
 __global__ void k_advance_nn(WaveCounters* ctr, int capacity) {
+    after_previous();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int n_next = ctr->n_next;
     const unsigned long long left = ctr->work_total - ctr->work_next;
@@ -1134,23 +1141,23 @@ __global__ void k_advance_nn(WaveCounters* ctr, int capacity) {
 void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                      unsigned long long* film, const float4* params, const NNPathData& PD, bool guided,
                      const DevBatchJob* jobs, cudaStream_t st) {
-    k_shade_nn<<<(B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st>>>(S, B, path_io(B, cur), path_io(B, 1 - cur), cur, P, ctr, film, params, PD, guided ? 1 : 0, jobs);
+    launch_after(k_shade_nn, (B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st, S, B, path_io(B, cur), path_io(B, 1 - cur), cur, P, ctr, film, params, PD, guided ? 1 : 0, jobs);
 }
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    k_shadow_nn<<<num_sms * kTraceBlocksPerSM, kTraceThreads, trace_smem(false, true, kTraceThreads), st>>>(S, B, ctr, film, PD, jobs);
+    launch_after(k_shadow_nn, num_sms * kTraceBlocksPerSM, kTraceThreads, trace_smem(false, true, kTraceThreads), st, S, B, ctr, film, PD, jobs);
 }
 void launch_nn_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
                         const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
     // a resident grid over the free slots (as the plain wavefront's)
-    k_generate_nn<<<std::max(1, std::min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st>>>(
+    launch_after(k_generate_nn, std::max(1, std::min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st, 
         path_io(B, 1 - cur), B.capacity, ctr, PD, jobs, n_jobs);
-    if (PD.rec_cap > 0) k_advance_nn<<<1, 32, 0, st>>>(ctr, B.capacity);
+    if (PD.rec_cap > 0) launch_after(k_advance_nn, 1, 32, 0, st, ctr, B.capacity);
     else launch_advance(ctr, B.capacity, cur, st);
 }
 void launch_nn_finish(const NNPathData& PD, WaveCounters* ctr, const DevNNJob* nnj, int max_depth, int capacity,
                       cudaStream_t st) {
-    k_finish_nn<<<(capacity + 255) / 256, 256, 0, st>>>(PD, ctr, nnj, max_depth);
+    launch_after(k_finish_nn, (capacity + 255) / 256, 256, 0, st, PD, ctr, nnj, max_depth);
 }
 
 }  // namespace cpppt_gb300

@@ -15,6 +15,7 @@
 
 #include <mutex>
 
+#include "launch.cuh"
 #include "kernels.h"
 #include "shade.cuh"
 #include "trace.cuh"
@@ -135,6 +136,7 @@ __device__ __forceinline__ void shadow_queue(const DevScene& S, uint32_t* s_stac
 template <bool COUNT>
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(DevScene S, PathIO in, float4* __restrict__ Hout,
                                                                            WaveCounters* ctr) {
+    after_previous();
     extern __shared__ uint32_t s_stack[];
     const int n = ctr->n_cur;
     if (n == 0) return;  // drained wavefront
@@ -170,6 +172,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_wave
                                                                                  float4* __restrict__ Hout, ShadowIO Q,
                                                                                  int cur, WaveCounters* ctr,
                                                                                  unsigned long long* __restrict__ film) {
+    after_previous();
     extern __shared__ uint32_t s_stack[];
     const int n = ctr->n_cur, m = cur ? ctr->n_shadow : ctr->n_shadow1;
     if (n == 0 && m == 0) return;
@@ -291,6 +294,7 @@ __global__ void __launch_bounds__(kShadeThreads, CPPPT_SHADE_BLOCKS) k_shade(Dev
                                                const float4* __restrict__ hit, int cur, WaveCounters* ctr,
                                                unsigned long long* __restrict__ film,
                                                const DevBatchJob* __restrict__ jobs) {
+    after_previous();
     const int n = ctr->n_cur;
     // an empty CTA of the capacity's grid: nothing to shade, no barriers to
     // wait at (Cornell box, 256x256, 64 spp, 3.65 -> 3.57 ms)
@@ -354,6 +358,7 @@ __device__ __forceinline__ int find_job(const DevBatchJob* __restrict__ jobs, in
 // (global over the jobs' pixel x sample ranges) selects job, sample, pixel.
 __global__ void __launch_bounds__(256) k_generate(PathIO nxt, int capacity, WaveCounters* ctr,
                                                   const DevBatchJob* __restrict__ jobs, int n_jobs) {
+    after_previous();
     const int n_next = ctr->n_next;
     const unsigned long long first = ctr->work_next, left = ctr->work_total - first;
     const int room = capacity - n_next;
@@ -406,6 +411,7 @@ __global__ void __launch_bounds__(256) k_generate(PathIO nxt, int capacity, Wave
 // k_trace_wave's order).  Once no work is left, the last finish_max paths are
 // handed to k_finish and the wavefront has none.
 __global__ void k_advance(WaveCounters* ctr, int capacity, int cur, int traced, int finish_max) {
+    after_previous();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int n_next = ctr->n_next;
     const unsigned long long left = ctr->work_total - ctr->work_next;
@@ -453,6 +459,7 @@ constexpr size_t kFinishAnyWord = trace_smem(true, false, kFinishThreads) / 4;
 __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
     DevScene S, PathIO b0, PathIO b1, ShadowIO Q, WaveCounters* ctr, unsigned long long* __restrict__ film,
     const DevBatchJob* __restrict__ jobs) {
+    after_previous();
     const unsigned full = 0xffffffffu;
     const int m = ctr->n_shadow + ctr->n_shadow1;  // at most one of them is non-zero
     extern __shared__ uint32_t s_stack[];
@@ -546,12 +553,12 @@ __global__ void k_resolve(const unsigned long long* __restrict__ film, float* __
 void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, int num_sms, cudaStream_t st,
                    bool count) {
     const int g = num_sms * kTraceBlocksPerSM;
-    if (count) k_extend<true><<<g, kTraceThreads, kClosestSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
-    else k_extend<false><<<g, kTraceThreads, kClosestSmem, st>>>(S, path_io(B, cur), B.hit, ctr);
+    if (count) launch_after(k_extend<true>, g, kTraceThreads, kClosestSmem, st, S, path_io(B, cur), B.hit, ctr);
+    else launch_after(k_extend<false>, g, kTraceThreads, kClosestSmem, st, S, path_io(B, cur), B.hit, ctr);
 }
 void launch_trace_wave(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                        int num_sms, cudaStream_t st) {
-    k_trace_wave<<<num_sms * kTraceBlocksPerSM, kTraceThreads, kBothSmem, st>>>(S, path_io(B, cur), B.hit,
+    launch_after(k_trace_wave, num_sms * kTraceBlocksPerSM, kTraceThreads, kBothSmem, st, S, path_io(B, cur), B.hit,
                                                                                      shadow_io(B), cur, ctr, film);
 }
 cudaError_t trace_kernels_setup() {
@@ -570,7 +577,7 @@ cudaError_t trace_kernels_setup() {
 
 void launch_shade(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                   const DevBatchJob* jobs, cudaStream_t st) {
-    k_shade<<<(B.capacity + kShadeThreads - 1) / kShadeThreads, kShadeThreads, 0, st>>>(S, path_io(B, cur), path_io(B, 1 - cur), shadow_io(B), B.hit, cur,
+    launch_after(k_shade, (B.capacity + kShadeThreads - 1) / kShadeThreads, kShadeThreads, 0, st, S, path_io(B, cur), path_io(B, 1 - cur), shadow_io(B), B.hit, cur,
                                                       ctr, film, jobs);
 }
 void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
@@ -583,11 +590,11 @@ void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const Dev
     // few of them or none, and a CTA per 256 slots of the capacity cost up to
     // 50 us a launch there (a quarter of the Cornell box's 64-spp render)
     const int g = max(1, min((B.capacity + 255) / 256, num_sms * 8));
-    k_generate<<<g, 256, 0, st>>>(path_io(B, 1 - cur), B.capacity, ctr, jobs, n_jobs);
-    k_advance<<<1, 32, 0, st>>>(ctr, B.capacity, cur, shadows_traced ? cur : 1 - cur, shadows_traced ? 0 : kFinishPaths);
+    launch_after(k_generate, g, 256, 0, st, path_io(B, 1 - cur), B.capacity, ctr, jobs, n_jobs);
+    launch_after(k_advance, 1, 32, 0, st, ctr, B.capacity, cur, shadows_traced ? cur : 1 - cur, shadows_traced ? 0 : kFinishPaths);
 }
 void launch_advance(WaveCounters* ctr, int capacity, int cur, cudaStream_t st) {
-    k_advance<<<1, 32, 0, st>>>(ctr, capacity, cur, 1 - cur, 0);
+    launch_after(k_advance, 1, 32, 0, st, ctr, capacity, cur, 1 - cur, 0);
 }
 void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                            const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
@@ -598,7 +605,7 @@ void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, Wav
 
 void launch_finish(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                    const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    k_finish<<<num_sms, kFinishThreads, kFinishSmem, st>>>(S, path_io(B, 0), path_io(B, 1),
+    launch_after(k_finish, num_sms, kFinishThreads, kFinishSmem, st, S, path_io(B, 0), path_io(B, 1),
                                                                             shadow_io(B), ctr, film, jobs);
 }
 
