@@ -475,19 +475,35 @@ __global__ void __launch_bounds__(kTcRows) k_nn_train_fb(const NNTrainTask* __re
 
 // dW_l = A_l^T dZ_l over the batch on the tensor cores.  blockIdx.y = layer,
 // blockIdx.z = network (task); the CTAs of a (layer, network) share its
-// records in K tiles of kWGK.  Per tile every thread takes one record and
-// writes its activation row and output-gradient row transposed into the
-// canonical K-major layout (A: input x record, B: output x record), then one
-// thread issues the K chain of MMAs, D (+)= A B^T, into an FP32 accumulator
+// records in K tiles of kWGK.  Per tile every warp writes the activation and
+// output-gradient rows of 32 records transposed into the canonical K-major
+// layout (A: input x record, B: output x record): a lane loads pairs of
+// adjacent inputs of a record, the fragments of 8x8 blocks, and a transposing
+// matrix store writes a block as one 128-byte core matrix.  Then one thread
+// issues the K chain of MMAs, D (+)= A B^T, into an FP32 accumulator
 // in tensor memory that persists over the CTA's tiles.  M = 128 with input
 // rows 64..127 of A kept zero (lane r of the accumulator = input r); N = 64
 // or 48 outputs.  The CTA's sum is read back once (tcgen05.ld, inputs
-// 0..63 = warps 0 and 1) and added to the FP32 gradient.
+// 0..63 = warps 0 and 1) and added to the FP32 gradient, four weights at a
+// time.  Bound by the 268 MB of rows read (262,144 records; about 39 us from
+// memory, less what the caches still hold): 34 us.  With two-byte stores by a
+// thread per record (four-way bank conflicts) and an addition per weight 88
+// us; matrix stores alone 67, with the next tile's rows loaded during the MMAs
+// 67, and the additions were the rest.
 constexpr int kWGK = 128;                               // records per K tile
 constexpr uint32_t kWGSbo = (kWGK / 8) * 128;           // K = 128: 16 core matrices per 8-row group
 constexpr int kWGABytes = kTcRows * kWGK * 2;           // A tile: 128 x 128 bf16
 constexpr int kWGBBytes = 64 * kWGK * 2;                // B tile: 64 x 128 bf16
 constexpr size_t kWGSmem = kWGABytes + kWGBBytes + 16;  // + barrier, tensor-memory address
+
+// Stores the transposes of four 8x8 blocks of 16-bit elements: lane l holds
+// elements (l / 4, 2 (l % 4)) and the next one of each block; `row` is the
+// shared address of row l % 8 of block l / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t row, const uint32_t v[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(row), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
 
 __global__ void __launch_bounds__(kTcRows) k_nn_wgrad(const NNTrainTask* __restrict__ tasks) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -501,7 +517,7 @@ __global__ void __launch_bounds__(kTcRows) k_nn_wgrad(const NNTrainTask* __restr
     unsigned char* s_b = smem + kWGABytes;
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_b + kWGBBytes);
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + 1);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // zero both tiles once: A's rows 64..127 and B's rows >= nout stay zero
     for (int e = tid; e < (kWGABytes + kWGBBytes) / 16; e += blockDim.x)
         reinterpret_cast<uint4*>(smem)[e] = make_uint4(0u, 0u, 0u, 0u);
@@ -512,21 +528,30 @@ __global__ void __launch_bounds__(kTcRows) k_nn_wgrad(const NNTrainTask* __restr
     uint32_t phase = 0;
     bool ok = true;
     int tiles = 0;
-    for (int r0 = blockIdx.x * kWGK; r0 < n && ok; r0 += gridDim.x * kWGK, tiles++) {
-        const int r = r0 + tid;  // this thread's record = column k = tid of both tiles
+    // a tile's fragments: four times eight of the warp's 32 records
+    uint32_t va[4][8], vg[4][8];
+    auto load = [&](int r0) {
 #pragma unroll
-        for (int g = 0; g < 8; g++) {
-            uint4 va = make_uint4(0u, 0u, 0u, 0u), vg = make_uint4(0u, 0u, 0u, 0u);
-            if (r < n) {
-                va = *reinterpret_cast<const uint4*>(A + (size_t)r * 64 + 8 * g);
-                if (8 * g < nout) vg = *reinterpret_cast<const uint4*>(G + (size_t)r * 64 + 8 * g);
+        for (int q = 0; q < 4; q++) {
+            const int r = r0 + warp * 32 + 8 * q + (lane >> 2);
+#pragma unroll
+            for (int g = 0; g < 8; g++) {
+                const size_t e = (size_t)r * 64 + 8 * g + 2 * (lane & 3);
+                va[q][g] = r < n ? *reinterpret_cast<const uint32_t*>(A + e) : 0u;
+                vg[q][g] = r < n && 8 * g < nout ? *reinterpret_cast<const uint32_t*>(G + e) : 0u;
             }
-            const uint16_t* ea = reinterpret_cast<const uint16_t*>(&va);
-            const uint16_t* eg = reinterpret_cast<const uint16_t*>(&vg);
+        }
+    };
+    load(blockIdx.x * kWGK);
+    for (int r0 = blockIdx.x * kWGK; r0 < n && ok; r0 += gridDim.x * kWGK, tiles++) {
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                *reinterpret_cast<uint16_t*>(s_a + umma_offset(8 * g + q, tid, kWGK)) = ea[q];
-                if (8 * g < nout) *reinterpret_cast<uint16_t*>(s_b + umma_offset(8 * g + q, tid, kWGK)) = eg[q];
+        for (int q = 0; q < 4; q++) {
+#pragma unroll
+            for (int h = 0; h < 8; h += 4) {
+                // row lane % 8 of block lane / 8
+                const uint32_t off = umma_offset(8 * h + lane, warp * 32 + 8 * q, kWGK);
+                stmatrix_x4_trans(a_addr + off, va[q] + h);
+                stmatrix_x4_trans(b_addr + off, vg[q] + h);
             }
         }
         fence_proxy_async_smem();
@@ -540,6 +565,7 @@ __global__ void __launch_bounds__(kTcRows) k_nn_wgrad(const NNTrainTask* __restr
                           umma_desc(b_addr + ks * 2 * kUmmaLBO, kWGSbo), idesc, (tiles > 0 || ks > 0) ? 1u : 0u);
             umma_commit(bar);
         }
+        load(r0 + gridDim.x * kWGK);  // the next tile's, while the MMAs run
         // the tiles are rewritten only after the MMAs that read them completed
         ok = __syncthreads_and(mbar_wait_bounded(bar, phase)) != 0;
         phase ^= 1u;
@@ -552,7 +578,8 @@ __global__ void __launch_bounds__(kTcRows) k_nn_wgrad(const NNTrainTask* __restr
             float v[16];
             tmem_ld16(t_row + (uint32_t)c0, v);
 #pragma unroll
-            for (int k = 0; k < 16; k++) atomicAdd(dst + c0 + k, v[k]);
+            for (int k = 0; k < 16; k += 4)  // rows of 48 or 64 floats: 16-byte aligned
+                atomicAdd(reinterpret_cast<float4*>(dst + c0 + k), make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]));
         }
     }
     tc_end(ok, tmem, bar, phase, status);
