@@ -728,17 +728,6 @@ __device__ __forceinline__ void film_add_nn(unsigned long long* film, size_t pix
     film_add_rgb(film, pix, c.x, c.y, c.z, ctr);
 }
 
-__device__ __forceinline__ int warp_append_nn(int* counter, bool pred) {
-    const unsigned mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return -1;
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    return pred ? base + __popc(mask & ((1u << lane) - 1u)) : -1;
-}
-
 // Vertex record k of a path slot (kNNVert float4): 0: pos xyz, n.x  1: n.yz, wo.xy
 // 2: wo.z, wi xyz  3: p_bsdf(wi), throughput before the bounce (rgb)
 // 4: film total after the vertex's own NEE (rgb), wi valid (non-delta)
@@ -947,45 +936,28 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
 // * the NEE direction, where the shadow ray was unoccluded:
 //   T = lum((S_after_nee_k - S_before_nee_k) / throughput_k).
 // S_after_nee of the last vertex is S_end (its shadow ray resolved before
-// this kernel runs).  visit_records calls emit(vertex record, wi,
-// p_bsdf(wi), T) for every record of the finished path f (slot, traced
-// vertices, recorded vertices).
-template <class Emit>
-__device__ __forceinline__ void visit_records(const NNPathData& PD, int4 f, int max_depth, Emit emit) {
-    const float4 Se = PD.acc[f.x];
-    const size_t vbase = (size_t)f.x * max_depth;
-    for (int k = 0; k < f.z; k++) {
-        const float4* vr = PD.vert + kNNVert * (vbase + k);
-        const float4 v2 = vr[2], v3 = vr[3], v4 = vr[4], v5 = vr[5], v6 = vr[6];
-        const f3 inv = mk(v3.y > 0.f ? 1.0f / v3.y : 0.f, v3.z > 0.f ? 1.0f / v3.z : 0.f,
-                          v3.w > 0.f ? 1.0f / v3.w : 0.f);
-        const f3 after = k < f.z - 1 || k < f.y ? mk(v4.x, v4.y, v4.z) : mk(Se.x, Se.y, Se.z);
-        if (v6.w != 0.f) {
-            const f3 dn = mk(after.x - v5.x, after.y - v5.y, after.z - v5.z);
-            const float T = luminance(mk(dn.x * inv.x, dn.y * inv.y, dn.z * inv.z));
-            if (T > 0.f && isfinite(T)) emit(vr, mk(v6.x, v6.y, v6.z), v5.w, T);
-        }
-        if (k < f.y && v4.w != 0.f) {
-            const f3 dS = mk(Se.x - after.x, Se.y - after.y, Se.z - after.z);
-            const float T = luminance(mk(dS.x * inv.x, dS.y * inv.y, dS.z * inv.z));
-            if (T > 0.f && isfinite(T)) emit(vr, mk(v2.y, v2.z, v2.w), v3.x, T);
-        }
-    }
-}
-
-// Finished paths: records are counted first, then one atomic per warp (all
-// lanes of the same job; per lane otherwise) reserves room in the job's
-// record buffer, then they are written (records beyond the buffer's
-// capacity are dropped); the slots go back to the free list.
-__global__ void __launch_bounds__(256) k_finish_nn(NNPathData PD, WaveCounters* ctr,
+// this kernel runs).
+//
+// A thread takes a recorded vertex of one of its CTA's finished paths, found
+// in the running total of their vertices: it yields up to two records, room
+// for which is reserved in the job's buffer by one atomic per CTA and 256
+// vertices (per lane in a CTA where several jobs meet; jobs are rendered in
+// order, so that is rare).  Records beyond the buffer's capacity are dropped.
+// The slots go back to the free list.  With a thread per path, which walked
+// its vertices twice (to count, then to write), and an atomic per warp,
+// the kernel waited on those chains: 551 -> 431 us in the 16 launches of a 640x360,
+// 4-spp training render (four vertices a thread at a time: 411, the render the same).
+constexpr int kFinishNNThreads = 256;
+__global__ void __launch_bounds__(kFinishNNThreads) k_finish_nn(NNPathData PD, WaveCounters* ctr,
                                                    const DevNNJob* __restrict__ nnj, int max_depth) {
     after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = ctr->n_fin;
-    if ((int)(blockIdx.x * blockDim.x) >= n) return;  // an empty CTA of the capacity's grid
-    const unsigned lane = threadIdx.x & 31u;
+    constexpr int kWarps = kFinishNNThreads / 32;
+    const int n = ctr->n_fin, first = (int)(blockIdx.x * blockDim.x);
+    if (first >= n) return;  // an empty CTA of the capacity's grid
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = first + (int)threadIdx.x;
     const bool release = i < n;
-    int4 f = make_int4(0, 0, 0, 0);
+    int4 f = make_int4(0, 0, 0, 0);  // slot, traced vertices, recorded vertices
     if (release) f = PD.fin[i];
     bool records = release && PD.rec_cap > 0;
     const int job = records ? PD.slot_job[f.x] : -1;
@@ -1003,41 +975,103 @@ __global__ void __launch_bounds__(256) k_finish_nn(NNPathData PD, WaveCounters* 
             records = (float)(h >> 8) * (1.0f / 16777216.0f) < keep;
         }
     }
-    int count = 0;
-    if (records) visit_records(PD, f, max_depth, [&](const float4*, f3, float, float) { count++; });
-    // one job for the whole warp (the usual case: jobs are rendered in order)?
-    const int job0 = __shfl_sync(0xffffffffu, job, 0);
-    const bool uniform = __all_sync(0xffffffffu, job == job0 || job < 0);
-    int base = 0, incl = count;
-    if (uniform) {
+    __shared__ int s_first[kFinishNNThreads], s_job[kFinishNNThreads], s_total[kWarps], s_lead[kWarps], s_base, s_free;
+    __shared__ int4 s_f[kFinishNNThreads];
+    // inclusive sums over the warp and, with s_total, the CTA
+    auto warp_scan = [&](int v) {
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (unsigned)o) incl += v;
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
         }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        const int lead_job = __reduce_max_sync(0xffffffffu, (unsigned)(job + 1)) - 1;
-        if (lane == 31 && total > 0) base = atomicAdd(nnj[lead_job].n_rec, total);
-        base = __shfl_sync(0xffffffffu, base, 31) + incl - count;
-    } else if (count > 0) {
-        base = atomicAdd(nnj[job].n_rec, count);
+        return v;
+    };
+    const int nv = records ? f.z : 0;
+    int incl = warp_scan(nv);
+    const int lead = __reduce_max_sync(0xffffffffu, (unsigned)(job + 1)) - 1;
+    const bool uniform = __all_sync(0xffffffffu, job == lead || job < 0);
+    if (lane == 31) {
+        s_total[warp] = incl;
+        s_lead[warp] = uniform ? lead : -2;
     }
-    if (records && count > 0) {
-        const DevNNJob& Jn = nnj[job];
-        int r = base;
-        visit_records(PD, f, max_depth, [&](const float4* vr, f3 wi, float pb, float T) {
-            if (r < Jn.rec_cap) {
-                float4* o = Jn.rec + 4 * (size_t)r;
-                o[0] = vr[0];
-                o[1] = vr[1];
-                o[2] = make_float4(vr[2].x, wi.x, wi.y, wi.z);
-                o[3] = make_float4(pb, T, 0.f, 0.f);
+    s_job[threadIdx.x] = job;
+    s_f[threadIdx.x] = f;
+    if (threadIdx.x == 0) s_free = atomicAdd(&ctr->free_top, min(kFinishNNThreads, n - first));
+    __syncthreads();
+    int before = 0, n_verts = 0, cta_job = -1;
+    bool one_job = true;
+    for (int w = 0; w < kWarps; w++) {
+        if (w < warp) before += s_total[w];
+        n_verts += s_total[w];
+        if (s_lead[w] == -1) continue;
+        if (s_lead[w] == -2 || (cta_job >= 0 && s_lead[w] != cta_job)) one_job = false;
+        cta_job = s_lead[w];
+    }
+    s_first[threadIdx.x] = before + incl - nv;
+    if (release) PD.slot_stack[s_free + (int)threadIdx.x] = f.x;
+    for (int j0 = 0; j0 < n_verts; j0 += kFinishNNThreads) {
+        __syncthreads();  // s_first is there; the chunk before has read s_total and s_base
+        const int j = j0 + (int)threadIdx.x;
+        float T1 = 0.f, T2 = 0.f;
+        float4 r0, r1, v2, v3, v5, v6;
+        int rjob = -1;
+        if (j < n_verts) {
+            int path = 0;  // the last one that starts at or before j; those without vertices start with their successor
+            for (int step = kFinishNNThreads / 2; step > 0; step >>= 1)
+                if (s_first[path + step] <= j) path += step;
+            const int k = j - s_first[path];
+            const int4 g = s_f[path];
+            rjob = s_job[path];
+            const float4* vr = PD.vert + kNNVert * ((size_t)g.x * max_depth + k);
+            const float4 Se = PD.acc[g.x], v4 = vr[4];
+            r0 = vr[0], r1 = vr[1], v2 = vr[2], v3 = vr[3], v5 = vr[5], v6 = vr[6];
+            const f3 inv = mk(v3.y > 0.f ? 1.0f / v3.y : 0.f, v3.z > 0.f ? 1.0f / v3.z : 0.f,
+                              v3.w > 0.f ? 1.0f / v3.w : 0.f);
+            const f3 after = k < g.z - 1 || k < g.y ? mk(v4.x, v4.y, v4.z) : mk(Se.x, Se.y, Se.z);
+            if (v6.w != 0.f) {
+                const f3 dn = mk(after.x - v5.x, after.y - v5.y, after.z - v5.z);
+                const float T = luminance(mk(dn.x * inv.x, dn.y * inv.y, dn.z * inv.z));
+                if (T > 0.f && isfinite(T)) T1 = T;
             }
-            r++;
-        });
+            if (k < g.y && v4.w != 0.f) {
+                const f3 dS = mk(Se.x - after.x, Se.y - after.y, Se.z - after.z);
+                const float T = luminance(mk(dS.x * inv.x, dS.y * inv.y, dS.z * inv.z));
+                if (T > 0.f && isfinite(T)) T2 = T;
+            }
+        }
+        const int count = (T1 > 0.f) + (T2 > 0.f);
+        int r = 0;
+        if (one_job) {
+            incl = warp_scan(count);
+            if (lane == 31) s_total[warp] = incl;
+            __syncthreads();
+            int below = 0, total = 0;
+            for (int w = 0; w < kWarps; w++) {
+                if (w < warp) below += s_total[w];
+                total += s_total[w];
+            }
+            if (threadIdx.x == 0 && total > 0) s_base = atomicAdd(nnj[cta_job].n_rec, total);
+            __syncthreads();
+            r = s_base + below + incl - count;
+        } else if (count > 0) {
+            r = atomicAdd(nnj[rjob].n_rec, count);
+        }
+        if (count > 0) {
+            const DevNNJob& J = nnj[rjob];
+            auto emit = [&](f3 wi, float pb, float T) {
+                if (r < J.rec_cap) {
+                    float4* o = J.rec + 4 * (size_t)r;
+                    o[0] = r0;
+                    o[1] = r1;
+                    o[2] = make_float4(v2.x, wi.x, wi.y, wi.z);
+                    o[3] = make_float4(pb, T, 0.f, 0.f);
+                }
+                r++;
+            };
+            if (T1 > 0.f) emit(mk(v6.x, v6.y, v6.z), v5.w, T1);
+            if (T2 > 0.f) emit(mk(v2.y, v2.z, v2.w), v3.x, T2);
+        }
     }
-    const int jr = warp_append_nn(&ctr->free_top, release);
-    if (release) PD.slot_stack[jr] = f.x;
 }
 
 // NEE shadow rays of the learned-guide integrator: unoccluded contributions
@@ -1184,7 +1218,7 @@ void launch_nn_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const 
 }
 void launch_nn_finish(const NNPathData& PD, WaveCounters* ctr, const DevNNJob* nnj, int max_depth, int capacity,
                       cudaStream_t st) {
-    launch_after(k_finish_nn, (capacity + 255) / 256, 256, 0, st, PD, ctr, nnj, max_depth);
+    launch_after(k_finish_nn, (capacity + kFinishNNThreads - 1) / kFinishNNThreads, kFinishNNThreads, 0, st, PD, ctr, nnj, max_depth);
 }
 
 }  // namespace cpppt_gb300

@@ -225,3 +225,31 @@ def test_frozen_render_after_other_renders(gpu_lib, spp):
     gs.nn_reset(3)
     again = gs.render(spp, max_depth=6, seed=2, mode=MODE_NN, flags=FLAG_NN_FREEZE)
     assert np.array_equal(again.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("res,spp,depth", [((1, 1), 1, 4), ((16, 16), 1, 1), ((257, 1), 1, 8), ((64, 33), 9, 15)],
+                         ids=["one_path", "full_block", "partial_block", "many_blocks"])
+def test_training_render_at_block_edges(gpu_lib, res, spp, depth):
+    """Records of the finished paths, taken per CTA: a training render that
+    ends in one round renders what a frozen guide of the same weights does,
+    and trains finite weights; two jobs of two scenes in one batch train both."""
+    from cpppt import scenes
+    from cpppt.lib import FLAG_NN_FREEZE, MODE_NN, GpuBatch, GpuScene
+    sc = scenes.slit_room(n_boxes=20, width=res[0], height=res[1])
+    train, frozen = GpuScene(sc), GpuScene(sc)
+    train.nn_configure(batch=1024)  # whole batches only are trained on
+    a = train.render(spp, max_depth=depth, seed=3, mode=MODE_NN)
+    b = frozen.render(spp, max_depth=depth, seed=3, mode=MODE_NN, flags=FLAG_NN_FREEZE)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    w, w0 = train.nn_weights(), frozen.nn_weights()
+    assert np.isfinite(w).all()
+    if spp * res[0] * res[1] > 1000:
+        assert not np.array_equal(w, w0)
+    pair = [GpuScene(sc), GpuScene(scenes.cornell(*res))]
+    batch = GpuBatch(pair)
+    jobs = [dict(scene=k, spp=spp, max_depth=depth, seed=3) for k in (0, 1, 0)]
+    imgs = batch.render(jobs, mode=MODE_NN)
+    assert all(np.isfinite(x).all() for x in imgs)
+    if depth <= 8:  # as one job: nothing trains before the round's end
+        assert np.array_equal(imgs[0].view(np.uint32), a.view(np.uint32))
+    assert all(np.isfinite(s.nn_weights()).all() for s in pair)
