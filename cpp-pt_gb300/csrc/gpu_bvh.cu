@@ -4,7 +4,8 @@
 //
 // Level-synchronous: every node of one tree level is a segment [start,
 // start + count) of the primitive array, processed by one CTA of 128
-// threads (nodes of more than kBigSeg primitives by several, k_big_*), which
+// threads (nodes of more than kBigSeg primitives by several, k_big_*; nodes of
+// at most 32 by a warp, level_warp), which
 //   1. reduces the node's bounds and centroid bounds,
 //   2. bins the centroids into 5 equal-width bins per axis (a primitive
 //      joins the first bin j with c < min + (max - min) * (j + 1) / 5) and
@@ -152,10 +153,12 @@ struct ChunkG {
     int32_t big, index;  // kBigChunk primitives from index * kBigChunk on
 };
 
-// The next level's segments, and its large nodes with their chunks.
-// counts: [0] segments, [1] nodes, [2] large nodes, [3] chunks
+// The next level's segments, those of at most 32 primitives in a list of
+// their own, and its large nodes with their chunks.
+// counts: [0] segments, [1] nodes, [2] large nodes, [3] chunks, [4] small segments
 struct LevelOut {
     SegG* segs;
+    SegG* small;
     BigG* big;
     ChunkG* chunks;
     int* counts;
@@ -163,8 +166,12 @@ struct LevelOut {
 
 __device__ __forceinline__ bool comp_is_min(int comp) { return comp < 3; }
 
-__device__ void emit_seg(const LevelOut& L, int k, const SegG& c) {
-    L.segs[k] = c;
+__device__ void emit_seg(const LevelOut& L, const SegG& c) {
+    if (c.count <= 32) {
+        L.small[atomicAdd(L.counts + 4, 1)] = c;
+        return;
+    }
+    L.segs[atomicAdd(L.counts, 1)] = c;
     if (c.count <= kBigSeg) return;
     const int bi = atomicAdd(L.counts + 2, 1), n = (c.count + kBigChunk - 1) / kBigChunk;
     BigG& B = L.big[bi];
@@ -177,7 +184,7 @@ __device__ void emit_seg(const LevelOut& L, int k, const SegG& c) {
     for (int j = 0; j < n; j++) L.chunks[B.first + j] = ChunkG{bi, j};
 }
 
-__global__ void k_root(LevelOut L, int n) { emit_seg(L, 0, SegG{0, n, -1, 0}); }
+__global__ void k_root(LevelOut L, int n) { emit_seg(L, SegG{0, n, -1, 0}); }
 
 // The 12 bounds keys of P[begin, end), reduced over a warp.
 __device__ __forceinline__ void bounds_keys(const PrimG* __restrict__ P, int begin, int end, unsigned long long k[12]) {
@@ -313,9 +320,8 @@ __device__ void emit_node(const SegG& seg, const float bounds[6], int nl, NodeG*
     nd.child[0] = nd.child[1] = -1;
     nodes[nid] = nd;
     if (seg.parent >= 0) nodes[seg.parent].child[seg.side] = nid;
-    const int k = atomicAdd(L.counts, 2);
-    emit_seg(L, k, SegG{seg.start, nl, nid, 0});
-    emit_seg(L, k + 1, SegG{seg.start + nl, seg.count - nl, nid, 1});
+    emit_seg(L, SegG{seg.start, nl, nid, 0});
+    emit_seg(L, SegG{seg.start + nl, seg.count - nl, nid, 1});
 }
 
 // P[begin, end) into Q in the bins' concatenation order (bin 0's primitives,
@@ -355,8 +361,192 @@ __device__ __forceinline__ void scatter_bins(const PrimG* __restrict__ P, PrimG*
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_level(const SegG* __restrict__ segs, const PrimG* __restrict__ pin,
-                                                    PrimG* __restrict__ pout, NodeG* __restrict__ nodes, LevelOut L,
+__device__ __forceinline__ float okey_value(uint32_t k) {
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+// One level of the nodes of at most 32 primitives, a warp each with a primitive per
+// lane and no barriers but the two around the CTA's additions to the counters.
+// Children of fewer than 4 primitives become leaves at once.  Bound by the
+// latency of its chain of warp reductions.  With a CTA of 128 threads, and two
+// atomics on the counters, per node (and leaf) scene creation took 11.1 ms for
+// the 192k-triangle room, now 10.4; 1M-triangle soup 22.8, now 18.9.
+//
+// The bounds are the reference's floats (the later of equal values); the bins'
+// boxes only enter costs, where -0.0 and +0.0 give the same.
+__device__ __forceinline__ void level_warp(const SegG* __restrict__ small, int n_small, int block,
+                                           const PrimG* __restrict__ pin, PrimG* __restrict__ pout,
+                                           NodeG* __restrict__ nodes, const LevelOut& L,
+                                           int32_t* __restrict__ final_id, int32_t* __restrict__ leaf_parent) {
+    constexpr unsigned full = 0xffffffffu;
+    const float inf = __int_as_float(0x7f800000);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w = block * kWarps + warp;
+    SegG seg{0, 0, -1, 0};
+    if (w < n_small) seg = small[w];
+    const int n = seg.count;
+    const bool on = lane < n;
+    PrimG p{};
+    if (on) p = pin[seg.start + lane];
+    float bound[6];  // lo xyz, hi xyz
+    int nl = 0, bin = -1;  // primitives of the first partition; this one's bin on the chosen axis
+    if (n >= 4) {  // fewer: a leaf (bvh.h:152-158)
+        uint32_t kl[3], kh[3];
+        float cb[6];  // centroid bounds
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const uint32_t kc = okey(p.c[j]);
+            kl[j] = okey(p.lo[j]);
+            kh[j] = okey(p.hi[j]);
+            auto later = [&](uint32_t key, uint32_t best, float v) {  // the last lane that holds the best key
+                return __shfl_sync(full, v, 31 - __clz(__ballot_sync(full, on && key == best)));
+            };
+            bound[j] = later(kl[j], __reduce_min_sync(full, on ? kl[j] : full), p.lo[j]);
+            bound[3 + j] = later(kh[j], __reduce_max_sync(full, on ? kh[j] : 0u), p.hi[j]);
+            cb[j] = later(kc, __reduce_min_sync(full, on ? kc : full), p.c[j]);
+            cb[3 + j] = later(kc, __reduce_max_sync(full, on ? kc : 0u), p.c[j]);
+        }
+        // thresholds: lane 4 axis + j
+        const int ax = (lane >> 2) % 3;
+        const float t = bin_threshold(ax == 0 ? cb[0] : (ax == 1 ? cb[1] : cb[2]),
+                                      ax == 0 ? cb[3] : (ax == 1 ? cb[4] : cb[5]), lane & 3);
+        // bins: lane kBins axis + b holds bin b's count and box
+        int b[3], cnt = 0;
+        float blo[3] = {inf, inf, inf}, bhi[3] = {-inf, -inf, -inf};
+#pragma unroll
+        for (int axis = 0; axis < 3; axis++) {
+            float thr[kBins - 1];
+#pragma unroll
+            for (int j = 0; j < kBins - 1; j++) thr[j] = __shfl_sync(full, t, 4 * axis + j);
+            b[axis] = on ? bin_of(p.c[axis], thr) : -1;
+#pragma unroll
+            for (int q = 0; q < kBins; q++) {
+                const bool in = b[axis] == q, mine = lane == kBins * axis + q;
+                const unsigned m = __ballot_sync(full, in);
+                if (m == 0) continue;
+                if (mine) cnt = __popc(m);
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const uint32_t lo = __reduce_min_sync(full, in ? kl[j] : full);
+                    const uint32_t hi = __reduce_max_sync(full, in ? kh[j] : 0u);
+                    if (mine) {
+                        blo[j] = okey_value(lo);
+                        bhi[j] = okey_value(hi);
+                    }
+                }
+            }
+        }
+        // split costs (bvh.h:57-149): lane 4 axis + i splits after bin i
+        const int i = lane & 3;
+        float llo[3] = {inf, inf, inf}, lhi[3] = {-inf, -inf, -inf}, rlo[3] = {inf, inf, inf}, rhi[3] = {-inf, -inf, -inf};
+        int lc = 0, rc = 0;
+#pragma unroll
+        for (int q = 0; q < kBins; q++) {
+            const int src = kBins * ax + q, c = __shfl_sync(full, cnt, src);
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const float lo = __shfl_sync(full, blo[j], src), hi = __shfl_sync(full, bhi[j], src);
+                if (c == 0) continue;
+                if (q <= i) {
+                    llo[j] = vmin1(llo[j], lo);
+                    lhi[j] = vmax1(lhi[j], hi);
+                } else {
+                    rlo[j] = vmin1(rlo[j], lo);
+                    rhi[j] = vmax1(rhi[j], hi);
+                }
+            }
+            if (q <= i) lc += c;
+            else rc += c;
+        }
+        const float pc = (lc == 0 || rc == 0) ? inf : __fadd_rn(ref_area(llo, lhi), ref_area(rlo, rhi));
+        float cost[3];
+        int best[3];
+#pragma unroll
+        for (int axis = 0; axis < 3; axis++) {  // the first strict minimum
+            cost[axis] = __shfl_sync(full, pc, 4 * axis);
+            best[axis] = 0;
+#pragma unroll
+            for (int j = 1; j < kBins - 1; j++) {
+                const float c = __shfl_sync(full, pc, 4 * axis + j);
+                if (c < cost[axis]) {
+                    cost[axis] = c;
+                    best[axis] = j;
+                }
+            }
+        }
+        const int axis = pick_axis(cost);
+        bin = axis == 0 ? b[0] : (axis == 1 ? b[1] : b[2]);
+        const int last = axis == 0 ? best[0] : (axis == 1 ? best[1] : best[2]);
+        nl = __popc(__ballot_sync(full, on && bin <= last));
+    }
+    const bool split = nl > 0 && nl < n;
+    const int nr = n - nl;
+    const int kids = split ? (nl >= 4) + (nr >= 4) : 0;
+    __shared__ int s_split[kWarps], s_kids[kWarps], s_node, s_seg;
+    if (lane == 0) {
+        s_split[warp] = split;
+        s_kids[warp] = kids;
+    }
+    __syncthreads();
+    int node = 0, kid = 0, n_nodes = 0, n_kids = 0;
+    for (int v = 0; v < kWarps; v++) {
+        if (v < warp) {
+            node += s_split[v];
+            kid += s_kids[v];
+        }
+        n_nodes += s_split[v];
+        n_kids += s_kids[v];
+    }
+    if (threadIdx.x == 0 && n_nodes > 0) s_node = atomicAdd(L.counts + 1, n_nodes);
+    if (threadIdx.x == 32 && n_kids > 0) s_seg = atomicAdd(L.counts + 4, n_kids);
+    __syncthreads();
+    if (!split) {
+        if (on) {
+            final_id[seg.start + lane] = p.id;
+            leaf_parent[seg.start + lane] = seg.parent;
+        }
+        return;
+    }
+    node += s_node;
+    kid += s_seg;
+    if (lane == 0) {
+        NodeG nd;
+        for (int j = 0; j < 3; j++) {
+            nd.lo[j] = bound[j];
+            nd.hi[j] = bound[3 + j];
+        }
+        nd.parent = seg.parent;
+        nd.side = seg.side;
+        nd.child[0] = nd.child[1] = -1;
+        nodes[node] = nd;
+        if (seg.parent >= 0) nodes[seg.parent].child[seg.side] = node;
+        if (nl >= 4) L.small[kid++] = SegG{seg.start, nl, node, 0};
+        if (nr >= 4) L.small[kid] = SegG{seg.start + nl, nr, node, 1};
+    }
+    // the bins' concatenation order (bvh.h:138-144)
+    int pos = 0, before = 0;
+#pragma unroll
+    for (int q = 0; q < kBins; q++) {
+        const unsigned m = __ballot_sync(full, bin == q);
+        if (bin == q) pos = before + __popc(m & ((1u << lane) - 1u));
+        before += __popc(m);
+    }
+    if (on) {
+        if ((pos < nl ? nl : nr) < 4) {
+            final_id[seg.start + pos] = p.id;
+            leaf_parent[seg.start + pos] = node;
+        } else {
+            pout[seg.start + pos] = p;
+        }
+    }
+}
+
+// One level: a CTA per node of the list, then CTAs of kWarps small nodes each
+// (one launch: a second one per level cost a 10k-triangle scene 0.15 ms).
+__global__ void __launch_bounds__(kThreads) k_level(const SegG* __restrict__ segs, int n_seg,
+                                                    const SegG* __restrict__ small, int n_small,
+                                                    const PrimG* __restrict__ pin, PrimG* __restrict__ pout,
+                                                    NodeG* __restrict__ nodes, LevelOut L,
                                                     int32_t* __restrict__ final_id, int32_t* __restrict__ leaf_parent) {
     __shared__ unsigned long long s_red[kWarps][12];
     __shared__ float s_bounds[12];  // lo xyz, hi xyz, centroid lo xyz, centroid hi xyz
@@ -366,6 +556,10 @@ __global__ void __launch_bounds__(kThreads) k_level(const SegG* __restrict__ seg
     __shared__ int s_axis, s_leaf;
     __shared__ float s_thr[3][kBins - 1];
     __shared__ int s_wbin[kWarps][kBins];
+    if ((int)blockIdx.x >= n_seg) {
+        level_warp(small, n_small, (int)blockIdx.x - n_seg, pin, pout, nodes, L, final_id, leaf_parent);
+        return;
+    }
     const SegG seg = segs[blockIdx.x];
     if (seg.count > kBigSeg) return;  // k_big_*
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -378,10 +572,6 @@ __global__ void __launch_bounds__(kThreads) k_level(const SegG* __restrict__ seg
             leaf_parent[seg.start + i] = seg.parent;
         }
     };
-    if (n < 4) {  // bvh.h:152-158
-        emit_leaf();
-        return;
-    }
     // 1. bounds and centroid bounds
     {
         unsigned long long k[12];
@@ -620,7 +810,7 @@ RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& sc
                        RefBuildStats* stats) {
     std::vector<void*>& owned = scratch.v;
     int* h_cnt = nullptr;  // pinned: LevelOut::counts
-    ck(cudaMallocHost(&h_cnt, 4 * sizeof(int)), "cudaMallocHost");
+    ck(cudaMallocHost(&h_cnt, 5 * sizeof(int)), "cudaMallocHost");
     struct FreeHost {
         int* p;
         ~FreeHost() { cudaFreeHost(p); }
@@ -631,7 +821,8 @@ RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& sc
     const int max_nodes = n;
     NodeG* nodes = dmalloc<NodeG>(owned, max_nodes);
     SegG* segs[2] = {dmalloc<SegG>(owned, n + 2), dmalloc<SegG>(owned, n + 2)};
-    int* d_cnt = dmalloc<int>(owned, 4);  // LevelOut::counts
+    SegG* small[2] = {dmalloc<SegG>(owned, n + 2), dmalloc<SegG>(owned, n + 2)};
+    int* d_cnt = dmalloc<int>(owned, 5);  // LevelOut::counts
     const int max_big = n / kBigSeg + 1, max_chunks = n / kBigChunk + max_big + 1;
     BigG* big[2] = {dmalloc<BigG>(owned, max_big), dmalloc<BigG>(owned, max_big)};
     ChunkG* chunks[2] = {dmalloc<ChunkG>(owned, max_chunks), dmalloc<ChunkG>(owned, max_chunks)};
@@ -639,17 +830,18 @@ RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& sc
     int32_t* final_id = dmalloc<int32_t>(owned, n);
     int32_t* leaf_parent = dmalloc<int32_t>(owned, n);
     k_prims<<<(n + 255) / 256, 256, 0, st>>>(d_tv, n, buf[0]);
-    ck(cudaMemsetAsync(d_cnt, 0, 4 * sizeof(int), st), "memset");
-    k_root<<<1, 1, 0, st>>>(LevelOut{segs[0], big[0], chunks[0], d_cnt}, n);
+    ck(cudaMemsetAsync(d_cnt, 0, 5 * sizeof(int), st), "memset");
+    k_root<<<1, 1, 0, st>>>(LevelOut{segs[0], small[0], big[0], chunks[0], d_cnt}, n);
     std::vector<int> level_nodes(1, 0);  // node count after each level
-    int n_seg = 1, cur = 0, levels = 0;
+    int n_seg = n > 32 ? 1 : 0, n_small = n > 32 ? 0 : 1, cur = 0, levels = 0;
     int n_big = n > kBigSeg ? 1 : 0, n_chunks = n_big ? (n + kBigChunk - 1) / kBigChunk : 0;
-    while (n_seg > 0) {
-        const LevelOut L{segs[1 - cur], big[1 - cur], chunks[1 - cur], d_cnt};
+    while (n_seg > 0 || n_small > 0) {
+        const LevelOut L{segs[1 - cur], small[1 - cur], big[1 - cur], chunks[1 - cur], d_cnt};
         // all but the node count
         ck(cudaMemsetAsync(d_cnt, 0, sizeof(int), st), "memset");
-        ck(cudaMemsetAsync(d_cnt + 2, 0, 2 * sizeof(int), st), "memset");
-        k_level<<<n_seg, kThreads, 0, st>>>(segs[cur], buf[cur], buf[1 - cur], nodes, L, final_id, leaf_parent);
+        ck(cudaMemsetAsync(d_cnt + 2, 0, 3 * sizeof(int), st), "memset");
+        k_level<<<n_seg + (n_small + kWarps - 1) / kWarps, kThreads, 0, st>>>(
+            segs[cur], n_seg, small[cur], n_small, buf[cur], buf[1 - cur], nodes, L, final_id, leaf_parent);
         if (n_big > 0) {
             k_big_bounds<<<n_chunks, kBigThreads, 0, st>>>(chunks[cur], big[cur], buf[cur]);
             k_big_bins<<<n_chunks, kBigThreads, 0, st>>>(chunks[cur], big[cur], buf[cur], chunk_cnt);
@@ -658,13 +850,14 @@ RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& sc
                                                             final_id, leaf_parent);
         }
         ck(cudaGetLastError(), "level kernels");
-        ck(cudaMemcpyAsync(h_cnt, d_cnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, st), "counts");
+        ck(cudaMemcpyAsync(h_cnt, d_cnt, 5 * sizeof(int), cudaMemcpyDeviceToHost, st), "counts");
         ck(cudaStreamSynchronize(st), "level");
         n_seg = h_cnt[0];
         n_big = h_cnt[2];
         n_chunks = h_cnt[3];
+        n_small = h_cnt[4];
         level_nodes.push_back(h_cnt[1]);
-        if (h_cnt[1] > max_nodes || n_seg > n + 2 || n_big > max_big || n_chunks > max_chunks)
+        if (h_cnt[1] > max_nodes || n_seg > n + 2 || n_small > n + 2 || n_big > max_big || n_chunks > max_chunks)
             throw std::runtime_error("device BVH build overflow");
         cur = 1 - cur;
         levels++;

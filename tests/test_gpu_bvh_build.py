@@ -70,6 +70,18 @@ def test_device_build_full_size(gpu_lib, make):
     _same(lib.ref_topology_device(sc), lib.ref_topology(sc))
 
 
+@pytest.mark.parametrize("n", [1, 3, 4, 7, 31, 32, 33, 34, 65, 129, 2047, 2048, 2049])
+def test_device_build_at_node_size_limits(gpu_lib, n):
+    """A leaf, a warp's node (up to 32), a CTA's (up to 2048), several CTAs'."""
+    from dataclasses import replace
+
+    from cpppt import lib
+    sc = scenes.soup(seed=3, n_spheres=40, freq=3, width=8, height=8)
+    tris = np.random.default_rng(n).permutation(sc.triangles)[:n]
+    sc = replace(sc, triangles=np.ascontiguousarray(tris))  # geometry only: the tree builds read nothing else
+    _same(lib.ref_topology_device(sc), lib.ref_topology(sc))
+
+
 def _same_wide(sc):
     from cpppt import lib
     dn, do, dd, df = lib.wide_bvh(sc, on_device=True)
