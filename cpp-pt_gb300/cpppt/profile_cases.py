@@ -28,10 +28,10 @@ from .lib import FLAG_NN_FREEZE, FLAG_TIME_KERNELS, FLAG_UNBIASED_MIS, MODE_MIS,
 
 def case_extend():
     """Renders with PT_FLAG_TIME_KERNELS: the same kernels launched one by one
-    (16 iterations per round) instead of inside the device-driven graph,
+    (20 iterations per round) instead of inside the device-driven graph,
     whose kernel nodes ncu cannot capture (a graph with a conditional node);
     each render here takes one round, so the second render's extension
-    launches start at launch 16."""
+    launches start at launch 20."""
     gs = GpuScene(scenes.soup(seed=2, width=1280, height=720))
     for _ in range(2):
         gs.render(1, max_depth=10, seed=1, mode=MODE_MIS, flags=FLAG_TIME_KERNELS)

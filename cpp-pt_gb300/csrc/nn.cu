@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
 // The slots go back to the free list.  With a thread per path, which walked
 // its vertices twice (to count, then to write), and an atomic per warp,
 // the kernel waited on those chains: 551 -> 431 us in the 16 launches of a 640x360,
-// 4-spp training render (four vertices a thread at a time: 411, the render the same).
+// 8-spp training render (four vertices a thread at a time: 411, the render the same).
 constexpr int kFinishNNThreads = 256;
 __global__ void __launch_bounds__(kFinishNNThreads) k_finish_nn(NNPathData PD, WaveCounters* ctr,
                                                    const DevNNJob* __restrict__ nnj, int max_depth) {
