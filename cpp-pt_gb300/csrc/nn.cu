@@ -156,14 +156,21 @@ __device__ __forceinline__ void tc_stage_wt(const __nv_bfloat16* wt, unsigned ch
     }
 }
 
-// get_in(i, NNIn& in, int& job) -> bool valid, with in.pn NOT yet
-// normalised (world position); put(i, const float* prm41).  All kTcRows
-// threads of the CTA must call it.  status: kStatusTensorTimeout when a
-// completion wait runs out (the CTA then stops, frees its tensor memory and
-// returns).
-template <bool ONEBLOB, class GetIn, class Put>
+// input: reads a sample's input in four steps, each of which uses what the one
+// before loaded -- first(i), second(), third(), last(NNIn&, int& job) -> bool
+// valid, with pn NOT yet normalised (world position); put(i, const float*
+// prm41).  All kTcRows threads of the CTA must call it.  status:
+// kStatusTensorTimeout when a completion wait runs out (the CTA then stops,
+// frees its tensor memory and returns).
+// A tile's steps run between the layers of the tile before it: 16 warps per SM
+// (shared memory holds the weights of four CTAs) do not hide a chain of three
+// loads.  k_nn_infer in a 640x360, 8-spp training render 1126 -> 1030 us (in two
+// steps 1071), guided 1280x720 9.88 -> 9.69 ms.  The one-blob encoding leaves no
+// registers for it (128 at four CTAs; 8.88 -> 8.91 ms with it), so there a
+// tile's steps run when the one before is done.
+template <bool ONEBLOB, class Input, class Put>
 __device__ __forceinline__ void tc_infer_loop(int n, unsigned char* smem, const DevNNJob* __restrict__ nnj,
-                                              uint32_t* status, GetIn get_in, Put put) {
+                                              uint32_t* status, Input input, Put put) {
     unsigned char* s_w = smem;
     unsigned char* s_a = smem + kNNLayers * kTcWLayerBytes;
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_a + kTcABytes);
@@ -177,13 +184,22 @@ __device__ __forceinline__ void tc_infer_loop(int n, unsigned char* smem, const 
     uint32_t phase = 0;
     bool ok = true;
     const __nv_bfloat16* staged = nullptr;
-    for (int base = blockIdx.x * kTcRows; base < n && ok; base += gridDim.x * kTcRows) {
-        const int i = base + row;
-        NNIn in;
-        in.pn = in.n = in.wo = mk(0.f, 0.f, 0.f);
-        int job = -1;
-        const bool valid = i < n && get_in(i, in, job);
-        bool pending = valid;
+    constexpr bool ahead = !ONEBLOB;
+    const int stride = gridDim.x * kTcRows;
+    int i = blockIdx.x * kTcRows + row;
+    NNIn in;
+    in.pn = in.n = in.wo = mk(0.f, 0.f, 0.f);
+    int job = -1;
+    if (i < n) {
+        input.first(i);
+        input.second();
+        input.third();
+    }
+    bool pending = i < n && input.last(in, job);
+    for (int base = blockIdx.x * kTcRows; base < n && ok; base += stride, i += stride) {
+        const bool more = i + stride < n;
+        int step = ahead ? 0 : 2;  // of the next tile's input
+        if (ahead && more) input.first(i + stride);
         while (ok) {
             // smallest job among the rows still waiting
             if (threadIdx.x == 0) *s_job = 0x7fffffff;
@@ -214,6 +230,13 @@ __device__ __forceinline__ void tc_infer_loop(int n, unsigned char* smem, const 
                 for (int c = 0; c < 64; c += 16)
                     if (c < nout) tmem_ld16(t_row + (uint32_t)c, v + c);
                 if (l < kNNLayers - 1) tc_store_row(s_a, row, v, true);
+                if (ahead && l == 0 && step == 0) {
+                    if (more) input.second();
+                    step = 1;
+                } else if (ahead && l == 1 && step == 1) {
+                    if (more) input.third();
+                    step = 2;
+                }
             }
             if (ok && mine) {
                 float prm[kNNParams];
@@ -222,9 +245,75 @@ __device__ __forceinline__ void tc_infer_loop(int n, unsigned char* smem, const 
             }
             pending = pending && !mine;
         }
+        if (more && (!ahead || step == 0)) {  // step == 0: a tile without work
+            if (!ahead) input.first(i + stride);
+            input.second();
+            input.third();
+        }
+        in.pn = in.n = in.wo = mk(0.f, 0.f, 0.f);
+        job = -1;
+        pending = more && input.last(in, job);
     }
     tc_end(ok, tmem, bar, phase, status);
 }
+
+struct DebugInput {
+    const float* in;
+    const float* p;
+    __device__ __forceinline__ void first(int i) { p = in + 9 * (size_t)i; }
+    __device__ __forceinline__ void second() {}
+    __device__ __forceinline__ void third() {}
+    __device__ __forceinline__ bool last(NNIn& v, int& job) {
+        v.pn = mk(p[0], p[1], p[2]);
+        v.n = mk(p[3], p[4], p[5]);
+        v.wo = mk(p[6], p[7], p[8]);
+        job = 0;
+        return true;
+    }
+};
+
+// A live path's hit.
+struct PathInput {
+    const DevScene& S;
+    const PathIO& in;
+    const float4* hit;
+    float4 H, O, D;
+    float4 n0, n1, n2;
+    int job_;
+    int4 vi;
+    bool valid;
+    __device__ __forceinline__ PathInput(const DevScene& S_, const PathIO& in_, const float4* hit_)
+        : S(S_), in(in_), hit(hit_) {}
+    __device__ __forceinline__ void first(int i) {
+        H = hit[i];
+        O = in.o[i];
+        D = in.d[i];
+        job_ = (int)((uint32_t)in.info[i].z >> kNNJobShift);
+    }
+    __device__ __forceinline__ void second() {
+        const int prim = __float_as_int(H.y);
+        vi = make_int4(0, 0, 0, -1);
+        if (prim >= 0) vi = __ldg(S.tri_vidx + prim);
+    }
+    __device__ __forceinline__ void third() {
+        valid = vi.w >= 0;
+        if (!valid) return;
+        n0 = __ldg(S.v_nrm + vi.x);
+        n1 = __ldg(S.v_nrm + vi.y);
+        n2 = __ldg(S.v_nrm + vi.z);
+        valid = S.mats[vi.w].kind != PT_MAT_EMISSIVE_;
+    }
+    __device__ __forceinline__ bool last(NNIn& v, int& job) {
+        if (!valid) return false;
+        const f3 d = mk(D.x, D.y, D.z);
+        const float beta = H.z, gamma = H.w, alpha = 1.0f - (gamma + beta);
+        v.pn = mk(O.x, O.y, O.z) + d * H.x;
+        v.n = normalized(f3of(n0) * alpha + f3of(n1) * beta + f3of(n2) * gamma);
+        v.wo = -d;
+        job = job_;
+        return true;
+    }
+};
 
 template <bool ONEBLOB>
 __global__ void __launch_bounds__(kTcInferThreads) k_nn_forward_debug(const DevNNJob* __restrict__ nnj,
@@ -232,15 +321,7 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_forward_debug(const DevN
                                                                       float* __restrict__ out, uint32_t* status) {
     extern __shared__ __align__(1024) unsigned char smem[];
     tc_infer_loop<ONEBLOB>(
-        n, smem, nnj, status,
-        [&](int i, NNIn& v, int& job) {
-            const float* p = in + 9 * (size_t)i;
-            v.pn = mk(p[0], p[1], p[2]);
-            v.n = mk(p[3], p[4], p[5]);
-            v.wo = mk(p[6], p[7], p[8]);
-            job = 0;
-            return true;
-        },
+        n, smem, nnj, status, DebugInput{in, nullptr},
         [&](int i, const float* prm) {
             for (int k = 0; k < kNNParams; k++) out[kNNParams * (size_t)i + k] = prm[k];
         });
@@ -249,7 +330,7 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_forward_debug(const DevN
 // Guide parameters for every live path's hit (run between extend and shade),
 // each path with its job's network.
 template <bool ONEBLOB>
-__global__ void __launch_bounds__(kTcInferThreads) k_nn_infer(DevScene S, PathIO in, const float4* __restrict__ hit, WaveCounters* ctr,
+__global__ void __launch_bounds__(kTcInferThreads, 4) k_nn_infer(DevScene S, PathIO in, const float4* __restrict__ hit, WaveCounters* ctr,
                                                               const DevNNJob* __restrict__ nnj,
                                                               float4* __restrict__ params) {
     after_previous();
@@ -257,23 +338,7 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_infer(DevScene S, PathIO
     const int n = ctr->n_cur;
     if (n == 0) return;
     tc_infer_loop<ONEBLOB>(
-        n, smem, nnj, &ctr->status,
-        [&](int i, NNIn& v, int& job) {
-            const float4 H = hit[i];
-            const int prim = __float_as_int(H.y);
-            if (prim < 0) return false;
-            const int4 vi = __ldg(S.tri_vidx + prim);
-            if (S.mats[vi.w].kind == PT_MAT_EMISSIVE_) return false;
-            const float4 O = in.o[i], D = in.d[i];
-            const f3 d = mk(D.x, D.y, D.z);
-            const float beta = H.z, gamma = H.w, alpha = 1.0f - (gamma + beta);
-            v.pn = mk(O.x, O.y, O.z) + d * H.x;
-            v.n = normalized(f3of(__ldg(S.v_nrm + vi.x)) * alpha + f3of(__ldg(S.v_nrm + vi.y)) * beta +
-                             f3of(__ldg(S.v_nrm + vi.z)) * gamma);
-            v.wo = -d;
-            job = (int)((uint32_t)in.info[i].z >> kNNJobShift);
-            return true;
-        },
+        n, smem, nnj, &ctr->status, PathInput(S, in, hit),
         [&](int i, const float* prm) { nn_pack_mixture(prm, params + kNNMixF4 * (size_t)i); });
 }
 

@@ -253,3 +253,16 @@ def test_training_render_at_block_edges(gpu_lib, res, spp, depth):
     if depth <= 8:  # as one job: nothing trains before the round's end
         assert np.array_equal(imgs[0].view(np.uint32), a.view(np.uint32))
     assert all(np.isfinite(s.nn_weights()).all() for s in pair)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 608 * 128, 608 * 128 + 1, 200001])
+@pytest.mark.parametrize("encoding", [0, 1], ids=["freq", "oneblob"])
+def test_forward_over_several_tiles(gpu_lib, encoding, n):
+    """A CTA reads a tile's input while it runs the tile before: every row of
+    a batch of several tiles per CTA (608 CTAs of 128 rows) is what the row
+    gives by itself in a batch of one tile per CTA, bit for bit."""
+    from cpppt import lib
+    w, x = random_weights(1), random_inputs(n, 5)
+    got = lib.nn_forward(w, LO, HI, x, encoding=encoding)
+    parts = [lib.nn_forward(w, LO, HI, x[k:k + 4000], encoding=encoding) for k in range(0, n, 4000)]
+    assert np.array_equal(got.view(np.uint32), np.concatenate(parts).view(np.uint32))
