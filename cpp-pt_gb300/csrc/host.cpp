@@ -253,11 +253,15 @@ void check_status(pt_scene* s, uint32_t status) {
     if (status & kStatusRoundLimit) throw Fail(PT_ERR_LIMIT, "render did not converge within the iteration bound");
 }
 
-void trace_device(pt_scene* s, const pt_ray* rays, int n, void* out, bool any, cudaStream_t st) {
+// status: the caller reads the status word afterwards.  Otherwise a batch with
+// a warp per ray needs no cleared words, and no launch before its own (any hit,
+// 100 and 1000 rays: 18.6 -> 16.6 and 20.8 -> 19.7 us, closest hit 23.0 -> 21.5).
+void trace_device(pt_scene* s, const pt_ray* rays, int n, void* out, bool any, cudaStream_t st, bool status) {
     if (n < 0) throw std::invalid_argument("negative ray count");
     if (n == 0) return;
     if (!rays || !out) throw std::invalid_argument("null buffer");
-    ck(cudaMemsetAsync(s->d_counter, 0, 2 * sizeof(int), st), "memset");
+    if (status || trace_needs_counter(n, s->num_sms))
+        ck(cudaMemsetAsync(s->d_counter, 0, 2 * sizeof(int), st), "memset");
     if (any)
         launch_trace_any(s->dev, reinterpret_cast<const float*>(rays), n, static_cast<uint8_t*>(out), s->d_counter,
                          s->d_status, s->num_sms, st);
@@ -277,7 +281,7 @@ void trace_host(pt_scene* s, const pt_ray* rays, int n, void* out, bool any) {
     ensure_io(s, out_off + out_bytes);
     char* base = static_cast<char*>(s->d_io);
     ck(cudaMemcpyAsync(base, rays, in_bytes, cudaMemcpyHostToDevice, s->stream), "copy rays");
-    trace_device(s, reinterpret_cast<const pt_ray*>(base), n, base + out_off, any, s->stream);
+    trace_device(s, reinterpret_cast<const pt_ray*>(base), n, base + out_off, any, s->stream, true);
     ck(cudaMemcpyAsync(out, base + out_off, out_bytes, cudaMemcpyDeviceToHost, s->stream), "copy hits");
     uint32_t status = 0;
     ck(cudaMemcpyAsync(&status, s->d_status, 4, cudaMemcpyDeviceToHost, s->stream), "copy status");
@@ -1177,12 +1181,12 @@ pt_status pt_trace_any(pt_scene* s, const pt_ray* rays, int32_t n, uint8_t* occl
 
 pt_status pt_trace_closest_device(pt_scene* s, const pt_ray* d_rays, int32_t n, pt_hit* d_hits, void* stream) {
     if (!s) { g_error = "null scene"; return PT_ERR_INVALID; }
-    return guarded([&] { trace_device(s, d_rays, n, d_hits, false, static_cast<cudaStream_t>(stream)); });
+    return guarded([&] { trace_device(s, d_rays, n, d_hits, false, static_cast<cudaStream_t>(stream), false); });
 }
 
 pt_status pt_trace_any_device(pt_scene* s, const pt_ray* d_rays, int32_t n, uint8_t* d_occ, void* stream) {
     if (!s) { g_error = "null scene"; return PT_ERR_INVALID; }
-    return guarded([&] { trace_device(s, d_rays, n, d_occ, true, static_cast<cudaStream_t>(stream)); });
+    return guarded([&] { trace_device(s, d_rays, n, d_occ, true, static_cast<cudaStream_t>(stream), false); });
 }
 
 pt_status pt_render(pt_scene* s, const pt_render_desc* desc, float* rgb_out) {

@@ -7,8 +7,11 @@
 
 namespace cpppt_gb300 {
 
+// Whether a trace launch takes rays from its counter: with no more rays than
+// warps each warp has its own.
+bool trace_needs_counter(int n, int num_sms);
 // Persistent-warp ray-batch kernels.  `rays` are 7 packed floats per ray;
-// `counter` is one zeroed int in device memory (work queue head);
+// `counter` is one int in device memory (work queue head), zeroed if needed;
 // `status` collects kStatus* bits.
 void launch_trace_closest(const DevScene& S, const float* rays, int n, float4* hits, int* counter,
                           uint32_t* status, int num_sms, cudaStream_t st);

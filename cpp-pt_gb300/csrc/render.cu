@@ -67,6 +67,10 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_any(
         [&](int i, const HitRec& h) { occ[i] = h.prim >= 0 ? 1 : 0; });
 }
 
+bool trace_needs_counter(int n, int num_sms) {
+    return n > min(num_sms * kTraceBlocksPerSM, n) * (kTraceThreads / 32);
+}
+
 void launch_trace_closest(const DevScene& S, const float* rays, int n, float4* hits, int* counter, uint32_t* status,
                           int num_sms, cudaStream_t st) {
     if (n <= 0) return;

@@ -126,3 +126,36 @@ def test_stacks_beyond_their_shared_part(gpu_lib):
     assert np.array_equal(gi, oi)
     assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
     assert np.array_equal(gs.trace_any(sh), osc.trace_any(sh))
+
+
+@pytest.mark.parametrize("n", [1, 33, 4863, 4864, 4865, 9728, 9729])
+def test_device_batches_with_a_warp_per_ray(gpu_lib, n):
+    """Batches of no more rays than the GPU has traversal warps (152 x 32) run
+    without a cleared ray counter: the same answers as the host call, also
+    after a batch that left the counter high, twice in a row."""
+    torch = pytest.importorskip("torch")
+    from cpppt.lib import GpuScene
+    sc = scenes.soup(seed=2, n_spheres=100, freq=3, width=64, height=64)
+    gs = GpuScene(sc)
+    rays = scenes.hit_ray_batch(sc, 1 << 15, seed=11)
+    d = torch.as_tensor(rays).cuda().contiguous()
+    hits = torch.zeros(len(rays), 4, device="cuda")
+    occ = torch.zeros(len(rays), dtype=torch.uint8, device="cuda")
+    gs.trace_closest_device(d.data_ptr(), len(rays), hits.data_ptr())
+    gs.trace_any_device(d.data_ptr(), len(rays), occ.data_ptr())
+    torch.cuda.synchronize()  # a scene's batches share its counter: one stream at a time
+    idx, t, _, _ = gs.trace_closest(rays[:n])
+    blocked = gs.trace_any(rays[:n])
+    gs.trace_closest_device(d.data_ptr(), len(rays), hits.data_ptr())
+    for _ in range(2):
+        hits.zero_()
+        occ.zero_()
+        torch.cuda.synchronize()
+        gs.trace_closest_device(d.data_ptr(), n, hits.data_ptr())
+        gs.trace_any_device(d.data_ptr(), n, occ.data_ptr())
+        torch.cuda.synchronize()
+        h = hits.cpu().numpy()
+        assert np.array_equal(h[:n, 1].view(np.int32), idx)
+        assert np.array_equal(h[:n, 0].view(np.uint32), t.view(np.uint32))
+        assert np.array_equal(occ.cpu().numpy()[:n], blocked)
+        assert (h[n:] == 0).all()
