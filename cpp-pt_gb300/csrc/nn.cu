@@ -815,6 +815,9 @@ __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, Pat
         const float4 O = in.o[i], D = in.d[i], Tp = in.thr[i];
         const int4 I = in.info[i];
         const float4 H = B.hit[i];
+        // the path's mixture (one line) is read after the hit's vertices: fetch
+        // it beside them (guided 1280x720 9.72 -> 9.56 ms)
+        if (guided) asm volatile("prefetch.global.L1 [%0];" ::"l"(params + kNNMixF4 * (size_t)i));
         const int prim = __float_as_int(H.y);
         const int pixel = I.x, sample = I.y, bounce = I.z & 0xffff;
         const bool sdelta = (I.z >> 16) & 1;
