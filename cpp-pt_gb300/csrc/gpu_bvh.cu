@@ -748,23 +748,37 @@ __global__ void __launch_bounds__(kBigThreads) k_big_scatter(const ChunkG* __res
     scatter_bins(P, pout + seg.start, begin, end, axis, s_thr[axis], run, s_wbin);
 }
 
-// Subtree sizes (internal nodes), one level of nodes [lo, hi), bottom-up.
-__global__ void k_sizes(const NodeG* __restrict__ nodes, int lo, int hi, int32_t* __restrict__ size) {
-    const int i = lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= hi) return;
-    const NodeG& nd = nodes[i];
-    size[i] = 1 + (nd.child[0] >= 0 ? size[nd.child[0]] : 0) + (nd.child[1] >= 0 ? size[nd.child[1]] : 0);
+// Subtree sizes (internal nodes), bottom-up: a thread starts at each node
+// without internal children and climbs; the last of a node's arrivals
+// (counted in `seen`, zeroed) finds its children's sizes and goes on.  One
+// launch bound by the depth's chain of loads.  With a launch per level here and
+// in k_preorder (92 for the 192k-triangle room) scene creation took 10.45 ms
+// there, now 10.3; a 10k-triangle scene 3.72, now 3.56.
+__global__ void k_sizes(const NodeG* __restrict__ nodes, int n, int32_t* __restrict__ seen, int32_t* __restrict__ size) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || nodes[i].child[0] >= 0 || nodes[i].child[1] >= 0) return;
+    __stcg(size + i, 1);
+    for (i = nodes[i].parent; i >= 0; i = nodes[i].parent) {
+        const int a = nodes[i].child[0], b = nodes[i].child[1];
+        __threadfence();
+        if (atomicAdd(seen + i, 1) + 1 < (a >= 0) + (b >= 0)) return;
+        __threadfence();
+        __stcg(size + i, 1 + (a >= 0 ? __ldcg(size + a) : 0) + (b >= 0 ? __ldcg(size + b) : 0));
+    }
 }
 
-// Pre-order numbers of the children of one level of nodes, top-down.
-__global__ void k_preorder(const NodeG* __restrict__ nodes, int lo, int hi, const int32_t* __restrict__ size,
+// Pre-order numbers: the parent, then the first partition's subtree, then the
+// second's, summed on the way to the root.
+__global__ void k_preorder(const NodeG* __restrict__ nodes, int n, const int32_t* __restrict__ size,
                            int32_t* __restrict__ pre) {
-    const int i = lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= hi) return;
-    const NodeG& nd = nodes[i];
-    const int p = pre[i];
-    if (nd.child[0] >= 0) pre[nd.child[0]] = p + 1;
-    if (nd.child[1] >= 0) pre[nd.child[1]] = p + 1 + (nd.child[0] >= 0 ? size[nd.child[0]] : 0);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int number = 0;
+    for (int k = i, p = nodes[i].parent; p >= 0; k = p, p = nodes[p].parent) {
+        const int first = nodes[p].child[0];
+        number += 1 + (nodes[k].side == 1 && first >= 0 ? size[first] : 0);
+    }
+    pre[i] = number;
 }
 
 __global__ void k_node_out(const NodeG* __restrict__ nodes, int n_nodes, const int32_t* __restrict__ pre,
@@ -832,7 +846,7 @@ RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& sc
     k_prims<<<(n + 255) / 256, 256, 0, st>>>(d_tv, n, buf[0]);
     ck(cudaMemsetAsync(d_cnt, 0, 5 * sizeof(int), st), "memset");
     k_root<<<1, 1, 0, st>>>(LevelOut{segs[0], small[0], big[0], chunks[0], d_cnt}, n);
-    std::vector<int> level_nodes(1, 0);  // node count after each level
+    int n_nodes = 0;
     int n_seg = n > 32 ? 1 : 0, n_small = n > 32 ? 0 : 1, cur = 0, levels = 0;
     int n_big = n > kBigSeg ? 1 : 0, n_chunks = n_big ? (n + kBigChunk - 1) / kBigChunk : 0;
     while (n_seg > 0 || n_small > 0) {
@@ -856,23 +870,18 @@ RefTree build_ref_tree(const float* d_tv, int n, cudaStream_t st, DeviceBufs& sc
         n_big = h_cnt[2];
         n_chunks = h_cnt[3];
         n_small = h_cnt[4];
-        level_nodes.push_back(h_cnt[1]);
+        n_nodes = h_cnt[1];
         if (h_cnt[1] > max_nodes || n_seg > n + 2 || n_small > n + 2 || n_big > max_big || n_chunks > max_chunks)
             throw std::runtime_error("device BVH build overflow");
         cur = 1 - cur;
         levels++;
     }
-    const int n_nodes = level_nodes.back();
     int32_t* size = dmalloc<int32_t>(owned, n_nodes);
     int32_t* pre = dmalloc<int32_t>(owned, n_nodes);
-    for (int L = (int)level_nodes.size() - 2; L >= 0; L--) {
-        const int lo = level_nodes[L], hi = level_nodes[L + 1];
-        if (hi > lo) k_sizes<<<(hi - lo + 255) / 256, 256, 0, st>>>(nodes, lo, hi, size);
-    }
-    if (n_nodes > 0) ck(cudaMemsetAsync(pre, 0, sizeof(int32_t), st), "root pre-order");  // node 0 is the root
-    for (size_t L = 0; L + 1 < level_nodes.size(); L++) {
-        const int lo = level_nodes[L], hi = level_nodes[L + 1];
-        if (hi > lo) k_preorder<<<(hi - lo + 255) / 256, 256, 0, st>>>(nodes, lo, hi, size, pre);
+    if (n_nodes > 0) {
+        ck(cudaMemsetAsync(pre, 0, sizeof(int32_t) * (size_t)n_nodes, st), "memset");  // arrivals, until the numbers
+        k_sizes<<<(n_nodes + 255) / 256, 256, 0, st>>>(nodes, n_nodes, pre, size);
+        k_preorder<<<(n_nodes + 255) / 256, 256, 0, st>>>(nodes, n_nodes, size, pre);
     }
     float4* d_box = dmalloc<float4>(keep.v, 2 * (size_t)n_nodes);
     int32_t* d_parent = dmalloc<int32_t>(owned, n_nodes);
