@@ -40,6 +40,50 @@ def test_traversal_step_limit_is_reported(gpu_lib):
     assert np.isfinite(gs.render(4, max_depth=4, seed=1)).all()
 
 
+def _layers():
+    """Eight slanted triangles one above the other: two leaves (or more) under the root."""
+    sc = _scene()
+    k = np.arange(8, dtype=np.float32)[:, None]
+    one = np.ones_like(k)
+    v = np.stack([np.hstack([0 * one, 0 * one, k]), np.hstack([4 * one, 0 * one, k]),
+                  np.hstack([0 * one, 4 * one, k + np.float32(.5)])], 1).reshape(-1, 3).astype(np.float32)
+    up, side = np.float32([[0, 0, 1]]), np.float32([[1, 0, 0]])
+    return dataclasses.replace(
+        sc, vertices=v, normals=np.repeat(up, len(v), 0), tangents=np.repeat(side, len(v), 0),
+        triangles=np.arange(len(v), dtype=np.int32).reshape(-1, 3), mesh_tri_offset=np.array([0, 8], np.int32),
+        mesh_vert_offset=np.array([0, len(v)], np.int32), mesh_material=np.array([0], np.int32))
+
+
+def test_traversal_step_limit_bounds_node_visits(gpu_lib):
+    """The limit is tested at each node visit, and there alone: a tree of one
+    node and several leaves is walked whole under a limit of one step, by rays
+    that test one leaf, every leaf or none, in batches whose warps hold rays of
+    all kinds; a tree of two levels runs out."""
+    from cpppt import lib
+    from cpppt.lib import GpuScene, PtError
+    sc = _layers()
+    assert lib.wide_bvh(sc, on_device=False)[2] == 1
+    gs = GpuScene(sc)
+    rng = np.random.default_rng(1)
+    n = 1 << 14
+    o = np.hstack([rng.uniform(-1, 5, (n, 2)), np.full((n, 1), 20.0)])
+    d = np.hstack([rng.uniform(-.3, .3, (n, 2)), np.full((n, 1), -1.0)])
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.hstack([o, d, rng.choice([5.0, 16.0, np.inf], (n, 1))]).astype(np.float32)
+    want, blocked = gs.trace_closest(rays), gs.trace_any(rays)
+    assert 0.05 < blocked.mean() < 0.95
+    assert gpu_lib.pt_debug_traversal_limits(gs.h, 1, 0) == 0
+    got = gs.trace_closest(rays)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1].view(np.uint32), want[1].view(np.uint32))
+    assert np.array_equal(gs.trace_any(rays), blocked)
+    deep = _scene()
+    ds = GpuScene(deep)
+    assert gpu_lib.pt_debug_traversal_limits(ds.h, 1, 0) == 0
+    for query in (ds.trace_closest, ds.trace_any):
+        with pytest.raises(PtError, match="step limit"):
+            query(scenes.hit_ray_batch(deep, 4096, seed=3))
+
+
 def test_traversal_stack_overflow_is_reported(gpu_lib):
     from cpppt.lib import GpuScene, PtError
     sc = _scene()
