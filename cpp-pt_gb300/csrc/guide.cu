@@ -122,7 +122,7 @@ __device__ __forceinline__ void sd_splat_warp(const DevSDTree& T, bool on, float
 
 constexpr int kShadePPGThreads = 256;
 __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, PathIO in, PathIO nxt,
-                                                   const float4* __restrict__ hit, RenderParams P, WaveCounters* ctr, unsigned long long* __restrict__ film,
+                                                   const float4* hit, RenderParams P, WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                    DevSDTree T, PPGVerts V, int* slot_stack) {
     after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

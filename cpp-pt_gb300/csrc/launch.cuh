@@ -12,6 +12,12 @@ namespace cpppt_gb300 {
 // render, Cornell box 128x128, 64 spp, 3.59 -> 3.17 ms; training 640x360 in the
 // 192k-triangle room 7.95 -> 7.73, guided 1280x720 10.05 -> 9.91; 640x360, 1
 // spp on the 1M-triangle soup 1.85 -> 1.82; long kernels (1080p) unchanged.
+//
+// A kernel's lifetime so overlaps the writes of the one before, and a load
+// through the read-only path is not ordered by the wait.  What another kernel of
+// the loop writes (path state, hits, mixtures, queues, counters) is therefore
+// never read through `const ... __restrict__` or __ldg, which are for what stands
+// before the render: scene arrays, the guide's tree, job tables.
 template <class... A, class... B>
 void launch_after(void (*kernel)(A...), int grid, int threads, size_t smem, cudaStream_t st, B&&... args) {
     cudaLaunchConfig_t c{};

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_forward_debug(const DevN
 // Guide parameters for every live path's hit (run between extend and shade),
 // each path with its job's network.
 template <bool ONEBLOB>
-__global__ void __launch_bounds__(kTcInferThreads, 4) k_nn_infer(DevScene S, PathIO in, const float4* __restrict__ hit, WaveCounters* ctr,
+__global__ void __launch_bounds__(kTcInferThreads, 4) k_nn_infer(DevScene S, PathIO in, const float4* hit, WaveCounters* ctr,
                                                               const DevNNJob* __restrict__ nnj,
                                                               float4* __restrict__ params) {
     after_previous();
@@ -801,7 +801,7 @@ constexpr int kNNVert = kNNVertFloat4;
 constexpr int kShadeNNThreads = 256;
 __global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, PathBuffers B, PathIO in, PathIO nxt, int cur, RenderParams P,
                                                   WaveCounters* ctr, unsigned long long* __restrict__ film,
-                                                  const float4* __restrict__ params, NNPathData PD, int guided,
+                                                  const float4* params, NNPathData PD, int guided,
                                                   const DevBatchJob* __restrict__ jobs) {
     after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

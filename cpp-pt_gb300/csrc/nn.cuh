@@ -209,7 +209,7 @@ __device__ __forceinline__ void nn_pack_mixture(const float* prm, float4* out /*
     out[7] = make_float4(prm[40], 0.f, 0.f, 0.f);
 }
 
-__device__ __forceinline__ void nn_unpack_mixture(const float4* __restrict__ p, NNMixture& M) {
+__device__ __forceinline__ void nn_unpack_mixture(const float4* p, NNMixture& M) {
     uint32_t hw[20];
 #pragma unroll
     for (int k = 0; k < 5; k++) {

@@ -100,8 +100,8 @@ __device__ __forceinline__ void film_add(unsigned long long* film, size_t pix, f
 template <bool COUNT>
 __device__ __forceinline__ void extend_queue(const DevScene& S, uint32_t* s_stack, const PathIO& in,
                                              float4* __restrict__ Hout, int n, WaveCounters* ctr, TraceCount& cnt) {
-    const float4* __restrict__ O = in.o;
-    const float4* __restrict__ D = in.d;
+    const float4* O = in.o;
+    const float4* D = in.d;
     persistent_trace<false, COUNT>(
         S, s_stack, n, &ctr->fetch_ext, &ctr->status, cnt,
         [&](int i, float3& o, float3& d, float& tmax, uint32_t& root) {
@@ -295,7 +295,7 @@ __device__ __forceinline__ void shade_vertex(DevScene S, const DevBatchJob* __re
 
 constexpr int kShadeThreads = 256;
 __global__ void __launch_bounds__(kShadeThreads, CPPPT_SHADE_BLOCKS) k_shade(DevScene S, PathIO in, PathIO nxt, ShadowIO Q,
-                                               const float4* __restrict__ hit, int cur, WaveCounters* ctr,
+                                               const float4* hit, int cur, WaveCounters* ctr,
                                                unsigned long long* __restrict__ film,
                                                const DevBatchJob* __restrict__ jobs) {
     after_previous();
