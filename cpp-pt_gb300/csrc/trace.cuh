@@ -2,6 +2,7 @@
 // closest-hit semantics (see bvh.h for why this reproduces BVH::intersect).
 #pragma once
 #include "dev_types.h"
+#include "ray_range.h"
 
 namespace cpppt_gb300 {
 
@@ -511,22 +512,6 @@ __device__ __forceinline__ void trav_round(const DevScene& S, Trav& T, Stack& K,
     }
 }
 
-// Rays per fetch when `left` rays remain for `nwarps` warps (`share` chunks
-// each): kChunk while there are many, down to one for the last ones, so that
-// a small batch (or the end of a large one) is spread over all warps.  A warp
-// whose rays take different ways through the tree runs the union of their
-// steps, and the launch ends with its slowest warp.  Measured (1M-triangle
-// soup) against 16 rays a fetch from one CTA per 1024 rays: 1000 shadow rays
-// 136 -> 54 us, 30,001 closest-hit rays 194 -> 125 us; the first fetch at half
-// the even share 144 us (30,001 rays), at a quarter 171 us, since half the rays
-// then wait for a second fetch.  kChunk 8, 16, 24, 32, 48, 64: 1080p at 16 spp
-// 92.0, 87.7, 87.2, 86.8, 86.6, 86.5 ms, 1M rays in the 192k-triangle room 336,
-// 291, 289, 283, 294, 319 us.
-constexpr int kChunk = 32;
-__device__ __forceinline__ int ray_chunk(int left, int nwarps, int share) {
-    return min(kChunk, max(1, left / (share * nwarps)));
-}
-
 // smem: the stacks' shared region (stack_bytes(ANY, THREADS)).
 // Persistent ray loop.  Each warp takes chunks of up to kChunk consecutive
 // rays (ray_chunk) into a warp-private range, the first one by its number and
@@ -552,38 +537,31 @@ __device__ __forceinline__ void persistent_trace(const DevScene& S, uint32_t* __
     // come from the counter
     const int nwarps = (int)(gridDim.x * (blockDim.x >> 5));
     const int c0 = own_first ? ray_chunk(n, nwarps, 1) : 0;
-    int pool_next = min((int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * c0, n);
-    int pool_end = min(pool_next + c0, n);
+    RayRange pool = fetched_range(0, (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * c0, c0, n);
     bool exhausted = nwarps * c0 >= n;
     while (true) {
         const unsigned idle = __ballot_sync(0xffffffffu, ray < 0);
         if (idle) {
-            const int want = __popc(idle), avail = pool_end - pool_next;
-            int next = pool_end, end = pool_end;  // the range after the present one
-            if (avail < want && !exhausted) {
-                const int chunk = ray_chunk(n - pool_end, nwarps, 2);
-                int base = 0;
-                if (lane == 0) base = atomicAdd(counter, chunk);
-                next = min(__shfl_sync(0xffffffffu, base, 0) + nwarps * c0, n);
-                end = min(next + chunk, n);
-                exhausted = end >= n;
+            const uint32_t want = __popc(idle);
+            RayRange after{pool.end, pool.end};  // the range after the present one
+            if (pool.end - pool.next < want && !exhausted) {
+                const int chunk = ray_chunk(n - (int)pool.end, nwarps, 2);
+                int taken = 0;
+                if (lane == 0) taken = atomicAdd(counter, chunk);
+                after = fetched_range(__shfl_sync(0xffffffffu, taken, 0), nwarps * c0, chunk, n);
+                exhausted = after.end == (uint32_t)n;
             }
-            const int r = __popc(idle & lt_mask);
-            const int i = r < avail ? pool_next + r : next + (r - avail);
-            if (ray < 0 && (r < avail || i < end)) {
-                ray = i;
+            uint32_t i;
+            const bool more = ray_of(__popc(idle & lt_mask), pool, after, i);
+            if (ray < 0 && more) {
+                ray = (int)i;
                 float3 o, d;
                 float tmax;
                 uint32_t root = S.n_tris > 0 ? 0u : kTravDone;
                 load(ray, o, d, tmax, root);
                 trav_init(T, K.base, o, d, tmax, root);
             }
-            if (avail >= want) {
-                pool_next += want;
-            } else {
-                pool_next = min(next + (want - avail), end);
-                pool_end = end;
-            }
+            pool = left_of(want, pool, after);
         }
         const unsigned act = __ballot_sync(0xffffffffu, ray >= 0);
         if (act == 0) break;
