@@ -336,7 +336,7 @@ int ensure_wave(pt_scene* s, int capacity, int film_n) {
         };
         release();
         if (s->graph) { cudaGraphExecDestroy(s->graph); s->graph = nullptr; }
-        for (int c = capacity;; c = std::max(1 << 20, c / 2)) {
+        for (int c = capacity;;) {
             try {
                 for (int k = 0; k < 2; k++) {
                     B.o[k] = dalloc<float4>(s->pb_owned, c);
@@ -353,7 +353,9 @@ int ensure_wave(pt_scene* s, int capacity, int film_n) {
             } catch (...) {
                 release();
                 cudaGetLastError();  // an allocation failure is not sticky
-                if (c <= (1 << 20)) throw;
+                if (s->ppg.bytes() > 0) s->ppg.release();  // of an earlier SD-tree render: once more without them
+                else if (c <= (1 << 20)) throw;
+                else c = std::max(1 << 20, c / 2);
             }
         }
     }
@@ -368,6 +370,8 @@ int ensure_wave(pt_scene* s, int capacity, int film_n) {
     }
     return std::min(capacity, s->pb.capacity);
 }
+
+constexpr size_t kKeptPPGBytes = 256 << 20;  // of an SD-tree render's buffers, kept for the scene's next one
 
 // PPG::render (src/renderer/ppg.h:149-215): passes of 1, 2, 4, ... spp while
 // below spp in total; the SD-tree learns from every pass (splats on the GPU,
@@ -388,8 +392,15 @@ void render_ppg(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     pb.capacity = capacity;
     // The buffers stay with the scene: allocated anew for every pass, their
     // cudaMalloc and cudaFree calls took 0.8 of 4.9 ms (Cornell box, 128x128, 64
-    // spp, six passes).
+    // spp, six passes).  A render whose records took more gives them back: they
+    // are up to 36 B x 2^20 paths x depth.
     Workspace& W = s->ppg;
+    struct GiveBack {
+        Workspace& w;
+        ~GiveBack() {
+            if (w.bytes() > kKeptPPGBytes) w.release();
+        }
+    } give_back{W};
     PPGVerts V;
     V.vp = W.get<float4>(0, (size_t)capacity * D);
     V.vd = W.get<float4>(1, (size_t)capacity * D);
@@ -581,7 +592,7 @@ int nn_path_buffers(pt_scene* s, int capacity, int depth, bool guided) {
         if (s->nn_params) cudaFree(s->nn_params);
         s->nn_params = nullptr;
         s->nn_params_cap = 0;
-        for (int c = capacity;; c = std::max(1 << 20, c / 2)) {
+        for (int c = capacity;;) {
             void* p = nullptr;
             const cudaError_t e = cudaMalloc(&p, sizeof(float4) * (size_t)c * kNNMixF4);
             if (e == cudaSuccess) {
@@ -589,8 +600,10 @@ int nn_path_buffers(pt_scene* s, int capacity, int depth, bool guided) {
                 s->nn_params_cap = c;
                 break;
             }
-            if (c <= (1 << 20)) ck(e, "cudaMalloc");
             cudaGetLastError();  // an allocation failure is not sticky
+            if (s->ppg.bytes() > 0) s->ppg.release();  // as in ensure_wave
+            else if (c <= (1 << 20)) ck(e, "cudaMalloc");
+            else c = std::max(1 << 20, c / 2);
         }
     }
     if (guided) capacity = std::min(capacity, s->nn_params_cap);

@@ -92,7 +92,7 @@ T* dupload(std::vector<void*>& owned, const std::vector<T>& v, cudaStream_t st) 
     return p;
 }
 
-// Device buffers by index, grown on demand and kept until the owner goes.
+// Device buffers by index, grown on demand and kept until they are released.
 struct Workspace {
     struct Buf {
         void* p = nullptr;
@@ -102,8 +102,15 @@ struct Workspace {
     Workspace() = default;
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
-    ~Workspace() {
+    ~Workspace() { release(); }
+    size_t bytes() const {
+        size_t n = 0;
+        for (const Buf& b : bufs) n += b.bytes;
+        return n;
+    }
+    void release() {
         for (Buf& b : bufs) cudaFree(b.p);
+        bufs.clear();
     }
     // Buffer i with room for n elements; what it held is lost when it grows
     // (no work that uses it may be in flight then).

@@ -97,7 +97,7 @@ typedef struct {
 
 /* Integrator modes. */
 #define PT_MODE_MIS 0       /* PathtracerMIS, reference estimator (default) */
-#define PT_MODE_SDTREE 1    /* SD-tree guided (practical path guiding) */
+#define PT_MODE_SDTREE 1    /* SD-tree guided (practical path guiding); the scene keeps up to 256 MB of its buffers */
 #define PT_MODE_NN 2        /* learned (MLP, vMF mixture) guiding */
 #define PT_MODE_NEE 3       /* Pathtracer: NEE without MIS (pathtracer.h:27-102) */
 #define PT_MODE_PT 4        /* PurePt: BSDF sampling only, no NEE (pure_pt.h:28-71) */

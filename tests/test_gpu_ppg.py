@@ -58,3 +58,22 @@ def test_ppg_splats_by_vertex(gpu_lib, res, depth):
     g, p = (np.array([x.astype(np.float64).mean() for x in v]) for v in (guided, plain))
     se = np.sqrt(g.var(ddof=1) / len(g) + p.var(ddof=1) / len(p))
     assert abs(g.mean() - p.mean()) <= 6 * se
+
+
+def test_ppg_gives_its_records_back(gpu_lib):
+    """The vertex records of long paths (36 B x 2^19 paths x 150 vertices, 2.8
+    GB) are freed when the render returns; a short render's are kept (at most
+    256 MB) and give the image of a fresh scene."""
+    torch = pytest.importorskip("torch")
+    from cpppt.lib import MODE_SDTREE, GpuScene
+    gs = GpuScene(scenes.cornell(256, 256))
+    gs.render(16, max_depth=4, seed=1)  # the wavefront's own buffers, which stay
+    gs.render(16, max_depth=2, seed=1, mode=MODE_SDTREE)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    gs.render(16, max_depth=150, rr_start=3, seed=1, mode=MODE_SDTREE)
+    assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
+    again = gs.render(16, max_depth=2, seed=5, mode=MODE_SDTREE)
+    assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
+    fresh = GpuScene(scenes.cornell(256, 256)).render(16, max_depth=2, seed=5, mode=MODE_SDTREE)
+    assert np.array_equal(again.view(np.uint32), fresh.view(np.uint32))
