@@ -27,7 +27,7 @@ EXPORTS = ["pt_scene_create", "pt_scene_load", "pt_scene_destroy", "pt_scene_inf
            "pt_trace_closest_device", "pt_trace_any_device", "pt_render", "pt_render_device",
            "pt_render_device_noalloc",
            "pt_render_stats_get", "pt_image_save", "pt_last_error", "pt_debug_ref_topology",
-           "pt_debug_sdtree_run", "pt_nn_get_weights", "pt_nn_set_weights", "pt_nn_reset", "pt_nn_stats",
+           "pt_debug_sdtree_run", "pt_debug_sdtree_splat", "pt_nn_get_weights", "pt_nn_set_weights", "pt_nn_reset", "pt_nn_stats",
            "pt_debug_nn_forward", "pt_debug_nn_forward_ex", "pt_debug_nn_grad", "pt_debug_nn_grad_ex", "pt_nn_configure", "pt_nn_config_get",
            "pt_batch_create", "pt_batch_destroy", "pt_batch_render", "pt_batch_render_device", "pt_batch_set_tuning",
            "pt_batch_get_tuning", "pt_batch_stats", "pt_batch_autotune", "pt_set_mesh_cache",
@@ -146,6 +146,8 @@ def load(path: str = LIB_PATH):
     lib.pt_batch_stats.argtypes = [P, C.POINTER(PtRenderStats)]
     lib.pt_batch_autotune.argtypes = [P, P, C.c_int32, C.c_int32, P, P]
     lib.pt_debug_sdtree_run.argtypes = [P, P, C.c_int32, P, P, C.c_int32, P, P, P, P, C.c_int32, P, P, P]
+    lib.pt_debug_sdtree_splat.argtypes = [P, P, C.c_int32, P, P, C.c_int32, P, P, C.c_int32, C.c_int32, P, C.c_int32,
+                                          P, P, P, P]
     for name in EXPORTS:
         getattr(lib, name).restype = C.c_int32 if name not in ("pt_scene_destroy", "pt_last_error",
                                                                "pt_batch_destroy", "pt_set_mesh_cache") else \
@@ -480,6 +482,23 @@ def sdtree_run(lo, hi, rounds, queries, max_leaves=1 << 20, fn=None, lib=None):
     total = int(lc[:n].sum())
     return {"leaves": leaves[:4 * total].reshape(-1, 4), "leaf_counts": lc[:n], "counts": cnt[:n],
             "flux": flux[:n], "pdf": pdf}
+
+
+def sdtree_splat(lo, hi, rounds, paths, on_device, max_slots=1 << 20, max_spatial=1 << 16):
+    """Splats of finished paths (pt_debug_sdtree_splat) on the tree that sdtree_run's rounds leave.  paths: list of
+    (n,9) arrays {pos, dir, factor}.  Returns the quadtree leaves' values and the spatial leaves' counts and flux."""
+    L = load()
+    lo, hi = (np.ascontiguousarray(x, np.float32) for x in (lo, hi))
+    ns = np.array([len(r) for r in rounds], np.int32)
+    sp = np.ascontiguousarray(np.concatenate(rounds) if rounds else np.zeros((0, 7)), np.float32)
+    nv = np.array([len(p) for p in paths], np.int32)
+    v = np.ascontiguousarray(np.concatenate(paths), np.float32)
+    values, counts, flux = np.zeros(max_slots, np.float32), np.zeros(max_spatial, np.int32), np.zeros(max_spatial, np.float32)
+    n, m = C.c_int32(), C.c_int32()
+    _check(L.pt_debug_sdtree_splat(_ptr(lo), _ptr(hi), len(rounds), _ptr(ns), _ptr(sp), len(paths), _ptr(nv), _ptr(v),
+                                   int(on_device), max_slots, _ptr(values), max_spatial, _ptr(counts), _ptr(flux),
+                                   C.byref(n), C.byref(m)))
+    return {"values": values[:n.value], "counts": counts[:m.value], "flux": flux[:m.value]}
 
 
 def debug_bsdf(cases: np.ndarray) -> np.ndarray:

@@ -121,6 +121,81 @@ __device__ __forceinline__ void sd_splat_warp(const DevSDTree& T, bool on, float
 }
 
 constexpr int kShadePPGThreads = 256;
+// Backward products and splats of the finished paths (ppg.h:131-141): vertex k
+// receives the largest channel of the product of the factors of vertices
+// k..n-1, taken from the last one down.  The path's thread puts the running
+// products in the place of the factors, four loads ahead; then a thread per
+// vertex of the CTA's finished paths, found in the running total of their
+// vertices, splats: the tree walks are chains of dependent loads, and one thread
+// walking for vertex after vertex left the SM at 6 % of its issue slots (Cornell
+// box 128x128, 64 spp: render 4.35 -> 3.60 ms with the sums per warp).  With the
+// products multiplied anew by each vertex's thread a path of n vertices cost
+// n^2 / 2 loads: that render 3.19 ms, now 3.10; the splats of 64 paths of 8000
+// vertices 218 ms, now 7.
+// slot: the thread's path, n_splat: its vertices (0: none to splat), last: the
+// last one's factor.  All threads of the CTA call it.
+__device__ __forceinline__ void splat_paths(const DevSDTree& T, const PPGVerts& V, int max_depth, int slot, int n_splat,
+                                            f3 last) {
+    constexpr int kWarps = kShadePPGThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (n_splat > 1) {
+        constexpr int kAhead = 4;  // factors read at a time
+        const size_t base = (size_t)slot * max_depth;
+        f3 acc = last;
+        for (int v = n_splat - 2; v >= 0; v -= kAhead) {
+            float2 b[kAhead];
+            float c[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; j++)
+                if (v >= j) {
+                    b[j] = reinterpret_cast<const float2*>(V.vd + base + v - j)[1];
+                    c[j] = V.vr[base + v - j];
+                }
+#pragma unroll
+            for (int j = 0; j < kAhead; j++)
+                if (v >= j) {
+                    acc = acc * mk(b[j].x, b[j].y, c[j]);
+                    reinterpret_cast<float2*>(V.vd + base + v - j)[1] = make_float2(acc.x, acc.y);
+                    V.vr[base + v - j] = acc.z;
+                }
+        }
+    }
+    __shared__ int s_first[kShadePPGThreads], s_slot[kShadePPGThreads], s_total[kWarps];
+    int incl = n_splat;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_total[warp] = incl;
+    __syncthreads();
+    int before = 0, n_verts = 0;
+    for (int w = 0; w < kWarps; w++) {
+        if (w < warp) before += s_total[w];
+        n_verts += s_total[w];
+    }
+    s_first[threadIdx.x] = before + incl - n_splat;
+    s_slot[threadIdx.x] = slot;
+    __syncthreads();
+    for (int j0 = 0; j0 < n_verts; j0 += kShadePPGThreads) {
+        const int j = j0 + (int)threadIdx.x;
+        const bool on = j < n_verts;
+        float rad = 0.f;
+        f3 vp = mk(0.f, 0.f, 0.f), vd = vp;
+        if (on) {
+            int path = 0;  // the last one that starts at or before j; those without vertices start with their successor
+            for (int step = kShadePPGThreads / 2; step > 0; step >>= 1)
+                if (s_first[path + step] <= j) path += step;
+            const int k = j - s_first[path];
+            const size_t vi = (size_t)s_slot[path] * max_depth + k;
+            const float4 a = V.vp[vi], b = V.vd[vi];
+            rad = fmaxf(b.z, fmaxf(b.w, V.vr[vi]));
+            vp = mk(a.x, a.y, a.z);
+            vd = mk(a.w, b.x, b.y);
+        }
+        sd_splat_warp(T, on, rad, vp, vd);
+    }
+}
+
 __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, PathIO in, PathIO nxt,
                                                    const float4* hit, RenderParams P, WaveCounters* ctr, unsigned long long* __restrict__ film,
                                                    DevSDTree T, PPGVerts V, int* slot_stack) {
@@ -132,6 +207,7 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
     float4 no, nd, nt;
     int4 ninfo;
     int slot = -1, n_splat = 0;  // vertices that take a splat (all of them, one per bounce, or none)
+    f3 last = mk(0.f, 0.f, 0.f);  // the last one's factor
     if (i < n) {
         const float4 O = in.o[i], D = in.d[i], Tp = in.thr[i];
         const int4 I = in.info[i];
@@ -209,60 +285,14 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
         }
         release = done;
         // ppg.h:131-141: splats only when the last vertex carries radiance
-        if (done && (vrad.x > 0.f || vrad.y > 0.f || vrad.z > 0.f)) n_splat = bounce;
+        if (done && (vrad.x > 0.f || vrad.y > 0.f || vrad.z > 0.f)) {
+            n_splat = bounce;
+            last = vrad;
+        }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kShadePPGThreads / 32;
-    // Backward products and splats of the finished paths (ppg.h:131-141):
-    // vertex k receives the largest channel of the product of the factors of
-    // vertices k..n-1, taken from the last one down.  A thread per vertex of
-    // the CTA's finished paths, found in the running total of their vertices:
-    // the tree walks are chains of dependent loads, and one thread walking for
-    // vertex after vertex left the SM at 6 % of its issue slots (Cornell box
-    // 128x128, 64 spp: render 4.35 -> 3.60 ms with the sums per warp).
-    __shared__ int s_first[kShadePPGThreads], s_slot[kShadePPGThreads], s_nv[kShadePPGThreads], s_total[kWarps];
-    int incl = n_splat;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) s_total[warp] = incl;
-    __syncthreads();
-    int before = 0, n_verts = 0;
-    for (int w = 0; w < kWarps; w++) {
-        if (w < warp) before += s_total[w];
-        n_verts += s_total[w];
-    }
-    s_first[threadIdx.x] = before + incl - n_splat;
-    s_slot[threadIdx.x] = slot;
-    s_nv[threadIdx.x] = n_splat;
-    __syncthreads();
-    for (int j0 = 0; j0 < n_verts; j0 += kShadePPGThreads) {
-        const int j = j0 + (int)threadIdx.x;
-        const bool on = j < n_verts;
-        float rad = 0.f;
-        f3 vp = mk(0.f, 0.f, 0.f), vd = vp;
-        if (on) {
-            int path = 0;  // the last one that starts at or before j; those without vertices start with their successor
-            for (int step = kShadePPGThreads / 2; step > 0; step >>= 1)
-                if (s_first[path + step] <= j) path += step;
-            const int k = j - s_first[path];
-            const size_t base = (size_t)s_slot[path] * P.max_depth;
-            int v = s_nv[path] - 1;
-            float4 b = V.vd[base + v];
-            f3 acc = mk(b.z, b.w, V.vr[base + v]);
-            while (v > k) {
-                v--;
-                b = V.vd[base + v];
-                acc = acc * mk(b.z, b.w, V.vr[base + v]);
-            }
-            const float4 a = V.vp[base + k];
-            rad = fmaxf(acc.x, fmaxf(acc.y, acc.z));
-            vp = mk(a.x, a.y, a.z);
-            vd = mk(a.w, b.x, b.y);
-        }
-        sd_splat_warp(T, on, rad, vp, vd);
-    }
+    splat_paths(T, V, P.max_depth, slot, n_splat, last);
     // one addition to each queue's counter per CTA (as k_shade)
     __shared__ int s_count[2][kWarps], s_base[2];
     const unsigned m_free = __ballot_sync(0xffffffffu, release), m_cont = __ballot_sync(0xffffffffu, push_cont);
@@ -290,6 +320,21 @@ __global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, Path
         nxt.thr[jc] = nt;
         nxt.info[jc] = ninfo;
     }
+}
+
+// The splats of paths that finished elsewhere: path i in slot i with n_verts[i]
+// vertices recorded (checks of splat_paths).
+__global__ void __launch_bounds__(kShadePPGThreads) k_debug_splat(DevSDTree T, PPGVerts V, const int* n_verts, int n,
+                                                                  int max_depth) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int n_splat = i < n ? n_verts[i] : 0;
+    f3 last = mk(0.f, 0.f, 0.f);
+    if (n_splat > 0) {
+        const size_t vi = (size_t)i * max_depth + n_splat - 1;
+        last = mk(V.vd[vi].z, V.vd[vi].w, V.vr[vi]);
+        if (!(last.x > 0.f || last.y > 0.f || last.z > 0.f)) n_splat = 0;
+    }
+    splat_paths(T, V, max_depth, i, n_splat, last);
 }
 
 // Camera paths for PPG (ppg.h:174-186: one jittered sample per pixel per
@@ -355,6 +400,11 @@ void launch_shade_ppg(const DevScene& S, const PathBuffers& B, int cur, const Re
                       cudaStream_t st) {
     launch_after(k_shade_ppg, (B.capacity + kShadePPGThreads - 1) / kShadePPGThreads, kShadePPGThreads, 0, st,
         S, path_io(B, cur), path_io(B, 1 - cur), B.hit, P, ctr, film, T, V, slot_stack);
+}
+void launch_debug_splat(const DevSDTree& T, const PPGVerts& V, const int* n_verts, int n, int max_depth,
+                        cudaStream_t st) {
+    k_debug_splat<<<(n + kShadePPGThreads - 1) / kShadePPGThreads, kShadePPGThreads, 0, st>>>(T, V, n_verts, n,
+                                                                                             max_depth);
 }
 void launch_generate_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                          const int* slot_stack, int num_sms, cudaStream_t st) {

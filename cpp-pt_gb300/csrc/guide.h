@@ -35,5 +35,7 @@ void launch_shade_ppg(const DevScene& S, const PathBuffers& B, int cur, const Re
                       cudaStream_t st);
 void launch_generate_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                          const int* slot_stack, int num_sms, cudaStream_t st);
+void launch_debug_splat(const DevSDTree& T, const PPGVerts& V, const int* n_verts, int n, int max_depth,
+                        cudaStream_t st);
 
 }  // namespace cpppt_gb300

@@ -371,6 +371,31 @@ int ensure_wave(pt_scene* s, int capacity, int film_n) {
     return std::min(capacity, s->pb.capacity);
 }
 
+// The tree's device image with zeroed accumulators, in buffers first .. first + 8.
+DevSDTree upload_tree(Workspace& W, size_t first, const SDTreeFlat& f, cudaStream_t st) {
+    DevSDTree T;
+    for (int k = 0; k < 3; k++) { T.lo[k] = f.lo[k]; T.hi[k] = f.hi[k]; }
+    std::vector<int2> sn(f.snode.size() / 2);
+    for (size_t i = 0; i < sn.size(); i++) sn[i] = make_int2(f.snode[2 * i], f.snode[2 * i + 1]);
+    T.snode = W.upload(first, sn, st);
+    T.dnode = W.upload(first + 1, f.dnode, st);
+    T.dtree_root = W.upload(first + 2, f.dtree_root, st);
+    T.leaf_off = W.upload(first + 3, f.dtree_leaf_off, st);
+    T.leaf_cnt = W.upload(first + 4, f.dtree_leaf_cnt, st);
+    std::vector<float4> lv(f.leaves.size() / 4);
+    for (size_t i = 0; i < lv.size(); i++)
+        lv[i] = make_float4(f.leaves[4 * i], f.leaves[4 * i + 1], f.leaves[4 * i + 2], f.leaves[4 * i + 3]);
+    T.leaves = W.upload(first + 5, lv, st);
+    const int n_dtree = (int)f.dtree_root.size();
+    T.slot_value = W.get<float>(first + 6, f.n_value_slots);
+    T.dtree_count = W.get<int>(first + 7, n_dtree);
+    T.dtree_rad = W.get<float>(first + 8, n_dtree);
+    ck(cudaMemsetAsync(T.slot_value, 0, sizeof(float) * std::max(1, f.n_value_slots), st), "memset");
+    ck(cudaMemsetAsync(T.dtree_count, 0, sizeof(int) * std::max(1, n_dtree), st), "memset");
+    ck(cudaMemsetAsync(T.dtree_rad, 0, sizeof(float) * std::max(1, n_dtree), st), "memset");
+    return T;
+}
+
 constexpr size_t kKeptPPGBytes = 256 << 20;  // of an SD-tree render's buffers, kept for the scene's next one
 
 // PPG::render (src/renderer/ppg.h:149-215): passes of 1, 2, 4, ... spp while
@@ -418,26 +443,8 @@ void render_ppg(pt_scene* s, const pt_render_desc* desc, float* d_dst) {
     double launches = 0;
     for (size_t l = 0; l < passes.size(); l++) {
         const SDTreeFlat f = tree.flatten();
-        DevSDTree T;
-        for (int k = 0; k < 3; k++) { T.lo[k] = f.lo[k]; T.hi[k] = f.hi[k]; }
-        std::vector<int2> sn(f.snode.size() / 2);
-        for (size_t i = 0; i < sn.size(); i++) sn[i] = make_int2(f.snode[2 * i], f.snode[2 * i + 1]);
-        T.snode = W.upload(4, sn, st);
-        T.dnode = W.upload(5, f.dnode, st);
-        T.dtree_root = W.upload(6, f.dtree_root, st);
-        T.leaf_off = W.upload(7, f.dtree_leaf_off, st);
-        T.leaf_cnt = W.upload(8, f.dtree_leaf_cnt, st);
-        std::vector<float4> lv(f.leaves.size() / 4);
-        for (size_t i = 0; i < lv.size(); i++)
-            lv[i] = make_float4(f.leaves[4 * i], f.leaves[4 * i + 1], f.leaves[4 * i + 2], f.leaves[4 * i + 3]);
-        T.leaves = W.upload(9, lv, st);
+        const DevSDTree T = upload_tree(W, 4, f, st);
         const int n_dtree = (int)f.dtree_root.size();
-        T.slot_value = W.get<float>(10, f.n_value_slots);
-        T.dtree_count = W.get<int>(11, n_dtree);
-        T.dtree_rad = W.get<float>(12, n_dtree);
-        ck(cudaMemsetAsync(T.slot_value, 0, sizeof(float) * std::max(1, f.n_value_slots), st), "memset");
-        ck(cudaMemsetAsync(T.dtree_count, 0, sizeof(int) * std::max(1, n_dtree), st), "memset");
-        ck(cudaMemsetAsync(T.dtree_rad, 0, sizeof(float) * std::max(1, n_dtree), st), "memset");
         ck(cudaMemsetAsync(s->film, 0, sizeof(unsigned long long) * film_n, st), "memset film");
         launch_init_slots(slots, capacity, st);
         P.spp = passes[l];
@@ -1611,6 +1618,80 @@ pt_status pt_debug_sdtree_run(const float* lo, const float* hi, int32_t n_iters,
             if (out_counts) out_counts[i] = cnt[i];
             if (out_flux) out_flux[i] = flux[i];
         }
+    });
+}
+
+pt_status pt_debug_sdtree_splat(const float* lo, const float* hi, int32_t n_iters, const int32_t* n_splats,
+                                const float* splats, int32_t n_paths, const int32_t* n_verts, const float* verts,
+                                int32_t on_device, int32_t max_slots, float* out_slots, int32_t max_spatial,
+                                int32_t* out_counts, float* out_flux, int32_t* n_slots, int32_t* n_spatial) {
+    if (!lo || !hi || n_iters < 0 || (n_iters > 0 && (!n_splats || !splats)) || n_paths < 1 || !n_verts || !verts ||
+        !out_slots || !out_counts || !out_flux || !n_slots || !n_spatial) {
+        g_error = "bad argument";
+        return PT_ERR_INVALID;
+    }
+    return guarded([&] {
+        SDTreeHost t(lo, hi);
+        size_t off = 0;
+        for (int it = 0; it < n_iters; it++) {
+            for (int k = 0; k < n_splats[it]; k++, off++) t.splat(splats[7 * off], splats + 7 * off + 1, splats + 7 * off + 4);
+            t.update();
+        }
+        t.clear_accumulators();
+        int depth = 1;
+        for (int i = 0; i < n_paths; i++) {
+            if (n_verts[i] < 0 || n_verts[i] > 0xffff) throw std::invalid_argument("vertices of a path must be in [0, 65535]");
+            depth = std::max(depth, n_verts[i]);
+        }
+        if (on_device) {
+            const SDTreeFlat f = t.flatten();
+            const size_t n = (size_t)n_paths * depth;
+            std::vector<float4> vp(n), vd(n);
+            std::vector<float> vr(n);
+            const float* v = verts;
+            for (int i = 0; i < n_paths; i++)
+                for (int k = 0; k < n_verts[i]; k++, v += 9) {
+                    const size_t j = (size_t)i * depth + k;
+                    vp[j] = make_float4(v[0], v[1], v[2], v[3]);
+                    vd[j] = make_float4(v[4], v[5], v[6], v[7]);
+                    vr[j] = v[8];
+                }
+            DebugCtx c;
+            Workspace W;
+            PPGVerts V{W.upload(0, vp, c.st), W.upload(1, vd, c.st), W.upload(2, vr, c.st)};
+            const int* d_n = W.upload(3, std::vector<int>(n_verts, n_verts + n_paths), c.st);
+            const DevSDTree T = upload_tree(W, 4, f, c.st);
+            launch_debug_splat(T, V, d_n, n_paths, depth, c.st);
+            ck(cudaGetLastError(), "launch");
+            std::vector<float> hv(f.n_value_slots), hr(f.dtree_root.size());
+            std::vector<int32_t> hc(f.dtree_root.size());
+            ck(cudaMemcpyAsync(hv.data(), T.slot_value, sizeof(float) * hv.size(), cudaMemcpyDeviceToHost, c.st), "copy");
+            ck(cudaMemcpyAsync(hc.data(), T.dtree_count, sizeof(int) * hc.size(), cudaMemcpyDeviceToHost, c.st), "copy");
+            ck(cudaMemcpyAsync(hr.data(), T.dtree_rad, sizeof(float) * hr.size(), cudaMemcpyDeviceToHost, c.st), "copy");
+            ck(cudaStreamSynchronize(c.st), "splats");
+            t.accumulate(hv.data(), hc.data(), hr.data());
+        } else {
+            const float* v = verts;
+            for (int i = 0; i < n_paths; v += 9 * (size_t)n_verts[i], i++) {
+                if (n_verts[i] == 0) continue;
+                float acc[3] = {1.0f, 1.0f, 1.0f};
+                const float* last = v + 9 * (size_t)(n_verts[i] - 1);
+                if (!(last[6] > 0.f || last[7] > 0.f || last[8] > 0.f)) continue;
+                for (const float* x = last; x >= v; x -= 9) {
+                    for (int a = 0; a < 3; a++) acc[a] *= x[6 + a];
+                    t.splat(std::max(acc[0], std::max(acc[1], acc[2])), x, x + 3);
+                }
+            }
+        }
+        std::vector<float> values, rad;
+        std::vector<int32_t> counts;
+        t.accumulators(&values, &counts, &rad);
+        *n_slots = (int32_t)values.size();
+        *n_spatial = (int32_t)counts.size();
+        if (*n_slots > max_slots || *n_spatial > max_spatial) throw Fail(PT_ERR_LIMIT, "the tree exceeds the given buffers");
+        std::copy(values.begin(), values.end(), out_slots);
+        std::copy(counts.begin(), counts.end(), out_counts);
+        std::copy(rad.begin(), rad.end(), out_flux);
     });
 }
 

@@ -180,6 +180,23 @@ void SDTreeHost::accumulate(const float* slot_values, const int32_t* counts, con
         [&](const SNodeH*, const DNodeH* d) { const_cast<DNodeH*>(d)->value += slot_values[slot++]; });
 }
 
+void SDTreeHost::accumulators(std::vector<float>* slot_values, std::vector<int32_t>* counts,
+                              std::vector<float>* radiance) const {
+    walk(
+        root_.get(),
+        [&](const SNodeH* s) {
+            counts->push_back(s->dtree->count);
+            radiance->push_back(s->dtree->radiance);
+        },
+        [&](const SNodeH*, const DNodeH* d) { slot_values->push_back(d->value); });
+}
+
+void SDTreeHost::clear_accumulators() {
+    walk(
+        root_.get(), [](const SNodeH* s) { s->dtree->count = 0, s->dtree->radiance = 0.0f; },
+        [](const SNodeH*, const DNodeH* d) { const_cast<DNodeH*>(d)->value = 0.0f; });
+}
+
 SDTreeFlat SDTreeHost::flatten() const {
     SDTreeFlat f;
     for (int k = 0; k < 3; k++) { f.lo[k] = lo_[k]; f.hi[k] = hi_[k]; }

@@ -67,6 +67,9 @@ public:
     // Folds one iteration's device accumulators (slot values in flatten()
     // order, per-dtree counts and flux) into the tree.
     void accumulate(const float* slot_values, const int32_t* counts, const float* radiance);
+    // The same accumulators: read, and set to zero.
+    void accumulators(std::vector<float>* slot_values, std::vector<int32_t>* counts, std::vector<float>* radiance) const;
+    void clear_accumulators();
     void update();  // SDTree::update: subdivide(12000, iteration); iteration++
     SDTreeFlat flatten() const;
     // Host versions of the device lookups (used by the host-only checks):

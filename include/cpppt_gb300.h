@@ -405,6 +405,18 @@ pt_status pt_debug_sdtree_run(const float* lo, const float* hi, int32_t n_iters,
                               const float* splats, int32_t max_leaves, float* out_leaves, int32_t* out_leaf_counts,
                               int32_t* out_counts, float* out_flux, int32_t n_queries, const float* queries,
                               float* out_pdf, int32_t* n_spatial);
+/* The splats of finished paths (ppg.h:131-141) on the tree that
+ * pt_debug_sdtree_run's rounds leave, its accumulators cleared: on_device = 1
+ * by the SD-tree render's own device code, 0 by a loop on the host (no CUDA
+ * call).  verts: 9 floats per vertex {pos xyz, dir xyz, factor rgb}, path after
+ * path, n_verts[i] of path i.  Outputs: the values of the quadtree leaves
+ * (spatial leaves depth first), the splat count and flux of each spatial leaf.
+ * PT_ERR_LIMIT when there are more than max_slots or max_spatial of them (their
+ * numbers are set). */
+pt_status pt_debug_sdtree_splat(const float* lo, const float* hi, int32_t n_iters, const int32_t* n_splats,
+                                const float* splats, int32_t n_paths, const int32_t* n_verts, const float* verts,
+                                int32_t on_device, int32_t max_slots, float* out_slots, int32_t max_spatial,
+                                int32_t* out_counts, float* out_flux, int32_t* n_slots, int32_t* n_spatial);
 
 /* Texture decoding as a material's image(...) texture sees it (host only):
  * the file's pixels as the reference's Image<Vec3> (rgb = 1) or

@@ -77,3 +77,63 @@ def test_ppg_gives_its_records_back(gpu_lib):
     assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
     fresh = GpuScene(scenes.cornell(256, 256)).render(16, max_depth=2, seed=5, mode=MODE_SDTREE)
     assert np.array_equal(again.view(np.uint32), fresh.view(np.uint32))
+
+
+def _finished_paths(seed, lengths):
+    """Paths whose backward products are powers of two in [1/16, 16]: every sum
+    of fewer than 2^16 of them is exact in any order."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for n in lengths:
+        pos = np.where(rng.random((n, 1)) < 0.7, rng.normal([2, 2, 2], 0.6, (n, 3)), rng.uniform(0, 10, (n, 3)))
+        d = rng.normal([0.3, -0.2, 0.8], 0.7, (n, 3))
+        d /= np.maximum(np.linalg.norm(d, axis=1, keepdims=True), 1e-9)
+        prod = 2.0 ** rng.integers(-4, 5, (n, 3))
+        factor = prod.copy()
+        factor[:-1] /= prod[1:]
+        out.append(np.hstack([pos, d, factor]).astype(np.float32))
+    return out
+
+
+@pytest.mark.parametrize("rounds", [[], [30000, 60000], [20000, 50000, 120000]], ids=["one_leaf", "split", "deep"])
+@pytest.mark.parametrize("lengths", [[1], [0, 0, 3], [7] * 255, [5] * 256, [4] * 257, "mixed", "long"], ids=str)
+def test_device_splats_equal_the_hosts(gpu_lib, rounds, lengths):
+    """Counts, flux and quadtree values of the device's splats of finished
+    paths against the host tree's, exactly: partial blocks, paths without
+    vertices, paths whose last vertex carries nothing, several spatial leaves
+    in a warp."""
+    from cpppt import lib
+    from tests.test_sdtree_host import make_rounds
+    rng = np.random.default_rng(4)
+    if lengths == "mixed":
+        lengths = rng.integers(0, 12, 3001)
+    elif lengths == "long":
+        lengths = [2000, 1, 1023, 0, 4097, 4]
+    paths = _finished_paths(5, lengths)
+    for p in paths[::5][1:]:
+        p[-1:, 6:] = 0
+    args = ([0, 0, 0], [10, 10, 10], make_rounds(7, rounds), paths)
+    host, dev = (lib.sdtree_splat(*args, on_device=k) for k in (False, True))
+    assert host["counts"].sum() == sum(len(p) for p in paths if len(p) and p[-1, 6:].max() > 0)
+    assert len(rounds) == 0 or len(host["counts"]) > 1
+    assert np.array_equal(dev["counts"], host["counts"])
+    for key in ("values", "flux"):
+        assert np.array_equal(dev[key].view(np.uint32), host[key].view(np.uint32)), key
+
+
+def test_splats_of_long_paths_take_linear_time(gpu_lib):
+    """64 paths of 8000 vertices against 64 of 2000: four times the work."""
+    import time
+
+    from cpppt import lib
+
+    def ms(n):
+        paths, best = _finished_paths(6, [n] * 64), 1e9
+        for _ in range(4):
+            t = time.perf_counter()
+            lib.sdtree_splat([0, 0, 0], [10, 10, 10], [], paths, on_device=True)
+            best = min(best, 1e3 * (time.perf_counter() - t))
+        return best
+    short, long = ms(2000), ms(8000)
+    print(f"{short:.1f} ms, {long:.1f} ms")
+    assert long <= 6 * short, (short, long)
