@@ -253,7 +253,9 @@ void ensure_buffers(pt_batch* b, int capacity, size_t film_n, int n_jobs) {
         for (void* p : b->pb_owned)
             if (p != ctr) cudaFree(p);
         b->pb_owned.assign(1, ctr);
+        if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         PathBuffers& B = b->pb;
+        B.capacity = 0;  // until the buffers are there (as the other sizes below)
         for (int k = 0; k < 2; k++) {
             B.o[k] = dalloc<float4>(b->pb_owned, capacity);
             B.d[k] = dalloc<float4>(b->pb_owned, capacity);
@@ -265,28 +267,29 @@ void ensure_buffers(pt_batch* b, int capacity, size_t film_n, int n_jobs) {
         B.sh_d = dalloc<float4>(b->pb_owned, capacity);
         B.sh_c = dalloc<float4>(b->pb_owned, capacity);
         B.capacity = capacity;
-        if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
     }
     if (b->film_cap < film_n) {
         if (b->film) cudaFree(b->film);
         if (b->d_out) cudaFree(b->d_out);
         b->film = nullptr;
         b->d_out = nullptr;
+        b->film_cap = b->out_cap = 0;
+        if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         ck(cudaMalloc(&b->film, sizeof(unsigned long long) * film_n), "cudaMalloc film");
         ck(cudaMalloc(&b->d_out, sizeof(float) * film_n), "cudaMalloc film");
         b->film_cap = film_n;
         b->out_cap = film_n;
-        if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
     }
     if (b->jobs_cap < n_jobs) {
         if (b->d_jobs) cudaFree(b->d_jobs);
         if (b->h_jobs) cudaFreeHost(b->h_jobs);
         b->d_jobs = nullptr;
         b->h_jobs = nullptr;
+        b->jobs_cap = 0;
+        if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         ck(cudaMalloc(&b->d_jobs, sizeof(DevBatchJob) * n_jobs), "cudaMalloc jobs");
         ck(cudaMallocHost(&b->h_jobs, sizeof(DevBatchJob) * n_jobs), "cudaMallocHost jobs");
         b->jobs_cap = n_jobs;
-        if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
     }
 }
 
@@ -418,15 +421,16 @@ NNPathData slot_buffers(pt_batch* b, int capacity, int depth, bool params) {
         b->pd_owned.clear();
         b->pd = NNPathData{};
         b->nn_params = nullptr;
-        b->pd_cap = std::max(capacity, b->pd_cap);
-        b->pd_depth = std::max(depth, b->pd_depth);
-        const int cap = b->pd_cap;
-        b->pd.vert = dalloc<float4>(b->pd_owned, (size_t)cap * std::max(1, b->pd_depth) * kNNVertFloat4);
+        const int cap = std::max(capacity, b->pd_cap), d = std::max(depth, b->pd_depth);
+        b->pd_cap = b->pd_depth = 0;  // until the buffers are there
+        b->pd.vert = dalloc<float4>(b->pd_owned, (size_t)cap * std::max(1, d) * kNNVertFloat4);
         b->pd.acc = dalloc<float4>(b->pd_owned, cap);
         b->pd.slot_stack = dalloc<int>(b->pd_owned, cap);
         b->pd.slot_job = dalloc<int>(b->pd_owned, cap);
         b->pd.fin = dalloc<int4>(b->pd_owned, cap);
         if (params) b->nn_params = dalloc<float4>(b->pd_owned, (size_t)cap * kNNMixF4);
+        b->pd_cap = cap;
+        b->pd_depth = d;
     }
     return b->pd;
 }
@@ -470,6 +474,7 @@ void render_batch_slot(pt_batch* b, const pt_batch_job* jobs, int n_jobs, float*
         if (b->h_nnjobs) cudaFreeHost(b->h_nnjobs);
         b->d_nnjobs = nullptr;
         b->h_nnjobs = nullptr;
+        b->nnjobs_cap = 0;
         ck(cudaMalloc(&b->d_nnjobs, sizeof(DevNNJob) * n_jobs), "cudaMalloc guide jobs");
         ck(cudaMallocHost(&b->h_nnjobs, sizeof(DevNNJob) * n_jobs), "cudaMallocHost guide jobs");
         b->nnjobs_cap = n_jobs;

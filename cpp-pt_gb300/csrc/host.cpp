@@ -618,14 +618,15 @@ int nn_path_buffers(pt_scene* s, int capacity, int depth, bool guided) {
         for (void* p : s->nnpd_owned) cudaFree(p);
         s->nnpd_owned.clear();
         s->nnpd = NNPathData{};
-        s->nnpd_cap = std::max(capacity, s->nnpd_cap);
-        s->nnpd_depth = std::max(depth, s->nnpd_depth);
-        const int cap = s->nnpd_cap;
-        s->nnpd.vert = dalloc<float4>(s->nnpd_owned, (size_t)cap * s->nnpd_depth * kNNVertFloat4);
+        const int cap = std::max(capacity, s->nnpd_cap), d = std::max(depth, s->nnpd_depth);
+        s->nnpd_cap = s->nnpd_depth = 0;  // until the buffers are there
+        s->nnpd.vert = dalloc<float4>(s->nnpd_owned, (size_t)cap * d * kNNVertFloat4);
         s->nnpd.acc = dalloc<float4>(s->nnpd_owned, cap);
         s->nnpd.slot_stack = dalloc<int>(s->nnpd_owned, cap);
         s->nnpd.slot_job = dalloc<int>(s->nnpd_owned, cap);
         s->nnpd.fin = dalloc<int4>(s->nnpd_owned, cap);
+        s->nnpd_cap = cap;
+        s->nnpd_depth = d;
     }
     return capacity;
 }

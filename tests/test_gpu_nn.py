@@ -266,3 +266,26 @@ def test_forward_over_several_tiles(gpu_lib, encoding, n):
     got = lib.nn_forward(w, LO, HI, x, encoding=encoding)
     parts = [lib.nn_forward(w, LO, HI, x[k:k + 4000], encoding=encoding) for k in range(0, n, 4000)]
     assert np.array_equal(got.view(np.uint32), np.concatenate(parts).view(np.uint32))
+
+
+def test_failed_allocation_leaves_scene_and_batch_usable(gpu_lib):
+    """A training render whose vertex records no device can hold (3.8 TB)
+    fails, and the next one, scene or batch, allocates its own and gives the
+    image of a fresh scene."""
+    from cpppt import scenes
+    from cpppt.lib import FLAG_NN_FREEZE, MODE_NN, GpuBatch, GpuScene, PtError
+    sc = scenes.slit_room(n_boxes=20, width=512, height=512)
+    want = GpuScene(sc).render(2, max_depth=6, seed=3, mode=MODE_NN, flags=FLAG_NN_FREEZE)
+    gs = GpuScene(sc)
+    with pytest.raises(PtError) as e:
+        gs.render(2, max_depth=65535, seed=3, mode=MODE_NN)
+    assert e.value.status == 3
+    got = gs.render(2, max_depth=6, seed=3, mode=MODE_NN)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    one = GpuScene(sc)
+    batch = GpuBatch([one])
+    with pytest.raises(PtError) as e:
+        batch.render([dict(scene=0, spp=2, max_depth=65535, seed=3)], mode=MODE_NN)
+    assert e.value.status == 3
+    got, = batch.render([dict(scene=0, spp=2, max_depth=6, seed=3)], mode=MODE_NN)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
