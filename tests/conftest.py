@@ -14,6 +14,20 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a GB300 (sm_103a) GPU")
 
 
+# Tests that compile or run the reference renderer's own sources, which
+# oracle/build_ref.sh copies where they are at hand; without the copy they
+# cannot run, and say so instead of failing.
+NEED_REFERENCE = ("test_adapter.py::test_adapter_", "test_gpu_ppg.py::test_ppg_matches_reference_ppg")
+
+
+def pytest_collection_modifyitems(items):
+    if os.path.isdir(os.path.join(ROOT, "oracle", "_ref", "src")):
+        return
+    for item in items:
+        if any(name in item.nodeid for name in NEED_REFERENCE):
+            item.add_marker(pytest.mark.skip(reason="the reference's sources are not here (oracle/build_ref.sh)"))
+
+
 @pytest.fixture(scope="session")
 def golden():
     def get(name):
