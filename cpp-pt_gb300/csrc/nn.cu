@@ -1149,7 +1149,7 @@ __global__ void __launch_bounds__(kTraceThreads) k_shadow_nn(DevScene S, PathBuf
                                                    unsigned long long* __restrict__ film, NNPathData PD,
                                                    const DevBatchJob* __restrict__ jobs) {
     after_previous();
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = ctr->n_shadow;
     if (n == 0) return;
     TraceCount cnt{0u, 0u};

@@ -38,7 +38,7 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src) {
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_closest(DevScene S, const float* __restrict__ rays, int n,
                                                                  float4* __restrict__ hits, int* counter,
                                                                  uint32_t* status) {
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     TraceCount cnt{0u, 0u};
     persistent_trace<false, false>(
         S, s_stack, n, counter, status, cnt,
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_clos
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_any(DevScene S, const float* __restrict__ rays, int n,
                                                              uint8_t* __restrict__ occ, int* counter,
                                                              uint32_t* status) {
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     TraceCount cnt{0u, 0u};
     persistent_trace<true, false>(
         S, s_stack, n, counter, status, cnt,
@@ -141,7 +141,7 @@ template <bool COUNT>
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(DevScene S, PathIO in, float4* __restrict__ Hout,
                                                                            WaveCounters* ctr) {
     after_previous();
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = ctr->n_cur;
     if (n == 0) return;  // drained wavefront
     TraceCount cnt{0u, 0u};
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(Dev
 
 __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(DevScene S, ShadowIO Q, int cur, WaveCounters* ctr,
                                                           unsigned long long* __restrict__ film) {
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = cur ? ctr->n_shadow1 : ctr->n_shadow;
     if (n == 0) return;
     shadow_queue<kTraceThreads>(S, s_stack, Q, n, ctr, film, true);
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_wave
                                                                                  int cur, WaveCounters* ctr,
                                                                                  unsigned long long* __restrict__ film) {
     after_previous();
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = ctr->n_cur, m = cur ? ctr->n_shadow : ctr->n_shadow1;
     if (n == 0 && m == 0) return;
     TraceCount cnt{0u, 0u};
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kFinishThreads, 1) k_finish(
     after_previous();
     const unsigned full = 0xffffffffu;
     const int m = ctr->n_shadow + ctr->n_shadow1;  // at most one of them is non-zero
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     if (m > 0) shadow_queue<kFinishThreads>(S, s_stack + kFinishAnyWord, Q, m, ctr, film, true);
     const int n = ctr->n_finish;
     if (n == 0) return;

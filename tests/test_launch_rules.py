@@ -52,3 +52,14 @@ def test_overlapping_launches_begin_with_the_wait():
             if head.startswith("__global__") and body.lstrip().startswith("after_previous();"):
                 waiting.add(re.search(r"\b(k_\w+)\(", head).group(1))
     assert launched and launched <= waiting, launched - waiting
+
+
+def test_traversal_stacks_are_aligned():
+    """Closest-hit stacks are read and written eight bytes at a time."""
+    found = 0
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            for decl in re.findall(r"extern __shared__[^;]*s_stack\[\];", open(os.path.join(CSRC, name)).read()):
+                found += 1
+                assert "__align__(16)" in decl, (name, decl)
+    assert found >= 6
