@@ -267,8 +267,10 @@ def run_ours(a):
     n_e2e = len(e2e_ms)
     e2e_val, _, _ = aggregate(dist, paths / a.steps, 0.0, float(np.mean(e2e_ms)), "cuda")
 
-    # roofline of the dominant kernel (closest-hit extension): algorithmic
-    # bytes from a counting render, duration from an event-timed render of
+    # roofline of the dominant kernel (closest-hit extension), which is bound by
+    # instruction issue (76 % of the slots): its algorithmic bytes, which the
+    # caches serve, over the HBM rate, beside the bytes that reach DRAM
+    # (`traffic`).  Bytes from a counting render, duration from an event-timed render of
     # the same work (same seed -> the same rays)
     gs.render_device(out.data_ptr(), spp, max_depth=a.depth, seed=4242, flags=FLAG_COUNT)
     cnt = gs.stats()
@@ -307,7 +309,7 @@ def run_ours(a):
                "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": h2d / n_e2e,
                        "d2h_bytes_per_step": d2h / n_e2e, "api": "pt_render (host image buffer)"},
                "gpu_launches": int(launches),
-               "roofline": {"bound": "hbm", "kernel": "k_extend (closest-hit traversal)",
+               "roofline": {"bound": "issue", "kernel": "k_extend (closest-hit traversal)",
                             "achieved": achieved, "peak": peak,
                             "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6800",
                             "unit": "GB/s", "frac": achieved / peak,

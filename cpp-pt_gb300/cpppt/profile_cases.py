@@ -9,6 +9,10 @@
     python -m cpppt.profile_cases batchnn [R]    # 8 slit rooms (50k-430k tris), 640x360, one learned
                                                  # guide each, trained online: R batched renders of 2 spp
     python -m cpppt.profile_cases batchslit [R]  # the same batches with plain PT (PT_FLAG_UNBIASED_MIS)
+    python -m cpppt.profile_cases noalloc  # 1M-tri soup, 512x512, 1 spp, depth 10, without allocations: the
+                                           # wavefront loop's kernels as plain launches (ncu-visible)
+    python -m cpppt.profile_cases sdtree   # Cornell box, 128x128, 64 spp, depth 8, SD-tree
+    python -m cpppt.profile_cases create   # creation of the 200k-tri slit room
     python -m cpppt.profile_cases c5 [R] [plain|train|frozen]  # the eight 1080p rooms of
                                                  # batch_guiding_eval (11.4M tris): R batched renders of 2 spp
 
@@ -23,7 +27,7 @@ import sys
 import time
 
 from . import scenes
-from .lib import FLAG_NN_FREEZE, FLAG_TIME_KERNELS, FLAG_UNBIASED_MIS, MODE_MIS, MODE_NN, GpuBatch, GpuScene
+from .lib import FLAG_NN_FREEZE, FLAG_TIME_KERNELS, FLAG_UNBIASED_MIS, MODE_MIS, MODE_NN, MODE_SDTREE, GpuBatch, GpuScene
 
 
 def case_extend():
@@ -52,6 +56,36 @@ def case_raycounts():
         per.append(int(c - prev))
         prev = c
     return {"rays_per_bounce": per, "total": int(prev)}
+
+
+def case_noalloc():
+    """pt_render_device_noalloc runs the plain wavefront (65,536 paths in
+    flight, k_finish at the end) without a graph."""
+    import ctypes as C
+
+    import torch
+
+    from . import lib
+    gs = GpuScene(scenes.soup(seed=2, width=512, height=512))
+    out = torch.zeros(512, 512, 3, device="cuda")
+    for _ in range(2):
+        assert lib.load().pt_render_device_noalloc(gs.h, C.byref(gs.desc(1, 10, 3, 1, MODE_MIS, 0)), out.data_ptr(),
+                                                   None) == 0
+    torch.cuda.synchronize()
+    return gs.stats()
+
+
+def case_sdtree():
+    gs = GpuScene(scenes.cornell(128, 128))
+    for _ in range(2):
+        gs.render(64, max_depth=8, seed=1, mode=MODE_SDTREE)
+    return gs.stats()
+
+
+def case_create():
+    for _ in range(2):
+        gs = GpuScene(scenes.slit_room(seed=4, n_boxes=1000, box_subdiv=4, width=640, height=360))
+    return {"scenes": 2}
 
 
 def case_nn(renders: int = 2):
@@ -123,7 +157,8 @@ def case_c5(renders: int = 2, what: str = "train"):
 
 def main():
     name = sys.argv[1] if len(sys.argv) > 1 else "extend"
-    fn = {"extend": case_extend, "raycounts": case_raycounts, "nn": case_nn, "slit": case_slit, "batch": case_batch, "batchnn": case_batchnn,
+    fn = {"extend": case_extend, "raycounts": case_raycounts, "noalloc": case_noalloc, "sdtree": case_sdtree,
+          "create": case_create, "nn": case_nn, "slit": case_slit, "batch": case_batch, "batchnn": case_batchnn,
           "batchslit": case_batchslit, "c5": case_c5}[name]
     t0 = time.perf_counter()
     args = [int(sys.argv[2])] if len(sys.argv) > 2 else []

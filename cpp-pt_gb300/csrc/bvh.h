@@ -83,7 +83,9 @@ WideBVH build_wide_bvh(const float* tri_v, int n_tris, int max_leaf = 4, int n_t
 // which it can stand as at most j children of one wide node: a leaf costs
 // nothing, an inner node either becomes one child (its area and the best
 // split of 4 slots between its two sides) or is dissolved, its slots split
-// between its sides.  Against opening the child of largest area first: 1M
+// between its sides.  (The dynamic program of Ylitie, Karras and Laine 2017,
+// "Efficient incoherent ray traversal on GPUs through compressed wide BVHs",
+// for leaves that stay as they are.)  Against opening the child of largest area first: 1M
 // triangle soup 21 % fewer nodes and 4 % less area, closest hit of 1.8M rays
 // 851 -> 754 us, any hit 601 -> 578; 192k-triangle room any hit 138 -> 124.
 //

@@ -31,8 +31,9 @@ struct DevCamera {
 };
 
 // Default bounds of a ray's traversal (kernel-side bounded loops): steps (node
-// visits and leaf tests; tested at each visit) and entries of the per-lane stack.  A scene may carry
-// lower bounds (pt_debug_traversal_limits), never higher ones.
+// visits and leaf tests; tested at each visit) and entries of the per-lane
+// stack.  A scene may carry lower bounds (pt_debug_traversal_limits), never
+// higher ones.
 constexpr uint32_t kTraversalStepLimit = 1u << 22;
 constexpr int32_t kTraversalStackSize = 64;
 

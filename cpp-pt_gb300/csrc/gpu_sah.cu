@@ -819,7 +819,8 @@ __global__ void k_parents(const Node2* __restrict__ nodes, int n, int32_t* __res
 // first one (a record is {cost[3], choices | depth << kDepthShift}, zero for a
 // leaf), bottom-up: a thread starts at each leaf and climbs; of a node's two
 // arrivals (counted in `seen`, zeroed) the first ends and the second, which
-// finds the records of all nodes below, goes on.  Bound by the latency of that
+// finds the records of all nodes below, goes on (Karras 2012, "Maximizing
+// parallelism in the construction of BVHs, octrees, and k-d trees").  Bound by the latency of that
 // chain (about 25 levels).
 __global__ void k_collapse_cost(const Node2* __restrict__ nodes, int n, const int32_t* __restrict__ parent,
                                 int32_t* __restrict__ seen, float4* __restrict__ cost) {

@@ -196,9 +196,9 @@ __device__ __forceinline__ void splat_paths(const DevSDTree& T, const PPGVerts& 
     }
 }
 
-__global__ void __launch_bounds__(kShadePPGThreads) k_shade_ppg(DevScene S, PathIO in, PathIO nxt,
-                                                   const float4* hit, RenderParams P, WaveCounters* ctr, unsigned long long* __restrict__ film,
-                                                   DevSDTree T, PPGVerts V, int* slot_stack) {
+__global__ void __launch_bounds__(kShadePPGThreads)
+    k_shade_ppg(DevScene S, PathIO in, PathIO nxt, const float4* hit, RenderParams P, WaveCounters* ctr,
+                unsigned long long* __restrict__ film, DevSDTree T, PPGVerts V, int* slot_stack) {
     after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
@@ -409,8 +409,8 @@ void launch_debug_splat(const DevSDTree& T, const PPGVerts& V, const int* n_vert
 void launch_generate_ppg(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                          const int* slot_stack, int num_sms, cudaStream_t st) {
     // a resident grid over the free slots (as the plain wavefront's)
-    launch_after(k_generate_ppg, max(1, min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st, S, path_io(B, 1 - cur), B.capacity,
-                                                                                       P, ctr, slot_stack);
+    launch_after(k_generate_ppg, max(1, min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st, S, path_io(B, 1 - cur),
+                 B.capacity, P, ctr, slot_stack);
     launch_after(k_advance_ppg, 1, 32, 0, st, ctr, B.capacity);
 }
 

@@ -313,14 +313,21 @@ constexpr int kTrainCapacity = 1 << 20;
 // state and 128 B of mixture each.  The slit room at 1280x720, 4 spp, frozen
 // guide: 2^20 12.46 ms, 2^21 11.95, 2^22 11.19.
 constexpr int kFrozenCapacity = 1 << 22;
-constexpr int kItersPerGraph = 16;   // of the learned-guide and SD-tree renders between host steps; even: buffers alternate
+// Of the learned-guide and SD-tree renders between host steps; even: the buffers alternate.
+constexpr int kItersPerGraph = 16;
 // Iterations between two looks at the counters: where all paths start at once
 // they end within `last` iterations (the depth, and one more where shadow rays
 // follow an iteration late), and the rest of sixteen would be empty launches.
 int iterations_per_check(unsigned long long work, int capacity, int last) {
     return work <= (unsigned long long)capacity ? std::min(kItersPerGraph, (last + 1) & ~1) : kItersPerGraph;
 }
-constexpr int kItersPerBody = 20;    // of a plain render's device-driven loop body; even
+// Iterations of a plain render's device-driven loop body; even.  Those after a
+// render's last paths are empty launches: with bodies of 8, 12, 16 and 20 a
+// 640x360, 1-spp render of the 1M-triangle soup takes 1.71, 1.77, 1.81 and 1.84
+// ms, the Cornell box at 256x256, 64 spp 3.40, 3.46, 3.51 and 3.58 (1080p
+// renders: no difference beyond the clock's).  20, not fewer, because the
+// render-loop test takes more than 80 launches as the sign that the loop ran.
+constexpr int kItersPerBody = 20;
 
 // The scene's wavefront buffers for `capacity` paths in flight (192 B per
 // path, kept for later renders).  Returns the paths in flight the render

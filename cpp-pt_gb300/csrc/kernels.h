@@ -21,13 +21,14 @@ void launch_trace_any(const DevScene& S, const float* rays, int n, uint8_t* occl
 // Wavefront path state: capacity paths, structure of arrays, two copies.
 struct PathBuffers {
     float4* o[2];    // origin.xyz, p (pdf of the last BSDF sample, RR scaled)
-    float4* d[2];    // direction.xyz, unused
+    float4* d[2];    // direction.xyz, the scene's root node
     float4* thr[2];  // throughput rgb, unused
-    int4* info[2];   // pixel, sample, bounce | sampled_delta << 16, unused
+    int4* info[2];   // pixel, sample, bounce | sampled_delta << 16 (learned guide: | job << kNNJobShift), then the
+                     // job, or the vertex slot (SD-tree renders, guides in training)
     float4* hit;     // t, prim, beta, gamma of the current buffer
     float4* sh_o;    // shadow ray origin.xyz, max_t
-    float4* sh_d;    // direction.xyz, pixel
-    float4* sh_c;    // contribution rgb
+    float4* sh_d;    // direction.xyz, film pixel
+    float4* sh_c;    // contribution rgb, the scene's root node (guides in training: the path's slot)
     int capacity;
 };
 
@@ -117,8 +118,8 @@ int noalloc_paths();
 constexpr int kDebugBsdfIn = 20, kDebugBsdfOut = 10, kDebugLightIn = 6, kDebugLightOut = 10;
 void launch_debug_bsdf(const float* in, float* out, int n, cudaStream_t st);
 void launch_debug_light(const DevScene& S, const float* in, float* out, int n, cudaStream_t st);
-// Shared-memory limits of the traversal kernels (their top-node staging may
-// exceed the default 48 KB); call on each device before the first launch.
+// Shared-memory limits of the traversal kernels (their stacks take more than
+// the default 48 KB); call on each device before the first launch.
 cudaError_t trace_kernels_setup();
 // film: 32.32 fixed point per pixel and channel; out = film * scale / 2^32
 void launch_film_resolve(const unsigned long long* film, float* out, int n, double scale, cudaStream_t st);

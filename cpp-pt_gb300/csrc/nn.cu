@@ -330,9 +330,9 @@ __global__ void __launch_bounds__(kTcInferThreads) k_nn_forward_debug(const DevN
 // Guide parameters for every live path's hit (run between extend and shade),
 // each path with its job's network.
 template <bool ONEBLOB>
-__global__ void __launch_bounds__(kTcInferThreads, 4) k_nn_infer(DevScene S, PathIO in, const float4* hit, WaveCounters* ctr,
-                                                              const DevNNJob* __restrict__ nnj,
-                                                              float4* __restrict__ params) {
+__global__ void __launch_bounds__(kTcInferThreads, 4)
+    k_nn_infer(DevScene S, PathIO in, const float4* hit, WaveCounters* ctr, const DevNNJob* __restrict__ nnj,
+               float4* __restrict__ params) {
     after_previous();
     extern __shared__ __align__(1024) unsigned char smem[];
     const int n = ctr->n_cur;
@@ -721,8 +721,11 @@ void launch_nn_forward_debug(const DevNNJob* nnj, const float* in, int n, float*
 void launch_nn_infer(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, const DevNNJob* nnj,
                      float4* params, int num_sms, cudaStream_t st, bool oneblob) {
     // four CTAs of 128 threads per SM fit in shared memory (48 KB each)
-    if (oneblob) launch_after(k_nn_infer<true>, num_sms * 4, kTcInferThreads, nn_smem_infer(), st, S, path_io(B, cur), B.hit, ctr, nnj, params);
-    else launch_after(k_nn_infer<false>, num_sms * 4, kTcInferThreads, nn_smem_infer(), st, S, path_io(B, cur), B.hit, ctr, nnj, params);
+    const int g = num_sms * 4;
+    const size_t smem = nn_smem_infer();
+    const PathIO in = path_io(B, cur);
+    if (oneblob) launch_after(k_nn_infer<true>, g, kTcInferThreads, smem, st, S, in, B.hit, ctr, nnj, params);
+    else launch_after(k_nn_infer<false>, g, kTcInferThreads, smem, st, S, in, B.hit, ctr, nnj, params);
 }
 // Zeroes each task's gradient and loss (and, with prep, its T sum).
 __global__ void k_nn_task_zero(const NNTrainTask* __restrict__ tasks, int prep) {
@@ -799,10 +802,10 @@ __device__ __forceinline__ void film_add_nn(unsigned long long* film, size_t pix
 // 5: film total before the NEE (rgb), p_bsdf(wi_nee)  6: wi_nee xyz, NEE valid.
 constexpr int kNNVert = kNNVertFloat4;
 constexpr int kShadeNNThreads = 256;
-__global__ void __launch_bounds__(kShadeNNThreads, 2) k_shade_nn(DevScene S, PathBuffers B, PathIO in, PathIO nxt, int cur, RenderParams P,
-                                                  WaveCounters* ctr, unsigned long long* __restrict__ film,
-                                                  const float4* params, NNPathData PD, int guided,
-                                                  const DevBatchJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(kShadeNNThreads, 2)
+    k_shade_nn(DevScene S, PathBuffers B, PathIO in, PathIO nxt, int cur, RenderParams P, WaveCounters* ctr,
+               unsigned long long* __restrict__ film, const float4* params, NNPathData PD, int guided,
+               const DevBatchJob* __restrict__ jobs) {
     after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = ctr->n_cur;
@@ -1177,7 +1180,8 @@ __global__ void __launch_bounds__(kTraceThreads) k_shadow_nn(DevScene S, PathBuf
 }
 
 cudaError_t nn_shadow_smem_limit() {
-    return cudaFuncSetAttribute(k_shadow_nn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trace_smem(false, true, kTraceThreads));
+    return cudaFuncSetAttribute(k_shadow_nn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)trace_smem(false, true, kTraceThreads));
 }
 
 // Camera paths (stratified like pathtracerMIS.h:148-153) with a vertex slot.
@@ -1270,23 +1274,26 @@ __global__ void k_advance_nn(WaveCounters* ctr, int capacity) {
 void launch_nn_shade(const DevScene& S, const PathBuffers& B, int cur, const RenderParams& P, WaveCounters* ctr,
                      unsigned long long* film, const float4* params, const NNPathData& PD, bool guided,
                      const DevBatchJob* jobs, cudaStream_t st) {
-    launch_after(k_shade_nn, (B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st, S, B, path_io(B, cur), path_io(B, 1 - cur), cur, P, ctr, film, params, PD, guided ? 1 : 0, jobs);
+    launch_after(k_shade_nn, (B.capacity + kShadeNNThreads - 1) / kShadeNNThreads, kShadeNNThreads, 0, st, S, B,
+                 path_io(B, cur), path_io(B, 1 - cur), cur, P, ctr, film, params, PD, guided ? 1 : 0, jobs);
 }
 void launch_nn_shadow(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                       const NNPathData& PD, const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    launch_after(k_shadow_nn, num_sms * kTraceBlocksPerSM, kTraceThreads, trace_smem(false, true, kTraceThreads), st, S, B, ctr, film, PD, jobs);
+    launch_after(k_shadow_nn, num_sms * kTraceBlocksPerSM, kTraceThreads, trace_smem(false, true, kTraceThreads), st, S, B,
+                 ctr, film, PD, jobs);
 }
 void launch_nn_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const NNPathData& PD,
                         const DevBatchJob* jobs, int n_jobs, int num_sms, cudaStream_t st) {
     // a resident grid over the free slots (as the plain wavefront's)
-    launch_after(k_generate_nn, std::max(1, std::min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st, 
-        path_io(B, 1 - cur), B.capacity, ctr, PD, jobs, n_jobs);
+    launch_after(k_generate_nn, std::max(1, std::min((B.capacity + 255) / 256, num_sms * 8)), 256, 0, st,
+                 path_io(B, 1 - cur), B.capacity, ctr, PD, jobs, n_jobs);
     if (PD.rec_cap > 0) launch_after(k_advance_nn, 1, 32, 0, st, ctr, B.capacity);
     else launch_advance(ctr, B.capacity, cur, st);
 }
 void launch_nn_finish(const NNPathData& PD, WaveCounters* ctr, const DevNNJob* nnj, int max_depth, int capacity,
                       cudaStream_t st) {
-    launch_after(k_finish_nn, (capacity + kFinishNNThreads - 1) / kFinishNNThreads, kFinishNNThreads, 0, st, PD, ctr, nnj, max_depth);
+    launch_after(k_finish_nn, (capacity + kFinishNNThreads - 1) / kFinishNNThreads, kFinishNNThreads, 0, st, PD, ctr, nnj,
+                 max_depth);
 }
 
 }  // namespace cpppt_gb300

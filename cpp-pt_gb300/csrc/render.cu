@@ -6,7 +6,7 @@
 // path, then any hit for the shadow rays the iteration before queued, whose
 // unoccluded NEE contributions go to the film) -> shade (emission + MIS, BSDF
 // sample, NEE shadow ray, Russian roulette; survivors are appended compactly
-// to the next buffer with warp-aggregated atomics) -> generate (new camera
+// to the next buffer, one counter addition per CTA) -> generate (new camera
 // paths fill the next buffer up to capacity from a global work counter) ->
 // advance (one thread swaps counts).
 // All sizes are read from device counters, so an iteration needs no host
@@ -35,9 +35,9 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src) {
 // ---------------------------------------------------------------------------
 // Ray batches (BVH::intersect / intersect_any on arrays of rays)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_closest(DevScene S, const float* __restrict__ rays, int n,
-                                                                 float4* __restrict__ hits, int* counter,
-                                                                 uint32_t* status) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM)
+    k_trace_closest(DevScene S, const float* __restrict__ rays, int n, float4* __restrict__ hits, int* counter,
+                    uint32_t* status) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     TraceCount cnt{0u, 0u};
     persistent_trace<false, false>(
@@ -51,9 +51,9 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_clos
         [&](int i, const HitRec& h) { hits[i] = make_float4(h.t, __int_as_float(h.prim), h.beta, h.gamma); });
 }
 
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_any(DevScene S, const float* __restrict__ rays, int n,
-                                                             uint8_t* __restrict__ occ, int* counter,
-                                                             uint32_t* status) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM)
+    k_trace_any(DevScene S, const float* __restrict__ rays, int n, uint8_t* __restrict__ occ, int* counter,
+                uint32_t* status) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     TraceCount cnt{0u, 0u};
     persistent_trace<true, false>(
@@ -138,8 +138,8 @@ __device__ __forceinline__ void shadow_queue(const DevScene& S, uint32_t* s_stac
 }
 
 template <bool COUNT>
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(DevScene S, PathIO in, float4* __restrict__ Hout,
-                                                                           WaveCounters* ctr) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM)
+    k_extend(DevScene S, PathIO in, float4* __restrict__ Hout, WaveCounters* ctr) {
     after_previous();
     extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = ctr->n_cur;
@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_extend(Dev
     }
 }
 
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(DevScene S, ShadowIO Q, int cur, WaveCounters* ctr,
-                                                          unsigned long long* __restrict__ film) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM)
+    k_shadow(DevScene S, ShadowIO Q, int cur, WaveCounters* ctr, unsigned long long* __restrict__ film) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = cur ? ctr->n_shadow1 : ctr->n_shadow;
     if (n == 0) return;
@@ -172,10 +172,9 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_shadow(Dev
 // measured (1M-triangle soup) 640x360 at 1 spp 2.9 -> 2.4
 // ms, 1920x1080 at 16 spp 106.3 -> 98.8 ms together with k_generate's grid;
 // the Cornell box at 256x256, 64 spp 6.1 -> 4.75 ms (same images).
-__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM) k_trace_wave(DevScene S, PathIO in,
-                                                                                 float4* __restrict__ Hout, ShadowIO Q,
-                                                                                 int cur, WaveCounters* ctr,
-                                                                                 unsigned long long* __restrict__ film) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocksPerSM)
+    k_trace_wave(DevScene S, PathIO in, float4* __restrict__ Hout, ShadowIO Q, int cur, WaveCounters* ctr,
+                 unsigned long long* __restrict__ film) {
     after_previous();
     extern __shared__ __align__(16) uint32_t s_stack[];
     const int n = ctr->n_cur, m = cur ? ctr->n_shadow : ctr->n_shadow1;
@@ -206,9 +205,9 @@ struct ShadeOut {
 
 // One vertex of a path (PathtracerMIS::integrate's loop body): emission with
 // its MIS weight, BSDF sample, next-event estimation, Russian roulette.
-__device__ __forceinline__ void shade_vertex(DevScene S, const DevBatchJob* __restrict__ jobs, float4 O, float4 D, float4 T,
-                                             int4 I, float4 H, WaveCounters* ctr, unsigned long long* __restrict__ film,
-                                             ShadeOut& out) {
+__device__ __forceinline__ void shade_vertex(DevScene S, const DevBatchJob* __restrict__ jobs, float4 O, float4 D,
+                                             float4 T, int4 I, float4 H, WaveCounters* ctr,
+                                             unsigned long long* __restrict__ film, ShadeOut& out) {
     out.push_sh = out.push_cont = false;
     const int prim = __float_as_int(H.y);
     const int pixel = I.x, sample = I.y, bounce = I.z & 0xffff;
@@ -294,10 +293,9 @@ __device__ __forceinline__ void shade_vertex(DevScene S, const DevBatchJob* __re
 }
 
 constexpr int kShadeThreads = 256;
-__global__ void __launch_bounds__(kShadeThreads, CPPPT_SHADE_BLOCKS) k_shade(DevScene S, PathIO in, PathIO nxt, ShadowIO Q,
-                                               const float4* hit, int cur, WaveCounters* ctr,
-                                               unsigned long long* __restrict__ film,
-                                               const DevBatchJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(kShadeThreads, CPPPT_SHADE_BLOCKS)
+    k_shade(DevScene S, PathIO in, PathIO nxt, ShadowIO Q, const float4* hit, int cur, WaveCounters* ctr,
+            unsigned long long* __restrict__ film, const DevBatchJob* __restrict__ jobs) {
     after_previous();
     const int n = ctr->n_cur;
     // an empty CTA of the capacity's grid: nothing to shade, no barriers to
@@ -563,7 +561,7 @@ void launch_extend(const DevScene& S, const PathBuffers& B, int cur, WaveCounter
 void launch_trace_wave(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                        int num_sms, cudaStream_t st) {
     launch_after(k_trace_wave, num_sms * kTraceBlocksPerSM, kTraceThreads, kBothSmem, st, S, path_io(B, cur), B.hit,
-                                                                                     shadow_io(B), cur, ctr, film);
+                 shadow_io(B), cur, ctr, film);
 }
 cudaError_t trace_kernels_setup() {
     const auto limit = [](const void* f, size_t bytes) {
@@ -581,8 +579,8 @@ cudaError_t trace_kernels_setup() {
 
 void launch_shade(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                   const DevBatchJob* jobs, cudaStream_t st) {
-    launch_after(k_shade, (B.capacity + kShadeThreads - 1) / kShadeThreads, kShadeThreads, 0, st, S, path_io(B, cur), path_io(B, 1 - cur), shadow_io(B), B.hit, cur,
-                                                      ctr, film, jobs);
+    launch_after(k_shade, (B.capacity + kShadeThreads - 1) / kShadeThreads, kShadeThreads, 0, st, S, path_io(B, cur),
+                 path_io(B, 1 - cur), shadow_io(B), B.hit, cur, ctr, film, jobs);
 }
 void launch_shadow(const DevScene& S, const PathBuffers& B, int cur, WaveCounters* ctr, unsigned long long* film,
                    int num_sms, cudaStream_t st) {
@@ -595,7 +593,8 @@ void launch_generate(const PathBuffers& B, int cur, WaveCounters* ctr, const Dev
     // 50 us a launch there (a quarter of the Cornell box's 64-spp render)
     const int g = max(1, min((B.capacity + 255) / 256, num_sms * 8));
     launch_after(k_generate, g, 256, 0, st, path_io(B, 1 - cur), B.capacity, ctr, jobs, n_jobs);
-    launch_after(k_advance, 1, 32, 0, st, ctr, B.capacity, cur, shadows_traced ? cur : 1 - cur, shadows_traced ? 0 : kFinishPaths);
+    launch_after(k_advance, 1, 32, 0, st, ctr, B.capacity, cur, shadows_traced ? cur : 1 - cur,
+                 shadows_traced ? 0 : kFinishPaths);
 }
 void launch_advance(WaveCounters* ctr, int capacity, int cur, cudaStream_t st) {
     launch_after(k_advance, 1, 32, 0, st, ctr, capacity, cur, 1 - cur, 0);
@@ -609,8 +608,8 @@ void launch_wave_iteration(const DevScene& S, const PathBuffers& B, int cur, Wav
 
 void launch_finish(const DevScene& S, const PathBuffers& B, WaveCounters* ctr, unsigned long long* film,
                    const DevBatchJob* jobs, int num_sms, cudaStream_t st) {
-    launch_after(k_finish, num_sms, kFinishThreads, kFinishSmem, st, S, path_io(B, 0), path_io(B, 1),
-                                                                            shadow_io(B), ctr, film, jobs);
+    launch_after(k_finish, num_sms, kFinishThreads, kFinishSmem, st, S, path_io(B, 0), path_io(B, 1), shadow_io(B),
+                 ctr, film, jobs);
 }
 
 // Body end of a device-driven render loop (build_render_graph).  One thread.
@@ -844,7 +843,8 @@ cudaError_t render_noalloc(const DevScene& S, const RenderParams& P, int num_sms
     WaveCounters h{};
     for (unsigned long long round = 0;; round++) {
         // a render of at most kFinishPaths paths goes straight to k_finish
-        for (int k = 0; k < iters && total > (unsigned long long)kFinishPaths; k++) launch_wave_iteration(S, B, k & 1, ctr, film, job, 1, num_sms, st);
+        for (int k = 0; k < iters && total > (unsigned long long)kFinishPaths; k++)
+            launch_wave_iteration(S, B, k & 1, ctr, film, job, 1, num_sms, st);
         e = cudaMemcpyAsync(&h, ctr, sizeof(h), cudaMemcpyDeviceToHost, st);
         if (e != cudaSuccess) return e;
         e = cudaStreamSynchronize(st);

@@ -6,6 +6,12 @@
 
 namespace cpppt_gb300 {
 
+// Figures in this file: the two or more sides of a choice, measured together on
+// the build of their time, on boxes whose clocks differ by several per cent.
+// They compare with each other, not with those of another comment.  The whole
+// now, in one session: 1.8M closest-hit rays 676 us, shadow rays 561 us, 1080p
+// at 16 spp 68.8 ms (1M-triangle soup).
+//
 // Launch shape of the traversal kernels: threads per CTA and resident CTAs
 // per SM (the grid is the latter times the SM count); 64 registers.  1024 x 1:
 // 1.8M closest-hit rays on the 1M-triangle soup 967 us, 512 x 2 981 us; more
@@ -523,8 +529,9 @@ __device__ __forceinline__ void trav_round(const DevScene& S, Trav& T, Stack& K,
 // load(i, o, d, tmax, root) fetches ray i; root arrives set to the scene's
 // own root and may be replaced (rays of a merged multi-scene arena).
 template <bool ANY, bool COUNT, int THREADS = kTraceThreads, class Load, class Store>
-__device__ __forceinline__ void persistent_trace(const DevScene& S, uint32_t* __restrict__ smem, int n, int* counter, uint32_t* status, TraceCount& cnt, Load load,
-                                                 Store store, bool own_first = true) {
+__device__ __forceinline__ void persistent_trace(const DevScene& S, uint32_t* __restrict__ smem, int n, int* counter,
+                                                 uint32_t* status, TraceCount& cnt, Load load, Store store,
+                                                 bool own_first = true) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     Trav T;
